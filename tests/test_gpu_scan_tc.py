@@ -1,0 +1,75 @@
+"""The tcgen05 corpus scan at the edges of its tiles and query widths: 128-row tiles, 64 / 128 / 256 query columns, rows of 64 /
+128 bf16 or 128 / 256 int8, with and without the sampled pivot, and row scales the int8 filter has to step aside for."""
+import numpy as np
+import pytest
+
+from oracle import phoenix_oracle as po
+
+pytestmark = pytest.mark.gpu
+
+
+def _topk(sh, users, k):
+    import torch
+    B = users.shape[0]
+    u = torch.from_numpy(users).cuda()
+    sc = torch.empty((B, k), dtype=torch.float32, device="cuda"); ids = torch.empty((B, k), dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    sh.topk_device(u, B, k, sc, ids)
+    sh.sync()
+    return sc.cpu().numpy(), ids.cpu().numpy()
+
+
+def _users(B, dim, seed):
+    u = np.random.default_rng(seed).standard_normal((B, dim)).astype(np.float32)
+    return u / np.linalg.norm(u, axis=1, keepdims=True)
+
+
+@pytest.mark.parametrize("dim", [128, 256])
+@pytest.mark.parametrize("N,B,k", [(127, 1, 5), (128, 64, 128), (129, 65, 3), (33000, 1, 50), (40001, 128, 60), (40000, 129, 60), (36900, 250, 17)])
+def test_int8_scan_bit_exact(dim, N, B, k):
+    """Ids and scores equal the oracle's; some rows have a zero or a negative scale (their order is turned round)."""
+    from x_algorithm_b200.engine import dispatch_counts
+    from x_algorithm_b200.retrieval import CorpusShard
+    r = np.random.default_rng(N + dim)
+    q8 = r.integers(-128, 128, size=(N, dim), dtype=np.int8)
+    q8[::31] = q8[3]
+    scales = (r.random(N, dtype=np.float32) * np.float32(0.01) + np.float32(1e-4)).astype(np.float32)
+    scales[::31] = scales[3]
+    scales[5::53] = 0.0
+    scales[7::59] *= -1.0
+    users = _users(B, dim, 2)
+    sh = CorpusShard(N, dim, row_offset=11, max_queries=B, max_k=k)
+    sh.upload_int8(0, q8, scales)
+    sh.set_int8(True)
+    before = dispatch_counts()["scan.tcgen05"]
+    got_s, got_i = _topk(sh, users, k)
+    assert dispatch_counts()["scan.tcgen05"] > before
+    want_s, want_i = po.top_k(po.int8_corpus_scores(users, q8, scales), k, row_offset=11)
+    np.testing.assert_array_equal(got_i, want_i)
+    np.testing.assert_array_equal(got_s, want_s)
+    sh.close()
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("N,B,k", [(127, 1, 5), (129, 64, 40), (33000, 65, 30), (50001, 128, 50), (40000, 129, 20)])
+def test_bf16_scan_against_64_bit_scores(dim, N, B, k):
+    """Every list is ordered, its scores are the bf16 roundings of the rows' own dot products and no row outside it beats
+    the last entry by more than a bf16 step (fp32 sums may round to either neighbour: 2^-8 relative)."""
+    from x_algorithm_b200.retrieval import CorpusShard
+    users = _users(B, dim, 5)
+    sh = CorpusShard(N, dim, max_queries=B, max_k=k)
+    sh.fill_synthetic(4)
+    got_s, got_i = _topk(sh, users, k)
+    sh.close()
+    corpus = po.bf16_from_bits(po.synthetic_corpus_rows(np.arange(N), dim, 4)).astype(np.float64)
+    full = po.bf16_round(users).astype(np.float64) @ corpus.T
+    step = 2.0 ** -8
+    for b in range(B):
+        own = full[b][got_i[b]]
+        assert np.all(np.abs(got_s[b] - own) <= step * np.abs(own) + 1e-6)
+        key = np.lexsort((got_i[b], -got_s[b].astype(np.float64)))
+        np.testing.assert_array_equal(key, np.arange(k))
+        assert len(set(got_i[b])) == k
+        rest = np.delete(full[b], got_i[b])
+        if rest.size:
+            assert rest.max() <= got_s[b][-1] + step * abs(got_s[b][-1]) + 1e-6

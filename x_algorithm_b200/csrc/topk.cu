@@ -473,15 +473,18 @@ struct phx_corpus {
   int* counts = nullptr;
   int* status = nullptr;
   int* err_flag = nullptr;       // raised by a bounded device-side wait that ran out
-  bool use_tc = false;           // tcgen05 scan (dim 64 / 128), else the mma.sync scan
+  bool use_tc = false;           // tcgen05 scan of the bf16 rows (dim 64 / 128), else the mma.sync scan
+  bool use_tc_i8 = false;        // the same of the int8 rows (dim 128 / 256)
   // int8 form of the corpus (phx_corpus_upload_int8 / phx_corpus_quantize_int8) and whether calls score with it
   signed char* q8 = nullptr;     // [rows, dim]
   float* row_scale = nullptr;    // [rows]
   float* user_scale = nullptr;   // [256]
   bool int8 = false;
   CUtensorMap map_corpus, map_users;
+  CUtensorMap map_corpus_i8, map_users_i8;
   CUtensorMap map_window;                    // corpus map of the last scanned window (phx_corpus_topk_window_device)
   long long win_begin = -1, win_end = -1;
+  bool win_i8 = false;
   unsigned int* mask = nullptr;              // eligibility bits of the shard's rows (phx_corpus_set_mask), null = all
   std::vector<unsigned int> mask_host;
   long long elig_begin = -1, elig_end = -1, elig_count = 0;   // eligible rows of the last window asked for
@@ -640,10 +643,12 @@ phx_status phx_corpus_create(int32_t device, int64_t rows, int32_t dim, int64_t 
 #undef CU
   {
     const char* force = getenv("PHX_TOPK");
-    c->use_tc = tc_scan_supported(dim) && prop.major == 10 && !(force && strcmp(force, "simt") == 0);
+    const bool tc = prop.major == 10 && !(force && strcmp(force, "simt") == 0);
+    c->use_tc = tc && tc_scan_supported(dim * 2);
+    c->use_tc_i8 = tc && tc_scan_supported(dim);
     if (c->use_tc) {
       std::string err;
-      phx_status s = tc_scan_make_maps(&c->map_corpus, &c->map_users, c->data, rows, dim, c->users_bf, err);
+      phx_status s = tc_scan_make_maps(&c->map_corpus, &c->map_users, c->data, rows, dim * 2, c->users_bf, err);
       if (s) { set_global_error(err); phx_corpus_destroy(c); return s; }
     }
   }
@@ -695,6 +700,7 @@ phx_status ensure_int8_buffers(phx_corpus* c) {
   if (!c->q8) PHX_CUDA_TRY(cudaMalloc(&c->q8, (size_t)c->rows * c->dim), c->err);
   if (!c->row_scale) PHX_CUDA_TRY(cudaMalloc(&c->row_scale, (size_t)c->rows * 4), c->err);
   if (!c->user_scale) PHX_CUDA_TRY(cudaMalloc(&c->user_scale, 256 * 4), c->err);
+  if (c->use_tc_i8) return tc_scan_make_maps(&c->map_corpus_i8, &c->map_users_i8, c->q8, c->rows, c->dim, c->users_bf, c->err);
   return PHX_OK;
 }
 }  // namespace
@@ -765,7 +771,8 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
   if (row_begin < 0 || row_end > c->rows || row_begin >= row_end) { c->err = "topk: window outside the shard's rows"; return PHX_E_ARG; }
   // the window [row_begin, row_end) of the shard scanned as a corpus of its own: rows, first row and global id of row 0
   const long long rows = row_end - row_begin, roff = c->row_offset + row_begin;
-  const bool tc = c->use_tc && !c->int8;   // the int8 corpus is scanned by the mma.sync kernel
+  const bool tc = c->int8 ? c->use_tc_i8 : c->use_tc;
+  const int row_bytes = c->int8 ? c->dim : c->dim * 2;
   const bf16* data = c->int8 ? reinterpret_cast<const bf16*>(c->q8 + row_begin * (long long)c->dim) : c->data + row_begin * (long long)c->dim;
   if (k > rows) { c->err = "topk: k exceeds the rows of the window"; return PHX_E_ARG; }
   if (c->mask) {
@@ -797,13 +804,14 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
     }
   }
   cudaSetDevice(c->device);
-  const CUtensorMap* map_corpus = &c->map_corpus;
+  const CUtensorMap* map_corpus = c->int8 ? &c->map_corpus_i8 : &c->map_corpus;
+  const CUtensorMap& map_users = c->int8 ? c->map_users_i8 : c->map_users;
   if (tc && (row_begin != 0 || row_end != c->rows)) {
-    if (c->win_begin != row_begin || c->win_end != row_end) {
+    if (c->win_begin != row_begin || c->win_end != row_end || c->win_i8 != c->int8) {
       CUtensorMap users_unused;
-      phx_status ms = tc_scan_make_maps(&c->map_window, &users_unused, data, rows, c->dim, c->users_bf, c->err);
+      phx_status ms = tc_scan_make_maps(&c->map_window, &users_unused, data, rows, row_bytes, c->users_bf, c->err);
       if (ms) return ms;
-      c->win_begin = row_begin; c->win_end = row_end;
+      c->win_begin = row_begin; c->win_end = row_end; c->win_i8 = c->int8;
     }
     map_corpus = &c->map_window;
   }
@@ -850,7 +858,8 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
   a.i8 = c->int8 ? 1 : 0; a.user_scale = c->user_scale; a.row_scale = c->int8 ? c->row_scale + row_begin : nullptr;
   TcScanArgs ta;
   ta.mask = c->mask; ta.mask_row0 = row_begin;
-  ta.rows = rows; ta.row_offset = roff; ta.dim = c->dim; ta.B = B; ta.stride = 1; ta.gmax = c->gmax; ta.n_groups = 0;
+  if (c->int8) { ta.user_scale = c->user_scale; ta.row_scale = c->row_scale + row_begin; }
+  ta.rows = rows; ta.row_offset = roff; ta.row_bytes = row_bytes; ta.B = B; ta.stride = 1; ta.gmax = c->gmax; ta.n_groups = 0;
   ta.pivot = c->pivot; ta.surv = c->surv; ta.counts = c->counts; ta.cap = c->cap;
   const long long n_tiles = (rows + tile_rows - 1) / tile_rows;
   int j = 0;
@@ -871,7 +880,7 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
     if (j < 1) j = 1;
     phx_status s;
     dispatch_note(tc ? DK_SCAN_TC : DK_SCAN_MMA);
-    if (tc) s = tc_scan_launch(*map_corpus, c->map_users, ta, 0, c->num_sms, c->err_flag, c->stream, c->err);
+    if (tc) s = tc_scan_launch(*map_corpus, map_users, ta, 0, c->num_sms, c->err_flag, c->stream, c->err);
     else s = run_scan(c, a, 0, (int)(sampled_tiles < c->num_sms * 2 ? sampled_tiles : c->num_sms * 2));
     if (s) return s;
   }
@@ -880,7 +889,7 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
   {
     phx_status s;
     dispatch_note(tc ? DK_SCAN_TC : DK_SCAN_MMA);
-    if (tc) s = tc_scan_launch(*map_corpus, c->map_users, ta, 1, c->num_sms, c->err_flag, c->stream, c->err);
+    if (tc) s = tc_scan_launch(*map_corpus, map_users, ta, 1, c->num_sms, c->err_flag, c->stream, c->err);
     else s = run_scan(c, a, 1, (int)(n_tiles < c->num_sms * 2 ? n_tiles : c->num_sms * 2));
     if (s) return s;
   }

@@ -8,7 +8,7 @@ namespace phx {
 struct TcScanArgs {
   long long rows;            // corpus rows of this shard
   long long row_offset;      // global id of local row 0
-  int dim, B;                // embedding dim (64 or 128), live queries (<= 256)
+  int row_bytes, B;          // bytes of a corpus row (128 or 256), live queries (<= 256)
   int stride;                // sample pass: tiles 0, stride, 2*stride, ...
   float* gmax;               // sample pass out: [B][n_groups] maxima of 32-row groups
   long long n_groups;        // sampled tiles * 4
@@ -20,6 +20,10 @@ struct TcScanArgs {
   // a row whose bit is clear is skipped like a row past the end.  null = every row is eligible
   const unsigned int* mask = nullptr;
   long long mask_row0 = 0;
+  // int8 corpus (recsys_two_tower_model.py:2518-2533): score = bf16((float(int32 dot) * user_scale[u]) * row_scale[row]);
+  // null = bf16 corpus
+  const float* user_scale = nullptr;   // [B]
+  const float* row_scale = nullptr;    // [rows]
 };
 
 __device__ __forceinline__ bool row_eligible(const unsigned int* mask, long long mask_row0, long long row) {
@@ -28,9 +32,11 @@ __device__ __forceinline__ bool row_eligible(const unsigned int* mask, long long
   return (mask[r >> 5] >> (r & 31)) & 1u;
 }
 
-bool tc_scan_supported(int dim);
-phx_status tc_scan_make_maps(CUtensorMap* map_corpus, CUtensorMap* map_users, const bf16* corpus, long long rows, int dim,
-                             const bf16* users_bf, std::string& err);
+// rows of 64 or 128 bf16, or of 128 or 256 int8
+bool tc_scan_supported(int row_bytes);
+// `queries`: [256][row_bytes], in the corpus' type
+phx_status tc_scan_make_maps(CUtensorMap* map_corpus, CUtensorMap* map_users, const void* corpus, long long rows, int row_bytes,
+                             const void* queries, std::string& err);
 // mode 0 = sample pass (group maxima), 1 = collect pass (survivors)
 phx_status tc_scan_launch(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, int mode,
                           int num_sms, int* err_flag, cudaStream_t stream, std::string& err);

@@ -1,15 +1,20 @@
 // Corpus scan of the exhaustive top-k on Blackwell tensor cores (reference: users_bf16 @ posts^T,
-// phoenix/xrex/models/recsys_two_tower_model.py:2455-2456): the score tile of 128 corpus rows x 256 queries is
-// formed in TMEM and consumed there, so the only HBM traffic is the corpus itself, read once.
+// phoenix/xrex/models/recsys_two_tower_model.py:2455-2456; its int8 form 2518-2533): the score tile of 128 corpus rows x NQ
+// queries is formed in TMEM and consumed there, so the only HBM traffic is the corpus itself, read once.
 //
-// Persistent kernel, one CTA per SM, 320 threads:
-//   warp 0      TMA producer: the query matrix once (stays in shared memory), then one 128 x dim corpus tile per
-//               stage (128-byte swizzle, 64-column boxes)
-//   warp 1      MMA issuer: tcgen05.mma M=128 (corpus rows) x N=256 (queries), K=16 steps, into one of two TMEM
-//               accumulators
-//   warps 2-9   consumers: each warp reads its 32-row lane quadrant and one half of the query columns with
+// Persistent kernel, one CTA per SM, 576 threads:
+//   warp 0      TMA producer: the query matrix once (stays in shared memory), then one corpus tile of 128 rows per
+//               stage (128-byte swizzle, 128-byte boxes: 64 bf16 or 128 int8 columns)
+//   warp 1      MMA issuer: tcgen05.mma M=128 (corpus rows) x N=NQ (queries), 32 bytes of a row per instruction
+//               (kind::f16: 16 bf16, fp32 sums; kind::i8: 32 int8, int32 sums), into one of two TMEM accumulators
+//   warps 2-17  consumers: each warp reads its 32-row lane quadrant and a quarter of the query columns with
 //               tcgen05.ld and either appends rows whose score reaches the query's threshold to the survivor list
 //               (collect pass) or reduces the 32-row maximum per query (sample pass)
+// An int8 row of 128 columns is the byte image of a bf16 row of 64: tiles, swizzle, descriptors and tensor maps are the
+// same, only the instruction kind and what a consumer makes of an accumulator differ.
+// Measured (256 queries, k = 1000, one 12.5 M-row shard of 128 columns, whole top-k call): int8 rows 3.98 ms on mma.sync ->
+// 1.49 ms here; bf16 rows 1.28 -> 1.17 ms with 16 consumer warps instead of 8; one query over 1 M rows 227 -> 213 us with 64
+// query columns instead of 256.
 // All mbarrier waits are bounded; on expiry *err_flag is raised and the kernel unwinds.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
@@ -21,8 +26,9 @@ namespace {
 using namespace sm100;
 
 constexpr int TC_ROWS = 128;      // corpus rows per tile
-constexpr int TC_Q = 256;         // query columns (padded)
-constexpr int TC_THREADS = 320;
+constexpr int TC_QBOX = 64;       // query rows per TMA box
+constexpr int TC_CWARPS = 16;     // consumer warps: four per scheduler, what hides the latency of the filter's chains
+constexpr int TC_THREADS = 64 + 32 * TC_CWARPS;
 constexpr int TC_STAGES = 4;
 constexpr int QCAP = 64;          // per-warp staging queue of survivors (records of 16 bytes)
 constexpr int QFLUSH = 24;        // flush a warp's queue once it holds this many records
@@ -62,20 +68,63 @@ __device__ __noinline__ void stage_hit(int* counts, unsigned long long* surv, in
   }
 }
 
-template <int MODE>
+// D[tmem] (+)= A[smem desc] * B[smem desc], signed int8 inputs, int32 accumulate, K = 32
+__device__ __forceinline__ void umma_s8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
+      : "memory");
+}
+// instruction descriptor of kind::i8: D int32, A / B signed, both K-major
+__host__ __device__ constexpr uint32_t make_idesc_s8(int M, int N) {
+  return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+template <int CH>
+__device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, uint32_t* r) {
+  if (CH == 32) tmem_ld32_nowait(taddr, r); else tmem_ld16_nowait(taddr, r);
+}
+// r[k] for a k known only at run time, without local memory: a tree of CH - 1 selects
+template <int CH>
+__device__ __forceinline__ uint32_t pick(const uint32_t (&r)[CH], int k) {
+  uint32_t t[CH / 2];
+#pragma unroll
+  for (int i = 0; i < CH / 2; ++i) t[i] = (k & 1) ? r[2 * i + 1] : r[2 * i];
+#pragma unroll
+  for (int n = CH / 4, b = 2; n >= 1; n >>= 1, b <<= 1)
+#pragma unroll
+    for (int i = 0; i < n; ++i) t[i] = (k & b) ? t[2 * i + 1] : t[2 * i];
+  return t[0];
+}
+// The int32 accumulator of an int8 dot product as fp32 (exact: |dot| <= 128 * 128 * 256 = 2^22) times the query's scale;
+// the row's scale follows: (float(dot) * query scale) * row scale, in that order.
+__device__ __forceinline__ float s8_value(uint32_t acc, float query_scale) { return (float)(int)acc * query_scale; }
+
+constexpr float S8_OFFSET = 12582912.0f;            // 1.5 * 2^23: its bit pattern plus an integer below 2^22 in size is the float of their sum
+constexpr uint32_t S8_OFFSET_BITS = 0x4B400000u;
+
+// Columns per group of the collect filter: the group's threshold is the smallest of its queries'.
+template <int NQ> struct ScanCfg {
+  static constexpr int CW = NQ / 4;                  // query columns per consumer warp
+  static constexpr int CH = CW < 32 ? CW : 32;       // columns per group
+  static constexpr int GROUPS = NQ / CH;
+};
+
+template <int MODE, bool I8, int NQ>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_constant__ CUtensorMap map_users,
                TcScanArgs a, int* err_flag) {
+  using cfg = ScanCfg<NQ>;
+  constexpr int CW = cfg::CW, CH = cfg::CH;
   extern __shared__ uint8_t smem_raw[];
-  const int kblk = a.dim / BK;                                   // 64-column k-blocks: 1 or 2
+  const int kblk = a.row_bytes / 128;                            // 128-byte k-blocks: 1 or 2
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t users_smem = smem_base;                         // kblk x [256 x 128 B]
-  const uint32_t users_bytes = (uint32_t)kblk * TC_Q * 128;
+  const uint32_t users_smem = smem_base;                         // kblk x [NQ x 128 B]
+  const uint32_t users_bytes = (uint32_t)kblk * NQ * 128;
   const uint32_t stage_bytes = (uint32_t)kblk * TC_ROWS * 128;
   const uint32_t stage_base = users_smem + users_bytes;
-  const uint32_t thr_smem = stage_base + TC_STAGES * stage_bytes;  // [256] float thresholds
-  const uint32_t queue_smem = thr_smem + TC_Q * 4 + 32;            // (+ [8] minima of the thresholds per 32 columns) [8 warps][QCAP] uint4 records + [8] counters
-  const uint32_t bars = queue_smem + 8 * QCAP * 16 + 64;
+  const uint32_t thr_smem = stage_base + TC_STAGES * stage_bytes;  // [256] thresholds, [256] query scales, [8] + [8] per group, [128] query scale pairs
+  const uint32_t queue_smem = thr_smem + 2 * 256 * 4 + 64 + 128 * 16;         // [consumer warps][QCAP] records, then their counters
+  const uint32_t bars = queue_smem + TC_CWARPS * QCAP * 16 + 64;
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (TC_STAGES + s); };
   auto tfull_bar = [&](int x) { return bars + 8u * (2 * TC_STAGES + x); };
@@ -84,10 +133,13 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   const uint32_t tmem_slot = bars + 8u * (2 * TC_STAGES + 5);
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
   float* s_thr = reinterpret_cast<float*>(smem_raw + (thr_smem - smem_u32(smem_raw)));
-  float* s_thr_min = s_thr + TC_Q;
+  float* s_us = s_thr + 256;
+  float* s_thr_min = s_us + 256;     // [8] smallest threshold of a group
+  float* s_us_max = s_thr_min + 8;   // [8] largest query scale of a group
+  float4* s_us2 = reinterpret_cast<float4*>(s_us_max + 8);   // [128] {scale, scale, -offset * scale, -offset * scale} of two queries
   uint4* s_queue = reinterpret_cast<uint4*>(smem_raw + (queue_smem - smem_u32(smem_raw)));
-  int* s_qcnt = reinterpret_cast<int*>(s_queue + 8 * QCAP);
-  if (threadIdx.x < 8) s_qcnt[threadIdx.x] = 0;
+  int* s_qcnt = reinterpret_cast<int*>(s_queue + TC_CWARPS * QCAP);
+  if (threadIdx.x < TC_CWARPS) s_qcnt[threadIdx.x] = 0;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* verr = err_flag;
@@ -97,14 +149,14 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-    for (int x = 0; x < 2; ++x) { mbar_init(tfull_bar(x), 1); mbar_init(tempty_bar(x), 256); }
+    for (int x = 0; x < 2; ++x) { mbar_init(tfull_bar(x), 1); mbar_init(tempty_bar(x), 32 * TC_CWARPS); }
     mbar_init(users_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (MODE == 1) {
-    // collect when acc >= thr, with thr a little below the midpoint under the pivot: a superset of
-    // { bf16(acc) >= pivot }; the exact selection happens later on the rounded scores
-    for (int u = threadIdx.x; u < TC_Q; u += TC_THREADS) {
+  for (int u = threadIdx.x; u < NQ; u += TC_THREADS) {
+    if (MODE == 1) {
+      // collect when the score >= thr, with thr a little below the midpoint under the pivot: a superset of
+      // { bf16(score) >= pivot }; the exact selection happens later on the rounded scores
       float t = INFINITY;
       if (u < a.B) {
         const float p = a.pivot[u];
@@ -112,26 +164,34 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
       }
       s_thr[u] = t;
     }
+    if (I8) s_us[u] = (u < a.B) ? a.user_scale[u] : 0.f;
   }
-  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  if (warp == 1) tmem_alloc(tmem_slot, 2 * NQ);
   tc_fence_before();
   __syncthreads();
+  if (MODE == 1) {   // per group: smallest threshold, largest query scale
+    if (threadIdx.x < cfg::GROUPS) {
+      float t = INFINITY, m = 0.f;
+      for (int k = 0; k < CH; ++k) {
+        t = fminf(t, s_thr[threadIdx.x * CH + k]);
+        if (I8) m = fmaxf(m, s_us[threadIdx.x * CH + k]);
+      }
+      s_thr_min[threadIdx.x] = t; s_us_max[threadIdx.x] = m;
+    }
+    if (I8 && threadIdx.x < NQ / 2) {
+      const float x = s_us[2 * threadIdx.x], y = s_us[2 * threadIdx.x + 1];
+      s_us2[threadIdx.x] = make_float4(x, y, -S8_OFFSET * x, -S8_OFFSET * y);
+    }
+    __syncthreads();
+  }
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
-  if (MODE == 1 && warp >= 2) {   // every consumer warp fills the same eight minima (same values, benign) for its own use
-    for (int g8 = 0; g8 < 8; ++g8) {
-      float t = s_thr[g8 * 32 + lane];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t = fminf(t, __shfl_xor_sync(0xffffffffu, t, o));
-      if (lane == 0) s_thr_min[g8] = t;
-    }
-    __syncwarp();
-  }
 
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(users_bar, users_bytes);
-      for (int kb = 0; kb < kblk; ++kb) tma_load_2d(users_smem + kb * TC_Q * 128, &map_users, users_bar, kb * BK, 0);
+      for (int kb = 0; kb < kblk; ++kb)
+        for (int q = 0; q < NQ; q += TC_QBOX) tma_load_2d(users_smem + (kb * NQ + q) * 128, &map_users, users_bar, kb * BK, q);
       int stage = 0; uint32_t phase = 0;
       for (long long w = blockIdx.x; w < n_work; w += gridDim.x) {
         const long long tile = (MODE == 0) ? w * a.stride : w;
@@ -145,7 +205,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(TC_ROWS, TC_Q);
+      constexpr uint32_t idesc = I8 ? make_idesc_s8(TC_ROWS, NQ) : make_idesc(TC_ROWS, NQ);
       bool ok = mbar_wait(users_bar, 0, verr);
       int stage = 0; uint32_t phase = 0, it = 0;
       for (long long w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++it) {
@@ -156,10 +216,12 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
         const uint32_t src = stage_base + stage * stage_bytes;
         for (int kb = 0; kb < kblk; ++kb) {
           const uint64_t adesc = make_smem_desc(src + kb * TC_ROWS * 128);
-          const uint64_t bdesc = make_smem_desc(users_smem + kb * TC_Q * 128);
+          const uint64_t bdesc = make_smem_desc(users_smem + kb * NQ * 128);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_bf16(tmem_base + acc * TC_Q, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+          for (int k = 0; k < 4; ++k) {   // 32 bytes of every row per instruction
+            if (I8) umma_s8(tmem_base + acc * NQ, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+            else umma_bf16(tmem_base + acc * NQ, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+          }
         }
         umma_commit(empty_bar(stage));
         umma_commit(tfull_bar(acc));
@@ -168,72 +230,100 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
     }
   } else {
     const int ew = warp - 2;
-    const int half = ew >> 2;        // which 128 query columns
+    const int part = ew >> 2;        // which quarter of the query columns
     const int quad = warp & 3;       // TMEM lane quadrant
     uint32_t it = 0;
     for (long long w = blockIdx.x; w < n_work; w += gridDim.x, ++it) {
       const long long tile = (MODE == 0) ? w * a.stride : w;
       const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
+      const long long row = tile * TC_ROWS + quad * 32 + lane;
+      const bool row_ok = row < a.rows && row_eligible(a.mask, a.mask_row0, row);
+      const float rs = (I8 && row < a.rows) ? __ldg(a.row_scale + row) : 0.f;
       bool ok = mbar_wait(tfull_bar(acc), acc_phase, verr);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const long long row = tile * TC_ROWS + quad * 32 + lane;
-      const bool row_ok = row < a.rows && row_eligible(a.mask, a.mask_row0, row);
-      const uint32_t taddr = tmem_base + acc * TC_Q + ((uint32_t)(quad * 32) << 16) + half * 128;
+      const uint32_t taddr = tmem_base + acc * NQ + ((uint32_t)(quad * 32) << 16) + part * CW;
       if (MODE == 1) {
-        // the warp's whole slice of the tile (32 rows x 128 queries) in one round trip to TMEM, then the accumulator
+        // the warp's whole slice of the tile (32 rows x CW queries) in one round trip to TMEM, then the accumulator
         // goes straight back to the MMA warp: the filtering below works from registers
-        uint32_t rr[4][32];
+        uint32_t rr[CW / CH][CH];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld32_nowait(taddr + c * 32, rr[c]);
+        for (int c = 0; c < CW / CH; ++c) tmem_ld_chunk<CH>(taddr + c * CH, rr[c]);
         tmem_ld_wait();
         tc_fence_before();
         mbar_arrive(tempty_bar(acc));
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t (&r)[32] = rr[c];
-          const int u0 = half * 128 + c * 32;
-          // First a filter: the largest of the row's 32 scores against the smallest of the 32 thresholds (16
-          // three-input max instructions).  Survivors are a few in 10^5 elements, so for almost every group the
-          // warp stops here; the exact per-column test below runs only when some lane's group passes.
-          float mx = max3(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]));
+        for (int c = 0; c < CW / CH; ++c) {
+          uint32_t (&r)[CH] = rr[c];
+          const int u0 = part * CW + c * CH;
+          // First a filter: the largest of the row's CH scores against the smallest of the CH thresholds.  Survivors
+          // are a few in 10^4 .. 10^5 elements, so for most groups the warp stops here; the exact per-column test below
+          // runs only when some lane's group passes.
+          bool pass;
+          if (I8) {
+            // float(dot) * query scale without a conversion per element (those run at a fraction of the fp32 rate):
+            // 1.5 * 2^23 + dot is the integer sum of the bit patterns, and the fma takes the offset's product off
+            // again.  That product is rounded: the value is off by at most 0.75 of the query scale, which the margin
+            // of one scale covers.  A row scale that is not positive turns the order round: no filter then.
+            float mx = -INFINITY;
 #pragma unroll
-          for (int k = 3; k + 1 < 32; k += 2) mx = max3(mx, __uint_as_float(r[k]), __uint_as_float(r[k + 1]));
-          mx = fmaxf(mx, __uint_as_float(r[31]));
-          if (!__any_sync(0xffffffffu, row_ok && mx >= s_thr_min[(u0 >> 5)])) continue;
-          // branch-free hit mask over the 32 columns, then the rare hits one by one: a taken branch per
-          // element (hit code laid out inline 32 times) made this loop instruction-fetch bound
+            for (int k = 0; k < CH; k += 2) {
+              const float4 s2 = s_us2[(u0 + k) >> 1];
+              const float2 x = make_float2(__uint_as_float(r[k] + S8_OFFSET_BITS), __uint_as_float(r[k + 1] + S8_OFFSET_BITS));
+              const float2 v = __ffma2_rn(x, make_float2(s2.x, s2.y), make_float2(s2.z, s2.w));
+              mx = max3(mx, v.x, v.y);
+            }
+            pass = !(rs > 0.f) || !((mx + s_us_max[u0 / CH]) * rs < s_thr_min[u0 / CH]);
+          } else {
+            float mx = max3(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]));
+#pragma unroll
+            for (int k = 3; k + 1 < CH; k += 2) mx = max3(mx, __uint_as_float(r[k]), __uint_as_float(r[k + 1]));
+            mx = fmaxf(mx, __uint_as_float(r[CH - 1]));
+            pass = mx >= s_thr_min[u0 / CH];
+          }
+          if (!__any_sync(0xffffffffu, row_ok && pass)) continue;
+          // branch-free hit mask over the columns, then the rare hits one by one: a taken branch per
+          // element (hit code laid out inline CH times) made this loop instruction-fetch bound
           uint32_t hits = 0;
 #pragma unroll
-          for (int k4 = 0; k4 < 8; ++k4) {
+          for (int k4 = 0; k4 < CH / 4; ++k4) {
             const float4 t4 = *reinterpret_cast<const float4*>(&s_thr[u0 + k4 * 4]);
-            hits |= (__uint_as_float(r[k4 * 4 + 0]) >= t4.x ? 1u : 0u) << (k4 * 4 + 0);
-            hits |= (__uint_as_float(r[k4 * 4 + 1]) >= t4.y ? 1u : 0u) << (k4 * 4 + 1);
-            hits |= (__uint_as_float(r[k4 * 4 + 2]) >= t4.z ? 1u : 0u) << (k4 * 4 + 2);
-            hits |= (__uint_as_float(r[k4 * 4 + 3]) >= t4.w ? 1u : 0u) << (k4 * 4 + 3);
+            float v[4];
+            if (I8) {
+              const float4 us4 = *reinterpret_cast<const float4*>(&s_us[u0 + k4 * 4]);
+              v[0] = s8_value(r[k4 * 4 + 0], us4.x) * rs; v[1] = s8_value(r[k4 * 4 + 1], us4.y) * rs;
+              v[2] = s8_value(r[k4 * 4 + 2], us4.z) * rs; v[3] = s8_value(r[k4 * 4 + 3], us4.w) * rs;
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) v[e] = __uint_as_float(r[k4 * 4 + e]);
+            }
+            hits |= (v[0] >= t4.x ? 1u : 0u) << (k4 * 4 + 0);
+            hits |= (v[1] >= t4.y ? 1u : 0u) << (k4 * 4 + 1);
+            hits |= (v[2] >= t4.z ? 1u : 0u) << (k4 * 4 + 2);
+            hits |= (v[3] >= t4.w ? 1u : 0u) << (k4 * 4 + 3);
           }
           if (!row_ok) hits = 0;
           while (hits) {
             const int k = __ffs(hits) - 1;
             hits &= hits - 1;
-            uint32_t bits = 0;
-#pragma unroll
-            for (int i = 0; i < 32; ++i) bits = (i == k) ? r[i] : bits;   // register select, no local memory
-            stage_hit(a.counts, a.surv, a.cap, s_queue + ew * QCAP, &s_qcnt[ew], u0 + k, __uint_as_float(bits),
-                      (uint32_t)(a.row_offset + row));
+            const uint32_t bits = pick<CH>(r, k);
+            const float v = I8 ? s8_value(bits, s_us[u0 + k]) * rs : __uint_as_float(bits);
+            stage_hit(a.counts, a.surv, a.cap, s_queue + ew * QCAP, &s_qcnt[ew], u0 + k, v, (uint32_t)(a.row_offset + row));
           }
         }
       } else {
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          tmem_ld32(taddr + c * 32, r);
-          const int u0 = half * 128 + c * 32;
+        for (int c = 0; c < CW / CH; ++c) {
+          uint32_t r[CH];
+          tmem_ld_chunk<CH>(taddr + c * CH, r);
+          tmem_ld_wait();
+          const int u0 = part * CW + c * CH;
           const long long grp = w * 4 + quad;
 #pragma unroll
-          for (int k = 0; k < 32; ++k) {
-            const uint32_t key = row_ok ? ord32(round_bf(__uint_as_float(r[k]))) : 0x007FFFFFu;  // ordered(-inf)
+          for (int k = 0; k < CH; ++k) {
+            const float v = I8 ? s8_value(r[k], s_us[u0 + k]) * rs : __uint_as_float(r[k]);
+            const uint32_t key = row_ok ? ord32(round_bf(v)) : 0x007FFFFFu;  // ordered(-inf)
             uint32_t mx;
             asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(mx) : "r"(key));
             const int u = u0 + k;
@@ -272,38 +362,53 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, 2 * NQ);
   }
+}
+
+template <int MODE, bool I8, int NQ>
+phx_status launch_scan_tc(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, int grid, int* err_flag,
+                          cudaStream_t stream, std::string& err) {
+  const int kblk = a.row_bytes / 128;
+  const size_t smem = (size_t)kblk * NQ * 128 + (size_t)TC_STAGES * kblk * TC_ROWS * 128 + 2 * 256 * 4 + 64 + 128 * 16 + TC_CWARPS * QCAP * 16 + 64 + 256 + 1024;
+  PHX_CUDA_TRY(cudaFuncSetAttribute(scan_tc_kernel<MODE, I8, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), err);
+  scan_tc_kernel<MODE, I8, NQ><<<grid, TC_THREADS, smem, stream>>>(map_corpus, map_users, a, err_flag);
+  PHX_CUDA_TRY(cudaGetLastError(), err);
+  return PHX_OK;
+}
+template <int MODE, bool I8>
+phx_status launch_scan_nq(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, int grid, int* err_flag,
+                          cudaStream_t stream, std::string& err) {
+  // query columns: the multiple of 64 that holds the batch (the tensor core and the consumers work on all NQ of them)
+  if (a.B <= 64) return launch_scan_tc<MODE, I8, 64>(map_corpus, map_users, a, grid, err_flag, stream, err);
+  if (a.B <= 128) return launch_scan_tc<MODE, I8, 128>(map_corpus, map_users, a, grid, err_flag, stream, err);
+  return launch_scan_tc<MODE, I8, 256>(map_corpus, map_users, a, grid, err_flag, stream, err);
 }
 
 }  // namespace
 
-bool tc_scan_supported(int dim) { return dim == 64 || dim == 128; }
+bool tc_scan_supported(int row_bytes) { return row_bytes == 128 || row_bytes == 256; }
 
-phx_status tc_scan_make_maps(CUtensorMap* map_corpus, CUtensorMap* map_users, const bf16* corpus, long long rows, int dim,
-                             const bf16* users_bf, std::string& err) {
-  phx_status s = sm100::make_map(map_corpus, corpus, rows, dim, TC_ROWS, err);
+phx_status tc_scan_make_maps(CUtensorMap* map_corpus, CUtensorMap* map_users, const void* corpus, long long rows, int row_bytes,
+                             const void* queries, std::string& err) {
+  // both are moved as 16-bit columns whatever they hold: the copies and the swizzle only see bytes
+  phx_status s = sm100::make_map(map_corpus, static_cast<const bf16*>(corpus), rows, row_bytes / 2, TC_ROWS, err);
   if (s) return s;
-  return sm100::make_map(map_users, users_bf, TC_Q, dim, TC_Q, err);
+  return sm100::make_map(map_users, static_cast<const bf16*>(queries), 256, row_bytes / 2, TC_QBOX, err);
 }
 
 phx_status tc_scan_launch(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, int mode,
                           int num_sms, int* err_flag, cudaStream_t stream, std::string& err) {
-  const int kblk = a.dim / BK;
-  const size_t smem = (size_t)kblk * TC_Q * 128 + (size_t)TC_STAGES * kblk * TC_ROWS * 128 + TC_Q * 4 + 32 + 8 * QCAP * 16 + 64 + 256 + 1024;
   const long long n_tiles = (a.rows + TC_ROWS - 1) / TC_ROWS;
   const long long n_work = (mode == 0) ? (n_tiles + a.stride - 1) / a.stride : n_tiles;
   const int grid = (int)(n_work < num_sms ? n_work : num_sms);
   if (grid <= 0) return PHX_OK;
-  if (mode == 0) {
-    PHX_CUDA_TRY(cudaFuncSetAttribute(scan_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), err);
-    scan_tc_kernel<0><<<grid, TC_THREADS, smem, stream>>>(map_corpus, map_users, a, err_flag);
-  } else {
-    PHX_CUDA_TRY(cudaFuncSetAttribute(scan_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), err);
-    scan_tc_kernel<1><<<grid, TC_THREADS, smem, stream>>>(map_corpus, map_users, a, err_flag);
-  }
-  PHX_CUDA_TRY(cudaGetLastError(), err);
-  return PHX_OK;
+  const bool i8 = a.row_scale != nullptr;
+  if (mode == 0)
+    return i8 ? launch_scan_nq<0, true>(map_corpus, map_users, a, grid, err_flag, stream, err)
+              : launch_scan_nq<0, false>(map_corpus, map_users, a, grid, err_flag, stream, err);
+  return i8 ? launch_scan_nq<1, true>(map_corpus, map_users, a, grid, err_flag, stream, err)
+            : launch_scan_nq<1, false>(map_corpus, map_users, a, grid, err_flag, stream, err);
 }
 
 }  // namespace phx
