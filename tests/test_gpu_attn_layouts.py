@@ -1,0 +1,35 @@
+"""The tcgen05 attention kernels under grouped q heads and the split token layout: the streaming kernel (head dim 128, histories
+past 128 keys) and the resident-history kernel (head dim 64), with and without a candidate-only tail, at the edges of the
+128-row query tiles and the 64 / 128-key blocks, against the oracle and against the mma.sync kernels."""
+import numpy as np
+import pytest
+
+from helpers import assert_heads_close, logits_of, make_pair, rel_l2, to_inputs
+from oracle import phoenix_oracle as po
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("S,C,dh,hq,hkv,tail", [(129, 1, 64, 4, 2, 1), (128, 129, 64, 4, 1, 0), (127, 40, 128, 4, 1, 1), (200, 130, 128, 2, 2, 2),
+                                                (257, 65, 64, 4, 4, 0), (64, 128, 128, 4, 2, 0), (1, 5, 128, 2, 1, 1)])
+def test_grouped_heads_and_split_rows(monkeypatch, S, C, dh, hq, hkv, tail):
+    from x_algorithm_b200.engine import dispatch_counts
+    B = 38 if dh == 64 and S <= 128 else 3              # the resident kernel starts at 148 (batch, head) pairs
+    kw = dict(max_batch=B, emb_size=256, num_q_heads=hq, num_kv_heads=hkv, key_size=dh, history_len=S, num_candidates=C, num_layers=2,
+              num_candidate_only_layers=tail)
+    ocfg, w, rows_fn, eng = make_pair(**kw)
+    b = po.make_batch(ocfg, B, seed=S + C, ragged=True)
+    before = dispatch_counts()
+    got = eng.rank(to_inputs(b))
+    ran = {k: v - before[k] for k, v in dispatch_counts().items() if k.startswith("attn.") and v != before[k]}
+    assert set(ran) == {"attn.pingpong" if dh == 64 and S <= 128 else "attn.tcgen05"}, ran
+    monkeypatch.setenv("PHX_ATTN", "mma")
+    other = eng.rank(to_inputs(b))
+    eng.close()
+    valid = b.cand_post_ids != 0
+    assert rel_l2(logits_of(got.log_probs[valid]), logits_of(other.log_probs[valid])) < 1e-2
+    few = slice(0, 3)
+    bb = po.RankBatch(*(getattr(b, f)[few] for f in ("hist_post_ids", "hist_author_ids", "hist_actions", "hist_surfaces", "cand_post_ids", "cand_author_ids")))
+    lp, cont, logits = po.rank_forward(ocfg, w, rows_fn, bb)
+    ok = bb.cand_post_ids != 0
+    assert_heads_close(got.log_probs[few][ok], got.continuous[few][ok], logits[ok], cont[ok], 2e-2, str(kw))

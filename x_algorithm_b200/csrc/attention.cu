@@ -673,12 +673,12 @@ phx_status ranker_attention_launch(const AttnArgs& a, cudaStream_t stream, std::
     const bool legacy = force && strcmp(force, "mma") == 0;
     const bool forced_tc = force && (strcmp(force, "tcgen05") == 0 || strcmp(force, "resident") == 0);
     // Histories longer than one key block (128 keys at head dim 64) and head dim 128 go to the streaming tcgen05
-    // kernel (measured on B200: 1.5 vs 4.6 ms for the mma.sync kernel at 1024 + 1024 tokens, 16 heads x 128); a
+    // kernel (measured on B200: 1.5 vs 4.6 ms for the mma.sync kernel at 1024 + 1024 tokens, 16 heads x 128; grouped heads
+    // and split rows: a two-layer forward with 16 / 4 heads of 128 and 1022 + 64 rows goes from 761 to 521 us); a
     // history of one key block is the resident-history kernels' case further down.
     const int n_hist = a.hist_len < a.T ? a.hist_len : a.T;
     const bool prefer_tc = forced_tc || a.dh == 128 || n_hist > 128;
-    const bool plain = !a.split && a.q_start == 0 && !a.pack.hist_off;   // the tcgen05 kernel's tensor maps assume [B, T] token rows
-    if (plain && !legacy && prefer_tc && a.err_flag && ranker_attention_tc_supported(a)) return ranker_attention_tc_launch(a, a.err_flag, stream, err);
+    if (!legacy && prefer_tc && a.err_flag && ranker_attention_tc_supported(a)) return ranker_attention_tc_launch(a, a.err_flag, stream, err);
   }
   {
     // Head dim 64 with a history of at most 128 keys: the persistent tcgen05 kernel with the history resident and two

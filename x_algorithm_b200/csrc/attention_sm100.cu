@@ -65,7 +65,16 @@ struct AttnTcArgs {
   float sm_scale, cap;
   int cap_method;
   int* err_flag;
+  // streaming kernel: a request's rows as a history block and a candidate block (plain or split token layout)
+  int q_group, q_group_stride;                                    // column of q head h: AttnArgs::q_col
+  int n_hist, n_cand, hist_tiles;                                 // hist_tiles = 0: history rows are keys only
+  long long hist_row0, hist_req_rows, cand_row0, cand_req_rows;   // token row of position 0 of request 0; rows per request
 };
+__device__ __forceinline__ int q_column(int h, int head_stride, int group, int group_stride) {
+  return group <= 1 ? h * head_stride : (h / group) * group_stride + (h % group) * head_stride;
+}
+// the tensor maps of a streaming launch: Q / out over the history block and over the candidate block, K / V over history
+struct TcMaps { CUtensorMap qh, qc, k, v, oh, oc; };
 
 // D[tmem] (+)= A[tmem] * B[smem desc]: the A operand (bf16 pairs, one row per lane) comes from tensor memory
 __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
@@ -110,9 +119,7 @@ __device__ __forceinline__ void tmem_ld_wait_on(float (&r)[32]) {
 
 template <int DH, bool CAP>
 __global__ void __launch_bounds__(A_THREADS, 2)
-ranker_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                           const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
-                           AttnTcArgs a) {
+ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
   constexpr int KBLK = (DH == 64) ? 128 : 64;   // keys per block (keeps shared memory at 80 KB: two CTAs per SM)
   constexpr int DCH = DH / 64;                  // 64-column chunks of the head dim
   // S is double-buffered in TMEM (and K in shared memory): S of block j+1 is computed while the softmax warps are
@@ -136,11 +143,14 @@ ranker_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
   uint32_t* mask_words = reinterpret_cast<uint32_t*>(smem_raw + (sMask - smem_u32(smem_raw)));
 
-  const int b = blockIdx.z, h = blockIdx.y, q0 = blockIdx.x * QT;
+  // query tile: of the history block, then of the candidate block (q0 counts inside the block)
+  const int b = blockIdx.z, h = blockIdx.y;
+  const bool cand_tile = (int)blockIdx.x >= a.hist_tiles;
+  const int q0 = ((int)blockIdx.x - (cand_tile ? a.hist_tiles : 0)) * QT;
   const int hk = h / (a.Hq / a.Hkv);
+  const int qcol = q_column(h, a.q_head_stride, a.q_group, a.q_group_stride);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int T = a.T;
-  const int n_hist = a.hist_len < T ? a.hist_len : T;
+  const int n_hist = a.n_hist;
   const int n_blocks = (n_hist + KBLK - 1) / KBLK;
   volatile int* verr = a.err_flag;
 
@@ -159,13 +169,13 @@ ranker_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     // ---------------- TMA producer ----------------
     if (lane == 0) {
       mbar_expect_tx(q_full, DCH * SLAB);
-      for (int c = 0; c < DCH; ++c) tma_load_3d(sQ + c * SLAB, &map_q, q_full, h * a.q_head_stride + c * 64, q0, b);
+      for (int c = 0; c < DCH; ++c) tma_load_3d(sQ + c * SLAB, cand_tile ? &maps.qc : &maps.qh, q_full, qcol + c * 64, q0, b);
       auto load_k = [&](int j) {   // K block j into buffer j % NSB, once S of block j - NSB has been computed
         const int kb = j % NSB; const uint32_t use = (uint32_t)(j / NSB);
         mbar_wait(k_empty(kb), (use & 1) ^ 1, verr);
         mbar_expect_tx(k_full(kb), DCH * KBLK * 128);
         for (int c = 0; c < DCH; ++c)
-          tma_load_3d(sK + (kb * DCH + c) * KBLK * 128, &map_k, k_full(kb), hk * a.k_head_stride + c * 64, j * KBLK, b);
+          tma_load_3d(sK + (kb * DCH + c) * KBLK * 128, &maps.k, k_full(kb), hk * a.k_head_stride + c * 64, j * KBLK, b);
       };
       for (int j = 0; j < NSB - 1 && j < n_blocks; ++j) load_k(j);
       for (int j = 0; j < n_blocks; ++j) {
@@ -174,7 +184,7 @@ ranker_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         mbar_wait(v_empty(vb), (uint32_t)((j >> 1) & 1) ^ 1u, verr);
         mbar_expect_tx(v_full(vb), DCH * KBLK * 128);
         for (int c = 0; c < DCH; ++c)
-          tma_load_3d(sV + (vb * DCH + c) * KBLK * 128, &map_v, v_full(vb), hk * a.v_head_stride + c * 64, j * KBLK, b);
+          tma_load_3d(sV + (vb * DCH + c) * KBLK * 128, &maps.v, v_full(vb), hk * a.v_head_stride + c * 64, j * KBLK, b);
       }
     }
   } else if (warp == 1) {
@@ -221,9 +231,11 @@ ranker_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     const int quad = warp & 3;
     const int r = quad * 32 + lane;
     const int sw = r & 7;
-    const int row = q0 + r;
-    const long long tok0 = (long long)b * T;
-    const int segq = (row < T) ? a.seg[tok0 + row] : 0;
+    // token row of this thread's query, and of the request's first history key
+    const bool in = q0 + r < (cand_tile ? a.n_cand : n_hist);
+    const long long hist0 = a.hist_row0 + (long long)b * a.hist_req_rows;
+    const long long tok = (cand_tile ? a.cand_row0 + (long long)b * a.cand_req_rows : hist0) + q0 + r;
+    const int segq = in ? a.seg[tok] : 0;
     const uint32_t lane_base = ((uint32_t)(quad * 32) << 16);
     const float csc = CAP ? 1.0f : a.sm_scale * 1.4426950408889634f;
     float m = -INFINITY, l = 0.f;
@@ -232,7 +244,7 @@ ranker_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     // in flight together instead of one exposed round trip per block)
     for (int j = 0; j < n_blocks; ++j) {
       const int key = j * KBLK + r;
-      const bool ok = (r < KBLK) && (key < n_hist) && (a.seg[tok0 + key] == 1);
+      const bool ok = (r < KBLK) && (key < n_hist) && (a.seg[hist0 + key] == 1);
       const uint32_t word = __ballot_sync(0xffffffffu, ok);
       if (lane == 0) mask_words[j * 4 + quad] = word;
     }
@@ -339,8 +351,7 @@ ranker_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       for (int k = 0; k < DH; ++k) o[k] = 0.f;
     }
     if (segq == -1) {
-      const long long tok = tok0 + row;
-      const uint4* qp = reinterpret_cast<const uint4*>(a.q + tok * a.q_tok_stride + (long long)h * a.q_head_stride);
+      const uint4* qp = reinterpret_cast<const uint4*>(a.q + tok * a.q_tok_stride + qcol);
       const uint4* kp = reinterpret_cast<const uint4*>(a.k + tok * a.k_tok_stride + (long long)hk * a.k_head_stride);
       const uint4* vp = reinterpret_cast<const uint4*>(a.v + tok * a.v_tok_stride + (long long)hk * a.v_head_stride);
       float dot = 0.f;
@@ -378,7 +389,7 @@ ranker_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     bar_sync_128();
     if (warp == 2 && lane == 0) {
-      for (int c = 0; c < DCH; ++c) tma_store_3d(&map_o, sQ + c * SLAB, h * DH + c * 64, q0, b);
+      for (int c = 0; c < DCH; ++c) tma_store_3d(cand_tile ? &maps.oc : &maps.oh, sQ + c * SLAB, h * DH + c * 64, q0, b);
       asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
@@ -681,7 +692,7 @@ constexpr int PP_NQ = 3;
 
 struct PingArgs {
   const int* seg;
-  int q_head_stride, k_head_stride, v_head_stride;
+  int q_head_stride, k_head_stride, v_head_stride, q_group, q_group_stride;
   int Hq, Hkv, n_hist, n_cand, n_items;
   long long hist_row0, hist_req_rows, cand_row0, cand_req_rows;   // token row of position 0 of request 0; rows per request
   int skip_hist;                                                  // 1: history rows are keys only (candidate-only layer)
@@ -748,6 +759,7 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
       for (int li = 0; li < my_items; ++li) {
         const int it = (int)blockIdx.x + li * (int)gridDim.x;
         const int b = it / a.Hq, h = it % a.Hq, hk = h / (a.Hq / a.Hkv);
+        const int qcol = q_column(h, a.q_head_stride, a.q_group, a.q_group_stride);
         const int kb = li & 1;
         mbar_wait(kv_free(kb), (uint32_t)(((li >> 1) & 1) ^ 1), verr);
         mbar_expect_tx(kv_full(kb), 2 * SLAB);
@@ -759,11 +771,11 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
           mbar_wait(q_free(st), (uint32_t)(((g / PP_NQ) & 1) ^ 1), verr);
           if (ti < n_htiles) {
             mbar_expect_tx(q_full(st), SLAB);
-            tma_load_3d(dst, &maps.qh, q_full(st), h * a.q_head_stride, ti * QT, b);
+            tma_load_3d(dst, &maps.qh, q_full(st), qcol, ti * QT, b);
           } else {
             const int r0 = (ti - n_htiles) * QT;
             mbar_expect_tx(q_full(st), 3 * SLAB);
-            tma_load_3d(dst, &maps.qc, q_full(st), h * a.q_head_stride, r0, b);
+            tma_load_3d(dst, &maps.qc, q_full(st), qcol, r0, b);
             tma_load_3d(dst + SLAB, &maps.kc, q_full(st), hk * a.k_head_stride, r0, b);
             tma_load_3d(dst + 2 * SLAB, &maps.vc, q_full(st), hk * a.v_head_stride, r0, b);
           }
@@ -1037,23 +1049,24 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
 }
 
 // tensor maps are cached: the engine calls with the same buffers every layer and every step
-typedef std::tuple<const void*, long long, int, int, long long, int> MapKey;
+// [B] requests of `rows` rows each, req_rows rows apart
+typedef std::tuple<const void*, long long, long long, long long, int, long long, int> MapKey;
 std::map<MapKey, CUtensorMap> g_map_cache;
 std::mutex g_map_mu;
 
-phx_status cached_map3d(const CUtensorMap** out, const bf16* ptr, long long cols, int T, int B, long long tok_stride,
-                        int box_rows, std::string& err) {
+phx_status cached_map3d(CUtensorMap* out, const bf16* ptr, long long cols, long long rows, long long req_rows, int B,
+                        long long tok_stride, int box_rows, std::string& err) {
   std::lock_guard<std::mutex> lk(g_map_mu);
-  MapKey key(ptr, cols, T, B, tok_stride, box_rows);
+  MapKey key(ptr, cols, rows, req_rows, B, tok_stride, box_rows);
   auto it = g_map_cache.find(key);
   if (it == g_map_cache.end()) {
     if (g_map_cache.size() > 4096) g_map_cache.clear();
     CUtensorMap m;
-    phx_status s = make_map3d(&m, ptr, cols, T, B, tok_stride * 2, (long long)T * tok_stride * 2, box_rows, err);
+    phx_status s = make_map3d(&m, ptr, cols, rows, B, tok_stride * 2, req_rows * tok_stride * 2, box_rows, err);
     if (s) return s;
     it = g_map_cache.emplace(key, m).first;
   }
-  *out = &it->second;
+  *out = it->second;
   return PHX_OK;
 }
 
@@ -1069,6 +1082,7 @@ phx_status launch_pingpong(const AttnArgs& a, int* err_flag, int num_sms, cudaSt
   const int n_cand = a.T - n_hist;
   PingArgs p;
   p.seg = a.seg;
+  p.q_group = a.q_group; p.q_group_stride = a.q_group_stride;
   p.q_head_stride = a.q_head_stride; p.k_head_stride = a.k_head_stride; p.v_head_stride = a.v_head_stride;
   p.Hq = a.Hq; p.Hkv = a.Hkv; p.n_hist = n_hist; p.n_cand = n_cand; p.n_items = a.B * a.Hq;
   p.hist_row0 = token_row(a.split, a.B, a.hist_len, a.T, 0, 0);
@@ -1080,16 +1094,16 @@ phx_status launch_pingpong(const AttnArgs& a, int* err_flag, int num_sms, cudaSt
   if (p.skip_hist && n_cand == 0) return PHX_OK;
   // eight maps per launch: the engine calls with the same buffers every layer and every step, so they are cached whole
   struct Key {
-    const void *q, *k, *v, *o; long long qs, ks, vs, h0, hr, c0, cr; int qh, kh, vh, Hq, Hkv, nh, nc, B;
+    const void *q, *k, *v, *o; long long qs, ks, vs, h0, hr, c0, cr; int qh, kh, vh, qg, qgs, Hq, Hkv, nh, nc, B;
     bool operator<(const Key& x) const {
-      return std::tie(q, k, v, o, qs, ks, vs, h0, hr, c0, cr, qh, kh, vh, Hq, Hkv, nh, nc, B) <
-             std::tie(x.q, x.k, x.v, x.o, x.qs, x.ks, x.vs, x.h0, x.hr, x.c0, x.cr, x.qh, x.kh, x.vh, x.Hq, x.Hkv, x.nh, x.nc, x.B);
+      return std::tie(q, k, v, o, qs, ks, vs, h0, hr, c0, cr, qh, kh, vh, qg, qgs, Hq, Hkv, nh, nc, B) <
+             std::tie(x.q, x.k, x.v, x.o, x.qs, x.ks, x.vs, x.h0, x.hr, x.c0, x.cr, x.qh, x.kh, x.vh, x.qg, x.qgs, x.Hq, x.Hkv, x.nh, x.nc, x.B);
     }
   };
   static std::map<Key, PingMaps> cache;
   static std::mutex mu;
   const Key key{a.q, a.k, a.v, a.out, a.q_tok_stride, a.k_tok_stride, a.v_tok_stride, p.hist_row0, p.hist_req_rows, p.cand_row0,
-                p.cand_req_rows, a.q_head_stride, a.k_head_stride, a.v_head_stride, a.Hq, a.Hkv, n_hist, n_cand, a.B};
+                p.cand_req_rows, a.q_head_stride, a.k_head_stride, a.v_head_stride, a.q_group, a.q_group_stride, a.Hq, a.Hkv, n_hist, n_cand, a.B};
   PingMaps pm;
   {
     std::lock_guard<std::mutex> lk(mu);
@@ -1098,7 +1112,7 @@ phx_status launch_pingpong(const AttnArgs& a, int* err_flag, int num_sms, cudaSt
       if (cache.size() > 1024) cache.clear();
       PingMaps m;
       phx_status s;
-      const long long qcols = (long long)(a.Hq - 1) * a.q_head_stride + 64, kcols = (long long)(a.Hkv - 1) * a.k_head_stride + 64,
+      const long long qcols = a.q_col(a.Hq - 1) + 64, kcols = (long long)(a.Hkv - 1) * a.k_head_stride + 64,
                       vcols = (long long)(a.Hkv - 1) * a.v_head_stride + 64, ocols = (long long)a.Hq * 64;
       const long long ostr = ocols;   // output rows are dense: [token][head][64]
       auto mk = [&](CUtensorMap* dst, const bf16* ptr, long long cols, long long rows, long long tok_stride, long long req_rows) {
@@ -1136,20 +1150,38 @@ phx_status launch_tc(const AttnArgs& a, int* err_flag, cudaStream_t stream, std:
     PHX_CUDA_TRY(cudaFuncSetAttribute(ranker_attention_tc_kernel<DH, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), err);
     attr_set = true;
   }
-  const CUtensorMap *mq, *mk, *mv, *mo;
-  phx_status s;
-  if ((s = cached_map3d(&mq, a.q, (long long)(a.Hq - 1) * a.q_head_stride + DH, a.T, a.B, a.q_tok_stride, QT, err))) return s;
-  if ((s = cached_map3d(&mk, a.k, (long long)(a.Hkv - 1) * a.k_head_stride + DH, a.T, a.B, a.k_tok_stride, KBLK, err))) return s;
-  if ((s = cached_map3d(&mv, a.v, (long long)(a.Hkv - 1) * a.v_head_stride + DH, a.T, a.B, a.v_tok_stride, KBLK, err))) return s;
-  if ((s = cached_map3d(&mo, a.out, (long long)a.Hq * DH, a.T, a.B, (long long)a.Hq * DH, QT, err))) return s;
   AttnTcArgs t;
   t.q = a.q; t.k = a.k; t.v = a.v; t.out = a.out;
   t.q_tok_stride = a.q_tok_stride; t.k_tok_stride = a.k_tok_stride; t.v_tok_stride = a.v_tok_stride;
   t.q_head_stride = a.q_head_stride; t.k_head_stride = a.k_head_stride; t.v_head_stride = a.v_head_stride;
+  t.q_group = a.q_group; t.q_group_stride = a.q_group_stride;
   t.seg = a.seg; t.B = a.B; t.T = a.T; t.Hq = a.Hq; t.Hkv = a.Hkv; t.hist_len = a.hist_len;
   t.sm_scale = a.sm_scale; t.cap = a.cap; t.cap_method = a.cap_method; t.err_flag = err_flag;
-  dim3 grid((a.T + QT - 1) / QT, a.Hq, a.B);
-  ranker_attention_tc_kernel<DH, CAP><<<grid, A_THREADS, smem, stream>>>(*mq, *mk, *mv, *mo, t);
+  t.n_hist = a.hist_len < a.T ? a.hist_len : a.T;
+  t.n_cand = a.T - t.n_hist;
+  t.hist_row0 = 0; t.hist_req_rows = a.split ? a.hist_len : a.T;
+  t.cand_row0 = t.n_cand > 0 ? token_row(a.split, a.B, a.hist_len, a.T, 0, t.n_hist) : 0;
+  t.cand_req_rows = a.split ? t.n_cand : a.T;
+  t.hist_tiles = a.q_start > 0 ? 0 : (t.n_hist + QT - 1) / QT;
+  const int cand_tiles = (t.n_cand + QT - 1) / QT;
+  if (t.hist_tiles + cand_tiles == 0) return PHX_OK;
+  TcMaps m;
+  phx_status s;
+  const long long qcols = a.q_col(a.Hq - 1) + DH, kcols = (long long)(a.Hkv - 1) * a.k_head_stride + DH,
+                  vcols = (long long)(a.Hkv - 1) * a.v_head_stride + DH, ocols = (long long)a.Hq * DH;
+  const long long hn = t.n_hist, hr = t.hist_req_rows, cn = t.n_cand, cr = t.cand_req_rows;
+  // an empty block's maps are never used: they stand over the other block
+  const bool no_hist = hn == 0, no_cand = cn == 0;
+  const long long h0 = no_hist ? t.cand_row0 : 0, hrows = no_hist ? cn : hn, hreq = no_hist ? cr : hr;
+  const long long c0 = no_cand ? h0 : t.cand_row0, crows = no_cand ? hrows : cn, creq = no_cand ? hreq : cr;
+  if ((s = cached_map3d(&m.qh, a.q + h0 * a.q_tok_stride, qcols, hrows, hreq, a.B, a.q_tok_stride, QT, err))) return s;
+  if ((s = cached_map3d(&m.qc, a.q + c0 * a.q_tok_stride, qcols, crows, creq, a.B, a.q_tok_stride, QT, err))) return s;
+  if ((s = cached_map3d(&m.k, a.k + h0 * a.k_tok_stride, kcols, hrows, hreq, a.B, a.k_tok_stride, KBLK, err))) return s;
+  if ((s = cached_map3d(&m.v, a.v + h0 * a.v_tok_stride, vcols, hrows, hreq, a.B, a.v_tok_stride, KBLK, err))) return s;
+  if ((s = cached_map3d(&m.oh, a.out + h0 * ocols, ocols, hrows, hreq, a.B, ocols, QT, err))) return s;
+  if ((s = cached_map3d(&m.oc, a.out + c0 * ocols, ocols, crows, creq, a.B, ocols, QT, err))) return s;
+  dim3 grid(t.hist_tiles + cand_tiles, a.Hq, a.B);
+  ranker_attention_tc_kernel<DH, CAP><<<grid, A_THREADS, smem, stream>>>(m, t);
   PHX_CUDA_TRY(cudaGetLastError(), err);
   return PHX_OK;
 }
@@ -1161,12 +1193,12 @@ phx_status launch_resident(const AttnArgs& a, int* err_flag, cudaStream_t stream
     PHX_CUDA_TRY(cudaFuncSetAttribute(ranker_attention_resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), err);
     attr_set = true;
   }
-  const CUtensorMap *mq, *mk, *mv, *mo;
+  CUtensorMap mq, mk, mv, mo;
   phx_status s;
-  if ((s = cached_map3d(&mq, a.q, (long long)(a.Hq - 1) * a.q_head_stride + 64, a.T, a.B, a.q_tok_stride, QT, err))) return s;
-  if ((s = cached_map3d(&mk, a.k, (long long)(a.Hkv - 1) * a.k_head_stride + 64, a.T, a.B, a.k_tok_stride, 128, err))) return s;
-  if ((s = cached_map3d(&mv, a.v, (long long)(a.Hkv - 1) * a.v_head_stride + 64, a.T, a.B, a.v_tok_stride, 128, err))) return s;
-  if ((s = cached_map3d(&mo, a.out, (long long)a.Hq * 64, a.T, a.B, (long long)a.Hq * 64, QT, err))) return s;
+  if ((s = cached_map3d(&mq, a.q, (long long)(a.Hq - 1) * a.q_head_stride + 64, a.T, a.T, a.B, a.q_tok_stride, QT, err))) return s;
+  if ((s = cached_map3d(&mk, a.k, (long long)(a.Hkv - 1) * a.k_head_stride + 64, a.T, a.T, a.B, a.k_tok_stride, 128, err))) return s;
+  if ((s = cached_map3d(&mv, a.v, (long long)(a.Hkv - 1) * a.v_head_stride + 64, a.T, a.T, a.B, a.v_tok_stride, 128, err))) return s;
+  if ((s = cached_map3d(&mo, a.out, (long long)a.Hq * 64, a.T, a.T, a.B, (long long)a.Hq * 64, QT, err))) return s;
   AttnTcArgs t;
   t.q = a.q; t.k = a.k; t.v = a.v; t.out = a.out;
   t.q_tok_stride = a.q_tok_stride; t.k_tok_stride = a.k_tok_stride; t.v_tok_stride = a.v_tok_stride;
@@ -1175,21 +1207,21 @@ phx_status launch_resident(const AttnArgs& a, int* err_flag, cudaStream_t stream
   t.sm_scale = a.sm_scale; t.cap = a.cap; t.cap_method = a.cap_method; t.err_flag = err_flag;
   const int cap_on = (a.cap_method != 0 && a.cap > 0.f) ? 1 : 0;
   dim3 grid(1, a.Hq, a.B);
-  ranker_attention_resident_kernel<<<grid, A_THREADS, smem, stream>>>(*mq, *mk, *mv, *mo, t, cap_on);
+  ranker_attention_resident_kernel<<<grid, A_THREADS, smem, stream>>>(mq, mk, mv, mo, t, cap_on);
   PHX_CUDA_TRY(cudaGetLastError(), err);
   return PHX_OK;
 }
 
 }  // namespace
 
-// the two-warpgroup resident-history kernel: head dim 64, 1..128 history keys, q heads not grouped, rows not packed
+// the two-warpgroup resident-history kernel: head dim 64, 1..128 history keys, rows not packed
 bool ranker_attention_pingpong_supported(const AttnArgs& a) {
   const int n_hist = a.hist_len < a.T ? a.hist_len : a.T;
-  if (a.dh != 64 || n_hist < 1 || n_hist > 128 || a.q_group > 1 || a.pack.hist_off || a.Hq % a.Hkv != 0) return false;
+  if (a.dh != 64 || n_hist < 1 || n_hist > 128 || a.pack.hist_off || a.Hq % a.Hkv != 0) return false;
   if (a.q_start != 0 && a.q_start != n_hist) return false;
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   return al(a.q) && al(a.k) && al(a.v) && al(a.out) && a.q_tok_stride % 8 == 0 && a.k_tok_stride % 8 == 0 &&
-         a.v_tok_stride % 8 == 0 && a.q_head_stride % 8 == 0 && a.k_head_stride % 8 == 0 && a.v_head_stride % 8 == 0;
+         a.v_tok_stride % 8 == 0 && a.q_group_stride % 8 == 0 && a.q_head_stride % 8 == 0 && a.k_head_stride % 8 == 0 && a.v_head_stride % 8 == 0;
 }
 
 phx_status ranker_attention_pingpong_launch(const AttnArgs& a, int* err_flag, cudaStream_t stream, std::string& err) {
@@ -1205,9 +1237,10 @@ phx_status ranker_attention_pingpong_launch(const AttnArgs& a, int* err_flag, cu
   return cap ? launch_pingpong<true>(a, err_flag, num_sms, stream, err) : launch_pingpong<false>(a, err_flag, num_sms, stream, err);
 }
 
+// the streaming kernel: head dim 64 or 128, any grouping of the q heads, plain or split rows (not packed ones)
 bool ranker_attention_tc_supported(const AttnArgs& a) {
   if (a.dh != 64 && a.dh != 128) return false;
-  if (a.q_group > 1) return false;   // grouped q heads of a merged QKV row: the mma.sync kernels address them
+  if (a.pack.hist_off || (a.q_start != 0 && a.q_start != (a.hist_len < a.T ? a.hist_len : a.T))) return false;
   {
     const int n_hist = a.hist_len < a.T ? a.hist_len : a.T;
     if ((n_hist + 63) / 64 > TC_MAX_BLOCKS) return false;   // validity table of the CTA
@@ -1215,7 +1248,7 @@ bool ranker_attention_tc_supported(const AttnArgs& a) {
   // TMA: 16-byte aligned bases and strides, head offsets that are multiples of 8 elements
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   return al(a.q) && al(a.k) && al(a.v) && al(a.out) && a.q_tok_stride % 8 == 0 && a.k_tok_stride % 8 == 0 &&
-         a.v_tok_stride % 8 == 0 && a.q_head_stride % 8 == 0 && a.k_head_stride % 8 == 0 && a.v_head_stride % 8 == 0;
+         a.v_tok_stride % 8 == 0 && a.q_group_stride % 8 == 0 && a.q_head_stride % 8 == 0 && a.k_head_stride % 8 == 0 && a.v_head_stride % 8 == 0;
 }
 
 phx_status ranker_attention_tc_launch(const AttnArgs& a, int* err_flag, cudaStream_t stream, std::string& err) {
@@ -1224,7 +1257,7 @@ phx_status ranker_attention_tc_launch(const AttnArgs& a, int* err_flag, cudaStre
     const char* force = getenv("PHX_ATTN");
     const bool resident = force && strcmp(force, "resident") == 0;
     const int n_hist = a.hist_len < a.T ? a.hist_len : a.T;
-    if (resident && a.dh == 64 && n_hist <= 128 && n_hist > 0) { dispatch_note(DK_ATTN_RESIDENT); return launch_resident(a, err_flag, stream, err); }
+    if (resident && a.dh == 64 && n_hist <= 128 && n_hist > 0 && a.q_group <= 1 && !a.split && a.q_start == 0) { dispatch_note(DK_ATTN_RESIDENT); return launch_resident(a, err_flag, stream, err); }
   }
   dispatch_note(DK_ATTN_TC);
   if (a.dh == 64) return cap ? launch_tc<64, true>(a, err_flag, stream, err) : launch_tc<64, false>(a, err_flag, stream, err);

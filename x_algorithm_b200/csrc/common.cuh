@@ -307,7 +307,7 @@ struct AttnArgs {
   int cap_method;
   int* err_flag;         // device int raised by a bounded wait that ran out (tcgen05 path); null = mma.sync path only
   // Split token layout (token_row): q / k / v / out / seg rows are the B * hist_len history rows followed by the
-  // candidate rows; mma.sync kernels only.  q_start > 0: query rows below it are not computed (candidate-only layers).
+  // candidate rows.  q_start > 0: query rows below it are not computed (candidate-only layers).
   int split = 0, q_start = 0;
   // Packed rows (PackMap): per-request history / candidate counts; T and hist_len are then the largest a request can
   // have (grid sizing), q_start > 0 means "history queries are not wanted".  mma.sync kernels only.
