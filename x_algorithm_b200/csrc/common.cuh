@@ -43,7 +43,8 @@ enum DispatchKind {
   DK_SCAN_MMA = 10,      // mma.sync corpus scan
   DK_TOPK_EXACT = 11,    // exact-threshold passes of the top-k (the sampled pivot missed)
   DK_ATTN_PINGPONG = 12, // tcgen05 / TMEM resident-history kernel with two softmax warpgroups
-  DK_COUNT = 13
+  DK_GEMM_SMALL = 13,    // tcgen05 GEMM, one tile per CTA (few tiles)
+  DK_COUNT = 14
 };
 void dispatch_note(int kind);
 
@@ -146,6 +147,7 @@ struct GemmPlan {
   int N = 0, K = 0, BN = 0;
   bool pair = false;   // two CTAs of a cluster share each 256-row tile (tcgen05 cta_group::2)
   bool ready = false;
+  bool w_stable = false;   // nothing writes Wt while launches of this plan are in flight or queued: it may be read ahead
   unsigned long long* counters = nullptr;  // optional device counters [8]: MMA issuer cycles total / waiting for
                                            // operands / waiting for a free accumulator (diagnostics)
 };

@@ -356,6 +356,8 @@ phx_status refresh_folded(phx_engine* e) {
     if ((s = fold_gain_launch(L.w_qkv_t, L.pre_attn_norm, L.w_qkv_f, e->QW, e->D, e->stream, e->err))) return s;
     if ((s = fold_gain_launch(L.w_up_t, L.pre_ffn_norm, L.w_up_f, e->F, e->D, e->stream, e->err))) return s;
   }
+  // once per parameter load: the GEMMs may read their weights ahead of the kernel in front of them (GemmPlan::w_stable)
+  PHX_CUDA_TRY(cudaStreamSynchronize(e->stream), e->err);
   e->folded_dirty = false;
   return PHX_OK;
 }
@@ -779,6 +781,7 @@ phx_status phx_engine_create(const phx_model_config* cfg, int32_t device, phx_en
     TRY(gemm_plan_create(&L.p_out, e->attn, L.w_out_t, M, e->D, e->HD, e->HD <= 1024 && !cfg->primer_norm, e->err));
     TRY(gemm_plan_create(&L.p_up, e->hbuf, L.w_up_t, M, e->F, e->D, false, e->err));
     TRY(gemm_plan_create(&L.p_down, e->ffn, L.w_down_t, M, e->D, e->F, false, e->err));
+    for (GemmPlan* p : {&L.p_qkv, &L.p_qkv_f, &L.p_out, &L.p_up, &L.p_up_f, &L.p_down}) p->w_stable = true;
 #ifdef PHX_DIAGNOSTICS
     if (getenv("PHX_GEMM_COUNTERS")) {   // diagnostics: MMA-issuer wait counters by role, summed over layers and forwards
       if (!e->gemm_counters) {
@@ -1595,7 +1598,8 @@ int32_t phx_dispatch_counts(int64_t* out, int32_t n) {
 
 const char* phx_dispatch_name(int32_t kind) {
   static const char* names[DK_COUNT] = {"attn.strip", "attn.stream", "attn.tcgen05", "attn.resident", "gemm.pair256", "gemm.pair128",
-                                        "gemm.cta256", "gemm.cta128", "gemm.simt", "scan.tcgen05", "scan.mma", "topk.exact", "attn.pingpong"};
+                                        "gemm.cta256", "gemm.cta128", "gemm.simt", "scan.tcgen05", "scan.mma", "topk.exact", "attn.pingpong",
+                                        "gemm.small"};
   return (kind >= 0 && kind < DK_COUNT) ? names[kind] : "";
 }
 

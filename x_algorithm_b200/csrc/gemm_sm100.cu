@@ -516,6 +516,274 @@ phx_status launch_e(const GemmPlan& p, int epilogue, const GemmRope& rp, const G
   return PHX_E_ARG;
 }
 
+// ---- small problems: one 128 x BN tile per CTA -----------------------------------------------------------------------
+// For calls whose 128 x BN tiles (BN = 64 or 128) do not outnumber the SMs: one request, or a few.  Such a GEMM is a chain of
+// latencies - launch, first operand bytes, k-steps, epilogue, last store - and the pair kernel above pays most of them on
+// a dozen CTA pairs.  Here every tile has a CTA of its own, no cluster hand-shake, at most two CTAs fit an SM, so the next
+// kernel's CTAs set up (and, for weights that nothing rewrites, fetch the W half of their ring) under the tail of this
+// one; each epilogue thread owns half a row's slab, has its residual / statistics loads in flight under the main loop and
+// stores its 64 bytes straight to global memory.
+//   warp 0 TMA producer, warp 1 MMA issuer, then BN / 32 epilogue groups of four warps: group g takes the half g & 1 of
+//   64-column slab g >> 1 (RoPE: the column pairs of pass g & 1)
+// Measured: a forward of one request (640 rows, 8 layers) 492 -> 431 us, 16 small requests through two layers 155 -> 143 us.
+// The arithmetic per element, the order of the row statistics included, is the pair kernel's: results are the same bits.
+template <int BN>
+struct SmallCfg {
+  static constexpr int NG = BN / 32;
+  static constexpr int THREADS = 64 + NG * 128;
+  static constexpr int STAGE_BYTES = (BM + BN) * BK * 2;
+  static constexpr int STAGES = 98304 / STAGE_BYTES;          // 96 KB of ring: 4 (BN = 64) or 3 (BN = 128) k-steps
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + (BN / 64) * BM * 4 + 128 + 1024;   // + partial row sums, barriers, alignment
+};
+
+template <int BN, int EPI>
+__global__ void __launch_bounds__(SmallCfg<BN>::THREADS, 1)
+gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, bf16* C, const bf16* R,
+                  GemmRope rope, GemmNorm norm, long long M, int N, int K, int early_w, int* err_flag) {
+  using cfg = SmallCfg<BN>;
+  constexpr bool RES = (EPI == EPI_RESIDUAL);
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t ss_base = smem_base + cfg::STAGES * cfg::STAGE_BYTES;     // [slab][128] first halves of the row sums
+  const uint32_t bars = ss_base + (BN / 64) * BM * 4;
+  auto full_bar = [&](int s) { return bars + 8u * s; };
+  auto empty_bar = [&](int s) { return bars + 8u * (cfg::STAGES + s); };
+  const uint32_t tfull_bar = bars + 8u * (2 * cfg::STAGES);
+  const uint32_t tmem_slot = tfull_bar + 8u;
+  uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_tiles = (N + BN - 1) / BN;
+  const int n0 = ((int)blockIdx.x % n_tiles) * BN;
+  const long long m0 = (long long)((int)blockIdx.x / n_tiles) * BM;
+  const int k_blocks = (K + BK - 1) / BK;
+  volatile int* verr = err_flag;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < cfg::STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+    mbar_init(tfull_bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, BN);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_d = *tmem_slot_ptr;
+
+  auto load_w = [&](int kb, int stage) {
+    const uint32_t dst = smem_base + stage * cfg::STAGE_BYTES + BM * BK * 2;
+    for (int c = 0; c < BN / 64; ++c) tma_load_2d(dst + c * 64 * BK * 2, &map_b, full_bar(stage), kb * BK, n0 + c * 64);
+  };
+  const int ahead = k_blocks < cfg::STAGES ? k_blocks : cfg::STAGES;
+  if (warp == 0 && lane == 0 && early_w) {
+    // weights that no kernel writes while forwards run need not wait for the kernel in front
+    for (int kb = 0; kb < ahead; ++kb) { mbar_expect_tx(full_bar(kb), cfg::STAGE_BYTES); load_w(kb, kb); }
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0; uint32_t phase = 0;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (kb >= ahead || !early_w) {
+          if (!mbar_wait(empty_bar(stage), phase ^ 1, verr)) break;
+          mbar_expect_tx(full_bar(stage), cfg::STAGE_BYTES);
+          load_w(kb, stage);
+        }
+        tma_load_2d(smem_base + stage * cfg::STAGE_BYTES, &map_a, full_bar(stage), kb * BK, (int)m0);
+        if (++stage == cfg::STAGES) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc(BM, BN);
+      int stage = 0; uint32_t phase = 0;
+      bool ok = true;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait(full_bar(stage), phase, verr)) { ok = false; break; }
+        tc_fence_after();
+        const uint64_t adesc = make_smem_desc(smem_base + stage * cfg::STAGE_BYTES);
+        const uint64_t bdesc = make_smem_desc(smem_base + stage * cfg::STAGE_BYTES + BM * BK * 2);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) umma_bf16(tmem_d, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (kb | k) != 0);
+        umma_commit(empty_bar(stage));
+        if (++stage == cfg::STAGES) { stage = 0; phase ^= 1; }
+      }
+      if (ok) umma_commit(tfull_bar);
+    }
+  } else {
+    const int gidx = (warp - 2) >> 2, slab = gidx >> 1, p = gidx & 1;
+    const int quad = warp & 3;
+    const int r = quad * 32 + lane;
+    const long long row = m0 + r;
+    const bool in = row < M;
+    const int c0 = n0 + slab * 64;                       // first column of the slab
+    // two runs of 16 columns: neighbours, or (RoPE) the halves of a head that are rotated against each other
+    const bool d64 = EPI == EPI_ROPE && rope.dh == 64;
+    const int lo_col = d64 ? 16 * p : 32 * p, hi_col = d64 ? 32 + 16 * p : 32 * p + 16;
+    // ---- everything that does not need the accumulator ----
+    uint4 res[4];
+    if (RES) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int col = c0 + (c < 2 ? lo_col : hi_col) + (c & 1) * 8;
+        res[c] = (in && col < N) ? *reinterpret_cast<const uint4*>(R + row * N + col) : make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
+    float rstd = 1.0f;
+    if (!RES && norm.ss_in != nullptr) {                 // partials summed in slot order
+      float ss = 0.f;
+      if (in) {
+        const float* sp = norm.ss_in + row * norm.slots_in;
+        if (norm.slots_in == 8) {
+          const float4 a = __ldg(reinterpret_cast<const float4*>(sp)), b = __ldg(reinterpret_cast<const float4*>(sp + 4));
+          ss += a.x; ss += a.y; ss += a.z; ss += a.w; ss += b.x; ss += b.y; ss += b.z; ss += b.w;
+        } else {
+          for (int t = 0; t < norm.slots_in; ++t) ss += __ldg(sp + t);
+        }
+      }
+      rstd = rsqrtf(ss * norm.inv_d + norm.eps);
+    }
+    float4 cs[4], sn[4];
+    bool rotate = false;
+    if (EPI == EPI_ROPE) {
+      const long long trow = row + rope.row_offset;
+      int pos = rope.pos_cap;
+      if (rope.pos_rows) pos = in ? rope.pos_rows[trow] : 0;
+      else if (rope.split_rows == 0 || trow < rope.split_rows) {
+        const int t = (int)(trow % rope.T);
+        pos = t < rope.pos_cap ? t : rope.pos_cap;
+      }
+      const int kind = d64 ? (c0 >> 6) % rope.group : ((c0 >> 5) + p) % rope.group;
+      rotate = kind <= rope.g;
+      if (rotate) {
+        const long long o = (long long)pos * (rope.dh >> 1) + (d64 ? 16 * p : 0);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          cs[j] = __ldg(reinterpret_cast<const float4*>(rope.cos_tab + o) + j);
+          sn[j] = __ldg(reinterpret_cast<const float4*>(rope.sin_tab + o) + j);
+        }
+      }
+    }
+    bool ok = mbar_wait(tfull_bar, 0, verr);
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok) {
+      tc_fence_after();
+      const uint32_t taddr = tmem_d + ((uint32_t)(quad * 32) << 16) + slab * 64;
+      uint32_t raw[32];
+      tmem_ld16_nowait(taddr + lo_col, raw);
+      tmem_ld16_nowait(taddr + hi_col, raw + 16);
+      tmem_ld_wait();
+      float v[32];
+#pragma unroll
+      for (int k = 0; k < 32; ++k) {
+        v[k] = round_bf(__uint_as_float(raw[k]) * rstd);              // Linear output is bf16
+        if (EPI == EPI_GELU) v[k] = gelu_tanh_f(v[k]);
+      }
+      if (EPI == EPI_ROPE && rotate) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float cc[4] = {cs[j].x, cs[j].y, cs[j].z, cs[j].w}, ss[4] = {sn[j].x, sn[j].y, sn[j].z, sn[j].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float x1 = v[j * 4 + e], x2 = v[16 + j * 4 + e];
+            v[j * 4 + e] = x1 * cc[e] - x2 * ss[e];
+            v[16 + j * 4 + e] = x2 * cc[e] + x1 * ss[e];
+          }
+        }
+      }
+      if (RES) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float2 a = unpack_bf2(res[c].x), b = unpack_bf2(res[c].y), d = unpack_bf2(res[c].z), e = unpack_bf2(res[c].w);
+          v[c * 8 + 0] += a.x; v[c * 8 + 1] += a.y; v[c * 8 + 2] += b.x; v[c * 8 + 3] += b.y;
+          v[c * 8 + 4] += d.x; v[c * 8 + 5] += d.y; v[c * 8 + 6] += e.x; v[c * 8 + 7] += e.y;
+        }
+      }
+      if (in) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int col = c0 + (c < 2 ? lo_col : hi_col) + (c & 1) * 8;
+          uint4 o;
+          o.x = pack_bf2(v[c * 8 + 0], v[c * 8 + 1]); o.y = pack_bf2(v[c * 8 + 2], v[c * 8 + 3]);
+          o.z = pack_bf2(v[c * 8 + 4], v[c * 8 + 5]); o.w = pack_bf2(v[c * 8 + 6], v[c * 8 + 7]);
+          if (col < N) *reinterpret_cast<uint4*>(C + row * N + col) = o;
+        }
+      }
+      if (RES && norm.ss_out != nullptr) {
+        // statistics of the fp32 sums, one chain over the slab's 64 columns: the second half's thread goes on from where
+        // the first half's stopped
+        const uint32_t slot = ss_base + (slab * BM + r) * 4;
+        float ss = 0.f;
+        if (p == 0) {
+#pragma unroll
+          for (int k = 0; k < 32; ++k) ss += v[k] * v[k];
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot), "f"(ss) : "memory");
+        }
+        asm volatile("bar.sync %0, 256;" ::"r"(1 + slab) : "memory");
+        if (p == 1) {
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(ss) : "r"(slot) : "memory");
+#pragma unroll
+          for (int k = 0; k < 32; ++k) ss += v[k] * v[k];
+          if (in && c0 < N) norm.ss_out[row * (long long)(N / SLAB_COLS) + c0 / SLAB_COLS] = ss;
+        }
+      }
+    } else if (RES && norm.ss_out != nullptr) {
+      asm volatile("bar.sync %0, 256;" ::"r"(1 + slab) : "memory");    // a warp that gave up never leaves the others parked
+    }
+  }
+
+  // ---------------- teardown ----------------
+  if (*verr != 0) __nanosleep(1000000);  // error path: let in-flight bulk copies land before the CTA retires
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_d, BN);
+  }
+}
+
+template <int BN, int EPI>
+phx_status launch_small_t(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C, const bf16* R, const GemmRope& rope,
+                          const GemmNorm& norm, int64_t M, int* err_flag, cudaStream_t stream, std::string& err) {
+  using cfg = SmallCfg<BN>;
+  auto kern = gemm_small_kernel<BN, EPI>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    PHX_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg::SMEM_BYTES), err);
+    attr_set = true;
+  }
+  cudaLaunchConfig_t lc;
+  memset(&lc, 0, sizeof(lc));
+  cudaLaunchAttribute attr[1];
+  static const bool pdl = !(getenv("PHX_PDL") && getenv("PHX_PDL")[0] == '0');
+  if (pdl) {
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr; lc.numAttrs = 1;
+  }
+  lc.gridDim = dim3((unsigned)(((M + BM - 1) / BM) * ((p.N + BN - 1) / BN)));
+  lc.blockDim = dim3(cfg::THREADS);
+  lc.dynamicSmemBytes = cfg::SMEM_BYTES;
+  lc.stream = stream;
+  long long Mll = M;
+  int N = p.N, K = p.K, early = p.w_stable ? 1 : 0;
+  PHX_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, p.map_a, map_b64, C, R, rope, norm, Mll, N, K, early, err_flag), err);
+  return PHX_OK;
+}
+template <int BN>
+phx_status launch_small(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C, const bf16* R, int epilogue, const GemmRope& rp,
+                        const GemmNorm& nm, int64_t M, int* err_flag, cudaStream_t stream, std::string& err) {
+  switch (epilogue) {
+    case EPI_STORE: return launch_small_t<BN, EPI_STORE>(p, map_b64, C, R, rp, nm, M, err_flag, stream, err);
+    case EPI_RESIDUAL: return launch_small_t<BN, EPI_RESIDUAL>(p, map_b64, C, R, rp, nm, M, err_flag, stream, err);
+    case EPI_GELU: return launch_small_t<BN, EPI_GELU>(p, map_b64, C, R, rp, nm, M, err_flag, stream, err);
+    case EPI_ROPE: return launch_small_t<BN, EPI_ROPE>(p, map_b64, C, R, rp, nm, M, err_flag, stream, err);
+  }
+  err = "gemm: unknown epilogue";
+  return PHX_E_ARG;
+}
+
 // ---- SIMT cross-check GEMM --------------------------------------------------------------------------
 template <int EPI>
 __global__ void gemm_simt_kernel(const bf16* __restrict__ A, const bf16* __restrict__ Wt, bf16* C,
@@ -610,6 +878,17 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
     phx_status s = make_map(&p.map_r, R, M, p.N, BM, err);
     if (s != PHX_OK) return s;
     p.r_ptr = R; p.r_rows = M;
+  }
+  if (p.pair) {
+    // Few tiles: one 128 x 64 (else 128 x 128) tile per CTA while they do not outnumber the SMs.  Beyond that a CTA would have
+    // a second tile with nothing overlapped, and the pair kernel's wide tiles fetch fewer operand bytes.
+    static const bool small_ok = !getenv("PHX_GEMM_TILES");
+    const CUtensorMap& map_b64 = p.BN == 256 ? p.map_b_narrow : p.map_b;   // boxes of 64 W rows, either way
+    const long long mt = (M + BM - 1) / BM, t64 = mt * ((p.N + 63) / 64), t128 = mt * ((p.N + 127) / 128);
+    if (small_ok && (p.BN != 256 || p.has_narrow)) {
+      if (t64 <= num_sms) { dispatch_note(DK_GEMM_SMALL); return launch_small<64>(p, map_b64, C, R, epilogue, rp, nm, M, err_flag, stream, err); }
+      if (t128 <= num_sms) { dispatch_note(DK_GEMM_SMALL); return launch_small<128>(p, map_b64, C, R, epilogue, rp, nm, M, err_flag, stream, err); }
+    }
   }
   if (p.BN == 256) {
     // latency regime: when even the 128-column tiles leave SMs idle, take them - the call's time is one tile's time
