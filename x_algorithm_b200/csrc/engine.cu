@@ -146,8 +146,11 @@ struct phx_engine {
   void* in_stage_dev = nullptr;
   void* in_stage_host = nullptr;
   size_t in_stage_bytes = 0;
-  float* lp_dev = nullptr; float* cont_dev = nullptr; double* score_dev = nullptr;
+  void* out_stage_dev = nullptr;
+  void* out_stage_host = nullptr;
+  float* lp_dev = nullptr; float* cont_dev = nullptr; double* score_dev = nullptr;      // inside out_stage_dev / _host
   float* lp_host = nullptr; float* cont_host = nullptr; double* score_host = nullptr;
+  int* flag_host = nullptr;   // pinned: err_flag[0] comes back with a call's results
 
   // token prefetch (phx_rank_prefetch_device): tokens of the next batch are built on a side stream into the
   // alternate residual buffer while the current forward runs
@@ -230,6 +233,18 @@ phx_status dev_alloc(phx_engine* e, Tp** p, size_t count) {
   PHX_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(p), count * sizeof(Tp)), e->err);
   return PHX_OK;
 }
+
+// Results of `rows` candidates as one block: f64 scores, log-probabilities, continuous values, each on a 256-byte boundary
+struct OutLayout {
+  size_t lp_off, cont_off, bytes;
+  OutLayout(size_t rows, int V, int NC) {
+    lp_off = (rows * 8 + 255) & ~(size_t)255;
+    cont_off = (lp_off + rows * (V > 0 ? V : 1) * 4 + 255) & ~(size_t)255;
+    bytes = cont_off + rows * (NC > 0 ? NC : 1) * 4;
+  }
+  float* lp(void* base) const { return (float*)((uint8_t*)base + lp_off); }
+  float* cont(void* base) const { return (float*)((uint8_t*)base + cont_off); }
+};
 
 HashFamilyDev to_dev(const phx_hash_family& f, int offset) {
   HashFamilyDev d;
@@ -811,12 +826,14 @@ phx_status phx_engine_create(const phx_model_config* cfg, int32_t device, phx_en
     CU(cudaMalloc(&e->in_stage_dev, e->in_stage_bytes));
     CU(cudaMallocHost(&e->in_stage_host, e->in_stage_bytes));
     const size_t rows = B * (size_t)(e->C > 0 ? e->C : 1);
-    TRY(dev_alloc(e, &e->lp_dev, rows * (e->V > 0 ? e->V : 1)));
-    TRY(dev_alloc(e, &e->cont_dev, rows * (e->NC > 0 ? e->NC : 1)));
-    TRY(dev_alloc(e, &e->score_dev, rows));
-    CU(cudaMallocHost(reinterpret_cast<void**>(&e->lp_host), rows * (e->V > 0 ? e->V : 1) * 4));
-    CU(cudaMallocHost(reinterpret_cast<void**>(&e->cont_host), rows * (e->NC > 0 ? e->NC : 1) * 4));
-    CU(cudaMallocHost(reinterpret_cast<void**>(&e->score_host), rows * 8));
+    // one block each side: scores, log-probabilities, continuous values of max_batch requests; a small call lays its own
+    // rows out in front of it, back to back, and fetches them with one copy
+    const OutLayout ol(rows, e->V, e->NC);
+    CU(cudaMalloc(&e->out_stage_dev, ol.bytes));
+    CU(cudaMallocHost(&e->out_stage_host, ol.bytes));
+    e->score_dev = (double*)e->out_stage_dev; e->lp_dev = ol.lp(e->out_stage_dev); e->cont_dev = ol.cont(e->out_stage_dev);
+    e->score_host = (double*)e->out_stage_host; e->lp_host = ol.lp(e->out_stage_host); e->cont_host = ol.cont(e->out_stage_host);
+    CU(cudaMallocHost(reinterpret_cast<void**>(&e->flag_host), sizeof(int)));
   }
   // the memsets above ran on the default stream; every later launch uses the engine's own non-blocking stream, which
   // does not order itself behind them
@@ -857,11 +874,10 @@ void phx_engine_destroy(phx_engine* e) {
   fr(e->proj_hist_t); fr(e->proj_cand_t); fr(e->cat_hist); fr(e->cat_cand); fr(e->tok_proj); fr(e->proj_user_t); fr(e->cat_user);
   for (int i = 0; i < PHX_MAX_HIST_CONT; ++i) { fr(e->cont_w1[i]); fr(e->cont_w2[i]); }
   fr(e->x32); fr(e->h32); fr(e->qkv32); fr(e->attn32); fr(e->ffn32); fr(e->tmp32); fr(e->hist32);
-  fr(e->x_alt); fr(e->seg_alt); fr(e->rowss_a_alt); fr(e->rowss_a); fr(e->rowss_f); fr(e->seg); fr(e->hashes); fr(e->err_flag); fr(e->in_stage_dev); fr(e->lp_dev); fr(e->cont_dev); fr(e->score_dev);
+  fr(e->x_alt); fr(e->seg_alt); fr(e->rowss_a_alt); fr(e->rowss_a); fr(e->rowss_f); fr(e->seg); fr(e->hashes); fr(e->err_flag); fr(e->in_stage_dev); fr(e->out_stage_dev);
   if (e->in_stage_host) cudaFreeHost(e->in_stage_host);
-  if (e->lp_host) cudaFreeHost(e->lp_host);
-  if (e->cont_host) cudaFreeHost(e->cont_host);
-  if (e->score_host) cudaFreeHost(e->score_host);
+  if (e->out_stage_host) cudaFreeHost(e->out_stage_host);
+  if (e->flag_host) cudaFreeHost(e->flag_host);
   if (e->ev0) cudaEventDestroy(e->ev0);
   if (e->ev1) cudaEventDestroy(e->ev1);
   for (auto& pe : e->prof_events) { cudaEventDestroy(pe.second.first); cudaEventDestroy(pe.second.second); }
@@ -1433,10 +1449,24 @@ phx_status phx_rank_forward(phx_engine* e, const phx_rank_batch* bh, const phx_r
     PHX_CUDA_TRY(cudaMemcpyAsync(dp, hp, off, cudaMemcpyHostToDevice, e->stream), e->err);
   }
   phx_rank_out od; od.log_probs = e->lp_dev; od.continuous = e->cont_dev; od.scores = e->score_dev;
+  const size_t rows = B * C;
+  // Small results (up to half a megabyte) lie back to back and come back in one copy, the flag right behind: in chunks the
+  // twelve copies of one request, each a few kilobytes, took longer than their bytes.
+  const OutLayout ol(rows, e->V, e->NC);
+  const bool one_copy = ol.bytes <= (512u << 10);
+  if (one_copy) { od.log_probs = ol.lp(e->out_stage_dev); od.continuous = ol.cont(e->out_stage_dev); }
   phx_status s = phx_rank_forward_device(e, &bd, &od);
   if (s) return s;
-  const size_t rows = B * C;
-  // results come back in four row chunks: while the host copies chunk i out of the pinned staging block, chunk i+1
+  if (one_copy) {
+    PHX_CUDA_TRY(cudaMemcpyAsync(e->out_stage_host, e->out_stage_dev, ol.bytes, cudaMemcpyDeviceToHost, e->stream), e->err);
+    PHX_CUDA_TRY(cudaMemcpyAsync(e->flag_host, e->err_flag, sizeof(int), cudaMemcpyDeviceToHost, e->stream), e->err);
+    PHX_CUDA_TRY(cudaStreamSynchronize(e->stream), e->err);
+    if (oh->log_probs) memcpy(oh->log_probs, ol.lp(e->out_stage_host), rows * e->V * 4);
+    if (oh->continuous) memcpy(oh->continuous, ol.cont(e->out_stage_host), rows * e->NC * 4);
+    if (oh->scores && e->has_blend) memcpy(oh->scores, e->score_host, rows * 8);
+    return *e->flag_host ? check_err_flag(e) : PHX_OK;
+  }
+  // larger results come back in four row chunks: while the host copies chunk i out of the pinned staging block, chunk i+1
   // is still on the bus
   constexpr int NCH = 4;
   const size_t step = (rows + NCH - 1) / NCH;
@@ -1450,6 +1480,7 @@ phx_status phx_rank_forward(phx_engine* e, const phx_rank_batch* bh, const phx_r
     if (!e->ev_chunk[i]) PHX_CUDA_TRY(cudaEventCreateWithFlags(&e->ev_chunk[i], cudaEventDisableTiming), e->err);
     PHX_CUDA_TRY(cudaEventRecord(e->ev_chunk[i], e->stream), e->err);
   }
+  PHX_CUDA_TRY(cudaMemcpyAsync(e->flag_host, e->err_flag, sizeof(int), cudaMemcpyDeviceToHost, e->stream), e->err);
   for (int i = 0; i < NCH; ++i) {
     PHX_CUDA_TRY(cudaEventSynchronize(e->ev_chunk[i]), e->err);
     const size_t r0 = i * step, r1 = (r0 + step < rows) ? r0 + step : rows;
@@ -1459,7 +1490,7 @@ phx_status phx_rank_forward(phx_engine* e, const phx_rank_batch* bh, const phx_r
     if (oh->scores && e->has_blend) memcpy(oh->scores + r0, e->score_host + r0, (r1 - r0) * 8);
   }
   PHX_CUDA_TRY(cudaStreamSynchronize(e->stream), e->err);
-  return check_err_flag(e);
+  return *e->flag_host ? check_err_flag(e) : PHX_OK;
 }
 
 // ---- pipelined host-buffer requests ------------------------------------------------------------------------------
@@ -1752,6 +1783,64 @@ phx_status phx_user_tower_device(phx_engine* e, const phx_rank_batch* bd, float*
   return PHX_OK;
 }
 
+namespace {
+// What a stand-alone operator call needs beside its operands: the kernels' error flag block, a pinned word it is read into
+// and two events.  Kept between calls (allocating and freeing them took longer than a small operator: cudaFree waits for the
+// device), one set per call in flight; at most eight idle ones are held, the rest and any set whose call failed are freed.
+struct OpScratch {
+  int device = -1;
+  int* flag = nullptr;        // device, zero between calls
+  int* flag_host = nullptr;   // pinned
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  bool create(int dev) {
+    device = dev;
+    return cudaMalloc(reinterpret_cast<void**>(&flag), 2 * sizeof(int)) == cudaSuccess && cudaMemset(flag, 0, 2 * sizeof(int)) == cudaSuccess &&
+           cudaMallocHost(reinterpret_cast<void**>(&flag_host), sizeof(int)) == cudaSuccess && cudaEventCreate(&e0) == cudaSuccess &&
+           cudaEventCreate(&e1) == cudaSuccess;
+  }
+  void destroy() {
+    if (flag) cudaFree(flag);
+    if (flag_host) cudaFreeHost(flag_host);
+    if (e0) cudaEventDestroy(e0);
+    if (e1) cudaEventDestroy(e1);
+    *this = OpScratch();
+  }
+};
+std::mutex g_op_mu;
+std::vector<OpScratch> g_op_idle;
+
+bool op_acquire(int device, OpScratch* s) {
+  {
+    std::lock_guard<std::mutex> lk(g_op_mu);
+    for (size_t i = 0; i < g_op_idle.size(); ++i)
+      if (g_op_idle[i].device == device) { *s = g_op_idle[i]; g_op_idle.erase(g_op_idle.begin() + i); return true; }
+  }
+  if (s->create(device)) return true;
+  cudaGetLastError();
+  s->destroy();
+  return false;
+}
+void op_release(OpScratch* s, bool clean) {
+  if (clean) {
+    std::lock_guard<std::mutex> lk(g_op_mu);
+    if (g_op_idle.size() < 8) { g_op_idle.push_back(*s); return; }
+  }
+  s->destroy();
+}
+// The end of a call whose launch returned `s`: wait, read the flag and the time, hand the scratch back.
+phx_status op_finish(OpScratch* sc, phx_status s, const char* what, float* device_ms, std::string& err) {
+  cudaError_t ce = cudaEventRecord(sc->e1, 0);
+  if (ce == cudaSuccess) ce = cudaMemcpyAsync(sc->flag_host, sc->flag, sizeof(int), cudaMemcpyDeviceToHost, 0);
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(0);
+  if (s == PHX_OK && ce != cudaSuccess) { err = cudaGetErrorString(ce); s = PHX_E_CUDA; }
+  if (s == PHX_OK && device_ms) cudaEventElapsedTime(device_ms, sc->e0, sc->e1);
+  const bool raised = ce == cudaSuccess && *sc->flag_host != 0;
+  if (s == PHX_OK && raised) { err = std::string("a bounded device-side wait ran out (") + what + " pipeline)"; s = PHX_E_TIMEOUT; }
+  op_release(sc, ce == cudaSuccess && !raised);
+  return s;
+}
+}  // namespace
+
 phx_status phx_ranker_attention_device(int32_t device, const uint16_t* q, const uint16_t* k, const uint16_t* v,
                                        const int32_t* seg, uint16_t* out, int32_t B, int32_t T, int32_t Hq,
                                        int32_t Hkv, int32_t dh, int32_t hist_len, float sm_scale, float cap,
@@ -1764,25 +1853,12 @@ phx_status phx_ranker_attention_device(int32_t device, const uint16_t* q, const 
   aa.q_head_stride = aa.k_head_stride = aa.v_head_stride = dh;
   aa.out = (bf16*)out; aa.seg = seg; aa.B = B; aa.T = T; aa.Hq = Hq; aa.Hkv = Hkv; aa.dh = dh; aa.hist_len = hist_len;
   aa.sm_scale = sm_scale; aa.cap = cap; aa.cap_method = cap > 0.f ? cap_method : 0;
-  int* flag = nullptr;
-  if (cudaMalloc(&flag, 2 * sizeof(int)) != cudaSuccess) { set_global_error("cudaMalloc failed"); return PHX_E_CUDA; }
-  cudaMemset(flag, 0, 2 * sizeof(int));
-  aa.err_flag = flag;
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0); cudaEventCreate(&e1);
-  cudaEventRecord(e0, 0);
+  OpScratch sc;
+  if (!op_acquire(device, &sc)) { set_global_error("cudaMalloc failed"); return PHX_E_CUDA; }
+  aa.err_flag = sc.flag;
+  cudaEventRecord(sc.e0, 0);
   phx_status s = ranker_attention_launch(aa, 0, err);
-  cudaEventRecord(e1, 0);
-  cudaError_t ce = cudaEventSynchronize(e1);
-  if (s == PHX_OK && ce != cudaSuccess) { err = cudaGetErrorString(ce); s = PHX_E_CUDA; }
-  if (s == PHX_OK && device_ms) cudaEventElapsedTime(device_ms, e0, e1);
-  if (s == PHX_OK) {
-    int hflag = 0;
-    cudaMemcpy(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost);
-    if (hflag) { err = "a bounded device-side wait ran out (attention pipeline)"; s = PHX_E_TIMEOUT; }
-  }
-  cudaFree(flag);
-  cudaEventDestroy(e0); cudaEventDestroy(e1);
+  s = op_finish(&sc, s, "attention", device_ms, err);
   if (s) set_global_error(err);
   return s;
 }
@@ -1791,38 +1867,26 @@ phx_status phx_gemm_device(int32_t device, const uint16_t* A, const uint16_t* Wt
                            int64_t M, int32_t N, int32_t K, int32_t epilogue, int32_t impl, float* device_ms) {
   std::string err;
   if (cudaSetDevice(device) != cudaSuccess) { set_global_error("cudaSetDevice failed"); return PHX_E_CUDA; }
-  cudaDeviceProp prop;
-  cudaGetDeviceProperties(&prop, device);
-  int* flag = nullptr;
-  if (cudaMalloc(&flag, 2 * sizeof(int)) != cudaSuccess) { set_global_error("cudaMalloc failed"); return PHX_E_CUDA; }
-  cudaMemset(flag, 0, 2 * sizeof(int));
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0); cudaEventCreate(&e1);
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  OpScratch sc;
+  if (!op_acquire(device, &sc)) { set_global_error("cudaMalloc failed"); return PHX_E_CUDA; }
   phx_status s = PHX_OK;
   unsigned long long* ctr = nullptr;   // PHX_GEMM_COUNTERS=1: print where the MMA issuer waited (diagnostics)
+  GemmPlan plan;
   if (impl == 1) {
-    cudaEventRecord(e0, 0);
+    cudaEventRecord(sc.e0, 0);
     s = gemm_simt_launch((const bf16*)A, (const bf16*)Wt, (bf16*)C, (const bf16*)R, M, N, K, epilogue, 0, err);
-    cudaEventRecord(e1, 0);
   } else {
-    GemmPlan plan;
     s = gemm_plan_create(&plan, (const bf16*)A, (const bf16*)Wt, M, N, K, epilogue == 1 && K <= 1024, err, impl == 2 ? 0 : -1);
 #ifdef PHX_DIAGNOSTICS
     if (getenv("PHX_GEMM_COUNTERS")) { cudaMalloc(&ctr, 64); cudaMemset(ctr, 0, 64); plan.counters = ctr; }
 #endif
-    cudaEventRecord(e0, 0);
+    cudaEventRecord(sc.e0, 0);
     if (s == PHX_OK && (epilogue < 0 || epilogue > 2)) { err = "phx_gemm_device: epilogue must be 0, 1 or 2"; s = PHX_E_ARG; }
-    if (s == PHX_OK) s = gemm_launch(plan, (const bf16*)A, (bf16*)C, (const bf16*)R, M, epilogue, nullptr, nullptr, flag, prop.multiProcessorCount, 0, err);
-    cudaEventRecord(e1, 0);
+    if (s == PHX_OK) s = gemm_launch(plan, (const bf16*)A, (bf16*)C, (const bf16*)R, M, epilogue, nullptr, nullptr, sc.flag, sms, 0, err);
   }
-  cudaError_t ce = cudaEventSynchronize(e1);
-  if (s == PHX_OK && ce != cudaSuccess) { err = cudaGetErrorString(ce); s = PHX_E_CUDA; }
-  if (s == PHX_OK && device_ms) cudaEventElapsedTime(device_ms, e0, e1);
-  int hflag = 0;
-  if (s == PHX_OK) {
-    cudaMemcpy(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost);
-    if (hflag) { err = "a bounded device-side wait ran out (GEMM pipeline)"; s = PHX_E_TIMEOUT; }
-  }
+  s = op_finish(&sc, s, "GEMM", device_ms, err);
   if (ctr) {
     unsigned long long h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     cudaMemcpy(h, ctr, 64, cudaMemcpyDeviceToHost);
@@ -1833,8 +1897,6 @@ phx_status phx_gemm_device(int32_t device, const uint16_t* A, const uint16_t* Wt
             100.0 * h[2] / (double)(h[0] ? h[0] : 1));
     cudaFree(ctr);
   }
-  cudaFree(flag);
-  cudaEventDestroy(e0); cudaEventDestroy(e1);
   if (s) set_global_error(err);
   return s;
 }
