@@ -27,6 +27,9 @@ def test_variants_give_the_same_bits(M, N, K, epi):
 
 @pytest.mark.parametrize("B,opts", [(1, dict(history_len=31, num_candidates=70)), (5, dict(history_len=32, num_candidates=8)),
                                     (3, dict(emb_size=256, num_q_heads=4, num_kv_heads=2, key_size=64, history_len=40, num_candidates=150)),
+                                    (2, dict(emb_size=256, num_q_heads=2, num_kv_heads=1, key_size=128, history_len=40, num_candidates=90)),
+                                    (40, dict(emb_size=1024, num_q_heads=4, num_kv_heads=2, key_size=128, history_len=40, num_candidates=90, num_layers=1)),
+                                    (90, dict(emb_size=256, num_q_heads=6, num_kv_heads=3, key_size=128, history_len=129, num_candidates=100, num_layers=1)),
                                     (64, dict(emb_size=512, num_q_heads=8, num_kv_heads=8, key_size=64, history_len=100, num_candidates=211, num_layers=1))])
 def test_engine_forward_same_bits(monkeypatch, B, opts):
     ocfg, w, rows_fn, eng = make_pair(max_batch=B, **opts)

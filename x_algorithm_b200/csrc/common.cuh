@@ -73,7 +73,7 @@ __device__ __forceinline__ float gelu_tanh_f(float x) {
 }
 
 // ---- GEMM ---------------------------------------------------------------------------------------
-enum GemmEpilogue { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_GELU = 2, EPI_ROPE = 3 };
+enum GemmEpilogue { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_GELU = 2, EPI_ROPE = 3, EPI_ROPE128 = 4 /* kernels only: EPI_ROPE with head dim 128 */ };
 
 // RoPE fused into the epilogue of the merged QKV projection: applied to the q and k head parts
 // (column part p of width dh is q or k when p % group <= g; group = g + 2, g = q heads per kv head).
@@ -82,7 +82,7 @@ struct GemmRope {
   const float* sin_tab;
   int T;                 // tokens per request: position = min(row % T, pos_cap)
   int pos_cap;
-  int dh;                // 32 or 64
+  int dh;                // 32, 64 or 128
   int group, g;
   // split token layout (all history rows, then all candidate rows): GEMM row r is token row r + row_offset; rows
   // below split_rows are history rows of `T` per request, the rows from split_rows on sit at position pos_cap.

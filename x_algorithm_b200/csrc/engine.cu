@@ -485,8 +485,9 @@ phx_status run_trunk(phx_engine* e, int B, int Tt, int pos_cap, int hist_len, bo
     GemmPlan& pq = fused ? L.p_qkv_f : L.p_qkv;
     GemmPlan& pu = fused ? L.p_up_f : L.p_up;
     const bf16* a_in = fused ? e->x : e->hbuf;
-    // RoPE rides in the QKV epilogue unless qk-norm has to run first or the head dim is 128
-    const bool fuse_rope = c.rotary && !c.qk_norm && !e->use_simt_gemm && (e->dh == 32 || e->dh == 64);
+    // RoPE rides in the QKV epilogue unless qk-norm has to run first (heads of 128 through a pass of their own: 522 us for a
+    // two-layer forward of 8 x 1086 rows, 465 us in the epilogue)
+    const bool fuse_rope = c.rotary && !c.qk_norm && !e->use_simt_gemm;
     if (fuse_rope) {
       GemmRope gr;
       gr.cos_tab = e->cos_tab; gr.sin_tab = e->sin_tab; gr.T = Tt; gr.pos_cap = pos_cap; gr.dh = e->dh;

@@ -86,7 +86,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   // C and R may be the same buffer (in-place residual update): a slab is fetched before it is written back,
   // and no other CTA touches the tile.
   using cfg = Cfg<BN, PAIR, NG>;
-  constexpr int SLABS = BN / SLAB_COLS;
+  // columns per epilogue work item: one 64-column slab, or a whole head of 128 whose halves RoPE rotates against each other
+  constexpr int ITEM_COLS = (EPI == EPI_ROPE128) ? 128 : SLAB_COLS;
+  constexpr int ITEM_SLABS = ITEM_COLS / SLAB_COLS;
+  constexpr int SLABS = BN / ITEM_COLS;      // items per tile
   // epilogue threads that drain one accumulator (a tile with fewer slabs than groups is shared by SLABS groups)
   constexpr int DRAIN_THREADS = (SLABS < NG ? SLABS : NG) * 128 * (PAIR ? 2 : 1);
   extern __shared__ uint8_t smem_raw[];
@@ -240,7 +243,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // slab buffers, an issuing thread and named barrier 1 + gidx.  Per item: TMEM -> registers -> fused op
     // -> swizzled shared-memory slab -> one TMA bulk store.  The residual slab arrives by TMA into the same
     // buffer (up to NB - 1 items ahead, at least one) and is updated in place.
-    constexpr int NB = cfg::NSLAB / NG;
+    constexpr int NB = cfg::NSLAB / NG / ITEM_SLABS;    // item buffers per group
+    static_assert(NB >= 1, "an item needs its slab buffers");
     constexpr bool RES = (EPI == EPI_RESIDUAL);
     constexpr int DIST = NB - 1;                        // residual prefetch distance (items of this group)
     const int ew = warp - 2;
@@ -259,12 +263,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     };
     const long long total_items = my_tiles * SLABS;
     const long long my_items = (total_items > gidx) ? (total_items - gidx + NG - 1) / NG : 0;
-    const uint32_t gslab = slab_base + gidx * NB * SLAB_BYTES;
+    const uint32_t gslab = slab_base + gidx * NB * ITEM_SLABS * SLAB_BYTES;
     auto coords = [&](long long i, long long& m0, int& c0) {   // i = item index inside this group
       const long long q = (long long)NG * i + gidx;
       const long long tile = first_tile + (q / SLABS) * tile_step;
       m0 = (tile / n_tiles) * TILE_M + rank * BM;
-      c0 = (int)(tile % n_tiles) * BN + (int)(q % SLABS) * SLAB_COLS;
+      c0 = (int)(tile % n_tiles) * BN + (int)(q % SLABS) * ITEM_COLS;
     };
     auto issue_res = [&](long long i) {
       long long m1; int c1; coords(i, m1, c1);
@@ -281,7 +285,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int s = (int)(q % SLABS);
       const uint32_t it = (uint32_t)(q / SLABS), acc = it & 1, acc_phase = (it >> 1) & 1;
       const int bi = (int)(i % NB);
-      const uint32_t slab = gslab + bi * SLAB_BYTES;
+      const uint32_t slab = gslab + bi * ITEM_SLABS * SLAB_BYTES;
       long long m0; int c0; coords(i, m0, c0);
       const bool first_of_tile = (s < NG);              // this group's first slab of the tile
       // RMSNorm folded into this GEMM: the row's 1/rms comes from the sum of squares its producer left behind
@@ -321,7 +325,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       }
       const uint32_t row_addr = slab + row_in_tile * 128;
       const int sw = row_in_tile & 7;
-      const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quad * 32) << 16) + s * SLAB_COLS;
+      const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quad * 32) << 16) + s * ITEM_COLS;
       if (!RES) {
         // the store that last read this buffer (item i - NB of this group) must have drained before it is rewritten
         if (issuer) bulk_wait_read<NB - 1>();
@@ -329,10 +333,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       }
       if (ok) {
         tc_fence_after();
-        if (EPI == EPI_ROPE) {
-          // RoPE on the q / k head parts of this slab (layers.py:52-67, 784-788), pairs (j, j + dh/2), in two
+        if (EPI == EPI_ROPE || EPI == EPI_ROPE128) {
+          // RoPE on the q / k head parts of this item (layers.py:52-67, 784-788), pairs (j, j + dh/2), in
           // passes of 16 pairs so that only 32 values are live: head dim 64 = one part per slab, pass p rotates
-          // columns [16p, 16p+16) against [32+16p, 48+16p); head dim 32 = pass p is the slab's p-th part.
+          // columns [16p, 16p+16) against [32+16p, 48+16p); head dim 32 = pass p is the slab's p-th part; head dim 128 =
+          // four passes, [16p, 16p+16) of the item's first slab against the same columns of its second.
+          constexpr bool D128 = EPI == EPI_ROPE128;
           const long long row = m0 + row_in_tile + rope.row_offset;
           int pos = rope.pos_cap;                       // split layout: the candidate block sits at the cap
           if (rope.pos_rows) {                          // packed rows: the position comes with the row
@@ -341,18 +347,18 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const int t = (int)(row % rope.T);
             pos = t < rope.pos_cap ? t : rope.pos_cap;
           }
-          const bool d64 = (rope.dh == 64);
+          const bool d64 = !D128 && (rope.dh == 64);
           const int half = rope.dh >> 1;
 #pragma unroll
-          for (int p = 0; p < 2; ++p) {
-            const int lo_col = d64 ? 16 * p : 32 * p;
-            const int hi_col = d64 ? 32 + 16 * p : 32 * p + 16;
+          for (int p = 0; p < (D128 ? 4 : 2); ++p) {
+            const int lo_col = (D128 || d64) ? 16 * p : 32 * p;
+            const int hi_col = D128 ? 64 + 16 * p : d64 ? 32 + 16 * p : 32 * p + 16;
             uint32_t rl[16], rh[16];
             tmem_ld16_nowait(taddr + lo_col, rl);
             tmem_ld16_nowait(taddr + hi_col, rh);
             tmem_ld_wait();
-            if (p == 1 && last_of_tile) release_acc(acc);
-            const int kind = d64 ? (c0 >> 6) % rope.group : ((c0 >> 5) + p) % rope.group;
+            if (p == (D128 ? 3 : 1) && last_of_tile) release_acc(acc);
+            const int kind = D128 ? (c0 >> 7) % rope.group : d64 ? (c0 >> 6) % rope.group : ((c0 >> 5) + p) % rope.group;
             float lo[16], hi[16];
 #pragma unroll
             for (int k = 0; k < 16; ++k) {   // Linear output is bf16
@@ -360,8 +366,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
               hi[k] = round_bf(__uint_as_float(rh[k]) * rstd);
             }
             if (kind <= rope.g) {   // q or k part (v parts pass through)
-              const float4* c4 = reinterpret_cast<const float4*>(rope.cos_tab + (long long)pos * half + (d64 ? 16 * p : 0));
-              const float4* s4 = reinterpret_cast<const float4*>(rope.sin_tab + (long long)pos * half + (d64 ? 16 * p : 0));
+              const float4* c4 = reinterpret_cast<const float4*>(rope.cos_tab + (long long)pos * half + ((D128 || d64) ? 16 * p : 0));
+              const float4* s4 = reinterpret_cast<const float4*>(rope.sin_tab + (long long)pos * half + ((D128 || d64) ? 16 * p : 0));
 #pragma unroll
               for (int jj = 0; jj < 4; ++jj) {
                 const float4 c = __ldg(c4 + jj), sn = __ldg(s4 + jj);
@@ -383,7 +389,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
               st_shared_v4(row_addr + ((uint32_t)(((lo_col >> 3) + h) ^ sw) << 4), o);
               o.x = pack_bf2(hi[h * 8 + 0], hi[h * 8 + 1]); o.y = pack_bf2(hi[h * 8 + 2], hi[h * 8 + 3]);
               o.z = pack_bf2(hi[h * 8 + 4], hi[h * 8 + 5]); o.w = pack_bf2(hi[h * 8 + 6], hi[h * 8 + 7]);
-              st_shared_v4(row_addr + ((uint32_t)(((hi_col >> 3) + h) ^ sw) << 4), o);
+              if (D128) st_shared_v4(row_addr + SLAB_BYTES + ((uint32_t)(((lo_col >> 3) + h) ^ sw) << 4), o);
+              else st_shared_v4(row_addr + ((uint32_t)(((hi_col >> 3) + h) ^ sw) << 4), o);
             }
           }
         } else {
@@ -424,6 +431,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       if (!epi_barrier_and(ok, 1 + gidx)) break;        // uniform over the group's 128 threads
       if (issuer && c0 < N && m0 < M) {
         tma_store_2d(&map_c, slab, c0, (int)m0);
+        if (ITEM_SLABS == 2) tma_store_2d(&map_c, slab + SLAB_BYTES, c0 + SLAB_COLS, (int)m0);
         bulk_commit();
       }
     }
@@ -449,7 +457,8 @@ phx_status launch_t(const GemmPlan& p, const GemmRope& rope, const GemmNorm& nor
   // the residual epilogues are fed by TMA prefetch and keep up with two groups; the others (RoPE, GELU, norm
   // scaling) are bound by the latency of each thread's instruction stream and get four groups where a pair's
   // smaller stages leave room for the slab buffers
-  constexpr int NG = (PAIR && EPI != EPI_RESIDUAL) ? 4 : 2;
+  // (heads of 128: two groups, each with the two slab buffers of its item)
+  constexpr int NG = (PAIR && EPI != EPI_RESIDUAL && EPI != EPI_ROPE128) ? 4 : 2;
   using cfg = Cfg<BN, PAIR, NG>;
   auto kern = gemm_tcgen05_kernel<BN, EPI, PAIR, NG>;
   static bool attr_set = false;
@@ -510,7 +519,12 @@ phx_status launch_e(const GemmPlan& p, int epilogue, const GemmRope& rp, const G
     case EPI_STORE: return launch_t<BN, EPI_STORE, PAIR>(p, rp, nm, M, err_flag, num_sms, stream, err);
     case EPI_RESIDUAL: return launch_t<BN, EPI_RESIDUAL, PAIR>(p, rp, nm, M, err_flag, num_sms, stream, err);
     case EPI_GELU: return launch_t<BN, EPI_GELU, PAIR>(p, rp, nm, M, err_flag, num_sms, stream, err);
-    case EPI_ROPE: return launch_t<BN, EPI_ROPE, PAIR>(p, rp, nm, M, err_flag, num_sms, stream, err);
+    case EPI_ROPE:
+      if (rp.dh == 128) {   // a single CTA's 256-column tiles leave no room for the item buffers: gemm_launch takes narrow ones
+        if constexpr (PAIR || BN == 128) return launch_t<BN, EPI_ROPE128, PAIR>(p, rp, nm, M, err_flag, num_sms, stream, err);
+        break;
+      }
+      return launch_t<BN, EPI_ROPE, PAIR>(p, rp, nm, M, err_flag, num_sms, stream, err);
   }
   err = "gemm: unknown epilogue";
   return PHX_E_ARG;
@@ -612,7 +626,9 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       if (ok) umma_commit(tfull_bar);
     }
   } else {
-    const int gidx = (warp - 2) >> 2, slab = gidx >> 1, p = gidx & 1;
+    // heads of 128 columns (BN = 128 only): the tile is one head, group p takes pass p of its four
+    const bool d128 = EPI == EPI_ROPE && BN == 128 && rope.dh == 128;
+    const int gidx = (warp - 2) >> 2, slab = d128 ? 0 : gidx >> 1, p = d128 ? gidx : gidx & 1;
     const int quad = warp & 3;
     const int r = quad * 32 + lane;
     const long long row = m0 + r;
@@ -620,7 +636,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const int c0 = n0 + slab * 64;                       // first column of the slab
     // two runs of 16 columns: neighbours, or (RoPE) the halves of a head that are rotated against each other
     const bool d64 = EPI == EPI_ROPE && rope.dh == 64;
-    const int lo_col = d64 ? 16 * p : 32 * p, hi_col = d64 ? 32 + 16 * p : 32 * p + 16;
+    const int lo_col = (d64 || d128) ? 16 * p : 32 * p, hi_col = d128 ? 64 + 16 * p : d64 ? 32 + 16 * p : 32 * p + 16;
     // ---- everything that does not need the accumulator ----
     uint4 res[4];
     if (RES) {
@@ -654,10 +670,10 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const int t = (int)(trow % rope.T);
         pos = t < rope.pos_cap ? t : rope.pos_cap;
       }
-      const int kind = d64 ? (c0 >> 6) % rope.group : ((c0 >> 5) + p) % rope.group;
+      const int kind = d128 ? (c0 >> 7) % rope.group : d64 ? (c0 >> 6) % rope.group : ((c0 >> 5) + p) % rope.group;
       rotate = kind <= rope.g;
       if (rotate) {
-        const long long o = (long long)pos * (rope.dh >> 1) + (d64 ? 16 * p : 0);
+        const long long o = (long long)pos * (rope.dh >> 1) + ((d64 || d128) ? 16 * p : 0);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           cs[j] = __ldg(reinterpret_cast<const float4*>(rope.cos_tab + o) + j);
@@ -862,8 +878,8 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
     p.A = A; p.a_rows = M;
   }
   if (epilogue == EPI_ROPE) {
-    if (!rope || (rope->dh != 32 && rope->dh != 64) || rope->T <= 0 || p.N % rope->dh != 0) {
-      err = "gemm: the RoPE epilogue needs head dim 32 or 64";
+    if (!rope || (rope->dh != 32 && rope->dh != 64 && rope->dh != 128) || rope->T <= 0 || p.N % rope->dh != 0) {
+      err = "gemm: the RoPE epilogue needs head dim 32, 64 or 128";
       return PHX_E_ARG;
     }
     rp = *rope;
@@ -886,7 +902,7 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
     const CUtensorMap& map_b64 = p.BN == 256 ? p.map_b_narrow : p.map_b;   // boxes of 64 W rows, either way
     const long long mt = (M + BM - 1) / BM, t64 = mt * ((p.N + 63) / 64), t128 = mt * ((p.N + 127) / 128);
     if (small_ok && (p.BN != 256 || p.has_narrow)) {
-      if (t64 <= num_sms) { dispatch_note(DK_GEMM_SMALL); return launch_small<64>(p, map_b64, C, R, epilogue, rp, nm, M, err_flag, stream, err); }
+      if (t64 <= num_sms && !(epilogue == EPI_ROPE && rp.dh == 128)) { dispatch_note(DK_GEMM_SMALL); return launch_small<64>(p, map_b64, C, R, epilogue, rp, nm, M, err_flag, stream, err); }
       if (t128 <= num_sms) { dispatch_note(DK_GEMM_SMALL); return launch_small<128>(p, map_b64, C, R, epilogue, rp, nm, M, err_flag, stream, err); }
     }
   }
@@ -896,7 +912,8 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
     const long long narrow_tiles = ((M + rows_per_tile - 1) / rows_per_tile) * ((p.N + 127) / 128);
     const long long slots = p.pair ? num_sms / 2 : num_sms;
     static const bool allow = !(getenv("PHX_GEMM_TILES") && strcmp(getenv("PHX_GEMM_TILES"), "wide") == 0);
-    if (allow && p.has_narrow && narrow_tiles <= slots) {
+    const bool must = !p.pair && epilogue == EPI_ROPE && rp.dh == 128;
+    if (p.has_narrow && (must || (allow && narrow_tiles <= slots))) {
       dispatch_note(p.pair ? DK_GEMM_PAIR128 : DK_GEMM_CTA128);
       GemmPlan q = p;
       q.map_b = p.map_b_narrow; q.BN = 128;
