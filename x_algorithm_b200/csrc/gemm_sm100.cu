@@ -77,6 +77,43 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint4 v) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
+// Epilogue arithmetic, two columns per instruction (packed fp32) and one conversion per pair: an epilogue thread's
+// instruction stream is what a tile with a short K waits for.  Measured: 163840 x 1024, K = 256, GELU 114.6 -> 94.2 us; a
+// forward of one request 384 -> 349 us, the user tower of 256 users 513 -> 492 us, 48 ragged requests 611 -> 597 us.
+// fp32 accumulators -> the Linear output, a bf16 pair: rounded once, kept in the form it is stored in
+__device__ __forceinline__ uint32_t linear_bf2(uint32_t a0, uint32_t a1, float2 rstd2) {
+  const float2 v = __fmul2_rn(make_float2(__uint_as_float(a0), __uint_as_float(a1)), rstd2);
+  return pack_bf2(v.x, v.y);
+}
+__device__ __forceinline__ float2 bf2_to_f2(uint32_t b) { return make_float2(__uint_as_float(b << 16), __uint_as_float(b & 0xFFFF0000u)); }
+// GELU, tanh form, of a bf16 pair (gelu_tanh_f's formula: sqrt(2/pi) (x + 0.044715 x^3) as x (c0 + c1 x^2))
+__device__ __forceinline__ uint32_t gelu_bf2(uint32_t b) {
+  const float2 x = bf2_to_f2(b);
+  const float2 p = __ffma2_rn(__fmul2_rn(x, x), make_float2(0.035677408136300125f, 0.035677408136300125f),
+                              make_float2(0.7978845608028654f, 0.7978845608028654f));
+  const float2 in = __fmul2_rn(x, p);
+  float2 t;
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t.x) : "f"(in.x));
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t.y) : "f"(in.y));
+  const float2 h = __fmul2_rn(x, make_float2(0.5f, 0.5f));
+  const float2 g = __ffma2_rn(h, t, h);
+  return pack_bf2(g.x, g.y);
+}
+// one RoPE pair of columns against its partner pair: (lo, hi) -> (lo c - hi s, hi c + lo s)
+__device__ __forceinline__ void rope_bf2(uint32_t& lo, uint32_t& hi, float c0, float c1, float s0, float s1) {
+  const float2 x1 = bf2_to_f2(lo), x2 = bf2_to_f2(hi), c = make_float2(c0, c1), sn = make_float2(s0, s1);
+  const float2 a = __fmul2_rn(x2, sn), b = __fmul2_rn(x1, sn);
+  const float2 l = __ffma2_rn(x1, c, make_float2(-a.x, -a.y)), h = __ffma2_rn(x2, c, b);
+  lo = pack_bf2(l.x, l.y); hi = pack_bf2(h.x, h.y);
+}
+// position of a token row: the row's slot in its request, at most pos_cap (GemmRope); token rows fit 31 bits
+__device__ __forceinline__ int rope_pos(const GemmRope& rope, long long row, bool in) {
+  if (rope.pos_rows) return in ? rope.pos_rows[row] : 0;
+  if (rope.split_rows != 0 && row >= rope.split_rows) return rope.pos_cap;
+  const int t = (int)((unsigned)row % (unsigned)rope.T);
+  return t < rope.pos_cap ? t : rope.pos_cap;
+}
+
 template <int BN, int EPI, bool PAIR, int NG>
 __global__ void __launch_bounds__(gemm_threads(NG), 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -309,6 +346,30 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
       }
       const bool last_of_tile = (s + NG >= SLABS);      // ... and its last
+      // RoPE: whether this item is rotated (q and k parts are), the row's position, and the first pass' angles, all before
+      // the wait on the accumulator
+      constexpr bool ROPE = EPI == EPI_ROPE || EPI == EPI_ROPE128, D128 = EPI == EPI_ROPE128;
+      const bool d64 = ROPE && !D128 && rope.dh == 64;
+      float4 cs[4], sn[4];
+      const float4 *cos_row = nullptr, *sin_row = nullptr;
+      auto part_rotated = [&](int p) {
+        const int part = D128 ? (c0 >> 7) : d64 ? (c0 >> 6) : (c0 >> 5) + p;
+        return part % rope.group <= rope.g;
+      };
+      auto load_angles = [&](int p) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          cs[j] = __ldg(cos_row + ((D128 || d64) ? 4 * p : 0) + j);
+          sn[j] = __ldg(sin_row + ((D128 || d64) ? 4 * p : 0) + j);
+        }
+      };
+      if (ROPE) {
+        const long long row = m0 + row_in_tile;
+        const long long o = (long long)rope_pos(rope, row + rope.row_offset, row < M) * (rope.dh >> 1);
+        cos_row = reinterpret_cast<const float4*>(rope.cos_tab + o);
+        sin_row = reinterpret_cast<const float4*>(rope.sin_tab + o);
+        if (part_rotated(0)) load_angles(0);
+      }
       if (RES && issuer && i + DIST < my_items) {
         // the buffer of item i + DIST was last used by item i - 1: its store must have drained
         bulk_wait_read<0>();
@@ -333,22 +394,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       }
       if (ok) {
         tc_fence_after();
-        if (EPI == EPI_ROPE || EPI == EPI_ROPE128) {
+        const float2 rstd2 = make_float2(rstd, rstd);
+        if (ROPE) {
           // RoPE on the q / k head parts of this item (layers.py:52-67, 784-788), pairs (j, j + dh/2), in
           // passes of 16 pairs so that only 32 values are live: head dim 64 = one part per slab, pass p rotates
           // columns [16p, 16p+16) against [32+16p, 48+16p); head dim 32 = pass p is the slab's p-th part; head dim 128 =
           // four passes, [16p, 16p+16) of the item's first slab against the same columns of its second.
-          constexpr bool D128 = EPI == EPI_ROPE128;
-          const long long row = m0 + row_in_tile + rope.row_offset;
-          int pos = rope.pos_cap;                       // split layout: the candidate block sits at the cap
-          if (rope.pos_rows) {                          // packed rows: the position comes with the row
-            pos = row < M + rope.row_offset ? rope.pos_rows[row] : 0;
-          } else if (rope.split_rows == 0 || row < rope.split_rows) {
-            const int t = (int)(row % rope.T);
-            pos = t < rope.pos_cap ? t : rope.pos_cap;
-          }
-          const bool d64 = !D128 && (rope.dh == 64);
-          const int half = rope.dh >> 1;
 #pragma unroll
           for (int p = 0; p < (D128 ? 4 : 2); ++p) {
             const int lo_col = (D128 || d64) ? 16 * p : 32 * p;
@@ -358,39 +409,26 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             tmem_ld16_nowait(taddr + hi_col, rh);
             tmem_ld_wait();
             if (p == (D128 ? 3 : 1) && last_of_tile) release_acc(acc);
-            const int kind = D128 ? (c0 >> 7) % rope.group : d64 ? (c0 >> 6) % rope.group : ((c0 >> 5) + p) % rope.group;
-            float lo[16], hi[16];
+            uint32_t lo[8], hi[8];
 #pragma unroll
-            for (int k = 0; k < 16; ++k) {   // Linear output is bf16
-              lo[k] = round_bf(__uint_as_float(rl[k]) * rstd);
-              hi[k] = round_bf(__uint_as_float(rh[k]) * rstd);
+            for (int k = 0; k < 8; ++k) {
+              lo[k] = linear_bf2(rl[2 * k], rl[2 * k + 1], rstd2);
+              hi[k] = linear_bf2(rh[2 * k], rh[2 * k + 1], rstd2);
             }
-            if (kind <= rope.g) {   // q or k part (v parts pass through)
-              const float4* c4 = reinterpret_cast<const float4*>(rope.cos_tab + (long long)pos * half + ((D128 || d64) ? 16 * p : 0));
-              const float4* s4 = reinterpret_cast<const float4*>(rope.sin_tab + (long long)pos * half + ((D128 || d64) ? 16 * p : 0));
+            if (part_rotated(p)) {   // v parts pass through
 #pragma unroll
-              for (int jj = 0; jj < 4; ++jj) {
-                const float4 c = __ldg(c4 + jj), sn = __ldg(s4 + jj);
-                const float cc[4] = {c.x, c.y, c.z, c.w}, ss[4] = {sn.x, sn.y, sn.z, sn.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const int j = jj * 4 + e;
-                  const float x1 = lo[j], x2 = hi[j];
-                  lo[j] = x1 * cc[e] - x2 * ss[e];
-                  hi[j] = x2 * cc[e] + x1 * ss[e];
-                }
+              for (int j = 0; j < 4; ++j) {
+                rope_bf2(lo[2 * j], hi[2 * j], cs[j].x, cs[j].y, sn[j].x, sn[j].y);
+                rope_bf2(lo[2 * j + 1], hi[2 * j + 1], cs[j].z, cs[j].w, sn[j].z, sn[j].w);
               }
             }
+            if (p + 1 < (D128 ? 4 : 2) && part_rotated(p + 1)) load_angles(p + 1);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-              uint4 o;
-              o.x = pack_bf2(lo[h * 8 + 0], lo[h * 8 + 1]); o.y = pack_bf2(lo[h * 8 + 2], lo[h * 8 + 3]);
-              o.z = pack_bf2(lo[h * 8 + 4], lo[h * 8 + 5]); o.w = pack_bf2(lo[h * 8 + 6], lo[h * 8 + 7]);
-              st_shared_v4(row_addr + ((uint32_t)(((lo_col >> 3) + h) ^ sw) << 4), o);
-              o.x = pack_bf2(hi[h * 8 + 0], hi[h * 8 + 1]); o.y = pack_bf2(hi[h * 8 + 2], hi[h * 8 + 3]);
-              o.z = pack_bf2(hi[h * 8 + 4], hi[h * 8 + 5]); o.w = pack_bf2(hi[h * 8 + 6], hi[h * 8 + 7]);
-              if (D128) st_shared_v4(row_addr + SLAB_BYTES + ((uint32_t)(((lo_col >> 3) + h) ^ sw) << 4), o);
-              else st_shared_v4(row_addr + ((uint32_t)(((hi_col >> 3) + h) ^ sw) << 4), o);
+              st_shared_v4(row_addr + ((uint32_t)(((lo_col >> 3) + h) ^ sw) << 4), make_uint4(lo[4 * h], lo[4 * h + 1], lo[4 * h + 2], lo[4 * h + 3]));
+              const uint32_t hi_addr = D128 ? row_addr + SLAB_BYTES + ((uint32_t)(((lo_col >> 3) + h) ^ sw) << 4)
+                                            : row_addr + ((uint32_t)(((hi_col >> 3) + h) ^ sw) << 4);
+              st_shared_v4(hi_addr, make_uint4(hi[4 * h], hi[4 * h + 1], hi[4 * h + 2], hi[4 * h + 3]));
             }
           }
         } else {
@@ -400,27 +438,26 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             uint32_t r[32];
             tmem_ld32(taddr + hh * 32, r);
             if (hh == 1 && last_of_tile) release_acc(acc);
-            float v[32];
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {
-              v[k] = round_bf(__uint_as_float(r[k]) * rstd);                   // Linear output is bf16
-              if (EPI == EPI_GELU) v[k] = gelu_tanh_f(v[k]);
-            }
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
               const uint32_t addr = row_addr + ((uint32_t)((hh * 4 + c) ^ sw) << 4);
+              uint32_t o[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                o[k] = linear_bf2(r[c * 8 + 2 * k], r[c * 8 + 2 * k + 1], rstd2);
+                if (EPI == EPI_GELU) o[k] = gelu_bf2(o[k]);
+              }
               if (RES) {
                 const uint4 rr = ld_shared_v4(addr);
-                const float2 a = unpack_bf2(rr.x), b = unpack_bf2(rr.y), cc = unpack_bf2(rr.z), d = unpack_bf2(rr.w);
-                v[c * 8 + 0] += a.x; v[c * 8 + 1] += a.y; v[c * 8 + 2] += b.x; v[c * 8 + 3] += b.y;
-                v[c * 8 + 4] += cc.x; v[c * 8 + 5] += cc.y; v[c * 8 + 6] += d.x; v[c * 8 + 7] += d.y;
+                const uint32_t rb[4] = {rr.x, rr.y, rr.z, rr.w};
 #pragma unroll
-                for (int k = 0; k < 8; ++k) ss_out += v[c * 8 + k] * v[c * 8 + k];   // statistics of the fp32 sums (pre-rounding)
+                for (int k = 0; k < 4; ++k) {
+                  const float2 v = __fadd2_rn(bf2_to_f2(o[k]), bf2_to_f2(rb[k]));
+                  ss_out += v.x * v.x; ss_out += v.y * v.y;          // statistics of the fp32 sums (pre-rounding)
+                  o[k] = pack_bf2(v.x, v.y);
+                }
               }
-              uint4 o;
-              o.x = pack_bf2(v[c * 8 + 0], v[c * 8 + 1]); o.y = pack_bf2(v[c * 8 + 2], v[c * 8 + 3]);
-              o.z = pack_bf2(v[c * 8 + 4], v[c * 8 + 5]); o.w = pack_bf2(v[c * 8 + 6], v[c * 8 + 7]);
-              st_shared_v4(addr, o);
+              st_shared_v4(addr, make_uint4(o[0], o[1], o[2], o[3]));
             }
           }
           if (RES && norm.ss_out != nullptr && m0 + row_in_tile < M && c0 < N)
@@ -663,13 +700,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     float4 cs[4], sn[4];
     bool rotate = false;
     if (EPI == EPI_ROPE) {
-      const long long trow = row + rope.row_offset;
-      int pos = rope.pos_cap;
-      if (rope.pos_rows) pos = in ? rope.pos_rows[trow] : 0;
-      else if (rope.split_rows == 0 || trow < rope.split_rows) {
-        const int t = (int)(trow % rope.T);
-        pos = t < rope.pos_cap ? t : rope.pos_cap;
-      }
+      const int pos = rope_pos(rope, row + rope.row_offset, in);
       const int kind = d128 ? (c0 >> 7) % rope.group : d64 ? (c0 >> 6) % rope.group : ((c0 >> 5) + p) % rope.group;
       rotate = kind <= rope.g;
       if (rotate) {
@@ -690,40 +721,38 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       tmem_ld16_nowait(taddr + lo_col, raw);
       tmem_ld16_nowait(taddr + hi_col, raw + 16);
       tmem_ld_wait();
-      float v[32];
+      const float2 rstd2 = make_float2(rstd, rstd);
+      uint32_t o[16];                                                 // column pairs: 8 of the low run, 8 of the high run
 #pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        v[k] = round_bf(__uint_as_float(raw[k]) * rstd);              // Linear output is bf16
-        if (EPI == EPI_GELU) v[k] = gelu_tanh_f(v[k]);
+      for (int k = 0; k < 16; ++k) {
+        o[k] = linear_bf2(raw[2 * k], raw[2 * k + 1], rstd2);
+        if (EPI == EPI_GELU) o[k] = gelu_bf2(o[k]);
       }
       if (EPI == EPI_ROPE && rotate) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float cc[4] = {cs[j].x, cs[j].y, cs[j].z, cs[j].w}, ss[4] = {sn[j].x, sn[j].y, sn[j].z, sn[j].w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float x1 = v[j * 4 + e], x2 = v[16 + j * 4 + e];
-            v[j * 4 + e] = x1 * cc[e] - x2 * ss[e];
-            v[16 + j * 4 + e] = x2 * cc[e] + x1 * ss[e];
-          }
+          rope_bf2(o[2 * j], o[8 + 2 * j], cs[j].x, cs[j].y, sn[j].x, sn[j].y);
+          rope_bf2(o[2 * j + 1], o[8 + 2 * j + 1], cs[j].z, cs[j].w, sn[j].z, sn[j].w);
         }
       }
+      float2 v[RES ? 16 : 1];
       if (RES) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          const float2 a = unpack_bf2(res[c].x), b = unpack_bf2(res[c].y), d = unpack_bf2(res[c].z), e = unpack_bf2(res[c].w);
-          v[c * 8 + 0] += a.x; v[c * 8 + 1] += a.y; v[c * 8 + 2] += b.x; v[c * 8 + 3] += b.y;
-          v[c * 8 + 4] += d.x; v[c * 8 + 5] += d.y; v[c * 8 + 6] += e.x; v[c * 8 + 7] += e.y;
+          const uint32_t rb[4] = {res[c].x, res[c].y, res[c].z, res[c].w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float2 x = __fadd2_rn(bf2_to_f2(o[4 * c + k]), bf2_to_f2(rb[k]));
+            v[RES ? 4 * c + k : 0] = x;
+            o[4 * c + k] = pack_bf2(x.x, x.y);
+          }
         }
       }
       if (in) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const int col = c0 + (c < 2 ? lo_col : hi_col) + (c & 1) * 8;
-          uint4 o;
-          o.x = pack_bf2(v[c * 8 + 0], v[c * 8 + 1]); o.y = pack_bf2(v[c * 8 + 2], v[c * 8 + 3]);
-          o.z = pack_bf2(v[c * 8 + 4], v[c * 8 + 5]); o.w = pack_bf2(v[c * 8 + 6], v[c * 8 + 7]);
-          if (col < N) *reinterpret_cast<uint4*>(C + row * N + col) = o;
+          if (col < N) *reinterpret_cast<uint4*>(C + row * N + col) = make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
         }
       }
       if (RES && norm.ss_out != nullptr) {
@@ -733,14 +762,14 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         float ss = 0.f;
         if (p == 0) {
 #pragma unroll
-          for (int k = 0; k < 32; ++k) ss += v[k] * v[k];
+          for (int k = 0; k < (RES ? 16 : 1); ++k) { ss += v[k].x * v[k].x; ss += v[k].y * v[k].y; }
           asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot), "f"(ss) : "memory");
         }
         asm volatile("bar.sync %0, 256;" ::"r"(1 + slab) : "memory");
         if (p == 1) {
           asm volatile("ld.shared.f32 %0, [%1];" : "=f"(ss) : "r"(slot) : "memory");
 #pragma unroll
-          for (int k = 0; k < 32; ++k) ss += v[k] * v[k];
+          for (int k = 0; k < (RES ? 16 : 1); ++k) { ss += v[k].x * v[k].x; ss += v[k].y * v[k].y; }
           if (in && c0 < N) norm.ss_out[row * (long long)(N / SLAB_COLS) + c0 / SLAB_COLS] = ss;
         }
       }
