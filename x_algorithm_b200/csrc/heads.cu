@@ -124,14 +124,19 @@ __device__ __forceinline__ void mma_bf16_16816_h(float (&c)[4], const uint32_t (
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <int NT>   // n-tiles of 8 outputs: V + NC <= 8 * NT
-__global__ void __launch_bounds__(HM_WARPS * 32) heads_mma_kernel(HeadsArgs a) {
+// NT: n-tiles of 8 outputs, V + NC <= 8 * NT.  WPS: warps per strip.  With enough strips every warp has its own (1); a small call
+// is one strip's chain of latencies, most of it the ten rounds of logarithms and f64 exponentials, so four warps form the
+// same sums and share the (row, output) items of one strip.  Same arithmetic, same bits.  One request of 512
+// candidates, whole call: 348.7 -> 346.4 us.
+template <int NT, int WPS>
+__global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_kernel(HeadsArgs a) {
+  constexpr int WARPS = WPS == 1 ? HM_WARPS : WPS;      // warps per CTA
   extern __shared__ __align__(16) uint8_t hsm[];
   const int D = a.D, NO = a.V + a.NC, WLD = D + HM_WPAD;
   bf16* sw = reinterpret_cast<bf16*>(hsm);                                   // [NT*8][WLD], rows >= NO are zero
   float* sgain = reinterpret_cast<float*>(sw + NT * 8 * WLD);                // [D]
   float* sC_all = sgain + D;                                                 // per warp [16][NT*8] fp32 sums
-  double* sD_all = reinterpret_cast<double*>(sC_all + HM_WARPS * 16 * NT * 8);   // per warp [16][NT*8] blend inputs
+  double* sD_all = reinterpret_cast<double*>(sC_all + WARPS * 16 * NT * 8);   // per strip [16][NT*8] blend inputs
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   for (int i = threadIdx.x; i < NT * 8 * (D / 8); i += blockDim.x) {
     const int n = i / (D / 8), ch = i % (D / 8);
@@ -145,11 +150,13 @@ __global__ void __launch_bounds__(HM_WARPS * 32) heads_mma_kernel(HeadsArgs a) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   __syncthreads();
   float* sC = sC_all + warp * 16 * NT * 8;
-  double* sD = sD_all + warp * 16 * NT * 8;
+  double* sD = sD_all + (WPS == 1 ? warp : 0) * 16 * NT * 8;
+  const int part = WPS == 1 ? 0 : warp;                 // this warp's share of the strip's items
   const long long nrows = a.out_index ? a.rows : (long long)a.B * a.C;
   const long long n_strips = (nrows + 15) / 16;
   const int groups = D / 32;
-  for (long long strip = (long long)blockIdx.x * HM_WARPS + warp; strip < n_strips; strip += (long long)gridDim.x * HM_WARPS) {
+  constexpr int CTA_STRIPS = WPS == 1 ? HM_WARPS : 1;
+  for (long long strip = (long long)blockIdx.x * CTA_STRIPS + (WPS == 1 ? warp : 0); strip < n_strips; strip += (long long)gridDim.x * CTA_STRIPS) {
     const long long r0 = strip * 16;
     const bf16* xr[2];
 #pragma unroll
@@ -160,6 +167,7 @@ __global__ void __launch_bounds__(HM_WARPS * 32) heads_mma_kernel(HeadsArgs a) {
     }
     // pass 1: sums of squares (a row's 32-column groups are spread over the 4 lanes of its quad)
     float ss[2] = {0.f, 0.f};
+#pragma unroll 8
     for (int gr = 0; gr < groups; ++gr) {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -209,7 +217,7 @@ __global__ void __launch_bounds__(HM_WARPS * 32) heads_mma_kernel(HeadsArgs a) {
       *reinterpret_cast<float2*>(sC + (g + 8) * (NT * 8) + j * 8 + 2 * t4) = make_float2(acc[j][2], acc[j][3]);
     }
     __syncwarp();
-    for (int idx = lane; idx < 16 * NO; idx += 32) {
+    for (int idx = lane + 32 * part; idx < 16 * NO; idx += 32 * WPS) {
       const int rr = idx / NO, oo = idx % NO;
       const long long r = r0 + rr;
       const long long orow = (a.out_index && r < nrows) ? a.out_index[r] : r;   // packed rows: the output slot this row answers
@@ -230,8 +238,8 @@ __global__ void __launch_bounds__(HM_WARPS * 32) heads_mma_kernel(HeadsArgs a) {
       }
       sD[rr * (NT * 8) + oo] = col;
     }
-    __syncwarp();
-    if (a.has_blend && a.scores && lane < 16 && r0 + lane < nrows) {
+    if (WPS == 1) __syncwarp(); else __syncthreads();
+    if (a.has_blend && a.scores && part == 0 && lane < 16 && r0 + lane < nrows) {
       double s = 0.0;   // terms summed left to right in f64
       for (int i = 0; i < a.blend.num_terms; ++i) s = s + sD[lane * (NT * 8) + a.blend.src[i]] * a.blend.weight[i];
       double out;
@@ -240,25 +248,26 @@ __global__ void __launch_bounds__(HM_WARPS * 32) heads_mma_kernel(HeadsArgs a) {
       else out = s + 0.001;
       a.scores[a.out_index ? a.out_index[r0 + lane] : r0 + lane] = out;
     }
-    __syncwarp();
+    if (WPS == 1) __syncwarp(); else __syncthreads();
   }
 }
 
-template <int NT>
-phx_status launch_heads_mma(const HeadsArgs& a, long long rows, cudaStream_t stream, std::string& err) {
+template <int NT, int WPS>
+phx_status launch_heads_wps(const HeadsArgs& a, long long strips, cudaStream_t stream, std::string& err) {
+  constexpr int WARPS = WPS == 1 ? HM_WARPS : WPS;
   const size_t smem = (size_t)NT * 8 * (a.D + HM_WPAD) * sizeof(bf16) + (size_t)a.D * sizeof(float) +
-                      (size_t)HM_WARPS * 16 * NT * 8 * (sizeof(float) + sizeof(double));
+                      (size_t)16 * NT * 8 * (WARPS * sizeof(float) + (WPS == 1 ? HM_WARPS : 1) * sizeof(double));
   if (smem > 200 * 1024) { err = "heads: head matrix does not fit shared memory"; return PHX_E_CAPACITY; }
   static bool attr_set = false;
   if (!attr_set) {
-    PHX_CUDA_TRY(cudaFuncSetAttribute(heads_mma_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), err);
+    PHX_CUDA_TRY(cudaFuncSetAttribute(heads_mma_kernel<NT, WPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), err);
     attr_set = true;
   }
-  long long blocks = ((rows + 15) / 16 + HM_WARPS - 1) / HM_WARPS;
+  long long blocks = WPS == 1 ? (strips + HM_WARPS - 1) / HM_WARPS : strips;
   if (blocks > 148 * 3) blocks = 148 * 3;
   cudaLaunchConfig_t lc;
   memset(&lc, 0, sizeof(lc));
-  lc.gridDim = dim3((unsigned)blocks); lc.blockDim = dim3(HM_WARPS * 32); lc.dynamicSmemBytes = smem; lc.stream = stream;
+  lc.gridDim = dim3((unsigned)blocks); lc.blockDim = dim3(WARPS * 32); lc.dynamicSmemBytes = smem; lc.stream = stream;
   cudaLaunchAttribute at[1];
   static const bool pdl = !(getenv("PHX_PDL") && getenv("PHX_PDL")[0] == '0');
   if (pdl) {   // start while the kernel in front drains; the kernel waits before it reads the residual stream
@@ -266,8 +275,15 @@ phx_status launch_heads_mma(const HeadsArgs& a, long long rows, cudaStream_t str
     at[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = at; lc.numAttrs = 1;
   }
-  PHX_CUDA_TRY(cudaLaunchKernelEx(&lc, heads_mma_kernel<NT>, a), err);
+  PHX_CUDA_TRY(cudaLaunchKernelEx(&lc, heads_mma_kernel<NT, WPS>, a), err);
   return PHX_OK;
+}
+template <int NT>
+phx_status launch_heads_mma(const HeadsArgs& a, long long rows, cudaStream_t stream, std::string& err) {
+  // up to two CTAs of a strip each per SM: beyond that the strips alone keep the SMs busy
+  const long long strips = (rows + 15) / 16;
+  if (strips <= 2 * 148) return launch_heads_wps<NT, 4>(a, strips, stream, err);
+  return launch_heads_wps<NT, 1>(a, strips, stream, err);
 }
 
 // users[b] = l2norm(mean over valid t of final_norm(x[b,t])), fp32; one CTA per user, one thread per column
