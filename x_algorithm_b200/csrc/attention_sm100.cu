@@ -733,8 +733,16 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
   const int n_htiles = a.skip_hist ? 0 : (a.n_hist + QT - 1) / QT;      // 0 or 1
   const int n_ctiles = (a.n_cand + QT - 1) / QT;
   const int nt = n_htiles + n_ctiles;                                   // query tiles per item
-  const int my_items = ((int)blockIdx.x < a.n_items) ? (a.n_items - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  const int G = my_items * nt;                                          // tiles this CTA works through
+  // Work of this CTA: whole items blockIdx.x, blockIdx.x + gridDim.x, ... while every CTA has one (the heads of a request
+  // run side by side: their rows share DRAM pages), then an even share of the remaining items' tiles.
+  const int rounds = a.n_items / (int)gridDim.x;
+  const int rest = (a.n_items - rounds * (int)gridDim.x) * nt;
+  const int r0 = (int)((long long)rest * blockIdx.x / gridDim.x), r1 = (int)((long long)rest * (blockIdx.x + 1) / gridDim.x);
+  const int ri0 = r0 / nt, rt0 = r0 - ri0 * nt;                         // item (of the remaining ones) and tile the share starts at
+  const int my_items = rounds + (r1 > r0 ? (r1 - 1) / nt - ri0 + 1 : 0);
+  const int G = rounds * nt + (r1 - r0);                                // tiles this CTA works through
+  auto item_at = [&](int li) { return li < rounds ? (int)blockIdx.x + li * (int)gridDim.x : rounds * (int)gridDim.x + ri0 + (li - rounds); };
+  auto first_tile = [&](int li) { return li == rounds ? rt0 : 0; };
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -757,7 +765,7 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
     if (lane == 0) {
       int g = 0;
       for (int li = 0; li < my_items; ++li) {
-        const int it = (int)blockIdx.x + li * (int)gridDim.x;
+        const int it = item_at(li);
         const int b = it / a.Hq, h = it % a.Hq, hk = h / (a.Hq / a.Hkv);
         const int qcol = q_column(h, a.q_head_stride, a.q_group, a.q_group_stride);
         const int kb = li & 1;
@@ -765,7 +773,7 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
         mbar_expect_tx(kv_full(kb), 2 * SLAB);
         tma_load_3d(sKV + (2 * kb) * SLAB, &maps.kh, kv_full(kb), hk * a.k_head_stride, 0, b);
         tma_load_3d(sKV + (2 * kb + 1) * SLAB, &maps.vh, kv_full(kb), hk * a.v_head_stride, 0, b);
-        for (int ti = 0; ti < nt; ++ti, ++g) {
+        for (int ti = first_tile(li); ti < nt && g < G; ++ti, ++g) {
           const int st = g % PP_NQ;
           const uint32_t dst = sQ + 3 * st * SLAB;
           mbar_wait(q_free(st), (uint32_t)(((g / PP_NQ) & 1) ^ 1), verr);
@@ -805,7 +813,7 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
       for (int li = 0; li < my_items; ++li) {
         const int kb = li & 1;
         mbar_wait(kv_full(kb), (uint32_t)((li >> 1) & 1), verr);
-        for (int ti = 0; ti < nt; ++ti, ++g) {
+        for (int ti = first_tile(li); ti < nt && g < G; ++ti, ++g) {
           const int st = g % PP_NQ, w = g & 1;
           mbar_wait(q_full(st), (uint32_t)((g / PP_NQ) & 1), verr);
           tc_fence_after();
@@ -826,7 +834,7 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
           }
           umma_commit(s_full(w));
           if (g > 0) issue_pv(g - 1, prev_kb, prev_last);
-          prev_kb = kb; prev_last = (ti == nt - 1);
+          prev_kb = kb; prev_last = (ti == nt - 1 || g == G - 1);
         }
       }
       if (G > 0) issue_pv(G - 1, prev_kb, prev_last);
@@ -834,9 +842,11 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
   } else if (warp == 10) {
     // ---------------- store warp: staged output rows -> global memory, then the stage goes back to the producer --------
     if (lane == 0) {
-      for (int g = 0; g < G; ++g) {
-        const int li = g / nt, ti = g - li * nt, st = g % PP_NQ, w = g & 1;
-        const int it = (int)blockIdx.x + li * (int)gridDim.x;
+      int li = 0, ti = first_tile(0);
+      for (int g = 0; g < G; ++g, ++ti) {
+        if (ti == nt) { ++li; ti = first_tile(li); }
+        const int st = g % PP_NQ, w = g & 1;
+        const int it = item_at(li);
         const int b = it / a.Hq, h = it % a.Hq;
         mbar_wait(o_staged(w), (uint32_t)((g >> 1) & 1), verr);
         if (ti < n_htiles) tma_store_3d(&maps.oh, sQ + 3 * st * SLAB, h * DH, ti * QT, b);
@@ -863,7 +873,7 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
     auto tile_at = [&](int li, int ti) {
       Tile t;
       t.li = li; t.ti = ti;
-      const int it = (int)blockIdx.x + li * (int)gridDim.x;
+      const int it = item_at(li);
       const int b = it / a.Hq;
       t.cand = ti >= n_htiles;
       const int p = (t.cand ? (ti - n_htiles) : ti) * QT + r;                        // position inside the block
@@ -873,9 +883,9 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
       t.hseg = (r < a.n_hist) ? a.seg[a.hist_row0 + (long long)b * a.hist_req_rows + r] : 0;   // history key r of the item
       return t;
     };
-    auto tile_after = [&](const Tile& c) {         // two tiles further on
-      int li = c.li, ti = c.ti + 2;
-      while (ti >= nt) { ti -= nt; ++li; }
+    auto tile_after = [&](int li, int ti, int n) {         // n tiles further on
+      for (; n > 0; --n)
+        if (++ti == nt) { ++li; ti = first_tile(li); }
       return tile_at(li, ti);
     };
 
@@ -883,13 +893,13 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
     bool all_ok = false;
     int mask_li = -1;
     Tile cur, nxt;
-    if (w < G) cur = tile_at(w / nt, w % nt);
+    if (w < G) cur = tile_after(0, first_tile(0), w);
     for (int g = w; g < G; g += 2) {
       const uint32_t ph = (uint32_t)((g >> 1) & 1);
       const int st = g % PP_NQ;
       const uint32_t stage = sQ + 3 * st * SLAB;
       const bool more = g + 2 < G;
-      if (more) nxt = tile_after(cur);
+      if (more) nxt = tile_after(cur.li, cur.ti, 2);
       if (cur.li != mask_li) {
         // validity of the item's history keys (the same for all of its tiles)
         const uint32_t word = __ballot_sync(0xffffffffu, cur.hseg == 1);
@@ -1133,7 +1143,8 @@ phx_status launch_pingpong(const AttnArgs& a, int* err_flag, int num_sms, cudaSt
     }
     pm = it->second;
   }
-  const int grid = p.n_items < num_sms ? p.n_items : num_sms;
+  const long long tiles = (long long)p.n_items * ((p.skip_hist ? 0 : (n_hist + QT - 1) / QT) + (n_cand + QT - 1) / QT);
+  const int grid = (int)(tiles < num_sms ? tiles : num_sms);
   ranker_attention_pingpong_kernel<CAP><<<grid, PP_THREADS, smem, stream>>>(pm, p);
   PHX_CUDA_TRY(cudaGetLastError(), err);
   return PHX_OK;
