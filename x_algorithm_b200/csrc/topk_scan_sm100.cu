@@ -12,9 +12,9 @@
 //               (collect pass) or reduces the 32-row maximum per query (sample pass)
 // An int8 row of 128 columns is the byte image of a bf16 row of 64: tiles, swizzle, descriptors and tensor maps are the
 // same, only the instruction kind and what a consumer makes of an accumulator differ.
-// Measured (256 queries, k = 1000, one 12.5 M-row shard of 128 columns, whole top-k call): int8 rows 3.98 ms on mma.sync ->
-// 1.49 ms here; bf16 rows 1.28 -> 1.17 ms with 16 consumer warps instead of 8; one query over 1 M rows 227 -> 213 us with 64
-// query columns instead of 256.
+// Measured (256 queries, k = 1000, one 12.5 M-row shard of 128 columns, whole top-k call): int8 rows 3.98 ms on mma.sync,
+// 1.49 ms when they moved here, 1.20 ms now; bf16 rows 1.28 ms with 8 consumer warps, 1.17 with 16, 0.96 now; one query over
+// 1 M rows 227 -> 213 us with 64 query columns instead of 256.
 // All mbarrier waits are bounded; on expiry *err_flag is raised and the kernel unwinds.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
@@ -38,11 +38,6 @@ __device__ __forceinline__ uint32_t ord32(float f) {
   const uint32_t u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-__device__ __forceinline__ float unord32(uint32_t o) {
-  const uint32_t u = (o & 0x80000000u) ? (o & 0x7FFFFFFFu) : ~o;
-  return __uint_as_float(u);
-}
-
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -323,15 +318,30 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
           tmem_ld_wait();
           const int u0 = part * CW + c * CH;
           const long long grp = w * 4 + quad;
+          float m[CH];
 #pragma unroll
           for (int k = 0; k < CH; ++k) {
             const float v = I8 ? s8_value(r[k], s_us[u0 + k]) * rs : __uint_as_float(r[k]);
-            const uint32_t key = row_ok ? ord32(round_bf(v)) : 0x007FFFFFu;  // ordered(-inf)
-            uint32_t mx;
-            asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(mx) : "r"(key));
-            const int u = u0 + k;
-            if (lane == 0 && u < a.B) a.gmax[(size_t)u * a.n_groups + grp] = unord32(mx);
+            m[k] = row_ok ? round_bf(v) : -INFINITY;
           }
+          // Maximum over the 32 rows for every column: at each exchange a lane keeps the half of its columns that its lane
+          // bit names and hands over the other half, so lane k ends with column k's and one store writes the group
+          // (a warp-wide reduction and a store of its own per column took 3 times the instructions: 995 -> 964 us for the whole
+          // call on bf16 rows, 1262 -> 1202 on int8).
+          if (CH == 16) {
+#pragma unroll
+            for (int k = 0; k < CH; ++k) m[k] = fmaxf(m[k], __shfl_xor_sync(0xffffffffu, m[k], 16));
+          }
+#pragma unroll
+          for (int o = CH / 2; o >= 1; o >>= 1) {
+            const bool upper = lane & o;
+#pragma unroll
+            for (int k = 0; k < o; ++k) {
+              const float keep = upper ? m[k + o] : m[k], give = upper ? m[k] : m[k + o];
+              m[k] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, give, o));
+            }
+          }
+          if (lane < CH && u0 + lane < a.B) a.gmax[(size_t)(u0 + lane) * a.n_groups + grp] = m[0];
         }
         tc_fence_before();
         mbar_arrive(tempty_bar(acc));
