@@ -1,6 +1,9 @@
 """The GEMM variants a call's size picks - one tile per CTA for few tiles, resident A rows for many tiles with a short K - against
 the single-CTA kernel, which multiplies and rounds in the same order: the same bits, at the edges of the 128-row and
 64 / 128 / 256-column tiles and of the 64-column k-steps, and through the engine for the RoPE, RMSNorm and statistics epilogues."""
+import ctypes
+import ctypes.util
+
 import numpy as np
 import pytest
 
@@ -40,3 +43,42 @@ def test_engine_forward_same_bits(monkeypatch, B, opts):
     want = eng.rank(to_inputs(b)); eng.close()
     np.testing.assert_array_equal(got.log_probs, want.log_probs)
     np.testing.assert_array_equal(got.continuous, want.continuous)
+
+
+@pytest.mark.parametrize("D,hq,hkv,dh,C,mode", [(512, 4, 4, 64, 512, None), (512, 4, 4, 64, 512, "pair"), (512, 4, 4, 64, 512, "cta1"),
+                                                (256, 8, 2, 32, 300, None), (256, 4, 1, 128, 300, None), (256, 2, 2, 128, 300, "pair"),
+                                                (128, 4, 4, 32, 300, "pair"), (128, 1, 1, 128, 300, "cta1")])
+def test_rope_epilogue_rounds_as_stated(monkeypatch, D, hq, hkv, dh, C, mode):
+    """The rotated q and k columns against their definition in 64 bits with the epilogue's roundings: (x1, x2) ->
+    (fma(x1, c, -fl(x2 s)), fma(x1, s, fl(x2 c))), heads of 128 (.., fma(x2, c, fl(x1 s))), then bf16.  Which product is rounded
+    shows in a few columns per million."""
+    S = 128
+    if mode:
+        monkeypatch.setenv("PHX_GEMM", mode)
+    kw = dict(max_batch=1, emb_size=D, num_q_heads=hq, num_kv_heads=hkv, key_size=dh, history_len=S, num_candidates=C, num_layers=1)
+    width = (hq + 2 * hkv) * dh
+    raw = []
+    for rotary in (False, True):
+        ocfg, w, rows_fn, eng = make_pair(rotary=rotary, **kw)
+        eng.rank(to_inputs(po.make_batch(ocfg, 1, seed=3)))
+        raw.append(po.bf16_from_bits(eng.debug_read("qkv", (S + C, width), np.uint16)))   # one request: rows in order in any layout
+        base = float(ocfg.rope_base)
+        eng.close()
+    libm = ctypes.CDLL(ctypes.util.find_library("m"))
+    for f in (libm.cosf, libm.sinf):
+        f.restype, f.argtypes = ctypes.c_float, [ctypes.c_float]
+    libm.powf.restype, libm.powf.argtypes = ctypes.c_float, [ctypes.c_float, ctypes.c_float]
+    f32, half = np.float32, dh // 2
+    inv = [f32(1) / f32(libm.powf(base, float(f32(2 * j) / f32(dh)))) for j in range(half)]
+    pos = np.minimum(np.arange(S + C), S)
+    tab = [np.array([[f(float(f32(p) * inv[j])) for j in range(half)] for p in range(S + 1)], f32)[pos].astype(np.float64)[:, None, None, :]
+           for f in (libm.cosf, libm.sinf)]
+    g = hq // hkv
+    x, got = (r.reshape(S + C, hkv, g + 2, dh) for r in raw)
+    np.testing.assert_array_equal(x[:, :, g + 1], got[:, :, g + 1])                       # v parts pass through
+    x1, x2 = (x[:, :, :g + 1, h * half:(h + 1) * half].astype(np.float64) for h in (0, 1))
+    fl = lambda v: v.astype(f32).astype(np.float64)
+    c, s = tab
+    np.testing.assert_array_equal(got[:, :, :g + 1, :half], po.bf16_round((x1 * c - fl(x2 * s)).astype(f32)))
+    hi = fl(x1 * s) + x2 * c if dh == 128 else x1 * s + fl(x2 * c)
+    np.testing.assert_array_equal(got[:, :, :g + 1, half:], po.bf16_round(hi.astype(f32)))

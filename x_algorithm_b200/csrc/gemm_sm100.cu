@@ -19,6 +19,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 
@@ -99,11 +101,15 @@ __device__ __forceinline__ uint32_t gelu_bf2(uint32_t b) {
   const float2 g = __ffma2_rn(h, t, h);
   return pack_bf2(g.x, g.y);
 }
-// one RoPE pair of columns against its partner pair: (lo, hi) -> (lo c - hi s, hi c + lo s)
+// one RoPE pair of columns against its partner pair: (lo, hi) -> (lo c - hi s, hi c + lo s).  Which of the two products of a sum is
+// rounded before the other goes into the fma shows in a few results per million: hi s and hi c, and with heads of 128
+// lo s instead of hi c.
+template <bool D128>
 __device__ __forceinline__ void rope_bf2(uint32_t& lo, uint32_t& hi, float c0, float c1, float s0, float s1) {
   const float2 x1 = bf2_to_f2(lo), x2 = bf2_to_f2(hi), c = make_float2(c0, c1), sn = make_float2(s0, s1);
-  const float2 a = __fmul2_rn(x2, sn), b = __fmul2_rn(x1, sn);
-  const float2 l = __ffma2_rn(x1, c, make_float2(-a.x, -a.y)), h = __ffma2_rn(x2, c, b);
+  const float2 a = __fmul2_rn(x2, sn);
+  const float2 l = __ffma2_rn(x1, c, make_float2(-a.x, -a.y));
+  const float2 h = D128 ? __ffma2_rn(x2, c, __fmul2_rn(x1, sn)) : __ffma2_rn(x1, sn, __fmul2_rn(x2, c));
   lo = pack_bf2(l.x, l.y); hi = pack_bf2(h.x, h.y);
 }
 // position of a token row: the row's slot in its request, at most pos_cap (GemmRope); token rows fit 31 bits
@@ -418,8 +424,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (part_rotated(p)) {   // v parts pass through
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                rope_bf2(lo[2 * j], hi[2 * j], cs[j].x, cs[j].y, sn[j].x, sn[j].y);
-                rope_bf2(lo[2 * j + 1], hi[2 * j + 1], cs[j].z, cs[j].w, sn[j].z, sn[j].w);
+                rope_bf2<D128>(lo[2 * j], hi[2 * j], cs[j].x, cs[j].y, sn[j].x, sn[j].y);
+                rope_bf2<D128>(lo[2 * j + 1], hi[2 * j + 1], cs[j].z, cs[j].w, sn[j].z, sn[j].w);
               }
             }
             if (p + 1 < (D128 ? 4 : 2) && part_rotated(p + 1)) load_angles(p + 1);
@@ -729,11 +735,14 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         if (EPI == EPI_GELU) o[k] = gelu_bf2(o[k]);
       }
       if (EPI == EPI_ROPE && rotate) {
+        auto rotate_all = [&](auto wide) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          rope_bf2(o[2 * j], o[8 + 2 * j], cs[j].x, cs[j].y, sn[j].x, sn[j].y);
-          rope_bf2(o[2 * j + 1], o[8 + 2 * j + 1], cs[j].z, cs[j].w, sn[j].z, sn[j].w);
-        }
+          for (int j = 0; j < 4; ++j) {
+            rope_bf2<wide.value>(o[2 * j], o[8 + 2 * j], cs[j].x, cs[j].y, sn[j].x, sn[j].y);
+            rope_bf2<wide.value>(o[2 * j + 1], o[8 + 2 * j + 1], cs[j].z, cs[j].w, sn[j].z, sn[j].w);
+          }
+        };
+        if (BN == 128 && d128) rotate_all(std::true_type()); else rotate_all(std::false_type());
       }
       float2 v[RES ? 16 : 1];
       if (RES) {
