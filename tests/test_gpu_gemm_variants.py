@@ -28,6 +28,21 @@ def test_variants_give_the_same_bits(M, N, K, epi):
     assert torch.equal(c, one)
 
 
+@pytest.mark.parametrize("rows", [8192, 65536])           # one tile per CTA; CTA pairs
+def test_gelu_of_every_value(rows):
+    """Every finite bf16 value through the GELU epilogue of each kernel: the value of the scalar formula (the SIMT kernel's), which
+    is written in another order; only a zero's sign may differ."""
+    import torch
+    from x_algorithm_b200.engine import gemm
+    v = torch.arange(65536, dtype=torch.int32, device="cuda").to(torch.int16).view(torch.bfloat16)
+    v = torch.where(torch.isfinite(v.float()), v, torch.ones_like(v)).reshape(8192, 8).repeat(rows // 8192, 1)
+    eye = torch.eye(8, dtype=torch.bfloat16, device="cuda")
+    want, _ = gemm(v, eye, None, 2, 1)
+    for impl in (0, 2):
+        got, _ = gemm(v, eye, None, 2, impl)
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("B,opts", [(1, dict(history_len=31, num_candidates=70)), (5, dict(history_len=32, num_candidates=8)),
                                     (3, dict(emb_size=256, num_q_heads=4, num_kv_heads=2, key_size=64, history_len=40, num_candidates=150)),
                                     (2, dict(emb_size=256, num_q_heads=2, num_kv_heads=1, key_size=128, history_len=40, num_candidates=90)),
