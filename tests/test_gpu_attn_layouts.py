@@ -33,3 +33,22 @@ def test_grouped_heads_and_split_rows(monkeypatch, S, C, dh, hq, hkv, tail):
     lp, cont, logits = po.rank_forward(ocfg, w, rows_fn, bb)
     ok = bb.cand_post_ids != 0
     assert_heads_close(got.log_probs[few][ok], got.continuous[few][ok], logits[ok], cont[ok], 2e-2, str(kw))
+
+
+@pytest.mark.parametrize("dh,S,cap", [(128, 300, -1.0), (64, 600, -1.0), (128, 300, 30.0)])
+def test_row_does_not_depend_on_its_neighbours(dh, S, cap):
+    """Streaming kernel: other queries beside a candidate (rows of the same warp, some far larger) leave its output bits alone."""
+    import torch
+    from x_algorithm_b200.engine import dispatch_counts, ranker_attention
+    g = torch.Generator(device="cuda").manual_seed(dh + S)
+    B, C, H = 2, 32, 4
+    q, k, v = (torch.randn(B, S + C, H, dh, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    seg = torch.ones((B, S + C), dtype=torch.int32, device="cuda")
+    seg[:, S:] = -1
+    before = dispatch_counts()["attn.tcgen05"]
+    a, _ = ranker_attention(q, k, v, seg, S, 0.2, cap, 1 if cap > 0 else 0)
+    q2 = q.clone()
+    q2[:, S + 1::2] *= 6.0
+    b, _ = ranker_attention(q2, k, v, seg, S, 0.2, cap, 1 if cap > 0 else 0)
+    assert dispatch_counts()["attn.tcgen05"] == before + 2
+    assert torch.equal(a[:, S::2], b[:, S::2]) and not torch.equal(a, b)

@@ -288,9 +288,10 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
       }
       // The reference point of the exponentials only has to bound them, not equal the running maximum: it moves
       // when the maximum has grown by more than 2^8 since it was set (P stays below 256, exact in bf16 up to the same
-      // power of two), which spares the rescaling of O in tensor memory for almost every block.
+      // power of two), which spares the rescaling of O in tensor memory for almost every block.  Each row moves its own:
+      // a row's bits depend on its query and the keys alone, not on the rows that share its warp.
       const float m_true = fmaxf(m, bm * csc);
-      const bool move = __any_sync(0xffffffffu, m_true > m + 8.0f || (m == -INFINITY && m_true != -INFINITY));
+      const bool move = m_true > m + 8.0f || (m == -INFINITY && m_true != -INFINITY);
       const float m_new = move ? m_true : m;
       const float mns = (m_new == -INFINITY) ? 0.f : m_new;   // finite stand-in while nothing is allowed yet
       const float alpha = ex2f(m - mns);                      // -inf - finite -> 0; unmoved: 1
