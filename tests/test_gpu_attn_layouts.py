@@ -52,3 +52,15 @@ def test_row_does_not_depend_on_its_neighbours(dh, S, cap):
     b, _ = ranker_attention(q2, k, v, seg, S, 0.2, cap, 1 if cap > 0 else 0)
     assert dispatch_counts()["attn.tcgen05"] == before + 2
     assert torch.equal(a[:, S::2], b[:, S::2]) and not torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dh,B", [(32, 2), (64, 2), (64, 40), (128, 2)])
+def test_negative_history_length_is_no_history(dh, B):
+    """A candidate without history keys attends to itself alone: its own value row, whatever the sign of the length given."""
+    import torch
+    from x_algorithm_b200.engine import ranker_attention
+    g = torch.Generator(device="cuda").manual_seed(dh + B)
+    q, k, v = (torch.randn(B, 131, 4, dh, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    seg = torch.full((B, 131), -1, dtype=torch.int32, device="cuda")
+    for hist_len in (0, -1, -200, -(1 << 31)):
+        assert torch.equal(ranker_attention(q, k, v, seg, hist_len, 0.2)[0], v)

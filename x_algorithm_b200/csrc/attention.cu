@@ -664,7 +664,9 @@ phx_status launch_strip(const AttnArgs& a, cudaStream_t stream, std::string& err
 
 }  // namespace
 
-phx_status ranker_attention_launch(const AttnArgs& a, cudaStream_t stream, std::string& err) {
+phx_status ranker_attention_launch(const AttnArgs& args, cudaStream_t stream, std::string& err) {
+  AttnArgs a = args;
+  if (a.hist_len < 0) a.hist_len = 0;   // no history; the kernels size their candidate blocks as T - hist_len
   if (a.Hq % a.Hkv != 0) { err = "attention: Hq must be a multiple of Hkv"; return PHX_E_ARG; }
   if (a.B == 0 || a.T == 0) return PHX_OK;
   if (a.B > 65535 || a.Hq > 65535) { err = "attention: batch or head count too large for one launch"; return PHX_E_CAPACITY; }
