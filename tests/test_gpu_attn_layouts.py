@@ -64,3 +64,19 @@ def test_negative_history_length_is_no_history(dh, B):
     seg = torch.full((B, 131), -1, dtype=torch.int32, device="cuda")
     for hist_len in (0, -1, -200, -(1 << 31)):
         assert torch.equal(ranker_attention(q, k, v, seg, hist_len, 0.2)[0], v)
+
+
+@pytest.mark.parametrize("S,C,dh,hq,hkv,B", [(128, 512, 64, 8, 8, 4), (128, 500, 64, 8, 4, 4), (128, 512, 64, 8, 8, 5), (200, 40, 64, 4, 2, 3),
+                                             (300, 65, 64, 4, 4, 2), (127, 40, 128, 4, 1, 3), (330, 130, 128, 2, 2, 3), (40, 24, 128, 2, 1, 2)])
+def test_candidate_only_last_layer_same_bits(monkeypatch, S, C, dh, hq, hkv, B):
+    """The last layer over its candidate rows only gives the candidate outputs of the last layer over every row, bit for bit:
+    long histories, heads of 128, grouped heads, and a batch whose tiles just fill the SMs with the history tile counted."""
+    kw = dict(max_batch=B, emb_size=256, num_q_heads=hq, num_kv_heads=hkv, key_size=dh, history_len=S, num_candidates=C, num_layers=2)
+    ocfg, w, rows_fn, eng = make_pair(**kw)
+    b = po.make_batch(ocfg, B, seed=S + B, ragged=True)
+    got = eng.rank(to_inputs(b)); eng.close()
+    monkeypatch.setenv("PHX_LAST_LAYER", "full")
+    _, _, _, eng = make_pair(**kw)
+    want = eng.rank(to_inputs(b)); eng.close()
+    np.testing.assert_array_equal(got.log_probs, want.log_probs)
+    np.testing.assert_array_equal(got.continuous, want.continuous)

@@ -686,7 +686,8 @@ phx_status ranker_attention_launch(const AttnArgs& args, cudaStream_t stream, st
     // Head dim 64 with a history of at most 128 keys: the persistent tcgen05 kernel with the history resident and two
     // softmax warpgroups, once there is an item (batch, head) for every SM, or long candidate lists with a tile for every SM
     // (8 requests of 640 rows: 17.5 against 20.1 us for the streaming mma.sync kernel, 16: 19.7 against 27.7; with one or two
-    // tiles per item the two are level at 148 items and below).  Measured on B200 at the ranking
+    // tiles per item the two are level at 148 items and below).  A candidate-only layer counts its history tile too: it takes
+    // the kernel the same layer over every row takes, and so has the same bits.  Measured on B200 at the ranking
     // benchmark's shape (B=256, S=128, C=512, 8 heads): 0.140 ms per layer against 0.206 ms for the mma.sync
     // resident-history kernel below (1.2-1.4 against 2.0 ms per step inside the forward), and 0.051 against 0.067 ms at
     // B=64; every byte it touches moves by bulk copies.  PHX_ATTN=strip keeps the mma.sync kernel, PHX_ATTN=pingpong
@@ -694,7 +695,7 @@ phx_status ranker_attention_launch(const AttnArgs& args, cudaStream_t stream, st
     const char* force = getenv("PHX_ATTN");
     const bool forced = force && strcmp(force, "pingpong") == 0;
     const int nh = a.hist_len < a.T ? a.hist_len : a.T;
-    const long long items = (long long)a.B * a.Hq, nt = (a.q_start > 0 ? 0 : (nh + 127) / 128) + (a.T - nh + 127) / 128;
+    const long long items = (long long)a.B * a.Hq, nt = (nh + 127) / 128 + (a.T - nh + 127) / 128;
     const bool fills = !force && (items >= 148 || (nt >= 4 && items * nt >= 148));
     if ((forced || fills) && a.err_flag && ranker_attention_pingpong_supported(a))
       return ranker_attention_pingpong_launch(a, a.err_flag, stream, err);
