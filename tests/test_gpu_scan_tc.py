@@ -73,3 +73,28 @@ def test_bf16_scan_against_64_bit_scores(dim, N, B, k):
         rest = np.delete(full[b], got_i[b])
         if rest.size:
             assert rest.max() <= got_s[b][-1] + step * abs(got_s[b][-1]) + 1e-6
+
+
+def test_masked_rows_stand_in_front_of_minus_infinity():
+    """Fewer eligible rows than k: masked rows fill the list at the bf16 minimum, and an eligible row whose score is -inf comes
+    behind them, as in a top-k over all scores."""
+    import torch
+    from x_algorithm_b200.retrieval import CorpusShard, Retriever
+    N, dim, k = 3000, 64, 9
+    rows = np.random.default_rng(3).standard_normal((N, dim)).astype(np.float32)
+    rows[1234, 0] = -np.inf
+    elig = np.zeros(N, bool)
+    elig[[7, 1234, 2000, 2999]] = True
+    sh = CorpusShard(N, dim, max_queries=2, max_k=k)
+    sh.upload(0, po.bf16_bits(rows))
+    sh.set_mask(elig)
+    users = np.abs(np.random.default_rng(4).standard_normal((2, dim))).astype(np.float32)
+    s, i = Retriever([sh]).retrieve(torch.from_numpy(users).cuda(), k)
+    s, i = s.cpu().numpy(), i.cpu().numpy()
+    sh.close()
+    scores = po.bf16_round(users).astype(np.float64) @ po.bf16_round(rows[[7, 2000, 2999]]).astype(np.float64).T
+    lowest = np.frombuffer(np.uint32(0xFF7F0000).tobytes(), np.float32)[0]
+    for b in range(2):
+        order = np.argsort(-scores[b])
+        assert list(i[b]) == [[7, 2000, 2999][o] for o in order] + [0, 1, 2, 3, 4] + [1234]
+        assert np.all(s[b, 3:8] == lowest) and s[b, 8] == -np.inf

@@ -18,6 +18,7 @@ class CorpusShard:
                  device: int = 0):
         self.rows, self.dim, self.row_offset, self.device = rows, dim, row_offset, device
         self.max_queries, self.max_k = max_queries, max_k
+        self.eligible_rows = rows
         self._h = C.c_void_p()
         st = lib.phx_corpus_create(device, rows, dim, row_offset, max_queries, max_k, C.byref(self._h))
         if st != 0:
@@ -74,11 +75,14 @@ class CorpusShard:
         (recsys_two_tower_model.py:2486-2493)."""
         if eligible is None:
             self._check(lib.phx_corpus_set_mask(self._h, None))
+            self.eligible_rows = self.rows
             return
-        bits = np.packbits(np.asarray(eligible, dtype=bool), bitorder="little")
+        eligible = np.asarray(eligible, dtype=bool)
+        bits = np.packbits(eligible, bitorder="little")
         words = np.zeros((len(eligible) + 31) // 32 * 4, np.uint8)
         words[:bits.size] = bits
         self._check(lib.phx_corpus_set_mask(self._h, words.view(np.uint32).ctypes.data))
+        self.eligible_rows = int(np.count_nonzero(eligible[:self.rows]))
 
     def topk_window_device(self, users, B: int, k: int, row_begin: int, row_end: int, scores, ids):
         """Top-k over shard-local rows [row_begin, row_end) only: one retrieval dataset of the reference's post table
@@ -185,8 +189,9 @@ class Retriever:
         out_i = torch.empty((B, k), dtype=torch.int64, device=dev)
         for sh in self.shards:
             sh.set_stream(stream)
-        if P == 1 and not multi:
-            # one list is its own merge: the shard writes scores and rows itself, an exact re-run rewrites them in place
+        if P == 1 and not multi and k <= self.shards[0].eligible_rows:
+            # one list is its own merge: the shard writes scores and rows itself, an exact re-run rewrites them in place.
+            # (A list completed with masked rows is merged: they stand at the bf16 minimum, in front of rows that score -inf.)
             try:
                 self.shards[0].topk_device(users, B, k, out_s, out_i)
                 if check:
