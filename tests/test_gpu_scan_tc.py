@@ -75,6 +75,28 @@ def test_bf16_scan_against_64_bit_scores(dim, N, B, k):
             assert rest.max() <= got_s[b][-1] + step * abs(got_s[b][-1]) + 1e-6
 
 
+@pytest.mark.parametrize("B", [16, 64, 200])
+def test_int8_scan_of_huge_queries(B):
+    """Query scales near the end of fp32's range (the filter's offset times the scale overflows): the list is complete without
+    an exact re-run, and equals the oracle's."""
+    from x_algorithm_b200.retrieval import CorpusShard
+    N, dim, k = 40001, 128, 30
+    r = np.random.default_rng(B)
+    q8 = r.integers(-127, 128, size=(N, dim), dtype=np.int8)
+    scales = (r.random(N, dtype=np.float32) * np.float32(0.01) + np.float32(1e-4)).astype(np.float32)
+    users = (_users(B, dim, 7) * np.float32(4e34)).astype(np.float32)
+    assert (np.abs(users).max(1) / 127 * np.float64(12582912.0)).min() > 3.5e38
+    sh = CorpusShard(N, dim, max_queries=B, max_k=k)
+    sh.upload_int8(0, q8, scales)
+    sh.set_int8(True)
+    got_s, got_i = _topk(sh, users, k)
+    assert sh.exact_runs() == 0
+    want_s, want_i = po.top_k(po.int8_corpus_scores(users, q8, scales), k)
+    sh.close()
+    np.testing.assert_array_equal(got_i, want_i)
+    np.testing.assert_array_equal(got_s, want_s)
+
+
 def test_masked_rows_stand_in_front_of_minus_infinity():
     """Fewer eligible rows than k: masked rows fill the list at the bf16 minimum, and an eligible row whose score is -inf comes
     behind them, as in a top-k over all scores."""

@@ -165,7 +165,8 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
         t = fminf(t, s_thr[threadIdx.x * CH + k]);
         if (I8) m = fmaxf(m, s_us[threadIdx.x * CH + k]);
       }
-      s_thr_min[threadIdx.x] = t; s_us_max[threadIdx.x] = m;
+      // a scale whose offset product overflows leaves no bound (-inf, NaN): such a group is not filtered
+      s_thr_min[threadIdx.x] = t; s_us_max[threadIdx.x] = (m * S8_OFFSET < INFINITY) ? m : INFINITY;
     }
     if (I8 && threadIdx.x < NQ / 2) {
       const float x = s_us[2 * threadIdx.x], y = s_us[2 * threadIdx.x + 1];
@@ -264,8 +265,10 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
           if (I8) {
             // float(dot) * query scale without a conversion per element (those run at a fraction of the fp32 rate):
             // 1.5 * 2^23 + dot is the integer sum of the bit patterns, and the fma takes the offset's product off
-            // again.  That product is rounded: the value is off by at most 0.75 of the query scale, which the margin
-            // of one scale covers.  A row scale that is not positive turns the order round: no filter then.
+            // again.  Two roundings: the product's, at most 0.75 of the query scale, and the fma's, at most 0.25 while
+            // |dot| < 2^22 (it is at most 128 * 127 * 256, which leaves 0.998 in all).  With the margin of one scale the bound
+            // is not below the unrounded dot * scale, so the roundings of the tested value, which keep order, cannot put it
+            // above the bound's.  A row scale that is not positive turns the order round: no filter then.
             float mx = -INFINITY;
 #pragma unroll
             for (int k = 0; k < CH; k += 2) {
