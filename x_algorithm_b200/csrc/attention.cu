@@ -339,11 +339,8 @@ template <int DH, bool CAP>
 phx_status launch_dh(const AttnArgs& a, cudaStream_t stream, std::string& err) {
   constexpr int LD = DH + 8;
   const size_t smem = (size_t)(3 * QROWS + 4 * KB) * LD * 2 + (2 * KB + 4) * sizeof(int);
-  static bool attr_set = false;
-  if (!attr_set) {
-    PHX_CUDA_TRY(cudaFuncSetAttribute(ranker_attention_kernel<DH, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), err);
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  PHX_CUDA_TRY(limit.raise(ranker_attention_kernel<DH, CAP>, (int)smem), err);
   dim3 grid((a.T + QROWS - 1) / QROWS, a.Hq, a.B);
   PHX_CUDA_TRY(launch_overlapped(ranker_attention_kernel<DH, CAP>, grid, ATT_THREADS, smem, stream, a), err);
   return PHX_OK;
@@ -652,11 +649,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) ranker_attention_strip_kernel(
 
 template <bool CAP>
 phx_status launch_strip(const AttnArgs& a, cudaStream_t stream, std::string& err) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    PHX_CUDA_TRY(cudaFuncSetAttribute(ranker_attention_strip_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, STRIP_SMEM), err);
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  PHX_CUDA_TRY(limit.raise(ranker_attention_strip_kernel<CAP>, STRIP_SMEM), err);
   dim3 grid(a.Hq, a.B);
   PHX_CUDA_TRY(launch_overlapped(ranker_attention_strip_kernel<CAP>, grid, ATT_THREADS, STRIP_SMEM, stream, a), err);
   return PHX_OK;

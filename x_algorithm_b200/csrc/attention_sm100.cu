@@ -1084,11 +1084,8 @@ phx_status cached_map3d(CUtensorMap* out, const bf16* ptr, long long cols, long 
 template <bool CAP>
 phx_status launch_pingpong(const AttnArgs& a, int* err_flag, int num_sms, cudaStream_t stream, std::string& err) {
   const size_t smem = (size_t)(4 + 3 * PP_NQ) * SLAB + 64 + 192 + 1024;
-  static bool attr_set = false;
-  if (!attr_set) {
-    PHX_CUDA_TRY(cudaFuncSetAttribute(ranker_attention_pingpong_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), err);
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  PHX_CUDA_TRY(limit.raise(ranker_attention_pingpong_kernel<CAP>, (int)smem), err);
   const int n_hist = a.hist_len < a.T ? a.hist_len : a.T;
   const int n_cand = a.T - n_hist;
   PingArgs p;
@@ -1157,11 +1154,8 @@ phx_status launch_tc(const AttnArgs& a, int* err_flag, cudaStream_t stream, std:
   constexpr int DCH = DH / 64;
   constexpr int NSB = (KBLK <= 64) ? 2 : 1;   // K buffers, as in the kernel
   const size_t smem = (size_t)DCH * SLAB + (NSB + 2) * (size_t)DCH * KBLK * 128 + TC_MAX_BLOCKS * 16 + 128 + 1024;
-  static bool attr_set = false;
-  if (!attr_set) {
-    PHX_CUDA_TRY(cudaFuncSetAttribute(ranker_attention_tc_kernel<DH, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), err);
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  PHX_CUDA_TRY(limit.raise(ranker_attention_tc_kernel<DH, CAP>, (int)smem), err);
   AttnTcArgs t;
   t.q = a.q; t.k = a.k; t.v = a.v; t.out = a.out;
   t.q_tok_stride = a.q_tok_stride; t.k_tok_stride = a.k_tok_stride; t.v_tok_stride = a.v_tok_stride;
@@ -1200,11 +1194,8 @@ phx_status launch_tc(const AttnArgs& a, int* err_flag, cudaStream_t stream, std:
 
 phx_status launch_resident(const AttnArgs& a, int* err_flag, cudaStream_t stream, std::string& err) {
   const size_t smem = 6 * (size_t)SLAB + 64 + 128 + 1024;
-  static bool attr_set = false;
-  if (!attr_set) {
-    PHX_CUDA_TRY(cudaFuncSetAttribute(ranker_attention_resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), err);
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  PHX_CUDA_TRY(limit.raise(ranker_attention_resident_kernel, (int)smem), err);
   CUtensorMap mq, mk, mv, mo;
   phx_status s;
   if ((s = cached_map3d(&mq, a.q, (long long)(a.Hq - 1) * a.q_head_stride + 64, a.T, a.T, a.B, a.q_tok_stride, QT, err))) return s;
@@ -1237,13 +1228,10 @@ bool ranker_attention_pingpong_supported(const AttnArgs& a) {
 }
 
 phx_status ranker_attention_pingpong_launch(const AttnArgs& a, int* err_flag, cudaStream_t stream, std::string& err) {
-  static int num_sms = 0;
-  if (!num_sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-    if (num_sms <= 0) num_sms = 148;
-  }
+  int num_sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+  if (num_sms <= 0) num_sms = 148;
   dispatch_note(DK_ATTN_PINGPONG);
   const bool cap = a.cap_method != 0 && a.cap > 0.f;
   return cap ? launch_pingpong<true>(a, err_flag, num_sms, stream, err) : launch_pingpong<false>(a, err_flag, num_sms, stream, err);

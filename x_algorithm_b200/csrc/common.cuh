@@ -10,6 +10,7 @@
 #include <string>
 
 #include "../../include/phoenix_b200.h"
+#include "launch_attr.cuh"
 
 namespace phx {
 

@@ -273,12 +273,9 @@ extern "C" phx_status phx_dpp_rescore_device(int32_t device, const phx_dpp_confi
   if (cudaSetDevice(device) != cudaSuccess) { set_global_error("phx_dpp_rescore_device: cudaSetDevice failed"); return PHX_E_CUDA; }
   constexpr int N1 = PHX_DPP_MAX_POOL + 1;
   const size_t smem = (size_t)(2 * N1 * N1 + N1 + 128) * sizeof(double) + (size_t)(3 * N1 + 128) * sizeof(int);
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(dpp_rescore_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-      set_global_error("phx_dpp_rescore_device: shared memory attribute"); return PHX_E_CUDA;
-    }
-    attr_set = true;
+  static SmemLimit limit;
+  if (limit.raise(dpp_rescore_kernel, (int)smem) != cudaSuccess) {
+    set_global_error("phx_dpp_rescore_device: shared memory attribute"); return PHX_E_CUDA;
   }
   DppKernelArgs a;
   a.cfg = *cfg; a.in = *in; a.out_index = out_index; a.out_score = out_score; a.out_count = out_count;

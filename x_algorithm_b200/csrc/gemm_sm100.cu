@@ -506,8 +506,9 @@ phx_status launch_t(const GemmPlan& p, const GemmRope& rope, const GemmNorm& nor
   constexpr int NG = (PAIR && EPI != EPI_RESIDUAL && EPI != EPI_ROPE128) ? 4 : 2;
   using cfg = Cfg<BN, PAIR, NG>;
   auto kern = gemm_tcgen05_kernel<BN, EPI, PAIR, NG>;
-  static bool attr_set = false;
-  static int max_pairs = 0;
+  static OncePerDevice once;
+  static std::atomic<int> pairs_of[LAUNCH_MAX_DEVICES];
+  int max_pairs = 0;
   cudaLaunchConfig_t lc;
   memset(&lc, 0, sizeof(lc));
   cudaLaunchAttribute attr[2];
@@ -529,20 +530,24 @@ phx_status launch_t(const GemmPlan& p, const GemmRope& rope, const GemmNorm& nor
     attr[lc.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     lc.numAttrs++;
   }
-  if (!attr_set) {
-    PHX_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg::SMEM_BYTES), err);
-    if (PAIR) {   // how many CTA pairs the device can hold at once (pairs need two SMs of one cluster-capable group)
+  int dev = 0;
+  PHX_CUDA_TRY(cudaGetDevice(&dev), err);
+  PHX_CUDA_TRY(once.run([&](int d) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg::SMEM_BYTES);
+    if (PAIR && e == cudaSuccess) {   // how many CTA pairs the device can hold at once (pairs need two SMs of one cluster-capable group)
       lc.gridDim = dim3(2 * (num_sms / 2));
       int n = 0;
       const int all_attrs = lc.numAttrs;
       lc.numAttrs = attrs_for_query;   // the occupancy query takes the cluster shape only
-      PHX_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, kern, &lc), err);
+      e = cudaOccupancyMaxActiveClusters(&n, kern, &lc);
       lc.numAttrs = all_attrs;
       max_pairs = n < num_sms / 2 ? n : num_sms / 2;
-      if (max_pairs <= 0) { err = "gemm: the device cannot hold a CTA pair of this kernel"; return PHX_E_CUDA; }
+      if (d < LAUNCH_MAX_DEVICES) pairs_of[d].store(max_pairs, std::memory_order_relaxed);
     }
-    attr_set = true;
-  }
+    return e;
+  }), err);
+  if (PAIR && max_pairs == 0 && dev < LAUNCH_MAX_DEVICES) max_pairs = pairs_of[dev].load(std::memory_order_relaxed);
+  if (PAIR && max_pairs <= 0) { err = "gemm: the device cannot hold a CTA pair of this kernel"; return PHX_E_CUDA; }
   constexpr int TILE_M = PAIR ? 2 * BM : BM;
   const long long tiles = ((M + TILE_M - 1) / TILE_M) * ((p.N + BN - 1) / BN);
   const int slots = PAIR ? max_pairs : num_sms;
@@ -804,11 +809,8 @@ phx_status launch_small_t(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C
                           const GemmNorm& norm, int64_t M, int* err_flag, cudaStream_t stream, std::string& err) {
   using cfg = SmallCfg<BN>;
   auto kern = gemm_small_kernel<BN, EPI>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    PHX_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cfg::SMEM_BYTES), err);
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  PHX_CUDA_TRY(limit.raise(kern, cfg::SMEM_BYTES), err);
   cudaLaunchConfig_t lc;
   memset(&lc, 0, sizeof(lc));
   cudaLaunchAttribute attr[1];

@@ -258,11 +258,8 @@ phx_status launch_heads_wps(const HeadsArgs& a, long long strips, cudaStream_t s
   const size_t smem = (size_t)NT * 8 * (a.D + HM_WPAD) * sizeof(bf16) + (size_t)a.D * sizeof(float) +
                       (size_t)16 * NT * 8 * (WARPS * sizeof(float) + (WPS == 1 ? HM_WARPS : 1) * sizeof(double));
   if (smem > 200 * 1024) { err = "heads: head matrix does not fit shared memory"; return PHX_E_CAPACITY; }
-  static bool attr_set = false;
-  if (!attr_set) {
-    PHX_CUDA_TRY(cudaFuncSetAttribute(heads_mma_kernel<NT, WPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), err);
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  PHX_CUDA_TRY(limit.raise(heads_mma_kernel<NT, WPS>, 200 * 1024), err);
   long long blocks = WPS == 1 ? (strips + HM_WARPS - 1) / HM_WARPS : strips;
   if (blocks > 148 * 3) blocks = 148 * 3;
   cudaLaunchConfig_t lc;
@@ -350,11 +347,8 @@ phx_status heads_launch(const HeadsArgs& a, cudaStream_t stream, std::string& er
     return launch_heads_mma<4>(a, rows, stream, err);
   }
   const size_t smem = (size_t)NO * a.D * sizeof(bf16);
-  static bool attr_set = false;
-  if (!attr_set && smem > 48 * 1024) {
-    PHX_CUDA_TRY(cudaFuncSetAttribute(heads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), err);
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  if (smem > 48 * 1024) PHX_CUDA_TRY(limit.raise(heads_kernel, 200 * 1024), err);
   if (smem > 200 * 1024) { err = "heads: head matrix does not fit shared memory"; return PHX_E_CAPACITY; }
   long long blocks = (rows + 7) / 8;
   if (blocks > 148 * 4) blocks = 148 * 4;
