@@ -80,3 +80,30 @@ def test_candidate_only_last_layer_same_bits(monkeypatch, S, C, dh, hq, hkv, B):
     want = eng.rank(to_inputs(b)); eng.close()
     np.testing.assert_array_equal(got.log_probs, want.log_probs)
     np.testing.assert_array_equal(got.continuous, want.continuous)
+
+
+@pytest.mark.parametrize("S,C,dh,hq,hkv,kw", [(160, 30, 64, 4, 4, {}), (40, 24, 128, 4, 1, {}), (130, 9, 64, 4, 2, dict(qk_norm=True)),
+                                              (20, 70, 128, 2, 2, dict(primer_norm=True))])
+def test_debug_taps_hold_every_row_in_request_order(monkeypatch, S, C, dh, hq, hkv, kw):
+    """phx_debug_read of the trunk is [B, T] with every row taken through every layer, although the engine keeps history and
+    candidate rows apart and skips the last layer's history rows: the bits of an engine that does neither."""
+    kw = dict(max_batch=3, emb_size=256, num_q_heads=hq, num_kv_heads=hkv, key_size=dh, history_len=S, num_candidates=C, num_layers=2, **kw)
+    taps = (("seg", 1, np.int32), ("qkv", (hq + 2 * hkv) * dh, np.uint16), ("attn", hq * dh, np.uint16), ("hidden", 256, np.uint16))
+
+    def read(eng, b):
+        first = eng.rank(to_inputs(b))
+        out = [eng.debug_read(n, (3, S + C, width), dt) for n, width, dt in taps + taps[-1:]]
+        for _ in range(3):                                # replayed launches
+            again = eng.rank(to_inputs(b))
+        out += [eng.debug_read("hidden", (3, S + C, 256), np.uint16), eng.debug_read("hidden", (S + C + 1, 256), np.uint16)]
+        np.testing.assert_array_equal(first.log_probs, again.log_probs)
+        eng.close()
+        return out
+
+    ocfg, w, rows_fn, eng = make_pair(**kw)
+    b = po.make_batch(ocfg, 3, seed=S, ragged=True)
+    got = read(eng, b)
+    monkeypatch.setenv("PHX_LAST_LAYER", "full")
+    _, _, _, eng = make_pair(**kw)
+    for a, c in zip(got, read(eng, b)):
+        np.testing.assert_array_equal(a, c)

@@ -93,6 +93,11 @@ struct phx_engine {
   // candidate block only
   bool split = false;
   int n_tail = 0;
+  // phx_debug_read of a plain model with heads of 128 or a history past one key block: every row of the trunk in [B, T] order,
+  // although the engine keeps split rows and its last layer leaves the history rows alone
+  bool taps_plain = false;
+  bool taps_of_rank = false;       // the last forward ranked candidates (the tower's rows are plain as they are)
+  bool history_done = false;       // its history rows have been taken through the last layer
   // packed rows (cfg.pack_ragged): every forward addresses its token rows through a PackMap; `full` covers all slots
   // of every request (device-pointer entry points, batches that are not front-filled), `ragged` the counts the
   // host-buffer call found in its batch
@@ -454,6 +459,67 @@ phx_status run_trunk_f32(phx_engine* e, int B, int Tt, int pos_cap, int hist_len
   return PHX_OK;
 }
 
+// attention of one layer over the rows of e->qkv; q_start > 0: history queries are not wanted
+phx_status layer_attention(phx_engine* e, int B, int Tt, int hist_len, bool split, int q_start, const phx_engine::PackState* pk) {
+  AttnArgs aa;
+  const phx_model_config& c = e->cfg;
+  const int g = e->Hq / e->Hkv;
+  aa.q = e->qkv; aa.k = e->qkv + (long long)g * e->dh; aa.v = e->qkv + (long long)(g + 1) * e->dh;
+  aa.q_tok_stride = aa.k_tok_stride = aa.v_tok_stride = e->QW;
+  // merged QKV row: per kv head [q_0..q_{g-1}, k, v] (layers.py:728-736): q head h sits at column
+  // ((h / g) * (g + 2) + h % g) * dh, kv head j's k at (j * (g + 2) + g) * dh
+  aa.q_head_stride = (g == 1) ? (g + 2) * e->dh : e->dh;
+  aa.q_group = g; aa.q_group_stride = (g + 2) * e->dh;
+  aa.k_head_stride = (g + 2) * e->dh; aa.v_head_stride = (g + 2) * e->dh;
+  aa.out = e->attn; aa.seg = e->seg; aa.B = B; aa.T = Tt; aa.Hq = e->Hq; aa.Hkv = e->Hkv; aa.dh = e->dh;
+  aa.hist_len = hist_len; aa.sm_scale = sqrtf(128.0f) / (float)c.key_size;  // phoenix/xrex/models/scaling.py:46-47
+  aa.cap = c.attn_logit_cap;
+  aa.cap_method = (c.attn_logit_cap > 0.f) ? c.cap_method : 0;
+  aa.err_flag = e->err_flag;
+  aa.split = split ? 1 : 0; aa.q_start = q_start;
+  aa.pack = pack_map(pk);
+  e->last_launches++;
+  ProfScope ps(e, KC_ATTN);
+  return ranker_attention_launch(aa, e->stream, e->err);
+}
+
+// out-projection and FFN of one layer over rows [off, off + Mu) of the residual stream
+phx_status layer_update(phx_engine* e, Layer& L, long long off, long long Mu) {
+  if (Mu == 0) return PHX_OK;                         // a candidate-only layer of a batch without candidates
+  const phx_model_config& c = e->cfg;
+  const bool fused = e->fused_norm;
+  const int slots = e->D / 64;
+  phx_status s;
+  GemmNorm n_attn_out = {nullptr, e->rowss_f ? e->rowss_f + off * slots : nullptr, 0, 0.f, 0.f};   // out-proj leaves stats for the FFN
+  GemmNorm n_ffn_in = {e->rowss_f ? e->rowss_f + off * slots : nullptr, nullptr, slots, 1.0f / (float)e->D, c.rms_eps};
+  GemmNorm n_ffn_out = {nullptr, e->rowss_a ? e->rowss_a + off * slots : nullptr, 0, 0.f, 0.f};    // down-proj leaves stats for the next layer
+  GemmPlan& pu = fused ? L.p_up_f : L.p_up;
+  bf16* xu = e->x + off * e->D;                       // the rows this layer updates
+  const bf16* attn_u = e->attn + off * e->HD;
+  bf16* ffn_u = e->ffn + off * e->F;
+  if (c.primer_norm) {
+    // x = x + post_attn_norm(out(attn)) (transformer.py:531-541)
+    if ((s = do_gemm(e, L.p_out, attn_u, e->tmp, nullptr, Mu, EPI_STORE))) return s;
+    { ProfScope ps(e, KC_NORM); if ((s = rmsnorm_launch(e->tmp, L.post_attn_norm, xu, xu, Mu, e->D, c.rms_eps, e->stream, e->err))) return s; }
+    e->last_launches++;
+  } else {
+    if ((s = do_gemm(e, L.p_out, attn_u, xu, xu, Mu, EPI_RESIDUAL, nullptr, fused ? &n_attn_out : nullptr))) return s;
+  }
+  if (!fused) {
+    { ProfScope ps(e, KC_NORM); if ((s = rmsnorm_launch(xu, L.pre_ffn_norm, e->hbuf, nullptr, Mu, e->D, c.rms_eps, e->stream, e->err))) return s; }
+    e->last_launches++;
+  }
+  if ((s = do_gemm(e, pu, fused ? xu : e->hbuf, ffn_u, nullptr, Mu, EPI_GELU, nullptr, fused ? &n_ffn_in : nullptr))) return s;
+  if (c.primer_norm) {
+    if ((s = do_gemm(e, L.p_down, ffn_u, e->tmp, nullptr, Mu, EPI_STORE))) return s;
+    { ProfScope ps(e, KC_NORM); if ((s = rmsnorm_launch(e->tmp, L.post_ffn_norm, xu, xu, Mu, e->D, c.rms_eps, e->stream, e->err))) return s; }
+    e->last_launches++;
+  } else {
+    if ((s = do_gemm(e, L.p_down, ffn_u, xu, xu, Mu, EPI_RESIDUAL, nullptr, fused ? &n_ffn_out : nullptr))) return s;
+  }
+  return PHX_OK;
+}
+
 // trunk over `Tt` tokens per request (history + candidates, or history only for the tower).
 // split: the rows are in split layout (token_row); the last `n_tail` layers then update the candidate rows only
 // (transformer.py:789-871): their QKV projection still covers every row - the history keys / values of a tail layer
@@ -464,7 +530,6 @@ phx_status run_trunk(phx_engine* e, int B, int Tt, int pos_cap, int hist_len, bo
   const phx_engine::PackState* pk = split ? nullptr : e->cur_pack;   // packed rows (ranking forward of a packing engine)
   const long long M = pk ? pk->M : (long long)B * Tt;
   const phx_model_config& c = e->cfg;
-  const float sm_scale = sqrtf(128.0f) / (float)c.key_size;  // phoenix/xrex/models/scaling.py:46-47
   phx_status s;
   for (int l = 0; l < c.num_layers; ++l) {
     Layer& L = e->layers[l];
@@ -472,18 +537,13 @@ phx_status run_trunk(phx_engine* e, int B, int Tt, int pos_cap, int hist_len, bo
     const int slots = e->D / 64;
     const bool tail = (split || pk) && l >= c.num_layers - n_tail;
     const long long off = tail ? (pk ? pk->Mh : (long long)B * hist_len) : 0;   // first row the out-projection and FFN update
-    const long long Mu = M - off;                                // rows they update
     GemmNorm n_attn_in = {e->rowss_a, nullptr, slots, 1.0f / (float)e->D, c.rms_eps};   // consume stats of x -> QKV
-    GemmNorm n_attn_out = {nullptr, e->rowss_f ? e->rowss_f + off * slots : nullptr, 0, 0.f, 0.f};   // out-proj leaves stats for the FFN
-    GemmNorm n_ffn_in = {e->rowss_f ? e->rowss_f + off * slots : nullptr, nullptr, slots, 1.0f / (float)e->D, c.rms_eps};
-    GemmNorm n_ffn_out = {nullptr, e->rowss_a ? e->rowss_a + off * slots : nullptr, 0, 0.f, 0.f};    // down-proj leaves stats for the next layer
     if (!fused) {
       { ProfScope ps(e, KC_NORM);
       if ((s = rmsnorm_launch(e->x, L.pre_attn_norm, e->hbuf, nullptr, M, e->D, c.rms_eps, e->stream, e->err))) return s; }
       e->last_launches++;
     }
     GemmPlan& pq = fused ? L.p_qkv_f : L.p_qkv;
-    GemmPlan& pu = fused ? L.p_up_f : L.p_up;
     const bf16* a_in = fused ? e->x : e->hbuf;
     // RoPE rides in the QKV epilogue unless qk-norm has to run first (heads of 128 through a pass of their own: 522 us for a
     // two-layer forward of 8 x 1086 rows, 465 us in the epilogue)
@@ -508,47 +568,8 @@ phx_status run_trunk(phx_engine* e, int B, int Tt, int pos_cap, int hist_len, bo
       { ProfScope ps(e, KC_ROPE); if ((s = qknorm_rope_launch(qa, e->stream, e->err))) return s; }
       e->last_launches++;
     }
-    AttnArgs aa;
-    const int g = e->Hq / e->Hkv;
-    aa.q = e->qkv; aa.k = e->qkv + (long long)g * e->dh; aa.v = e->qkv + (long long)(g + 1) * e->dh;
-    aa.q_tok_stride = aa.k_tok_stride = aa.v_tok_stride = e->QW;
-    // merged QKV row: per kv head [q_0..q_{g-1}, k, v] (layers.py:728-736): q head h sits at column
-    // ((h / g) * (g + 2) + h % g) * dh, kv head j's k at (j * (g + 2) + g) * dh
-    aa.q_head_stride = (g == 1) ? (g + 2) * e->dh : e->dh;
-    aa.q_group = g; aa.q_group_stride = (g + 2) * e->dh;
-    aa.k_head_stride = (g + 2) * e->dh; aa.v_head_stride = (g + 2) * e->dh;
-    aa.out = e->attn; aa.seg = e->seg; aa.B = B; aa.T = Tt; aa.Hq = e->Hq; aa.Hkv = e->Hkv; aa.dh = e->dh;
-    aa.hist_len = hist_len; aa.sm_scale = sm_scale; aa.cap = c.attn_logit_cap;
-    aa.cap_method = (c.attn_logit_cap > 0.f) ? c.cap_method : 0;
-    aa.err_flag = e->err_flag;
-    aa.split = split ? 1 : 0; aa.q_start = tail ? hist_len : 0;
-    aa.pack = pack_map(pk);
-    { ProfScope ps(e, KC_ATTN); if ((s = ranker_attention_launch(aa, e->stream, e->err))) return s; }
-    e->last_launches++;
-    if (Mu == 0) continue;                              // a candidate-only layer of a batch without candidates
-    bf16* xu = e->x + off * e->D;                       // the rows this layer updates
-    const bf16* attn_u = e->attn + off * e->HD;
-    bf16* ffn_u = e->ffn + off * e->F;
-    if (c.primer_norm) {
-      // x = x + post_attn_norm(out(attn)) (transformer.py:531-541)
-      if ((s = do_gemm(e, L.p_out, attn_u, e->tmp, nullptr, Mu, EPI_STORE))) return s;
-      { ProfScope ps(e, KC_NORM); if ((s = rmsnorm_launch(e->tmp, L.post_attn_norm, xu, xu, Mu, e->D, c.rms_eps, e->stream, e->err))) return s; }
-      e->last_launches++;
-    } else {
-      if ((s = do_gemm(e, L.p_out, attn_u, xu, xu, Mu, EPI_RESIDUAL, nullptr, fused ? &n_attn_out : nullptr))) return s;
-    }
-    if (!fused) {
-      { ProfScope ps(e, KC_NORM); if ((s = rmsnorm_launch(xu, L.pre_ffn_norm, e->hbuf, nullptr, Mu, e->D, c.rms_eps, e->stream, e->err))) return s; }
-      e->last_launches++;
-    }
-    if ((s = do_gemm(e, pu, fused ? xu : e->hbuf, ffn_u, nullptr, Mu, EPI_GELU, nullptr, fused ? &n_ffn_in : nullptr))) return s;
-    if (c.primer_norm) {
-      if ((s = do_gemm(e, L.p_down, ffn_u, e->tmp, nullptr, Mu, EPI_STORE))) return s;
-      { ProfScope ps(e, KC_NORM); if ((s = rmsnorm_launch(e->tmp, L.post_ffn_norm, xu, xu, Mu, e->D, c.rms_eps, e->stream, e->err))) return s; }
-      e->last_launches++;
-    } else {
-      if ((s = do_gemm(e, L.p_down, ffn_u, xu, xu, Mu, EPI_RESIDUAL, nullptr, fused ? &n_ffn_out : nullptr))) return s;
-    }
+    if ((s = layer_attention(e, B, Tt, hist_len, split, tail ? hist_len : 0, pk))) return s;
+    if ((s = layer_update(e, L, off, M - off))) return s;
   }
   return PHX_OK;
 }
@@ -689,7 +710,10 @@ phx_status phx_engine_create(const phx_model_config* cfg, int32_t device, phx_en
   {
     const char* ll = getenv("PHX_LAST_LAYER");
     const bool keep_full = ll && strcmp(ll, "full") == 0;
-    if (e->C > 0 && !e->fp32 && !keep_full && e->n_tail == 0) e->n_tail = 1;
+    if (e->C > 0 && !e->fp32 && !keep_full && e->n_tail == 0) {
+      e->n_tail = 1;
+      e->taps_plain = !e->pack && (e->dh == 128 || e->S > 128);
+    }
   }
   e->split = e->n_tail > 0 && !e->fp32 && !e->pack;   // packed rows carry their own history-first order
   const long long M = e->max_tokens;
@@ -1090,7 +1114,7 @@ phx_status phx_rank_forward_device(phx_engine* e, const phx_rank_batch* bd, cons
   if (!params_complete(e, true) || !shards_complete(e)) return PHX_E_STATE;
   cudaSetDevice(e->device);
   const int B = bd->batch;
-  e->last_batch = B; e->last_launches = 0; e->prof_used = 0;
+  e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = true; e->history_done = false;
   e->cur_pack = e->pack ? (planned ? planned : &e->pack_full) : nullptr;
   if (B == 0) return PHX_OK;
   PHX_CUDA_TRY(cudaEventRecord(e->ev0, e->stream), e->err);
@@ -1220,7 +1244,7 @@ phx_status phx_rank_forward_rows_device(phx_engine* e, const phx_rank_batch* bd,
   if (!params_complete(e, true)) return PHX_E_STATE;
   cudaSetDevice(e->device);
   const int B = bd->batch;
-  e->last_batch = B; e->last_launches = 0; e->prof_used = 0;
+  e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = true; e->history_done = false;
   e->prefetch_valid = false;
   e->graph_key_valid = false;
   e->cur_pack = e->pack ? &e->pack_full : nullptr;
@@ -1238,7 +1262,7 @@ namespace {
 phx_status forward_hashed_core(phx_engine* e, const HashedIn& in, int B, const phx_rank_out* od) {
   if (!params_complete(e, true) || !shards_complete(e)) return PHX_E_STATE;
   cudaSetDevice(e->device);
-  e->last_batch = B; e->last_launches = 0; e->prof_used = 0;
+  e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = true; e->history_done = false;
   e->prefetch_valid = false;
   e->graph_key_valid = false;   // plain launches: the graph cache is keyed on id batches
   e->cur_pack = e->pack ? &e->pack_full : nullptr;
@@ -1724,6 +1748,7 @@ phx_status phx_debug_read(phx_engine* e, const char* what, void* host, size_t nb
   const std::string w(what);
   const size_t M = (size_t)e->last_batch * e->T;
   const void* src = nullptr; size_t avail = 0;
+  const bool plain = e->taps_plain && e->taps_of_rank && (w == "hidden" || w == "seg" || w == "attn" || w == "qkv");
   if (w == "hidden" && e->fp32) { src = e->x32; avail = M * e->D * 4; }   // full-precision path: fp32 rows
   else if (w == "hidden") { src = e->x; avail = M * e->D * 2; }
   else if (w == "seg") { src = e->seg; avail = M * 4; }
@@ -1733,8 +1758,28 @@ phx_status phx_debug_read(phx_engine* e, const char* what, void* host, size_t nb
   else if (w == "hashes" && e->debug_taps) { src = e->hashes; avail = M * 2 * e->cfg.item.num_hashes * 4; }
   else { e->err = "phx_debug_read: unknown tap (tokens / hashes need PHX_DEBUG_TAPS=1): " + w; return PHX_E_ARG; }
   if (nbytes > avail) { e->err = "phx_debug_read: more bytes requested than the tap holds"; return PHX_E_ARG; }
+  if (plain && !e->history_done && nbytes > 0 && (w == "hidden" || w == "attn")) {
+    // the history rows' share of the last layer: q, k and v are there, the rows stand where the layer found them
+    const int launches = e->last_launches;
+    const size_t profiled = e->prof_used;
+    phx_status s = layer_attention(e, e->last_batch, e->T, e->S, true, 0, nullptr);
+    if (s == PHX_OK) s = layer_update(e, e->layers.back(), 0, (long long)e->last_batch * e->S);
+    e->last_launches = launches; e->prof_used = profiled;
+    if (s) return s;
+    e->history_done = true;
+  }
   PHX_CUDA_TRY(cudaStreamSynchronize(e->stream), e->err);
-  PHX_CUDA_TRY(cudaMemcpy(host, src, nbytes, cudaMemcpyDeviceToHost), e->err);
+  if (!plain) {
+    PHX_CUDA_TRY(cudaMemcpy(host, src, nbytes, cudaMemcpyDeviceToHost), e->err);
+    return PHX_OK;
+  }
+  std::vector<uint8_t> rows(avail);
+  PHX_CUDA_TRY(cudaMemcpy(rows.data(), src, avail, cudaMemcpyDeviceToHost), e->err);
+  const size_t width = M > 0 ? avail / M : 0;
+  for (size_t r = 0; r < M && r * width < nbytes; ++r) {
+    const size_t from = (size_t)token_row(1, e->last_batch, e->S, e->T, (int)(r / e->T), (int)(r % e->T)) * width;
+    memcpy((uint8_t*)host + r * width, rows.data() + from, nbytes - r * width < width ? nbytes - r * width : width);
+  }
   return PHX_OK;
 }
 
@@ -1769,7 +1814,7 @@ phx_status phx_user_tower_device(phx_engine* e, const phx_rank_batch* bd, float*
   if (!params_complete(e, false) || !shards_complete(e)) return PHX_E_STATE;
   cudaSetDevice(e->device);
   const int B = bd->batch;
-  e->last_batch = B; e->last_launches = 0; e->prof_used = 0;
+  e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = false;
   if (B == 0) return PHX_OK;
   PHX_CUDA_TRY(cudaEventRecord(e->ev0, e->stream), e->err);
   phx_status s;
