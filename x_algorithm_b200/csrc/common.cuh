@@ -135,8 +135,7 @@ struct GemmNorm {
 struct GemmPlan {
   CUtensorMap map_a;
   CUtensorMap map_b;
-  CUtensorMap map_b_narrow;   // W map for 128-column tiles, used when a call has too few wide tiles to fill the device
-  bool has_narrow = false;
+  CUtensorMap map_b_narrow;   // BN = 256: W map for narrower tiles, used when a call has too few wide tiles to fill the device
   CUtensorMap map_c;   // output map, re-encoded when the output pointer or M changes
   CUtensorMap map_r;   // residual map, likewise
   const bf16* c_ptr = nullptr; const bf16* r_ptr = nullptr;
@@ -147,6 +146,7 @@ struct GemmPlan {
   int64_t a_rows = 0;   // rows the A map was encoded over (rows_max, or the M of the call that moved A)
   int N = 0, K = 0, BN = 0;
   bool pair = false;   // two CTAs of a cluster share each 256-row tile (tcgen05 cta_group::2)
+  bool small_ok = false;   // calls of few tiles take one tile per CTA (gemm_small_kernel)
   bool ready = false;
   bool w_stable = false;   // nothing writes Wt while launches of this plan are in flight or queued: it may be read ahead
   unsigned long long* counters = nullptr;  // optional device counters [8]: MMA issuer cycles total / waiting for

@@ -882,9 +882,11 @@ phx_status gemm_plan_create(GemmPlan* plan, const bf16* A, const bf16* Wt, int64
   { const char* t = getenv("PHX_GEMM_TILES");   // diagnostics: wide | narrow overrides the caller's choice
     if (t && strcmp(t, "wide") == 0) narrow_tiles = false;
     if (t && strcmp(t, "narrow") == 0) narrow_tiles = true; }
-  // CTA pairs by default; PHX_GEMM=cta1 keeps every CTA on its own tile (for comparison)
+  // CTA pairs, and one tile per CTA for few tiles, by default; for comparison PHX_GEMM=pair takes pairs at every size and
+  // PHX_GEMM=cta1 the persistent kernel with single CTAs
   const char* mode = getenv("PHX_GEMM");
   plan->pair = pair >= 0 ? (pair != 0) : !(mode && strcmp(mode, "cta1") == 0);
+  plan->small_ok = plan->pair && !(mode && strcmp(mode, "pair") == 0);
   // a pair fills 128 + BN/2 operand rows per CTA and k-step: the wide tile is the cheaper one per FLOP there
   // (out-projection, N = K = 512: 0.100 ms wide against 0.146 ms narrow)
   if (plan->pair && !(getenv("PHX_GEMM_TILES") && strcmp(getenv("PHX_GEMM_TILES"), "narrow") == 0)) narrow_tiles = false;
@@ -893,10 +895,9 @@ phx_status gemm_plan_create(GemmPlan* plan, const bf16* A, const bf16* Wt, int64
   if (s != PHX_OK) return s;
   s = make_map(&plan->map_b, Wt, N, K, plan->pair ? plan->BN / 2 : plan->BN, err);
   if (s != PHX_OK) return s;
-  if (plan->BN == 256) {   // small calls (a single request) run 128-column tiles: twice the CTAs, half the work per tile
+  if (plan->BN == 256) {   // the narrow tiles' W box: one tile per CTA, and single CTAs in gemm_launch's latency regime
     s = make_map(&plan->map_b_narrow, Wt, N, K, plan->pair ? 64 : 128, err);
     if (s != PHX_OK) return s;
-    plan->has_narrow = true;
   }
   plan->ready = true;
   return PHX_OK;
@@ -937,30 +938,27 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
     if (s != PHX_OK) return s;
     p.r_ptr = R; p.r_rows = M;
   }
-  if (p.pair) {
+  if (p.small_ok) {
     // Few tiles: one 128 x 64 (else 128 x 128) tile per CTA while they do not outnumber the SMs.  Beyond that a CTA would have
     // a second tile with nothing overlapped, and the pair kernel's wide tiles fetch fewer operand bytes.
-    static const bool small_ok = !getenv("PHX_GEMM_TILES");
     const CUtensorMap& map_b64 = p.BN == 256 ? p.map_b_narrow : p.map_b;   // boxes of 64 W rows, either way
     const long long mt = (M + BM - 1) / BM, t64 = mt * ((p.N + 63) / 64), t128 = mt * ((p.N + 127) / 128);
-    if (small_ok && (p.BN != 256 || p.has_narrow)) {
-      if (t64 <= num_sms && !(epilogue == EPI_ROPE && rp.dh == 128)) { dispatch_note(DK_GEMM_SMALL); return launch_small<64>(p, map_b64, C, R, epilogue, rp, nm, M, err_flag, stream, err); }
-      if (t128 <= num_sms) { dispatch_note(DK_GEMM_SMALL); return launch_small<128>(p, map_b64, C, R, epilogue, rp, nm, M, err_flag, stream, err); }
-    }
+    if (t64 <= num_sms && !(epilogue == EPI_ROPE && rp.dh == 128)) { dispatch_note(DK_GEMM_SMALL); return launch_small<64>(p, map_b64, C, R, epilogue, rp, nm, M, err_flag, stream, err); }
+    if (t128 <= num_sms) { dispatch_note(DK_GEMM_SMALL); return launch_small<128>(p, map_b64, C, R, epilogue, rp, nm, M, err_flag, stream, err); }
   }
   if (p.BN == 256) {
-    // latency regime: when even the 128-column tiles leave SMs idle, take them - the call's time is one tile's time
-    const long long rows_per_tile = p.pair ? 2 * BM : BM;
-    const long long narrow_tiles = ((M + rows_per_tile - 1) / rows_per_tile) * ((p.N + 127) / 128);
-    const long long slots = p.pair ? num_sms / 2 : num_sms;
-    static const bool allow = !(getenv("PHX_GEMM_TILES") && strcmp(getenv("PHX_GEMM_TILES"), "wide") == 0);
-    const bool must = !p.pair && epilogue == EPI_ROPE && rp.dh == 128;
-    if (p.has_narrow && (must || (allow && narrow_tiles <= slots))) {
-      dispatch_note(p.pair ? DK_GEMM_PAIR128 : DK_GEMM_CTA128);
-      GemmPlan q = p;
-      q.map_b = p.map_b_narrow; q.BN = 128;
-      return q.pair ? launch_e<128, true>(q, epilogue, rp, nm, M, err_flag, num_sms, stream, err)
-                    : launch_e<128, false>(q, epilogue, rp, nm, M, err_flag, num_sms, stream, err);
+    if (!p.pair) {
+      // single CTAs, latency regime: when even the 128-column tiles leave SMs idle, take them - the call's time is one tile's
+      // time (a pair's call of that size has gone to one tile per CTA above).  Heads of 128 always: a single CTA's 256-column
+      // tiles leave no room for the buffers of a rotated head.
+      const long long narrow_tiles = ((M + BM - 1) / BM) * ((p.N + 127) / 128);
+      static const bool allow = !(getenv("PHX_GEMM_TILES") && strcmp(getenv("PHX_GEMM_TILES"), "wide") == 0);
+      if ((epilogue == EPI_ROPE && rp.dh == 128) || (allow && narrow_tiles <= num_sms)) {
+        dispatch_note(DK_GEMM_CTA128);
+        GemmPlan q = p;
+        q.map_b = p.map_b_narrow; q.BN = 128;
+        return launch_e<128, false>(q, epilogue, rp, nm, M, err_flag, num_sms, stream, err);
+      }
     }
     dispatch_note(p.pair ? DK_GEMM_PAIR256 : DK_GEMM_CTA256);
     return p.pair ? launch_e<256, true>(p, epilogue, rp, nm, M, err_flag, num_sms, stream, err)
