@@ -107,3 +107,32 @@ def test_debug_taps_hold_every_row_in_request_order(monkeypatch, S, C, dh, hq, h
     _, _, _, eng = make_pair(**kw)
     for a, c in zip(got, read(eng, b)):
         np.testing.assert_array_equal(a, c)
+
+
+@pytest.mark.parametrize("B,S,C,hkv", [(8, 128, 512, 8), (13, 128, 500, 8), (5, 97, 512, 4), (18, 128, 257, 2)])
+def test_fewer_items_than_sms_split_by_tiles(monkeypatch, B, S, C, hkv):
+    """The resident-history kernel with fewer (batch, head) pairs than SMs and more query tiles: a CTA's share begins inside one
+    item and runs into the next, in full layers and (the last one) without the history tile.  Ragged requests, against the
+    mma.sync kernel and the oracle."""
+    from x_algorithm_b200.engine import dispatch_counts
+    assert B * 8 < 148 <= B * 8 * (1 + -(-C // 128))
+    kw = dict(max_batch=B, emb_size=256, num_q_heads=8, num_kv_heads=hkv, key_size=64, history_len=S, num_candidates=C, num_layers=2)
+    ocfg, w, rows_fn, eng = make_pair(**kw)
+    b = po.make_batch(ocfg, B, seed=S + C, ragged=True)
+    before = dispatch_counts()
+    got = eng.rank(to_inputs(b))
+    ran = {k: v - before[k] for k, v in dispatch_counts().items() if k.startswith("attn.") and v != before[k]}
+    assert ran == {"attn.pingpong": 2}, ran
+    monkeypatch.setenv("PHX_ATTN", "mma")
+    other = eng.rank(to_inputs(b))
+    eng.close()
+    valid = b.cand_post_ids != 0
+    for r in range(B):                                   # request by request: a mixed-up tile cannot hide in the sum
+        v = valid[r]
+        if v.any():
+            assert rel_l2(logits_of(got.log_probs[r][v]), logits_of(other.log_probs[r][v])) < 1e-2, r
+    few = slice(B // 2, B // 2 + 2)
+    bb = po.RankBatch(*(getattr(b, f)[few] for f in ("hist_post_ids", "hist_author_ids", "hist_actions", "hist_surfaces", "cand_post_ids", "cand_author_ids")))
+    lp, cont, logits = po.rank_forward(ocfg, w, rows_fn, bb)
+    ok = bb.cand_post_ids != 0
+    assert_heads_close(got.log_probs[few][ok], got.continuous[few][ok], logits[ok], cont[ok], 2e-2, str(kw))
