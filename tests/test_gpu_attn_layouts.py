@@ -136,3 +136,20 @@ def test_fewer_items_than_sms_split_by_tiles(monkeypatch, B, S, C, hkv):
     lp, cont, logits = po.rank_forward(ocfg, w, rows_fn, bb)
     ok = bb.cand_post_ids != 0
     assert_heads_close(got.log_probs[few][ok], got.continuous[few][ok], logits[ok], cont[ok], 2e-2, str(kw))
+
+
+@pytest.mark.parametrize("B,S,C,hq,hkv,kind", [(5, 65, 385, 8, 8, "pingpong"), (5, 64, 512, 8, 8, "stream"), (7, 20, 512, 8, 8, "stream"), (4, 65, 384, 8, 8, "stream"),
+                                               (19, 64, 385, 8, 2, "pingpong"), (19, 64, 384, 8, 2, "strip"), (19, 65, 64, 8, 2, "pingpong"), (19, 65, 63, 8, 2, "strip"),
+                                               (19, 30, 20, 8, 8, "pingpong")])
+def test_which_kernel_takes_a_short_history(B, S, C, hq, hkv, kind):
+    """Both sides of the lines between the resident-history tcgen05 kernel and the mma.sync kernels at head dim 64; in the
+    candidate-only last layer as in the full one."""
+    from x_algorithm_b200.engine import dispatch_counts
+    kw = dict(max_batch=B, emb_size=128, num_q_heads=hq, num_kv_heads=hkv, key_size=64, history_len=S, num_candidates=C, num_layers=2)
+    ocfg, w, rows_fn, eng = make_pair(**kw)
+    b = po.make_batch(ocfg, B, seed=S + C)
+    before = dispatch_counts()
+    eng.rank(to_inputs(b))
+    ran = {k: v - before[k] for k, v in dispatch_counts().items() if k.startswith("attn.") and v != before[k]}
+    eng.close()
+    assert ran == {"attn." + kind: 2}, ran

@@ -678,19 +678,24 @@ phx_status ranker_attention_launch(const AttnArgs& args, cudaStream_t stream, st
   }
   {
     // Head dim 64 with a history of at most 128 keys: the persistent tcgen05 kernel with the history resident and two
-    // softmax warpgroups, once there is an item (batch, head) for every SM, or long candidate lists with a tile for every SM
-    // (8 requests of 640 rows: 17.5 against 20.1 us for the streaming mma.sync kernel, 16: 19.7 against 27.7; with one or two
-    // tiles per item the two are level at 148 items and below).  A candidate-only layer counts its history tile too: it takes
-    // the kernel the same layer over every row takes, and so has the same bits.  Measured on B200 at the ranking
-    // benchmark's shape (B=256, S=128, C=512, 8 heads): 0.140 ms per layer against 0.206 ms for the mma.sync
-    // resident-history kernel below (1.2-1.4 against 2.0 ms per step inside the forward), and 0.051 against 0.067 ms at
-    // B=64; every byte it touches moves by bulk copies.  PHX_ATTN=strip keeps the mma.sync kernel, PHX_ATTN=pingpong
-    // takes this one at any batch size.
+    // softmax warpgroups.  Measured on B200 at the ranking benchmark's shape (B=256, S=128, C=512, 8 heads): 0.140 ms per layer
+    // against 0.206 ms for the mma.sync resident-history kernel below (1.2-1.4 against 2.0 ms per step inside the forward), and
+    // 0.051 against 0.067 ms at B=64; every byte it touches moves by bulk copies.  It is taken
+    //  - with an item (batch, head) for every SM.  Grouped heads then need rows enough: it works on whole 128-key, 128-row
+    //    tiles and starts after the kernel in front has ended, the mma.sync kernels on 64-key blocks and ahead of that.
+    //    Three-layer forwards, 19-128 requests, mma.sync time over this kernel's: 128 history + 64 candidate rows 1.01-1.06,
+    //    100 + 64 1.01-1.08, 100 + 24 0.95-1.00; up to 64 history rows 0.86-0.99 with up to 257 candidates, 1.03-1.04 with 512.
+    //  - with fewer items, for lists long enough that every SM has a tile, and more than one 64-key block of history: 4-18
+    //    requests of 128 + 512 rows 1.01-1.07, 128 + 257 1.00-1.05, 100 + 400 0.98-1.03; 64 + 512 0.97-1.01, 20 + 257 0.95-0.98;
+    //    with one or two tiles per item the two are level.  A candidate-only layer counts its history tile too: it takes the
+    //    kernel the same layer over every row takes, and so has the same bits.
+    // PHX_ATTN=strip keeps the mma.sync kernel, PHX_ATTN=pingpong takes this one at any batch size.
     const char* force = getenv("PHX_ATTN");
     const bool forced = force && strcmp(force, "pingpong") == 0;
     const int nh = a.hist_len < a.T ? a.hist_len : a.T;
     const long long items = (long long)a.B * a.Hq, nt = (nh + 127) / 128 + (a.T - nh + 127) / 128;
-    const bool fills = !force && (items >= 148 || (nt >= 4 && items * nt >= 148));
+    const bool rows_enough = a.q_group <= 1 || (nh > 64 ? a.T > 128 : nt > 4);
+    const bool fills = !force && (items >= 148 ? rows_enough : nh > 64 && nt >= 4 && items * nt >= 148);
     if ((forced || fills) && a.err_flag && ranker_attention_pingpong_supported(a))
       return ranker_attention_pingpong_launch(a, a.err_flag, stream, err);
   }
