@@ -45,7 +45,9 @@ enum DispatchKind {
   DK_TOPK_EXACT = 11,    // exact-threshold passes of the top-k (the sampled pivot missed)
   DK_ATTN_PINGPONG = 12, // tcgen05 / TMEM resident-history kernel with two softmax warpgroups
   DK_GEMM_SMALL = 13,    // tcgen05 GEMM, one tile per CTA (few tiles)
-  DK_COUNT = 14
+  DK_GATHER = 14,        // stand-alone gather-sum, a lane group per id
+  DK_GATHER_BULK = 15,   // ... many ids per warp
+  DK_COUNT = 16
 };
 void dispatch_note(int kind);
 

@@ -343,13 +343,10 @@ __global__ void __launch_bounds__(256) gather_sum_kernel(HashFamilyDev fam, Tabl
   }
 }
 
-// Measured (256 columns, 4 hashes): 4 M Zipf ids 2095 -> 977 us, 256 k 143 -> 74, 16 k 18.0 -> 12.2, 4 k 11.7 -> 10.3; at 2 k ids
-// there are too few warps' worth of rounds (9.9 against 10.3 us), hence the line.
-constexpr long long GATHER_BULK_IDS = 1 << 12;
-
 // The same for many ids: a warp takes 32 / H ids at a time (H = hash count rounded up to a power of two), lane l hashes slot
 // l % H of id l / H - every lane one hash, where the kernel above has 32 lanes wait for 4 - and the rows of 16 / H ids per
 // lane group are requested before the first is summed; the next ids are already on their way.  Same order of additions.
+// Measured (256 columns, 4 hashes): 4 M Zipf ids 2095 -> 977 us, 256 k 143 -> 74, 16 k 18.4 -> 12.9, 4 k 11.5 -> 10.8.
 template <int LANES, int H>
 __global__ void __launch_bounds__(256, 2) gather_sum_bulk_kernel(HashFamilyDev fam, TableView table, int D,
                                                                  const long long* __restrict__ ids, long long n,
@@ -408,6 +405,18 @@ __global__ void __launch_bounds__(256, 2) gather_sum_bulk_kernel(HashFamilyDev f
       }
     }
   }
+}
+
+// From how many ids on.  A round of a warp is 32 / H ids and a pass over its columns for every 256 of them: too few rounds
+// leave SMs idle where the kernel above has a warp for every id or two.  Time of that kernel over this one's, Zipf ids:
+//   1 hash:   256 columns 0.83 at 4 k ids, 1.00 at 8 k, 512 columns 0.81 at 8 k, 1.13 at 16 k, 1024 columns 0.83 at 16 k, 1.00 at 32 k;
+//             64 and 128 columns 0.90-0.94 at 4 k, 1.12 at 8 k
+//   2 hashes: 256 columns 0.91 at 2 k, 1.01 at 4 k, 512 columns 0.85 at 4 k, 1.10 at 8 k, 1024 columns 0.88 at 8 k, 1.13 at 16 k
+//   4 hashes: 256 columns 1.06 at 4 k, 512 columns 0.90 at 4 k, 1.05 at 6 k, 1024 columns 0.85 at 6 k, 1.00 at 12 k
+inline bool gather_in_bulk(int num_hashes, int D, long long n) {
+  const int H = num_hashes <= 1 ? 1 : (num_hashes <= 2 ? 2 : 4);
+  const long long per_column = H == 4 ? 12 : 32 / H;
+  return n >= (H == 1 ? 8192 : 4096) && n >= per_column * D;
 }
 
 template <int LANES>
@@ -518,7 +527,9 @@ phx_status gather_sum_launch(const HashFamilyDev& fam, const TableView& table, i
                              const long long* ids, long long n, bf16* out, cudaStream_t stream, std::string& err) {
   if (D % 8 != 0) { err = "gather_sum: D must be a multiple of 8"; return PHX_E_ARG; }
   if (n == 0) return PHX_OK;
-  if (n >= GATHER_BULK_IDS) {
+  const bool bulk = gather_in_bulk(fam.num_hashes, D, n);
+  dispatch_note(bulk ? DK_GATHER_BULK : DK_GATHER);
+  if (bulk) {
     if (D <= 128) gather_sum_bulk<16>(fam, table, D, ids, n, out, stream);
     else gather_sum_bulk<32>(fam, table, D, ids, n, out, stream);
   } else if (D <= 128) {
