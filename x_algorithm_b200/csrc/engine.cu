@@ -1476,7 +1476,8 @@ phx_status phx_rank_forward(phx_engine* e, const phx_rank_batch* bh, const phx_r
   phx_rank_out od; od.log_probs = e->lp_dev; od.continuous = e->cont_dev; od.scores = e->score_dev;
   const size_t rows = B * C;
   // Small results (up to half a megabyte) lie back to back and come back in one copy, the flag right behind: in chunks the
-  // twelve copies of one request, each a few kilobytes, took longer than their bytes.
+  // twelve copies of one request, each a few kilobytes, took longer than their bytes.  Whole calls, chunks against one copy:
+  // 44 KB 94 against 78 us, 484 KB 138 against 124, 704 KB 161 against 150, 1.4 MB 244 against 260.
   const OutLayout ol(rows, e->V, e->NC);
   const bool one_copy = ol.bytes <= (512u << 10);
   if (one_copy) { od.log_probs = ol.lp(e->out_stage_dev); od.continuous = ol.cont(e->out_stage_dev); }

@@ -81,7 +81,7 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint4 v) {
 
 // Epilogue arithmetic, two columns per instruction (packed fp32) and one conversion per pair: an epilogue thread's
 // instruction stream is what a tile with a short K waits for.  Measured: 163840 x 1024, K = 256, GELU 114.6 -> 94.2 us; a
-// forward of one request 384 -> 349 us, the user tower of 256 users 513 -> 492 us, 48 ragged requests 611 -> 597 us.
+// forward of one request 384 -> 349 us; full batches, the user tower and ragged batches gain no more than runs differ.
 // fp32 accumulators -> the Linear output, a bf16 pair: rounded once, kept in the form it is stored in
 __device__ __forceinline__ uint32_t linear_bf2(uint32_t a0, uint32_t a1, float2 rstd2) {
   const float2 v = __fmul2_rn(make_float2(__uint_as_float(a0), __uint_as_float(a1)), rstd2);
@@ -940,7 +940,10 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
   }
   if (p.small_ok) {
     // Few tiles: one 128 x 64 (else 128 x 128) tile per CTA while they do not outnumber the SMs.  Beyond that a CTA would have
-    // a second tile with nothing overlapped, and the pair kernel's wide tiles fetch fewer operand bytes.
+    // a second tile with nothing overlapped, and the pair kernel's wide tiles fetch fewer operand bytes.  Pair time over this
+    // kernel's, each alone: 8-40 tiles of 64 columns (128 and 640 rows, N = 512) 1.28-1.30; 144-148 tiles of 128: N = 2048 1.11-1.15,
+    // N = 1024 1.12-1.18 up to K = 4096, N = 512 1.02 at K = 512 and 1.11-1.13 at 2048 and 4096, N = 128 0.97-1.00.  Three-layer
+    // forwards: D = 512, 640 rows a request 1.31 with one, 1.04 with four, 0.99 with eight (only the last layer's narrow ones are few).
     const CUtensorMap& map_b64 = p.BN == 256 ? p.map_b_narrow : p.map_b;   // boxes of 64 W rows, either way
     const long long mt = (M + BM - 1) / BM, t64 = mt * ((p.N + 63) / 64), t128 = mt * ((p.N + 127) / 128);
     if (t64 <= num_sms && !(epilogue == EPI_ROPE && rp.dh == 128)) { dispatch_note(DK_GEMM_SMALL); return launch_small<64>(p, map_b64, C, R, epilogue, rp, nm, M, err_flag, stream, err); }

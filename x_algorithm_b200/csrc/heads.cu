@@ -126,8 +126,8 @@ __device__ __forceinline__ void mma_bf16_16816_h(float (&c)[4], const uint32_t (
 
 // NT: n-tiles of 8 outputs, V + NC <= 8 * NT.  WPS: warps per strip.  With enough strips every warp has its own (1); a small call
 // is one strip's chain of latencies, most of it the ten rounds of logarithms and f64 exponentials, so four warps form the
-// same sums and share the (row, output) items of one strip.  Same arithmetic, same bits.  One request of 512
-// candidates, whole call: 348.7 -> 346.4 us.
+// same sums and share the (row, output) items of one strip.  Same arithmetic, same bits.  Kernel at D = 512, 20 outputs: 512 rows
+// 21.0 -> 18.9 us, 1024 and 2048 rows 23.0 -> 18.9, 4608 rows 23.0 -> 20.9, from 4736 rows (296 strips) on level at 23.0.
 template <int NT, int WPS>
 __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_kernel(HeadsArgs a) {
   constexpr int WARPS = WPS == 1 ? HM_WARPS : WPS;      // warps per CTA
@@ -277,7 +277,7 @@ phx_status launch_heads_wps(const HeadsArgs& a, long long strips, cudaStream_t s
 }
 template <int NT>
 phx_status launch_heads_mma(const HeadsArgs& a, long long rows, cudaStream_t stream, std::string& err) {
-  // up to two CTAs of a strip each per SM: beyond that the strips alone keep the SMs busy
+  // up to two CTAs of a strip each per SM: there and beyond the strips alone keep the SMs busy (level at 296 strips)
   const long long strips = (rows + 15) / 16;
   if (strips <= 2 * 148) return launch_heads_wps<NT, 4>(a, strips, stream, err);
   return launch_heads_wps<NT, 1>(a, strips, stream, err);
