@@ -356,7 +356,9 @@ phx_status phx_last_launch_count(phx_engine* e, int32_t* n);
 
 /* Debug / parity taps after a forward (device -> host copies of internal buffers):
  * "hashes" int32 [B,T,2H] (post hashes then author hashes per token), "tokens" bf16 bits [B,T,D]
- * (the gather-sum output before scaling), "hidden" bf16 bits [B,T,D] (trunk output). */
+ * (the gather-sum output before scaling), "hidden" bf16 bits [B,T,D] (trunk output).  "hidden" of a packing engine, of one
+ * with candidate-only layers, and of one with heads below 128 and at most 128 history rows holds the rows in the engine's own
+ * order (all history rows, as the last full layer left them, then all candidate rows). */
 phx_status phx_debug_read(phx_engine* e, const char* what, void* host, size_t nbytes);
 
 /* ---- row-sharded table, exchange by all-to-all ------------------------------------------------------------------
