@@ -81,8 +81,10 @@ enum GemmEpilogue { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_GELU = 2, EPI_ROPE = 3,
 // RoPE fused into the epilogue of the merged QKV projection: applied to the q and k head parts
 // (column part p of width dh is q or k when p % group <= g; group = g + 2, g = q heads per kv head).
 struct GemmRope {
-  const float* cos_tab;  // [pos_cap + 1, dh / 2]
-  const float* sin_tab;
+  // [dh / 4][n_pos] {cos 2t, cos 2t+1, sin 2t, sin 2t+1} of column pairs 2t and 2t + 1: positions are neighbours, so the 32 rows
+  // of an epilogue warp (consecutive positions, or all at the cap) read 512 contiguous bytes or one 16-byte word
+  const float4* angles;
+  int n_pos;
   int T;                 // tokens per request: position = min(row % T, pos_cap)
   int pos_cap;
   int dh;                // 32, 64 or 128

@@ -134,7 +134,8 @@ struct phx_engine {
   bf16* unembed_t = nullptr;  // [V+NC, D]
   std::vector<Layer> layers;
   std::map<std::string, bool> loaded;
-  float *cos_tab = nullptr, *sin_tab = nullptr;
+  float *cos_tab = nullptr, *sin_tab = nullptr;   // [S + 1][dh / 2]
+  float4* angles = nullptr;                       // the same values as GemmRope::angles
   phx_blend_spec blend;
   bool has_blend = false;
 
@@ -550,7 +551,7 @@ phx_status run_trunk(phx_engine* e, int B, int Tt, int pos_cap, int hist_len, bo
     const bool fuse_rope = c.rotary && !c.qk_norm && !e->use_simt_gemm;
     if (fuse_rope) {
       GemmRope gr;
-      gr.cos_tab = e->cos_tab; gr.sin_tab = e->sin_tab; gr.T = Tt; gr.pos_cap = pos_cap; gr.dh = e->dh;
+      gr.angles = e->angles; gr.n_pos = e->S + 1; gr.T = Tt; gr.pos_cap = pos_cap; gr.dh = e->dh;
       gr.g = e->Hq / e->Hkv; gr.group = gr.g + 2;
       if (split) { gr.T = hist_len; gr.split_rows = (long long)B * hist_len; }
       if (pk) gr.pos_rows = pk->pos_rows;
@@ -804,6 +805,14 @@ phx_status phx_engine_create(const phx_model_config* cfg, int32_t device, phx_en
     TRY(dev_alloc(e, &e->cos_tab, ct.size())); TRY(dev_alloc(e, &e->sin_tab, st.size()));
     CU(cudaMemcpy(e->cos_tab, ct.data(), ct.size() * 4, cudaMemcpyHostToDevice));
     CU(cudaMemcpy(e->sin_tab, st.data(), st.size() * 4, cudaMemcpyHostToDevice));
+    std::vector<float4> ang((size_t)(half / 2) * npos);
+    for (int t = 0; t < half / 2; ++t)
+      for (int p = 0; p < npos; ++p) {
+        const size_t o = (size_t)p * half + 2 * t;
+        ang[(size_t)t * npos + p] = make_float4(ct[o], ct[o + 1], st[o], st[o + 1]);
+      }
+    TRY(dev_alloc(e, &e->angles, ang.size()));
+    CU(cudaMemcpy(e->angles, ang.data(), ang.size() * sizeof(float4), cudaMemcpyHostToDevice));
   }
   e->layers.resize(cfg->num_layers);
   for (auto& L : e->layers) {
@@ -894,7 +903,7 @@ void phx_engine_destroy(phx_engine* e) {
     fr(L.pre_attn_norm); fr(L.pre_ffn_norm); fr(L.post_attn_norm); fr(L.post_ffn_norm); fr(L.q_norm); fr(L.k_norm);
     fr(L.w_qkv_t); fr(L.w_out_t); fr(L.w_up_t); fr(L.w_down_t); fr(L.w_qkv_f); fr(L.w_up_f);
   }
-  fr(e->cos_tab); fr(e->sin_tab); fr(e->x); fr(e->hbuf); fr(e->qkv); fr(e->attn); fr(e->ffn); fr(e->tmp); fr(e->tokens);
+  fr(e->cos_tab); fr(e->sin_tab); fr(e->angles); fr(e->x); fr(e->hbuf); fr(e->qkv); fr(e->attn); fr(e->ffn); fr(e->tmp); fr(e->tokens);
   for (phx_engine::PackState* ps : {&e->pack_full, &e->pack_ragged}) { fr(ps->hist_off); fr(ps->cand_off); fr(ps->pos_rows); fr(ps->out_index); }
   fr(e->proj_hist_t); fr(e->proj_cand_t); fr(e->cat_hist); fr(e->cat_cand); fr(e->tok_proj); fr(e->proj_user_t); fr(e->cat_user);
   for (int i = 0; i < PHX_MAX_HIST_CONT; ++i) { fr(e->cont_w1[i]); fr(e->cont_w2[i]); }

@@ -358,24 +358,23 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       // the wait on the accumulator
       constexpr bool ROPE = EPI == EPI_ROPE || EPI == EPI_ROPE128, D128 = EPI == EPI_ROPE128;
       const bool d64 = ROPE && !D128 && rope.dh == 64;
-      float4 cs[4], sn[4];
-      const float4 *cos_row = nullptr, *sin_row = nullptr;
+      // A thread is a row.  With one table row per position every lane of a load touched a cache line of its own, 32 tag
+      // look-ups an instruction and 5.5 k cycles a 256-column tile, which is what the tile waited for; with positions
+      // as the fast index a load touches four lines at most.  User tower (32768 rows, K = 256, four layers) 517 -> 489 us,
+      // two layers of 8 x 1086 rows with heads of 128 455 -> 449 us; full batches (K = 512) gain no more than runs differ.
+      float4 ang[8];
+      const float4* ang_col = nullptr;
       auto part_rotated = [&](int p) {
         const int part = D128 ? (c0 >> 7) : d64 ? (c0 >> 6) : (c0 >> 5) + p;
         return part % rope.group <= rope.g;
       };
       auto load_angles = [&](int p) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          cs[j] = __ldg(cos_row + ((D128 || d64) ? 4 * p : 0) + j);
-          sn[j] = __ldg(sin_row + ((D128 || d64) ? 4 * p : 0) + j);
-        }
+        for (int t = 0; t < 8; ++t) ang[t] = __ldg(ang_col + (((D128 || d64) ? 8 * p : 0) + t) * rope.n_pos);
       };
       if (ROPE) {
         const long long row = m0 + row_in_tile;
-        const long long o = (long long)rope_pos(rope, row + rope.row_offset, row < M) * (rope.dh >> 1);
-        cos_row = reinterpret_cast<const float4*>(rope.cos_tab + o);
-        sin_row = reinterpret_cast<const float4*>(rope.sin_tab + o);
+        ang_col = rope.angles + rope_pos(rope, row + rope.row_offset, row < M);
         if (part_rotated(0)) load_angles(0);
       }
       if (RES && issuer && i + DIST < my_items) {
@@ -425,10 +424,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
             if (part_rotated(p)) {   // v parts pass through
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                rope_bf2<D128>(lo[2 * j], hi[2 * j], cs[j].x, cs[j].y, sn[j].x, sn[j].y);
-                rope_bf2<D128>(lo[2 * j + 1], hi[2 * j + 1], cs[j].z, cs[j].w, sn[j].z, sn[j].w);
-              }
+              for (int t = 0; t < 8; ++t) rope_bf2<D128>(lo[t], hi[t], ang[t].x, ang[t].y, ang[t].z, ang[t].w);
             }
             if (p + 1 < (D128 ? 4 : 2) && part_rotated(p + 1)) load_angles(p + 1);
 #pragma unroll
@@ -710,19 +706,16 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       }
       rstd = rsqrtf(ss * norm.inv_d + norm.eps);
     }
-    float4 cs[4], sn[4];
+    float4 ang[8];
     bool rotate = false;
     if (EPI == EPI_ROPE) {
       const int pos = rope_pos(rope, row + rope.row_offset, in);
       const int kind = d128 ? (c0 >> 7) % rope.group : d64 ? (c0 >> 6) % rope.group : ((c0 >> 5) + p) % rope.group;
       rotate = kind <= rope.g;
       if (rotate) {
-        const long long o = (long long)pos * (rope.dh >> 1) + ((d64 || d128) ? 16 * p : 0);
+        const float4* col = rope.angles + pos + ((d64 || d128) ? 8 * p : 0) * rope.n_pos;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          cs[j] = __ldg(reinterpret_cast<const float4*>(rope.cos_tab + o) + j);
-          sn[j] = __ldg(reinterpret_cast<const float4*>(rope.sin_tab + o) + j);
-        }
+        for (int t = 0; t < 8; ++t) ang[t] = __ldg(col + t * rope.n_pos);
       }
     }
     bool ok = mbar_wait(tfull_bar, 0, verr);
@@ -744,10 +737,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       if (EPI == EPI_ROPE && rotate) {
         auto rotate_all = [&](auto wide) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            rope_bf2<wide.value>(o[2 * j], o[8 + 2 * j], cs[j].x, cs[j].y, sn[j].x, sn[j].y);
-            rope_bf2<wide.value>(o[2 * j + 1], o[8 + 2 * j + 1], cs[j].z, cs[j].w, sn[j].z, sn[j].w);
-          }
+          for (int t = 0; t < 8; ++t) rope_bf2<wide.value>(o[t], o[8 + t], ang[t].x, ang[t].y, ang[t].z, ang[t].w);
         };
         if (BN == 128 && d128) rotate_all(std::true_type()); else rotate_all(std::false_type());
       }
