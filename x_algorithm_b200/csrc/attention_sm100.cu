@@ -149,7 +149,7 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
   const int q0 = ((int)blockIdx.x - (cand_tile ? a.hist_tiles : 0)) * QT;
   const int hk = h / (a.Hq / a.Hkv);
   const int qcol = q_column(h, a.q_head_stride, a.q_group, a.q_group_stride);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_hist = a.n_hist;
   const int n_blocks = (n_hist + KBLK - 1) / KBLK;
   volatile int* verr = a.err_flag;
@@ -167,7 +167,7 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, DCH * SLAB);
       for (int c = 0; c < DCH; ++c) tma_load_3d(sQ + c * SLAB, cand_tile ? &maps.qc : &maps.qh, q_full, qcol + c * 64, q0, b);
       auto load_k = [&](int j) {   // K block j into buffer j % NSB, once S of block j - NSB has been computed
@@ -189,7 +189,7 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc(QT, KBLK);
       constexpr uint32_t idesc_o = make_idesc_b_mn(QT, DH);
       mbar_wait(q_full, 0, verr);
@@ -389,7 +389,7 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     bar_sync_128();
-    if (warp == 2 && lane == 0) {
+    if (warp == 2 && elect_one()) {
       for (int c = 0; c < DCH; ++c) tma_store_3d(cand_tile ? &maps.oc : &maps.oh, sQ + c * SLAB, h * DH + c * 64, q0, b);
       asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -433,7 +433,7 @@ ranker_attention_resident_kernel(const __grid_constant__ CUtensorMap map_q, cons
 
   const int b = blockIdx.z, h = blockIdx.y;
   const int hk = h / (a.Hq / a.Hkv);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int T = a.T;
   const int n_hist = a.hist_len < T ? a.hist_len : T;
   const int n_tiles = (T + QT - 1) / QT;
@@ -452,7 +452,7 @@ ranker_attention_resident_kernel(const __grid_constant__ CUtensorMap map_q, cons
   const uint32_t tmem = *tmem_slot_ptr;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(kv_full, 2 * SLAB);
       tma_load_3d(sK, &map_k, kv_full, hk * a.k_head_stride, 0, b);
       tma_load_3d(sV, &map_v, kv_full, hk * a.v_head_stride, 0, b);
@@ -464,7 +464,7 @@ ranker_attention_resident_kernel(const __grid_constant__ CUtensorMap map_q, cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc(QT, KBLK);
       constexpr uint32_t idesc_o = make_idesc_b_mn(QT, DH);
       mbar_wait(kv_full, 0, verr);
@@ -729,7 +729,7 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
   uint32_t* mask_words = reinterpret_cast<uint32_t*>(smem_raw + (sMask - smem_u32(smem_raw)));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   volatile int* verr = a.err_flag;
   const int n_htiles = a.skip_hist ? 0 : (a.n_hist + QT - 1) / QT;      // 0 or 1
   const int n_ctiles = (a.n_cand + QT - 1) / QT;
@@ -763,7 +763,7 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int g = 0;
       for (int li = 0; li < my_items; ++li) {
         const int it = item_at(li);
@@ -793,7 +793,7 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc(QT, 128);
       constexpr uint32_t idesc_o = make_idesc_b_mn(QT, DH);
       auto issue_pv = [&](int gp, int kbp, bool last_of_item) {      // O[w] = P[w] V for tile gp, P from tensor memory
@@ -842,7 +842,7 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
     }
   } else if (warp == 10) {
     // ---------------- store warp: staged output rows -> global memory, then the stage goes back to the producer --------
-    if (lane == 0) {
+    if (elect_one()) {
       int li = 0, ti = first_tile(0);
       for (int g = 0; g < G; ++g, ++ti) {
         if (ti == nt) { ++li; ti = first_tile(li); }

@@ -150,7 +150,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const uint32_t tmem_slot = bars + 8u * (2 * cfg::STAGES + 4 + cfg::NSLAB);
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (counters && blockIdx.x == 0 && threadIdx.x == 0) counters[3] = globaltimer_ns();   // diagnostics: kernel entry
   constexpr int TILE_M = PAIR ? 2 * BM : BM;          // rows of one work tile (of the CTA pair)
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u; // 0 = the CTA that issues the pair's MMAs
@@ -187,7 +187,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       for (long long tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
@@ -225,7 +225,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // One thread, and the pipe only stays fed if this loop is short: the thread shares its scheduler with four
     // epilogue warps, so every instruction here costs several cycles of wall time.  Stage addresses and descriptors
     // are carried as running values (no per-step address arithmetic), the wait counters exist only when asked for.
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = make_idesc(TILE_M, BN);
       constexpr uint64_t DESC_STEP = (uint64_t)(cfg::STAGE_BYTES >> 4);    // descriptor address field: bytes / 16
       const uint64_t adesc0 = make_smem_desc(smem_base);
@@ -296,7 +296,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int gidx = ew >> 2;
     const int quad = warp & 3;                          // TMEM lane quadrant this warp may read
     const int row_in_tile = quad * 32 + lane;
-    const bool issuer = ((ew & 3) == 0 && lane == 0);
+    const bool issuer_warp = (ew & 3) == 0;             // one lane of it issues the group's copies
     const long long my_tiles = (total_tiles > first_tile) ? (total_tiles - first_tile + tile_step - 1) / tile_step : 0;
     // the accumulator-drained signal goes to the CTA that issues the MMAs
     const uint32_t tempty0 = PAIR ? mapa_shared(tempty_bar(0), 0) : tempty_bar(0);
@@ -321,7 +321,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       mbar_expect_tx(res_bar(gidx * NB + bi), SLAB_BYTES);
       tma_load_2d(gslab + bi * SLAB_BYTES, &map_r, res_bar(gidx * NB + bi), c1, (int)m1);
     };
-    if (RES && issuer) {
+    if (RES && issuer_warp && elect_one()) {
       for (int i = 0; i < DIST && i < my_items; ++i) issue_res(i);
     }
     float rstd = 1.0f;   // 1/rms of this thread's row, refreshed at each tile
@@ -377,7 +377,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         ang_col = rope.angles + rope_pos(rope, row + rope.row_offset, row < M);
         if (part_rotated(0)) load_angles(0);
       }
-      if (RES && issuer && i + DIST < my_items) {
+      if (RES && issuer_warp && i + DIST < my_items && elect_one()) {
         // the buffer of item i + DIST was last used by item i - 1: its store must have drained
         bulk_wait_read<0>();
         issue_res(i + DIST);
@@ -396,7 +396,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quad * 32) << 16) + s * ITEM_COLS;
       if (!RES) {
         // the store that last read this buffer (item i - NB of this group) must have drained before it is rewritten
-        if (issuer) bulk_wait_read<NB - 1>();
+        if (issuer_warp && elect_one()) bulk_wait_read<NB - 1>();
         ok = epi_barrier_and(ok, 1 + gidx);
       }
       if (ok) {
@@ -470,13 +470,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         fence_async_smem();
       }
       if (!epi_barrier_and(ok, 1 + gidx)) break;        // uniform over the group's 128 threads
-      if (issuer && c0 < N && m0 < M) {
+      if (issuer_warp && c0 < N && m0 < M && elect_one()) {
         tma_store_2d(&map_c, slab, c0, (int)m0);
         if (ITEM_SLABS == 2) tma_store_2d(&map_c, slab + SLAB_BYTES, c0 + SLAB_COLS, (int)m0);
         bulk_commit();
       }
     }
-    if (issuer) bulk_wait_all();
+    if (issuer_warp && elect_one()) bulk_wait_all();
   }
 
   // ---------------- teardown ----------------
@@ -611,7 +611,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const uint32_t tfull_bar = bars + 8u * (2 * cfg::STAGES);
   const uint32_t tmem_slot = tfull_bar + 8u;
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_tiles = (N + BN - 1) / BN;
   const int n0 = ((int)blockIdx.x % n_tiles) * BN;
   const long long m0 = (long long)((int)blockIdx.x / n_tiles) * BM;
@@ -634,7 +634,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     for (int c = 0; c < BN / 64; ++c) tma_load_2d(dst + c * 64 * BK * 2, &map_b, full_bar(stage), kb * BK, n0 + c * 64);
   };
   const int ahead = k_blocks < cfg::STAGES ? k_blocks : cfg::STAGES;
-  if (warp == 0 && lane == 0 && early_w) {
+  if (warp == 0 && early_w && elect_one()) {
     // weights that no kernel writes while forwards run need not wait for the kernel in front
     for (int kb = 0; kb < ahead; ++kb) { mbar_expect_tx(full_bar(kb), cfg::STAGE_BYTES); load_w(kb, kb); }
   }
@@ -642,7 +642,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0; uint32_t phase = 0;
       for (int kb = 0; kb < k_blocks; ++kb) {
         if (kb >= ahead || !early_w) {
@@ -655,7 +655,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(BM, BN);
       int stage = 0; uint32_t phase = 0;
       bool ok = true;

@@ -130,7 +130,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   float4* s_us2 = reinterpret_cast<float4*>(s_us_max + 8);   // [128] {scale, scale, -offset * scale, -offset * scale} of two queries
   uint4* s_queue = reinterpret_cast<uint4*>(smem_raw + (queue_smem - smem_u32(smem_raw)));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   volatile int* verr = err_flag;
   // work list: MODE 1 every tile; MODE 0 tiles 0, stride, 2*stride, ...
   const long long n_tiles = (a.rows + TC_ROWS - 1) / TC_ROWS;
@@ -178,7 +178,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   const uint32_t tmem_base = *tmem_slot_ptr;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(users_bar, users_bytes);
       for (int kb = 0; kb < kblk; ++kb)
         for (int q = 0; q < NQ; q += TC_QBOX) tma_load_2d(users_smem + (kb * NQ + q) * 128, &map_users, users_bar, kb * BK, q);
@@ -194,7 +194,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = I8 ? make_idesc_s8(TC_ROWS, NQ) : make_idesc(TC_ROWS, NQ);
       bool ok = mbar_wait(users_bar, 0, verr);
       int stage = 0; uint32_t phase = 0, it = 0;
