@@ -1,0 +1,62 @@
+"""The plain token build takes 1, 2, 4 or 8 tokens a warp by the call's size; with debug taps the general kernel builds the tokens,
+one a warp.  Same sums and roundings: the forwards agree bit for bit, at sizes that leave a partly filled warp, widths that leave
+a partly filled 256-column step, every hash count, and packed rows.  The tower's pooling with rows in shared memory and without
+against the oracle, and both heads kernels against each other."""
+import numpy as np
+import pytest
+
+from helpers import make_pair, rel_l2, to_inputs
+from oracle import phoenix_oracle as po
+
+pytestmark = pytest.mark.gpu
+TOL = 2e-2        # bf16 trunk against the oracle: the bound of the other parity tests
+
+
+@pytest.mark.parametrize("B,S,C,D,H,pack", [
+    (1, 9, 5, 128, 2, False), (3, 33, 40, 576, 1, False), (2, 33, 500, 1024, 4, False), (7, 33, 100, 320, 3, True),
+    (31, 33, 100, 128, 2, False), (31, 33, 100, 320, 4, True),                       # 4123 tokens: two a warp
+    (63, 33, 98, 576, 2, True), (63, 33, 98, 64, 3, False), (63, 33, 98, 256, 1, False),   # 8253: four
+    (251, 33, 98, 128, 2, False), (251, 33, 98, 192, 1, True), (251, 33, 98, 64, 4, False)])  # 32881: eight (four of 3-4 hashes)
+def test_tokens_a_warp(monkeypatch, B, S, C, D, H, pack):
+    kw = dict(max_batch=B, emb_size=D, num_layers=1, num_q_heads=2, num_kv_heads=2, key_size=32, history_len=S, num_candidates=C, num_hashes=H,
+              engine_kw=dict(pack_ragged=pack))
+    ocfg, w, rows_fn, eng = make_pair(**kw)
+    b = po.make_batch(ocfg, B, seed=5, ragged=True)
+    got = eng.rank(to_inputs(b))
+    eng.close()
+    monkeypatch.setenv("PHX_DEBUG_TAPS", "1")
+    _, _, _, eng = make_pair(**kw)
+    want = eng.rank(to_inputs(b))
+    eng.close()
+    np.testing.assert_array_equal(got.log_probs, want.log_probs)
+    np.testing.assert_array_equal(got.continuous, want.continuous)
+
+
+@pytest.mark.parametrize("S,D,B", [(140, 256, 3), (144, 256, 3), (33, 128, 5), (200, 256, 2)])   # 72 KB of rows and statistics: 143 x 256
+def test_pooling_keeps_rows_where_they_fit(S, D, B):
+    import torch
+    ocfg, w, rows_fn, eng = make_pair(max_batch=B, emb_size=D, num_candidates=0, history_len=S, num_layers=1)
+    b = po.make_batch(po.ModelConfig(history_len=S, num_candidates=1), B, seed=5, ragged=True)
+    want = po.user_tower(ocfg, w, rows_fn, b)
+    users = torch.empty((B, D), dtype=torch.float32, device="cuda")
+    dev = [torch.from_numpy(a).cuda() for a in (b.hist_post_ids, b.hist_author_ids, b.hist_actions, b.hist_surfaces)]
+    eng.user_tower_device(B, *dev, users)
+    eng.sync()
+    eng.close()
+    ok = b.hist_post_ids[:, 0] != 0
+    assert rel_l2(users.cpu().numpy()[ok], want[ok]) < TOL
+
+
+@pytest.mark.parametrize("D", [128, 1024])
+def test_heads_with_and_without_staged_rows(D):
+    """296 strips of 16 candidates take eight warps a strip with its rows in shared memory, 297 a warp a strip: the same bits."""
+    kw = dict(emb_size=D, num_layers=1, num_q_heads=2, num_kv_heads=2, key_size=64, history_len=9, num_candidates=16)
+    ocfg, w, rows_fn, eng = make_pair(max_batch=297, **kw)
+    b = po.make_batch(ocfg, 297, seed=5, ragged=True)
+    whole = eng.rank(to_inputs(b))
+    part = type(b)(*[np.ascontiguousarray(a[:296]) for a in (b.hist_post_ids, b.hist_author_ids, b.hist_actions, b.hist_surfaces,
+                                                            b.cand_post_ids, b.cand_author_ids)])
+    some = eng.rank(to_inputs(part))
+    eng.close()
+    np.testing.assert_array_equal(some.log_probs, whole.log_probs[:296])
+    np.testing.assert_array_equal(some.continuous, whole.continuous[:296])

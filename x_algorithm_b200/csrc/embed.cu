@@ -56,9 +56,8 @@ __device__ __forceinline__ void acc_chunk(float (&acc)[8], uint4 u) {
 
 // One warp per token.  History token slots: post h0.., author h0.., action row, surface row;
 // candidate token slots: post h0.., author h0...  x = bf16(bf16(sum) * input_scale).
-// GENERAL = false is the benchmark's path with the optional inputs and outputs compiled out (packed rows, pre-hashed
-// rows, landing buffer, projected tokens, action sets, fp32 rows, debug taps, rows-only): same arithmetic, fewer
-// instructions in a kernel that is bound by how many loads it keeps in flight.
+// This kernel carries every optional input and output (packed rows, pre-hashed rows, landing buffer, projected tokens, action
+// sets, fp32 rows, debug taps, rows-only); the plain build has its own below.
 // Continuous history actions (project_continuous_value_to_embedding, recsys_model.py:1850-1886).  Hidden activations
 // of every configured column for one token, gelu(norm(v) * w1), into hid[c][0..hidden): the warp's scratch.
 __device__ __forceinline__ void cont_hidden(const TokenBuildArgs& a, const float* __restrict__ vals, int lane, float (*hid)[64]) {
@@ -87,11 +86,10 @@ __device__ __forceinline__ void cont_add(const TokenBuildArgs& a, const float (*
   }
 }
 
-template <bool GENERAL>
-__global__ void __launch_bounds__(256, GENERAL ? 3 : 5) build_tokens_kernel(TokenBuildArgs a) {
+__global__ void __launch_bounds__(256, 3) build_tokens_kernel(TokenBuildArgs a) {
   // (no early launch signal here: the GEMM behind this kernel would park its CTAs - registers and all - on the SMs
   // while this bandwidth-bound kernel still needs every warp slot it can get)
-  __shared__ float hid_s[GENERAL ? 8 : 1][PHX_MAX_HIST_CONT][64];
+  __shared__ float hid_s[8][PHX_MAX_HIST_CONT][64];
   const int T = a.S + a.C;
   const long long tok = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -99,15 +97,15 @@ __global__ void __launch_bounds__(256, GENERAL ? 3 : 5) build_tokens_kernel(Toke
   // request and slot by 32-bit division (the launcher refuses B * T >= 2^31): a 64-bit '/' and '%' here cost more
   // instructions than the rest of the warp's prologue
   const int b = (int)((unsigned)tok / (unsigned)T), t = (int)((unsigned)tok - (unsigned)b * (unsigned)T);
-  const int P = GENERAL ? a.P : 0;
+  const int P = a.P;
   const bool is_front = t < a.S;              // rows in front of the candidates: user prefix + history
-  const bool is_user = GENERAL && t < P;
+  const bool is_user = t < P;
   const bool is_hist = is_front && !is_user;
   const int Sh = a.S - P;                     // history slots of the input arrays
   const int H = a.item.num_hashes;
   const long long slot = is_user ? (long long)b : is_hist ? (long long)b * Sh + (t - P) : (long long)b * a.C + (t - a.S);
   long long orow;   // where this token's row goes
-  if (GENERAL && a.pack.on() && !a.rows_only) {
+  if (a.pack.on() && !a.rows_only) {
     // packed rows: slots past the request's counts are not built at all (one token per warp: the whole warp leaves)
     if (is_front ? t >= a.pack.hist_cnt(b) : (t - a.S) >= a.pack.cand_cnt(b)) return;
     orow = is_front ? (long long)a.pack.hist_off[b] + t : a.pack.cand_base + a.pack.cand_off[b] + (t - a.S);
@@ -116,13 +114,13 @@ __global__ void __launch_bounds__(256, GENERAL ? 3 : 5) build_tokens_kernel(Toke
   }
   // lanes 0..H-1 hold the post rows, lanes H..2H-1 the author rows: hashed here, or taken as given; the user token
   // holds its user rows in lanes 0..Hu-1 and its IP rows behind them
-  const int n_ip = (GENERAL && a.user_ip_hashes) ? a.Hip : 0;
+  const int n_ip = (a.user_ip_hashes) ? a.Hip : 0;
   const int nrow = is_user ? a.Hu + n_ip : 2 * H;
   int my_idx = 0;
   if (is_user) {
     if (lane < a.Hu) my_idx = a.user_hashes[(long long)b * a.Hu + lane];
     else if (lane < nrow) my_idx = a.user_ip_hashes[(long long)b * a.Hip + (lane - a.Hu)];
-  } else if (GENERAL && a.pre_hist_post) {
+  } else if (a.pre_hist_post) {
     if (lane < H) my_idx = (is_hist ? a.pre_hist_post : a.pre_cand_post)[slot * H + lane];
     else if (lane < 2 * H) my_idx = (is_hist ? a.pre_hist_author : a.pre_cand_author)[slot * H + (lane - H)];
   } else {
@@ -134,41 +132,41 @@ __global__ void __launch_bounds__(256, GENERAL ? 3 : 5) build_tokens_kernel(Toke
       my_idx = hash_one(auth_id, a.author.scales[j], a.author.biases[j], a.author);
     }
   }
-  if (GENERAL && a.hashes && lane < 2 * H) a.hashes[tok * (2 * H) + lane] = my_idx;
-  if (GENERAL && a.rows_only) return;   // uniform over the grid: the caller only wants the rows (exchange outside the kernel)
+  if (a.hashes && lane < 2 * H) a.hashes[tok * (2 * H) + lane] = my_idx;
+  if (a.rows_only) return;   // uniform over the grid: the caller only wants the rows (exchange outside the kernel)
   const int first_hash = __shfl_sync(0xffffffffu, my_idx, 0);
   if (lane == 0) a.seg[orow] = (first_hash != 0) ? (is_front ? 1 : -1) : 0;
   int act = 0, srf = 0;
   if (is_hist) {
-    if (GENERAL && a.hist_actions_bool) {   // the action set as the batch-prep hands it over: one byte per flag
+    if (a.hist_actions_bool) {   // the action set as the batch-prep hands it over: one byte per flag
       const unsigned char* f = a.hist_actions_bool + slot * a.num_action_types;
       act = (int)__ballot_sync(0xffffffffu, lane < a.num_action_types && f[lane] != 0);
     } else {
       act = a.hist_actions[slot];
     }
     srf = a.hist_surfaces[slot];
-    if (!(GENERAL && a.action_multi_hot)) act = act < 0 ? 0 : (act > a.num_action_types ? a.num_action_types : act);
-  } else if (GENERAL && !is_front && a.cand_surfaces) {
+    if (!(a.action_multi_hot)) act = act < 0 ? 0 : (act > a.num_action_types ? a.num_action_types : act);
+  } else if (!is_front && a.cand_surfaces) {
     srf = a.cand_surfaces[slot];
   }
   srf = srf < 0 ? 0 : (srf > a.num_surfaces ? a.num_surfaces : srf);
-  const bool has_srf = is_hist || (GENERAL && !is_front && a.cand_surfaces);
-  const bool has_cont = GENERAL && is_hist && a.n_cont > 0;
-  float (*hid)[64] = hid_s[GENERAL ? (threadIdx.x >> 5) : 0];
+  const bool has_srf = is_hist || (!is_front && a.cand_surfaces);
+  const bool has_cont = is_hist && a.n_cont > 0;
+  float (*hid)[64] = hid_s[threadIdx.x >> 5];
   if (has_cont && !a.concat_hist) cont_hidden(a, a.hist_cont + slot * PHX_PREP_CONTINUOUS, lane, hid);
   // every lane takes part in these shuffles (lanes whose column chunk lies past D skip the loop below, so a
   // shuffle inside the loop would leave the warp split across two different shuffle instructions)
   const bf16* rowp[2 * PHX_MAX_HASHES];
   int my_pos = 0;   // exchanged rows: where slot `lane` of this token sits in the landing buffer
-  if (GENERAL && a.landing && lane < 2 * H) my_pos = a.pos[tok * (2 * H) + lane];
+  if (a.landing && lane < 2 * H) my_pos = a.pos[tok * (2 * H) + lane];
 #pragma unroll
   for (int j = 0; j < 2 * PHX_MAX_HASHES; ++j) {
     const int jj = j < nrow ? j : 0;
     const int idx = __shfl_sync(0xffffffffu, my_idx, jj);
     const int ps = __shfl_sync(0xffffffffu, my_pos, jj);
-    rowp[j] = (GENERAL && a.landing) ? a.landing + (long long)ps * a.D : a.table.row_ptr(idx, a.D);
+    rowp[j] = (a.landing) ? a.landing + (long long)ps * a.D : a.table.row_ptr(idx, a.D);
   }
-  if (GENERAL && a.concat_hist) {
+  if (a.concat_hist) {
     // projected tokens: the gathered rows side by side - post rows, author rows, then the action and surface rows
     // (history) or the surface row (candidates that carry one); the user rows alone for the user token - as one GEMM
     // operand row (recsys_model.py:1903-1918, 2190-2221, 2307-2329); the projection, the addends, the scaling and
@@ -181,7 +179,7 @@ __global__ void __launch_bounds__(256, GENERAL ? 3 : 5) build_tokens_kernel(Toke
       for (int j = 0; j < 2 * PHX_MAX_HASHES; ++j)
         if (j < ngat) *reinterpret_cast<uint4*>(dst + (long long)j * a.D + col) = __ldg(reinterpret_cast<const uint4*>(rowp[j] + col));
       if (is_hist)
-        *reinterpret_cast<uint4*>(dst + (long long)ngat * a.D + col) = action_chunk(a, act, col, GENERAL && a.action_multi_hot);
+        *reinterpret_cast<uint4*>(dst + (long long)ngat * a.D + col) = action_chunk(a, act, col, a.action_multi_hot);
       if (has_srf)
         *reinterpret_cast<uint4*>(dst + (long long)(nslot - 1) * a.D + col) =
             __ldg(reinterpret_cast<const uint4*>(a.surface_table + (long long)srf * a.D + col));
@@ -194,18 +192,18 @@ __global__ void __launch_bounds__(256, GENERAL ? 3 : 5) build_tokens_kernel(Toke
 #pragma unroll
     for (int j = 0; j < 2 * PHX_MAX_HASHES; ++j)
       if (j < nrow) acc_row(acc, rowp[j], col);
-    if (is_hist) acc_chunk(acc, action_chunk(a, act, col, GENERAL && a.action_multi_hot));
+    if (is_hist) acc_chunk(acc, action_chunk(a, act, col, a.action_multi_hot));
     if (has_srf) acc_row(acc, a.surface_table + (long long)srf * a.D, col);
     float tv[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) tv[i] = round_bf(acc[i]);
     if (has_cont) cont_add(a, hid, col, tv);
     uint4 o;
-    if (GENERAL && a.tokens) {
+    if (a.tokens) {
       o.x = pack_bf2(tv[0], tv[1]); o.y = pack_bf2(tv[2], tv[3]); o.z = pack_bf2(tv[4], tv[5]); o.w = pack_bf2(tv[6], tv[7]);
       *reinterpret_cast<uint4*>(a.tokens + tok * a.D + col) = o;
     }
-    if (GENERAL && a.x32) {   // full-precision path: the token is the bf16 sum, its scaled value stays fp32
+    if (a.x32) {   // full-precision path: the token is the bf16 sum, its scaled value stays fp32
       float* dst = a.x32 + orow * a.D + col;
 #pragma unroll
       for (int i = 0; i < 8; ++i) dst[i] = tv[i] * a.input_scale;
@@ -222,6 +220,124 @@ __global__ void __launch_bounds__(256, GENERAL ? 3 : 5) build_tokens_kernel(Toke
     for (int o = 16; o > 0; o >>= 1) row_ss += __shfl_xor_sync(0xffffffffu, row_ss, o);
     if (lane < a.ss_slots) a.row_ss[orow * a.ss_slots + lane] = (lane == 0) ? row_ss : 0.f;
   }
+}
+
+// The plain token build (ids in, bf16 rows out; packed rows or not) for calls of many tokens.  The kernel above spends most of its
+// instructions on the hash of one token - 64-bit multiplications and remainders on 2H lanes while the others wait - and
+// on its prologue.  Here a warp takes TPW tokens: lane l hashes slot l % SL of token l / SL (SL = 2H rounded up to a power of
+// two), then the warp walks over (token, 256 columns) pairs, the rows of two pairs in flight.  Same order of additions and
+// roundings: the same bits.  Kernel,
+// one token a warp / this one: 640 tokens of 512 columns 7.7 / 5.6 us, 10240: 19.9 / 13.7, 81920: 103.5 / 56.9 (419 MB of
+// rows, ids and results: HBM); 32768 of 256 columns 35.8 / 22.1; a ragged batch of 48 packed requests 44.6 / 20.9.
+template <int SL, int TPW>
+__global__ void __launch_bounds__(256, SL == 8 ? 2 : 3) build_tokens_bulk_kernel(TokenBuildArgs a) {
+  static_assert(SL * TPW <= 32, "a lane per hash");
+  const int lane = threadIdx.x & 31, H = a.item.num_hashes;
+  const unsigned T = (unsigned)(a.S + a.C), n_tok = (unsigned)a.B * T;      // the launcher refuses B * T >= 2^31
+  const unsigned tok0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * TPW;
+  if (tok0 >= n_tok) return;
+  // ---- lane (k, slot): token k's facts and one of its hashes ----
+  const int slot = lane % SL;
+  const unsigned tok = tok0 + lane / SL;
+  int orow = -1, aux = 0;            // where the token's row goes (-1: nowhere); its action (slot 0) and surface (slot 1)
+  bool front = false;
+  unsigned long long rowp = reinterpret_cast<unsigned long long>(a.table.base[0]);
+  if (lane < SL * TPW && tok < n_tok) {
+    const unsigned b = tok / T, t = tok - b * T;
+    front = t < (unsigned)a.S;
+    if (!a.pack.on()) orow = (int)token_row(a.split, a.B, a.S, (int)T, (int)b, (int)t);
+    else if (front) orow = (int)t < a.pack.hist_cnt(b) ? a.pack.hist_off[b] + (int)t : -1;
+    else orow = (int)(t - a.S) < a.pack.cand_cnt(b) ? (int)a.pack.cand_base + a.pack.cand_off[b] + (int)(t - a.S) : -1;
+    if (orow >= 0) {
+      const long long s = front ? (long long)b * a.S + t : (long long)b * a.C + (t - a.S);
+      int idx = 0;
+      if (slot < 2 * H) {
+        const bool post = slot < H;
+        const HashFamilyDev& f = post ? a.item : a.author;
+        const long long id = __ldg((post ? (front ? a.hist_post : a.cand_post) : (front ? a.hist_author : a.cand_author)) + s);
+        const int j = post ? slot : slot - H;
+        idx = hash_one(id, f.scales[j], f.biases[j], f);
+        rowp = reinterpret_cast<unsigned long long>(a.table.row_ptr(idx, a.D));
+      }
+      if (slot == 0) a.seg[orow] = idx != 0 ? (front ? 1 : -1) : 0;
+      if (front && slot < 2) {
+        aux = __ldg((slot == 0 ? a.hist_actions : a.hist_surfaces) + s);
+        const int top = slot == 0 ? a.num_action_types : a.num_surfaces;
+        aux = aux < 0 ? 0 : (aux > top ? top : aux);
+      }
+    }
+  }
+  __syncwarp();
+  // ---- (token, 256 columns) pairs, two at a time; `on` and `hist` are uniform over the warp ----
+  struct Pair { uint4 r[SL + 2]; int row; bool on, hist; };
+  auto request = [&](int k, int col, bool there, Pair& p) {
+    const int l0 = (k * SL) & 31;
+    p.row = __shfl_sync(0xffffffffu, orow, l0);
+    p.on = there && p.row >= 0;
+    p.hist = __shfl_sync(0xffffffffu, (int)front, l0) != 0;
+    const int act = __shfl_sync(0xffffffffu, aux, l0), srf = __shfl_sync(0xffffffffu, aux, l0 + 1);
+#pragma unroll
+    for (int j = 0; j < SL; ++j) {
+      const bf16* src = reinterpret_cast<const bf16*>(__shfl_sync(0xffffffffu, rowp, l0 + j));
+      if (p.on && j < 2 * H && col < a.D) p.r[j] = __ldg(reinterpret_cast<const uint4*>(src + col));
+    }
+    if (p.on && p.hist && col < a.D) {
+      p.r[SL] = __ldg(reinterpret_cast<const uint4*>(a.action_table + (long long)act * a.D + col));
+      p.r[SL + 1] = __ldg(reinterpret_cast<const uint4*>(a.surface_table + (long long)srf * a.D + col));
+    }
+  };
+  auto add = [](float2 (&acc)[4], const uint4& u) {
+    acc[0] = __fadd2_rn(acc[0], unpack_bf2(u.x)); acc[1] = __fadd2_rn(acc[1], unpack_bf2(u.y));
+    acc[2] = __fadd2_rn(acc[2], unpack_bf2(u.z)); acc[3] = __fadd2_rn(acc[3], unpack_bf2(u.w));
+  };
+  float row_ss = 0.f;
+  const float2 scale = make_float2(a.input_scale, a.input_scale);
+  auto finish = [&](int col, bool first, bool last, const Pair& p) {
+    if (!p.on) return;
+    if (first) row_ss = 0.f;
+    if (col < a.D) {
+      float2 acc[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+      for (int j = 0; j < SL; ++j)
+        if (j < 2 * H) add(acc, p.r[j]);
+      if (p.hist) { add(acc, p.r[SL]); add(acc, p.r[SL + 1]); }
+      uint32_t o[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {       // the token is rounded, then scaled and rounded again
+        const float2 s = __fmul2_rn(unpack_bf2(pack_bf2(acc[i].x, acc[i].y)), scale);
+        o[i] = pack_bf2(s.x, s.y);
+        const float2 v = unpack_bf2(o[i]);
+        row_ss += v.x * v.x; row_ss += v.y * v.y;
+      }
+      *reinterpret_cast<uint4*>(a.x + (long long)p.row * a.D + col) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    if (last && a.row_ss) {               // statistics of the bf16 row for the first fused RMSNorm
+      float ss = row_ss;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (lane < a.ss_slots) a.row_ss[(long long)p.row * a.ss_slots + lane] = (lane == 0) ? ss : 0.f;
+    }
+  };
+  const int span = (a.D + 255) & ~255;    // columns of a token's walk
+  int k0 = 0, c0 = 0;
+  while (k0 < TPW) {
+    int k1 = k0, c1 = c0 + 256;
+    if (c1 == span) { c1 = 0; ++k1; }
+    Pair p0, p1;
+    request(k0, c0 + lane * 8, true, p0);
+    request(k1, c1 + lane * 8, k1 < TPW, p1);
+    finish(c0 + lane * 8, c0 == 0, c0 + 256 == span, p0);
+    finish(c1 + lane * 8, c1 == 0, c1 + 256 == span, p1);
+    k0 = k1; c0 = c1 + 256;
+    if (c0 == span) { c0 = 0; ++k0; }
+  }
+}
+template <int TPW>
+void build_tokens_bulk(const TokenBuildArgs& a, long long toks, cudaStream_t stream) {
+  const unsigned grid = (unsigned)((toks + 8 * TPW - 1) / (8 * TPW));
+  if (a.item.num_hashes == 1) build_tokens_bulk_kernel<2, TPW><<<grid, 256, 0, stream>>>(a);
+  else if (a.item.num_hashes == 2) build_tokens_bulk_kernel<4, TPW><<<grid, 256, 0, stream>>>(a);
+  else if constexpr (TPW <= 4) build_tokens_bulk_kernel<8, TPW><<<grid, 256, 0, stream>>>(a);
 }
 
 // Projected tokens, last step: x = bf16(token * input_scale) at the token's row of the residual stream (plain or
@@ -476,6 +592,14 @@ __global__ void corpus_fill_kernel(bf16* rows_ptr, long long global_row0, long l
 
 }  // namespace
 
+namespace {
+// Tokens a warp of the plain build takes.  Few tokens want a warp each (every warp is one round trip for ids and one for rows), many
+// want the hash shared.  1 / 2 / 4 / 8 tokens, us (2 hashes): D = 512: 2560 tokens 6.0 / 6.7 / 8.3 / 12.4, 5120: 8.8 / 8.4 / 9.5 /
+// 13.6, 10240: 15.5 / 14.4 / 13.9 / 18.4, 20480: 25.9 / 21.3 / 21.3 / 21.8, 81920: 88 / 70 / 61 / 57; D = 256: 2048: 4.7 / 4.7 / 6.0 /
+// 8.3, 8192: 11.0 / 9.8 / 7.7 / 9.3, 32768: 36.7 / 25.8 / 22.3 / 21.9; D = 1024: 8688: 21.1 / 21.3 / 19.8 / 28.0.
+inline int tokens_per_warp(long long toks) { return toks < 4096 ? 1 : toks < 8192 ? 2 : toks < 32768 ? 4 : 8; }
+}  // namespace
+
 phx_status build_tokens_launch(const TokenBuildArgs& a, cudaStream_t stream, std::string& err) {
   if (a.D % 8 != 0 || a.item.num_hashes != a.author.num_hashes || 2 * a.item.num_hashes > 32) {
     err = "build_tokens: D must be a multiple of 8 and hash counts must match";
@@ -485,12 +609,18 @@ phx_status build_tokens_launch(const TokenBuildArgs& a, cudaStream_t stream, std
   if (toks == 0) return PHX_OK;
   if (toks >= (1ll << 31)) { err = "build_tokens: more than 2^31 tokens in one call"; return PHX_E_CAPACITY; }
   const int warps = 8;
-  const bool general = a.pack.hist_off || a.pre_hist_post || a.landing || a.concat_hist || a.action_multi_hot || a.x32 ||
-                       a.tokens || a.hashes || a.rows_only || a.P || a.hist_actions_bool || a.cand_surfaces || a.n_cont;
   if (a.P && (a.Hu <= 0 || a.Hu + a.Hip > 2 * PHX_MAX_HASHES || !a.user_hashes)) { err = "build_tokens: user-prefix arguments"; return PHX_E_ARG; }
   if (a.n_cont && (a.cont_hidden <= 0 || a.cont_hidden > 64 || !a.hist_cont)) { err = "build_tokens: continuous-action arguments"; return PHX_E_ARG; }
-  if (general) build_tokens_kernel<true><<<(unsigned)((toks + warps - 1) / warps), warps * 32, 0, stream>>>(a);
-  else build_tokens_kernel<false><<<(unsigned)((toks + warps - 1) / warps), warps * 32, 0, stream>>>(a);
+  const bool plain = !(a.pre_hist_post || a.landing || a.concat_hist || a.action_multi_hot || a.x32 || a.tokens || a.hashes || a.rows_only ||
+                       a.P || a.hist_actions_bool || a.cand_surfaces || a.n_cont);
+  const int H = a.item.num_hashes;
+  int tpw = plain && H <= 4 ? tokens_per_warp(toks) : 0;
+  if (tpw == 8 && H > 2) tpw = 4;        // 2H lanes a token
+  if (tpw == 8) build_tokens_bulk<8>(a, toks, stream);
+  else if (tpw == 4) build_tokens_bulk<4>(a, toks, stream);
+  else if (tpw == 2) build_tokens_bulk<2>(a, toks, stream);
+  else if (tpw == 1) build_tokens_bulk<1>(a, toks, stream);
+  else build_tokens_kernel<<<(unsigned)((toks + warps - 1) / warps), warps * 32, 0, stream>>>(a);
   PHX_CUDA_TRY(cudaGetLastError(), err);
   return PHX_OK;
 }
