@@ -18,6 +18,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 constexpr int MAX_OUT = 32;  // V + NC
+constexpr size_t POOL_SMEM = 72 * 1024;   // three CTAs of the pooling kernel an SM
 
 __global__ void __launch_bounds__(256) heads_kernel(HeadsArgs a) {
   extern __shared__ __align__(16) uint8_t hsm[];
@@ -125,9 +126,10 @@ __device__ __forceinline__ void mma_bf16_16816_h(float (&c)[4], const uint32_t (
 }
 
 // NT: n-tiles of 8 outputs, V + NC <= 8 * NT.  WPS: warps per strip.  With enough strips every warp has its own (1); a small call
-// is one strip's chain of latencies, most of it the ten rounds of logarithms and f64 exponentials, so four warps form the
-// same sums and share the (row, output) items of one strip.  Same arithmetic, same bits.  Kernel at D = 512, 20 outputs: 512 rows
-// 21.0 -> 18.9 us, 1024 and 2048 rows 23.0 -> 18.9, 4608 rows 23.0 -> 20.9, from 4736 rows (296 strips) on level at 23.0.
+// is one strip's chain of latencies - round trips to its rows, then rounds of logarithms and f64 exponentials - so eight warps
+// fetch the strip's rows into shared memory in one go, form the same sums and share the (row, output) items.  Same arithmetic,
+// same bits.  Kernel at 20 outputs, parameters not yet staged (one warp / eight): D = 512: 512 to 2048 rows 18.5 / 11.5 us, 4096
+// rows 18.7 / 14.9, 8192 rows 20.4 / 27.2; D = 1024: 512 rows 29.0 / 18.3, 4800 rows 28.3 / 38.3; D = 128: 128 rows 12.7 / 6.6.
 template <int NT, int WPS>
 __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_kernel(HeadsArgs a) {
   constexpr int WARPS = WPS == 1 ? HM_WARPS : WPS;      // warps per CTA
@@ -137,8 +139,10 @@ __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_ke
   float* sgain = reinterpret_cast<float*>(sw + NT * 8 * WLD);                // [D]
   float* sC_all = sgain + D;                                                 // per warp [16][NT*8] fp32 sums
   double* sD_all = reinterpret_cast<double*>(sC_all + WARPS * 16 * NT * 8);   // per strip [16][NT*8] blend inputs
+  bf16* sX = reinterpret_cast<bf16*>(sD_all + (WPS == 1 ? HM_WARPS : 1) * 16 * NT * 8);   // WPS > 1: [16][WLD] the strip's rows
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-  for (int i = threadIdx.x; i < NT * 8 * (D / 8); i += blockDim.x) {
+#pragma unroll 4
+  for (int i = threadIdx.x; i < NT * 8 * (D / 8); i += WARPS * 32) {
     const int n = i / (D / 8), ch = i % (D / 8);
     uint4 w = make_uint4(0u, 0u, 0u, 0u);
     if (n < NO) w = *reinterpret_cast<const uint4*>(a.unembed_t + (long long)n * D + ch * 8);
@@ -159,11 +163,27 @@ __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_ke
   for (long long strip = (long long)blockIdx.x * CTA_STRIPS + (WPS == 1 ? warp : 0); strip < n_strips; strip += (long long)gridDim.x * CTA_STRIPS) {
     const long long r0 = strip * 16;
     const bf16* xr[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      long long r = r0 + g + 8 * i;
+    auto row_of = [&](int i) {
+      long long r = r0 + i;
       if (r >= nrows) r = nrows - 1;
-      xr[i] = (a.out_index ? a.x + r * (long long)D : a.x + ((r / a.C) * a.T + a.S + (r % a.C)) * (long long)D) + 8 * t4;
+      if (a.out_index) return a.x + r * (long long)D;
+      const unsigned b = (unsigned)r / (unsigned)a.C, c = (unsigned)r - b * (unsigned)a.C;     // rows fit 31 bits
+      return a.x + ((long long)b * a.T + a.S + c) * (long long)D;
+    };
+    if (WPS == 1) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) xr[i] = row_of(g + 8 * i) + 8 * t4;
+    } else {
+      // one round trip for the whole strip instead of one per 32 columns and pass
+      const int per_row = D / 8;
+#pragma unroll 8
+      for (int i = threadIdx.x; i < 16 * per_row; i += WARPS * 32) {
+        const int rr = i / per_row, ch = i - rr * per_row;
+        *reinterpret_cast<uint4*>(sX + rr * WLD + ch * 8) = *reinterpret_cast<const uint4*>(row_of(rr) + ch * 8);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 2; ++i) xr[i] = sX + (g + 8 * i) * WLD + 8 * t4;
     }
     // pass 1: sums of squares (a row's 32-column groups are spread over the 4 lanes of its quad)
     float ss[2] = {0.f, 0.f};
@@ -187,6 +207,7 @@ __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_ke
     float acc[NT][4];
 #pragma unroll
     for (int j = 0; j < NT; ++j) { acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f; }
+#pragma unroll 4
     for (int gr = 0; gr < groups; ++gr) {
       const float4 ga = *reinterpret_cast<const float4*>(sgain + gr * 32 + 8 * t4);
       const float4 gb = *reinterpret_cast<const float4*>(sgain + gr * 32 + 8 * t4 + 4);
@@ -241,6 +262,7 @@ __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_ke
     if (WPS == 1) __syncwarp(); else __syncthreads();
     if (a.has_blend && a.scores && part == 0 && lane < 16 && r0 + lane < nrows) {
       double s = 0.0;   // terms summed left to right in f64
+#pragma unroll 4
       for (int i = 0; i < a.blend.num_terms; ++i) s = s + sD[lane * (NT * 8) + a.blend.src[i]] * a.blend.weight[i];
       double out;
       if (a.blend.total_sum == 0.0) out = s > 0.0 ? s : 0.0;
@@ -256,7 +278,8 @@ template <int NT, int WPS>
 phx_status launch_heads_wps(const HeadsArgs& a, long long strips, cudaStream_t stream, std::string& err) {
   constexpr int WARPS = WPS == 1 ? HM_WARPS : WPS;
   const size_t smem = (size_t)NT * 8 * (a.D + HM_WPAD) * sizeof(bf16) + (size_t)a.D * sizeof(float) +
-                      (size_t)16 * NT * 8 * (WARPS * sizeof(float) + (WPS == 1 ? HM_WARPS : 1) * sizeof(double));
+                      (size_t)16 * NT * 8 * (WARPS * sizeof(float) + (WPS == 1 ? HM_WARPS : 1) * sizeof(double)) +
+                      (WPS == 1 ? 0 : (size_t)16 * (a.D + HM_WPAD) * sizeof(bf16));
   if (smem > 200 * 1024) { err = "heads: head matrix does not fit shared memory"; return PHX_E_CAPACITY; }
   static SmemLimit limit;
   PHX_CUDA_TRY(limit.raise(heads_mma_kernel<NT, WPS>, 200 * 1024), err);
@@ -277,42 +300,76 @@ phx_status launch_heads_wps(const HeadsArgs& a, long long strips, cudaStream_t s
 }
 template <int NT>
 phx_status launch_heads_mma(const HeadsArgs& a, long long rows, cudaStream_t stream, std::string& err) {
-  // up to two CTAs of a strip each per SM: there and beyond the strips alone keep the SMs busy (level at 296 strips)
+  // up to two CTAs of a strip each per SM; a third round of them costs more than a warp a strip (measured beside the kernel)
   const long long strips = (rows + 15) / 16;
-  if (strips <= 2 * 148) return launch_heads_wps<NT, 4>(a, strips, stream, err);
+  if (strips <= 2 * 148) return launch_heads_wps<NT, 8>(a, strips, stream, err);
   return launch_heads_wps<NT, 1>(a, strips, stream, err);
 }
 
-// users[b] = l2norm(mean over valid t of final_norm(x[b,t])), fp32; one CTA per user, one thread per column
-template <bool F32>   // F32: fp32 rows, nothing rounded (the full-precision path)
+// users[b] = l2norm(mean over valid t of final_norm(x[b,t])), fp32; one CTA per user, one thread per column.  Two passes
+// over the user's rows (row statistics, then the mean): a chain of latencies, so the rows are fetched once, all loads in
+// flight together, and kept in shared memory (STAGED) where they fit beside those of two more CTAs.
+// 128 rows of 256 columns: one user 20.0 -> 11.8 us, 256 users 24.3 -> 17.1.
+template <bool F32, bool STAGED>   // F32: fp32 rows, nothing rounded (the full-precision path)
 __global__ void tower_pool_kernel(const void* __restrict__ xv, const float* __restrict__ gain, const int* __restrict__ seg,
                                   int T, int D, float eps, float* __restrict__ users) {
-  auto ld = [&](long long i) { return F32 ? reinterpret_cast<const float*>(xv)[i] : bf2f(reinterpret_cast<const bf16*>(xv)[i]); };
-  extern __shared__ float psm[];  // [T] rstd (0 for invalid) + reduction scratch
-  float* rstd = psm;
-  float* red = psm + T;
+  extern __shared__ __align__(16) float psm[];  // STAGED: [T][D] rows; [T] rstd (0 for invalid) + reduction scratch
   const int b = blockIdx.x;
+  const char* rows = reinterpret_cast<const char*>(xv) + (long long)b * T * D * (F32 ? 4 : 2);
+  float* rstd = psm;
+  if (STAGED) {
+    const int n = T * D * (F32 ? 4 : 2) / 16;    // 16-byte units
+    rstd = psm + n * 4;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < n; i += blockDim.x) reinterpret_cast<uint4*>(psm)[i] = reinterpret_cast<const uint4*>(rows)[i];
+    rows = reinterpret_cast<const char*>(psm);
+    __syncthreads();
+  }
+  auto ld = [&](long long i) { return F32 ? reinterpret_cast<const float*>(rows)[i] : bf2f(reinterpret_cast<const bf16*>(rows)[i]); };
+  float* red = rstd + T;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int t = warp; t < T; t += nw) {
-    const long long r0 = ((long long)b * T + t) * D;
-    float ss = 0.f;
-    for (int k = lane; k < D; k += 32) { float v = ld(r0 + k); ss += v * v; }
-    ss = warp_sum(ss);
-    if (lane == 0) rstd[t] = (seg[(long long)b * T + t] != 0) ? (F32 ? 1.0f / sqrtf(ss / (float)D + eps) : rsqrtf(ss / (float)D + eps)) : 0.f;
+  // Both passes keep several rows' loads in flight; the order of every sum is that of one row after the other
+  constexpr int RU = 4;
+  for (int t0 = warp * RU; t0 < T; t0 += nw * RU) {
+    float ss[RU] = {0.f, 0.f, 0.f, 0.f};
+    int ok[RU];
+#pragma unroll
+    for (int i = 0; i < RU; ++i) ok[i] = t0 + i < T ? seg[(long long)b * T + t0 + i] : 0;
+    const long long r0 = (long long)t0 * D;
+#pragma unroll 4
+    for (int k = lane; k < D; k += 32) {
+#pragma unroll
+      for (int i = 0; i < RU; ++i) {
+        const float v = t0 + i < T ? ld(r0 + (long long)i * D + k) : 0.f;
+        ss[i] += v * v;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < RU; ++i) {
+      const float s = warp_sum(ss[i]);
+      if (lane == 0 && t0 + i < T) rstd[t0 + i] = ok[i] != 0 ? (F32 ? 1.0f / sqrtf(s / (float)D + eps) : rsqrtf(s / (float)D + eps)) : 0.f;
+    }
   }
   __syncthreads();
-  float cnt = 0.f;
-  for (int t = 0; t < T; ++t) cnt += (rstd[t] != 0.f) ? 1.f : 0.f;
+  float cnt = 0.f;     // whole numbers: exact in any order
+  for (int t = lane; t < T; t += 32) cnt += (rstd[t] != 0.f) ? 1.f : 0.f;
+  cnt = warp_sum(cnt);
   float sq = 0.f;
   float vals[8];  // D <= 8 * blockDim.x
   int nv = 0;
   for (int k = threadIdx.x; k < D; k += blockDim.x, ++nv) {
     float acc = 0.f;
     const float gk = gain[k];
-    for (int t = 0; t < T; ++t) {  // fixed order over positions
-      if (rstd[t] != 0.f) {
-        const float v = ld(((long long)b * T + t) * D + k) * rstd[t] * gk;
-        acc = acc + (F32 ? v : round_bf(v));
+    constexpr int TU = 16;
+    for (int t0 = 0; t0 < T; t0 += TU) {  // fixed order over positions
+      float x[TU];
+#pragma unroll
+      for (int i = 0; i < TU; ++i) x[i] = t0 + i < T ? ld((long long)(t0 + i) * D + k) : 0.f;
+#pragma unroll
+      for (int i = 0; i < TU; ++i) {
+        const float rs = t0 + i < T ? rstd[t0 + i] : 0.f;
+        const float v = x[i] * rs * gk;
+        if (rs != 0.f) acc = acc + (F32 ? v : round_bf(v));
       }
     }
     const float rep = acc / fmaxf(cnt, 1.0f);
@@ -362,9 +419,21 @@ phx_status tower_pool_launch(const void* x, const float* final_gain, const int* 
   if (B == 0) return PHX_OK;
   int threads = 256;
   if (D > 8 * threads) { err = "tower_pool: D too large"; return PHX_E_CAPACITY; }
-  const size_t smem = (size_t)(T + 32) * sizeof(float);
-  if (x_is_f32) tower_pool_kernel<true><<<B, threads, smem, stream>>>(x, final_gain, seg, T, D, eps, users);
-  else tower_pool_kernel<false><<<B, threads, smem, stream>>>(x, final_gain, seg, T, D, eps, users);
+  const size_t small = (size_t)(T + 32) * sizeof(float), rows = (size_t)T * D * (x_is_f32 ? 4 : 2);
+  const bool staged = rows % 16 == 0 && small + rows <= POOL_SMEM;
+  const size_t smem = small + (staged ? rows : 0);
+  static SmemLimit limit_bf16, limit_f32;
+  if (staged && x_is_f32) {
+    PHX_CUDA_TRY(limit_f32.raise(tower_pool_kernel<true, true>, (int)POOL_SMEM), err);
+    tower_pool_kernel<true, true><<<B, threads, smem, stream>>>(x, final_gain, seg, T, D, eps, users);
+  } else if (staged) {
+    PHX_CUDA_TRY(limit_bf16.raise(tower_pool_kernel<false, true>, (int)POOL_SMEM), err);
+    tower_pool_kernel<false, true><<<B, threads, smem, stream>>>(x, final_gain, seg, T, D, eps, users);
+  } else if (x_is_f32) {
+    tower_pool_kernel<true, false><<<B, threads, smem, stream>>>(x, final_gain, seg, T, D, eps, users);
+  } else {
+    tower_pool_kernel<false, false><<<B, threads, smem, stream>>>(x, final_gain, seg, T, D, eps, users);
+  }
   PHX_CUDA_TRY(cudaGetLastError(), err);
   return PHX_OK;
 }
