@@ -120,3 +120,28 @@ def test_masked_rows_stand_in_front_of_minus_infinity():
         order = np.argsort(-scores[b])
         assert list(i[b]) == [[7, 2000, 2999][o] for o in order] + [0, 1, 2, 3, 4] + [1234]
         assert np.all(s[b, 3:8] == lowest) and s[b, 8] == -np.inf
+
+
+@pytest.mark.parametrize("N,B,k", [(3_000_000, 1, 1), (3_000_000, 1, 900), (400_000, 256, 3), (400_000, 16, 10), (70_000, 3, 1)])
+@pytest.mark.parametrize("int8", [False, True])
+def test_sampled_pivot_of_short_lists(N, B, k, int8):
+    """How many rows the pivot lets through follows the corpus and the batch, not k alone: the lists equal those of the exact
+    passes, and no call had to be done again."""
+    from x_algorithm_b200.retrieval import CorpusShard
+    sh = CorpusShard(N, 128, max_queries=B, max_k=k)
+    sh.fill_synthetic(4)
+    if int8:
+        sh.quantize_int8()
+        sh.set_int8(True)
+    users = _users(B, 128, 6)
+    got_s, got_i = _topk(sh, users, k)
+    assert sh.exact_runs() == 0
+    sh.set_exact(True)
+    want_s, want_i = _topk(sh, users, k)
+    sh.close()
+    if int8:                                       # integer sums: the same bits
+        np.testing.assert_array_equal(got_i, want_i)
+        np.testing.assert_array_equal(got_s, want_s)
+    else:                                          # the two scans sum in another order: a bf16 step at a rounding edge
+        np.testing.assert_allclose(got_s, want_s, rtol=2.0 ** -7)
+        assert (got_i == want_i).mean() > 0.9

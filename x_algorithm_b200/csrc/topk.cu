@@ -4,7 +4,7 @@
 //
 //   1. sample pass   every `stride`-th 64-row tile is scored; per user and 16-row group the maximum
 //                    score is kept; the pivot of a user is the j-th largest group maximum, with j
-//                    chosen so that about 3k corpus rows are expected at or above it
+//                    chosen so that about 3k corpus rows (more for short lists) are expected at or above it
 //   2. collect pass  the whole shard is scored once (corpus read once from HBM, scores live only in
 //                    registers); rows with bf16(score) >= pivot are appended to the user's survivor
 //                    list as 64-bit keys  ordered(score) << 32 | ~global_row
@@ -877,8 +877,13 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
   int j = 0;
   // a window whose eligible rows all fit the survivor buffer needs no pivot: every eligible row is collected
   if (rows > c->cap && !(c->mask && c->elig_count <= c->cap)) {
-    // sample every stride-th tile so that about 48 of the wanted ~3k rows fall into the sample
-    const double want = 3.0 * k_real;
+    // Rows wanted at or above the pivot: 3k, and for short lists as many as keep the sample small.  Every stride-th tile is sampled
+    // so that about 48 of them fall into the sample: with 3k alone a list of 10 had every tile scored twice.  A wanted row
+    // costs about 0.14 ns a query in the collect pass and the select, a sampled tile as much as a collected one: the sum is
+    // smallest at sqrt(17.5 rows / queries).  Whole calls, 3k rows / this rule: 256 queries, 12.5 M rows, k = 10 1393 -> 739 us,
+    // k = 100 911 -> 752; one query 1170 -> 542; 3 M rows, k = 10 574 -> 262; 700 k rows, 16 queries 160 -> 125.
+    const double balanced = sqrt(17.5 * (double)rows / (double)B);
+    const double want = fmax(3.0 * k_real, fmin(3000.0, balanced));
     long long stride = (long long)(want / 48.0);
     if (stride < 1) stride = 1;
     long long sampled_tiles = (n_tiles + stride - 1) / stride;
