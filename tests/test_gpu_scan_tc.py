@@ -145,3 +145,31 @@ def test_sampled_pivot_of_short_lists(N, B, k, int8):
     else:                                          # the two scans sum in another order: a bf16 step at a rounding edge
         np.testing.assert_allclose(got_s, want_s, rtol=2.0 ** -7)
         assert (got_i == want_i).mean() > 0.9
+
+
+@pytest.mark.parametrize("dim", [128, 256])
+@pytest.mark.parametrize("kind", ["far_apart", "large_sums", "one_scale", "all_below_zero"])
+def test_int8_threshold_in_the_sum(dim, kind):
+    """Corpora whose thresholds the bias of the int8 sum cannot express, or only coarsely - row scales over six decades, dot products
+    beyond its range, sums below zero throughout - and the plain one: lists and scores equal the oracle's, without an exact re-run."""
+    from x_algorithm_b200.retrieval import CorpusShard
+    N, B, k = 40001, 70, 25
+    r = np.random.default_rng(dim)
+    scales = np.full(N, 0.01, np.float32)
+    if kind == "far_apart":
+        scales = (10.0 ** r.uniform(-6, 0, N)).astype(np.float32)
+    users = _users(B, dim, 3)
+    if kind in ("large_sums", "all_below_zero"):
+        q8 = r.integers(60, 128, size=(N, dim), dtype=np.int8)
+        users = np.abs(users) if kind == "large_sums" else -np.abs(users)
+    else:
+        q8 = r.integers(-127, 128, size=(N, dim), dtype=np.int8)
+    sh = CorpusShard(N, dim, max_queries=B, max_k=k)
+    sh.upload_int8(0, q8, scales)
+    sh.set_int8(True)
+    got_s, got_i = _topk(sh, users, k)
+    assert sh.exact_runs() == 0
+    want_s, want_i = po.top_k(po.int8_corpus_scores(users, q8, scales), k)
+    sh.close()
+    np.testing.assert_array_equal(got_i, want_i)
+    np.testing.assert_array_equal(got_s, want_s)

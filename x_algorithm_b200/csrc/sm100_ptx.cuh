@@ -209,6 +209,15 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// K-major operand with rows of 32 bytes, 32-byte swizzle, 8-row groups 256 bytes apart
+__device__ __forceinline__ uint64_t make_smem_desc_32b(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
+  d |= (uint64_t)(256 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)6 << 61;                               // layout: SWIZZLE_32B
+  return d;
+}
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows of 128 bytes, 8-row
 // groups 1024 bytes apart (stride byte offset), descriptor version 1 (Blackwell).
 __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {

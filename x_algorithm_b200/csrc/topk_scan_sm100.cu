@@ -7,13 +7,14 @@
 //               stage (128-byte swizzle, 128-byte boxes: 64 bf16 or 128 int8 columns)
 //   warp 1      MMA issuer: tcgen05.mma M=128 (corpus rows) x N=NQ (queries), 32 bytes of a row per instruction
 //               (kind::f16: 16 bf16, fp32 sums; kind::i8: 32 int8, int32 sums), into one of two TMEM accumulators
+//   (int8 collect pass: warps 18, 19 write the rows' side of the threshold bias, see bias_x)
 //   warps 2-17  consumers: each warp reads its 32-row lane quadrant and a quarter of the query columns with
 //               tcgen05.ld and either appends rows whose score reaches the query's threshold to the survivor list
 //               (collect pass) or reduces the 32-row maximum per query (sample pass)
 // An int8 row of 128 columns is the byte image of a bf16 row of 64: tiles, swizzle, descriptors and tensor maps are the
 // same, only the instruction kind and what a consumer makes of an accumulator differ.
 // Measured (256 queries, k = 1000, one 12.5 M-row shard of 128 columns, whole top-k call): int8 rows 3.98 ms on mma.sync,
-// 1.49 ms when they moved here, 1.20 ms now; bf16 rows 1.28 ms with 8 consumer warps, 1.17 with 16, 0.96 now; one query over
+// 1.49 ms when they moved here, 1.20 before their threshold went into the sum, 0.85 now (64 queries 0.68 -> 0.42); bf16 rows 1.28 ms with 8 consumer warps, 1.17 with 16, 0.96 now; one query over
 // 1 M rows 227 -> 213 us with 64 query columns instead of 256.
 // All mbarrier waits are bounded; on expiry *err_flag is raised and the kernel unwinds.
 #include "common.cuh"
@@ -30,6 +31,11 @@ constexpr int TC_QBOX = 64;       // query rows per TMA box
 constexpr int TC_CWARPS = 16;     // consumer warps: four per scheduler, what hides the latency of the filter's chains
 constexpr int TC_THREADS = 64 + 32 * TC_CWARPS;
 constexpr int TC_STAGES = 4;
+constexpr int TC_BWARPS = 2;      // int8 collect pass: warps that write the rows' side of the bias
+// the int8 collect pass has rows of two k-blocks in one stage less, beside its bias operands
+__host__ __device__ constexpr int scan_threads(int mode, bool i8) { return TC_THREADS + (mode == 1 && i8 ? 32 * TC_BWARPS : 0); }
+__host__ __device__ constexpr int scan_stages(int mode, bool i8, int kblk) { return mode == 1 && i8 && kblk == 2 ? TC_STAGES - 1 : TC_STAGES; }
+__host__ __device__ constexpr int scan_bias_bytes(int mode, bool i8, int nq) { return mode == 1 && i8 ? TC_STAGES * TC_ROWS * 32 + nq * 32 + nq * 4 : 0; }
 constexpr int QCAP = 64;          // per-warp queue of survivors (records of 16 bytes)
 constexpr int QFLUSH = 20;        // flush a warp's queue once it holds this many records
 
@@ -85,6 +91,24 @@ template <int CH>
 __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, uint32_t* r) {
   if (CH == 32) tmem_ld32_nowait(taddr, r); else tmem_ld16_nowait(taddr, r);
 }
+// The threshold inside the int8 sum.  One more MMA step of 32 bytes adds -x(row) * t(query) to every dot product: the row's
+// 32 bytes all hold x = floor(c / row scale), the query's 32 bytes sum to -t, t = floor(threshold / (query scale * c)) a little
+// reduced, so that x t is at most the smallest dot product whose score can reach the threshold.  A sum below zero is then no
+// hit, whatever its query, and 32 columns are tested by and-ing sign bits: no conversion, no scale, no group's smallest threshold.
+// c maps the 7/8 quantile of 1 / row scale (over 32 rows of the corpus) to x = 100; x ends at 127 and t at 4096, which only
+// lets more rows through to the second filter.
+constexpr float BIAS_X = 100.0f;
+constexpr int BIAS_T_MAX = 4096;
+__device__ __forceinline__ int bias_x(float c, float row_scale) {
+  float inv;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(row_scale));   // 1 ulp, covered by the reduction of t
+  return row_scale > 0.f ? (int)fminf(c * inv, 127.f) : 0;
+}
+__device__ __forceinline__ int bias_t(float c, float thr, float query_scale) {
+  // no statement about thresholds that are not positive (or close to the denormals), or where dot * scale may overflow
+  if (!(thr >= 1e-30f) || !(query_scale * 4194304.f < INFINITY) || !(c > 0.f)) return 0;
+  return (int)fminf(__fdiv_rn(__fdiv_rn(thr, query_scale), c) * 0.999f, (float)BIAS_T_MAX);
+}
 // The int32 accumulator of an int8 dot product as fp32 (exact: |dot| <= 128 * 128 * 256 = 2^22) times the query's scale;
 // the row's scale follows: (float(dot) * query scale) * row scale, in that order.
 __device__ __forceinline__ float s8_value(uint32_t acc, float query_scale) { return (float)(int)acc * query_scale; }
@@ -100,11 +124,12 @@ template <int NQ> struct ScanCfg {
 };
 
 template <int MODE, bool I8, int NQ>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(scan_threads(MODE, I8), 1)
 scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_constant__ CUtensorMap map_users,
                TcScanArgs a, int* err_flag) {
   using cfg = ScanCfg<NQ>;
   constexpr int CW = cfg::CW, CH = cfg::CH;
+  constexpr bool BIAS = MODE == 1 && I8;
   extern __shared__ uint8_t smem_raw[];
   const int kblk = a.row_bytes / 128;                            // 128-byte k-blocks: 1 or 2
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -112,7 +137,10 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   const uint32_t users_bytes = (uint32_t)kblk * NQ * 128;
   const uint32_t stage_bytes = (uint32_t)kblk * TC_ROWS * 128;
   const uint32_t stage_base = users_smem + users_bytes;
-  const uint32_t thr_smem = stage_base + TC_STAGES * stage_bytes;  // [256] thresholds, [256] query scales, [8] + [8] per group, [128] query scale pairs
+  const int stages = scan_stages(MODE, I8, kblk);
+  const uint32_t bias_smem = stage_base + stages * stage_bytes;    // BIAS: per stage [128 x 32 B] of x; [NQ x 32 B] of -t, [NQ] t
+  const uint32_t bias_q = bias_smem + TC_STAGES * TC_ROWS * 32;
+  const uint32_t thr_smem = bias_smem + scan_bias_bytes(MODE, I8, NQ);  // [256] thresholds, [256] query scales, [8] + [8] per group, [128] query scale pairs
   const uint32_t queue_smem = thr_smem + 2 * 256 * 4 + 64 + 128 * 16;         // [consumer warps][QCAP] records
   const uint32_t rows_smem = queue_smem + TC_CWARPS * QCAP * 16;   // [consumer warps][32] scores of one corpus row
   const uint32_t bars = rows_smem + TC_CWARPS * 128;
@@ -121,12 +149,14 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   auto tfull_bar = [&](int x) { return bars + 8u * (2 * TC_STAGES + x); };
   auto tempty_bar = [&](int x) { return bars + 8u * (2 * TC_STAGES + 2 + x); };
   const uint32_t users_bar = bars + 8u * (2 * TC_STAGES + 4);
-  const uint32_t tmem_slot = bars + 8u * (2 * TC_STAGES + 5);
+  auto xfull_bar = [&](int s) { return bars + 8u * (2 * TC_STAGES + 5 + s); };
+  const uint32_t tmem_slot = bars + 8u * (3 * TC_STAGES + 5);
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
   float* s_thr = reinterpret_cast<float*>(smem_raw + (thr_smem - smem_u32(smem_raw)));
   float* s_us = s_thr + 256;
   float* s_thr_min = s_us + 256;     // [8] smallest threshold of a group
   float* s_us_max = s_thr_min + 8;   // [8] largest query scale of a group
+  int* s_t = reinterpret_cast<int*>(smem_raw + (bias_q + NQ * 32 - smem_u32(smem_raw)));   // BIAS: [NQ] t
   float4* s_us2 = reinterpret_cast<float4*>(s_us_max + 8);   // [128] {scale, scale, -offset * scale, -offset * scale} of two queries
   uint4* s_queue = reinterpret_cast<uint4*>(smem_raw + (queue_smem - smem_u32(smem_raw)));
 
@@ -139,10 +169,11 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     for (int x = 0; x < 2; ++x) { mbar_init(tfull_bar(x), 1); mbar_init(tempty_bar(x), 32 * TC_CWARPS); }
+    for (int s = 0; s < TC_STAGES; ++s) mbar_init(xfull_bar(s), 1);
     mbar_init(users_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int u = threadIdx.x; u < NQ; u += TC_THREADS) {
+  for (int u = threadIdx.x; u < NQ; u += scan_threads(MODE, I8)) {
     if (MODE == 1) {
       // collect when the score >= thr, with thr a little below the midpoint under the pivot: a superset of
       // { bf16(score) >= pivot }; the exact selection happens later on the rounded scores
@@ -154,6 +185,38 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
       s_thr[u] = t;
     }
     if (I8) s_us[u] = (u < a.B) ? a.user_scale[u] : 0.f;
+  }
+  float bias_c = 0.f;
+  if (BIAS) {
+    // reference of the rows' factor, the same in every thread: each warp ranks the scales of 32 rows spread over the corpus
+    // (rows without a positive scale left out)
+    float s = __ldg(a.row_scale + ((long long)lane * (a.rows - 1)) / 31);
+    if (!(s > 0.f && s < INFINITY)) s = INFINITY;
+    const int n_pos = __popc(__ballot_sync(0xffffffffu, s < INFINITY));
+    int below = 0;                                   // smaller scales, equal ones in front counted too
+#pragma unroll
+    for (int l = 0; l < 32; ++l) {
+      const float o = __shfl_sync(0xffffffffu, s, l);
+      below += (o < s || (o == s && l < lane)) ? 1 : 0;
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, n_pos > 0 && below == n_pos / 8);
+    if (m) bias_c = BIAS_X * __shfl_sync(0xffffffffu, s, __ffs(m) - 1);
+    __syncthreads();                                 // thresholds and query scales are written
+    for (int u = threadIdx.x; u < NQ; u += scan_threads(MODE, I8)) {
+      const int t = u < a.B ? bias_t(bias_c, s_thr[u], s_us[u]) : BIAS_T_MAX;
+      s_t[u] = t;
+      const int each = t >> 5, more = t & 31;        // 32 bytes that sum to -t
+      uint32_t w[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        w[i] = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) w[i] |= (uint32_t)((-(each + (4 * i + b < more ? 1 : 0))) & 0xFF) << (8 * b);
+      }
+      uint4* dst = reinterpret_cast<uint4*>(smem_raw + (bias_q - smem_u32(smem_raw)) + u * 32);
+      dst[0] = make_uint4(w[0], w[1], w[2], w[3]); dst[1] = make_uint4(w[4], w[5], w[6], w[7]);   // (a swizzle only permutes the addends)
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(tmem_slot, 2 * NQ);
   tc_fence_before();
@@ -190,7 +253,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
         mbar_expect_tx(full_bar(stage), stage_bytes);
         for (int kb = 0; kb < kblk; ++kb)
           tma_load_2d(dst + kb * TC_ROWS * 128, &map_corpus, full_bar(stage), kb * BK, (int)(tile * TC_ROWS));
-        if (++stage == TC_STAGES) { stage = 0; phase ^= 1; }
+        if (++stage == stages) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
@@ -213,9 +276,56 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
             else umma_bf16(tmem_base + acc * NQ, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (kb | k) != 0);
           }
         }
+        if (BIAS) {
+          if (!mbar_wait(xfull_bar(stage), phase, verr)) break;
+          tc_fence_after();
+          umma_s8(tmem_base + acc * NQ, make_smem_desc_32b(bias_smem + stage * TC_ROWS * 32), make_smem_desc_32b(bias_q), idesc, 1);
+        }
         umma_commit(empty_bar(stage));
         umma_commit(tfull_bar(acc));
-        if (++stage == TC_STAGES) { stage = 0; phase ^= 1; }
+        if (++stage == stages) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (BIAS && warp >= 2 + TC_CWARPS) {
+    // ---- the rows' side of the bias: each warp every other tile, four rows a lane, into the tile's stage ----
+    // scales of AHEAD tiles are on their way (a tile takes less than a round trip to memory); the loop over them is unrolled
+    // because moving a register that a load has yet to fill waits for it
+    constexpr int AHEAD = 3;
+    const int first = warp - (2 + TC_CWARPS);
+    const long long step = (long long)TC_BWARPS * gridDim.x;
+    float s[AHEAD][4];
+    auto fetch = [&](long long w, float (&v)[4]) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const long long row = w * TC_ROWS + i * 32 + lane;
+        v[i] = (w < n_work && row < a.rows) ? __ldg(a.row_scale + row) : 0.f;
+      }
+    };
+    const long long w_first = blockIdx.x + (long long)first * gridDim.x;
+#pragma unroll
+    for (int d = 0; d < AHEAD; ++d) fetch(w_first + d * step, s[d]);
+    int stage = first; uint32_t phase = 0;             // TC_BWARPS <= stages
+    bool ok = true;
+    for (long long w0 = w_first; w0 < n_work && ok; w0 += AHEAD * step) {
+#pragma unroll
+      for (int d = 0; d < AHEAD; ++d) {
+        const long long w = w0 + d * step;
+        if (w < n_work && ok) {
+          // the stage is free once the MMAs of the tile before it are done, as for the copies
+          ok = __all_sync(0xffffffffu, mbar_wait(empty_bar(stage), phase ^ 1, verr));
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t x = (uint32_t)bias_x(bias_c, s[d][i]) * 0x01010101u;
+            uint4* dst = reinterpret_cast<uint4*>(smem_raw + (bias_smem - smem_u32(smem_raw)) + stage * TC_ROWS * 32 + (i * 32 + lane) * 32);
+            dst[0] = make_uint4(x, x, x, x); dst[1] = make_uint4(x, x, x, x);
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0 && ok) mbar_arrive(xfull_bar(stage));
+          fetch(w + AHEAD * step, s[d]);
+          stage += TC_BWARPS;
+          if (stage >= stages) { stage -= stages; phase ^= 1; }
+        }
       }
     }
   } else {
@@ -228,10 +338,12 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
     Flight flight;
     // threshold and query scale of the column this lane tests in each group
     float t_lane[CW / CH], us_lane[CW / CH];
+    int bt_lane[CW / CH];            // t of that column
 #pragma unroll
     for (int c = 0; c < CW / CH; ++c) {
       t_lane[c] = (MODE == 1 && lane < CH) ? s_thr[part * CW + c * CH + lane] : INFINITY;
       us_lane[c] = (I8 && lane < CH) ? s_us[part * CW + c * CH + lane] : 0.f;
+      bt_lane[c] = (BIAS && lane < CH) ? s_t[part * CW + c * CH + lane] : 0;
     }
     uint32_t it = 0;
     for (long long w = blockIdx.x; w < n_work; w += gridDim.x, ++it) {
@@ -239,7 +351,10 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
       const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
       const long long row = tile * TC_ROWS + quad * 32 + lane;
       const bool row_ok = row < a.rows && row_eligible(a.mask, a.mask_row0, row);
-      const float rs = (I8 && row < a.rows) ? __ldg(a.row_scale + row) : 0.f;
+      // sample pass: the row's scale; collect pass: fetched only when a row passes the filter
+      float rs = (I8 && MODE == 0 && row < a.rows) ? __ldg(a.row_scale + row) : 0.f;
+      bool have_rs = false;
+      int x_row = 0;
       bool ok = mbar_wait(tfull_bar(acc), acc_phase, verr);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
@@ -258,37 +373,54 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
         for (int c = 0; c < CW / CH; ++c) {
           uint32_t (&r)[CH] = rr[c];
           const int u0 = part * CW + c * CH;
-          // First a filter: the largest of the row's CH scores against the smallest of the CH thresholds.  Survivors
-          // are a few in 10^4 .. 10^5 elements, so for most groups the warp stops here; the exact per-column test below
-          // runs only when some lane's group passes.
+          // First a filter.  Survivors are a few in 10^4 .. 10^5 elements, so for most groups the warp stops here; the exact
+          // per-column test below runs only for the rows that pass.
           bool pass;
           if (I8) {
-            // float(dot) * query scale without a conversion per element (those run at a fraction of the fp32 rate):
-            // 1.5 * 2^23 + dot is the integer sum of the bit patterns, and the fma takes the offset's product off
-            // again.  Two roundings: the product's, at most 0.75 of the query scale, and the fma's, at most 0.25 while
-            // |dot| < 2^22 (it is at most 128 * 127 * 256, which leaves 0.998 in all).  With the margin of one scale the bound
-            // is not below the unrounded dot * scale, so the roundings of the tested value, which keep order, cannot put it
-            // above the bound's.  A row scale that is not positive turns the order round: no filter then.
-            float mx = -INFINITY;
+            // sums below zero are no hits (the threshold is part of the sum); a row scale that is not positive would turn the order
+            // round: no filter in a corpus that has one
+            uint32_t sign = r[0] & r[1];
 #pragma unroll
-            for (int k = 0; k < CH; k += 2) {
-              const float4 s2 = s_us2[(u0 + k) >> 1];
-              const float2 x = make_float2(__uint_as_float(r[k] + S8_OFFSET_BITS), __uint_as_float(r[k + 1] + S8_OFFSET_BITS));
-              const float2 v = __ffma2_rn(x, make_float2(s2.x, s2.y), make_float2(s2.z, s2.w));
-              mx = max3(mx, v.x, v.y);
-            }
-            pass = !(rs > 0.f) || !((mx + s_us_max[u0 / CH]) * rs < s_thr_min[u0 / CH]);
+            for (int k = 2; k < CH; k += 2) sign &= r[k] & r[k + 1];
+            pass = (int)sign >= 0 || !a.scales_positive;
           } else {
+            // the largest of the row's CH scores against the smallest of the CH thresholds
             float mx = max3(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]));
 #pragma unroll
             for (int k = 3; k + 1 < CH; k += 2) mx = max3(mx, __uint_as_float(r[k]), __uint_as_float(r[k + 1]));
             mx = fmaxf(mx, __uint_as_float(r[CH - 1]));
             pass = mx >= s_thr_min[u0 / CH];
           }
+          uint32_t rows_left = __ballot_sync(0xffffffffu, row_ok && pass);
+          if (BIAS && rows_left && !have_rs) {
+            rs = row < a.rows ? __ldg(a.row_scale + row) : 0.f;
+            x_row = bias_x(bias_c, rs);
+            have_rs = true;
+          }
+          if (BIAS && __popc(rows_left) > 4) {
+            // More rows than are worth testing one by one: the bias said nothing about some query (its threshold is not
+            // positive, or out of the bias' range), or the rows' scales lie too far apart.  The largest of the row's
+            // scores against the smallest threshold, then.  float(dot) * query scale without a conversion per element (those run
+            // at a fraction of the fp32 rate): 1.5 * 2^23 + dot is the integer sum of the bit patterns, and the fma takes the
+            // offset's product off again.  Two roundings: the product's, at most 0.75 of the query scale, and the fma's, at
+            // most 0.25 while |dot| < 2^22 (it is at most 128 * 127 * 256, which leaves 0.998 in all).  With the margin of one
+            // scale the bound is not below the unrounded dot * scale, so the roundings of the tested value, which keep order,
+            // cannot put it above the bound's.
+            float mx = -INFINITY;
+#pragma unroll
+            for (int k = 0; k < CH; k += 2) {
+              const float4 s2 = s_us2[(u0 + k) >> 1];
+              const uint32_t d0 = r[k] + (uint32_t)(x_row * s_t[u0 + k]), d1 = r[k + 1] + (uint32_t)(x_row * s_t[u0 + k + 1]);
+              const float2 x = make_float2(__uint_as_float(d0 + S8_OFFSET_BITS), __uint_as_float(d1 + S8_OFFSET_BITS));
+              const float2 v = __ffma2_rn(x, make_float2(s2.x, s2.y), make_float2(s2.z, s2.w));
+              mx = max3(mx, v.x, v.y);
+            }
+            pass = pass && (!(rs > 0.f) || !((mx + s_us_max[u0 / CH]) * rs < s_thr_min[u0 / CH]));
+            rows_left = __ballot_sync(0xffffffffu, row_ok && pass);
+          }
           // The few rows that pass, one at a time: the row's scores go through shared memory so that lane k holds column
           // k's, every lane compares with its own column's threshold, and the hits line up in the queue by ballot.  (Each
           // lane testing its own row over all columns cost the warp 150 instructions per group and 90 per hit.)
-          uint32_t rows_left = __ballot_sync(0xffffffffu, row_ok && pass);
           while (rows_left) {
             const int src = __ffs(rows_left) - 1;
             rows_left &= rows_left - 1;
@@ -298,7 +430,8 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
             }
             __syncwarp();
             const uint32_t word = lane < CH ? s_row[lane] : 0u;
-            const float v = I8 ? s8_value(word, us_lane[c]) * __shfl_sync(0xffffffffu, rs, src) : __uint_as_float(word);
+            const int dot = I8 ? (int)word + __shfl_sync(0xffffffffu, x_row, src) * bt_lane[c] : 0;
+            const float v = I8 ? s8_value((uint32_t)dot, us_lane[c]) * __shfl_sync(0xffffffffu, rs, src) : __uint_as_float(word);
             const bool hit = lane < CH && v >= t_lane[c];
             const uint32_t hm = __ballot_sync(0xffffffffu, hit);
             if (hm) {
@@ -374,9 +507,9 @@ template <int MODE, bool I8, int NQ>
 phx_status launch_scan_tc(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, int grid, int* err_flag,
                           cudaStream_t stream, std::string& err) {
   const int kblk = a.row_bytes / 128;
-  const size_t smem = (size_t)kblk * NQ * 128 + (size_t)TC_STAGES * kblk * TC_ROWS * 128 + 2 * 256 * 4 + 64 + 128 * 16 + TC_CWARPS * (QCAP * 16 + 128) + 256 + 1024;
+  const size_t smem = (size_t)kblk * NQ * 128 + (size_t)scan_stages(MODE, I8, kblk) * kblk * TC_ROWS * 128 + scan_bias_bytes(MODE, I8, NQ) + 2 * 256 * 4 + 64 + 128 * 16 + TC_CWARPS * (QCAP * 16 + 128) + 256 + 1024;
   PHX_CUDA_TRY(cudaFuncSetAttribute(scan_tc_kernel<MODE, I8, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), err);
-  scan_tc_kernel<MODE, I8, NQ><<<grid, TC_THREADS, smem, stream>>>(map_corpus, map_users, a, err_flag);
+  scan_tc_kernel<MODE, I8, NQ><<<grid, scan_threads(MODE, I8), smem, stream>>>(map_corpus, map_users, a, err_flag);
   PHX_CUDA_TRY(cudaGetLastError(), err);
   return PHX_OK;
 }
