@@ -35,7 +35,7 @@ constexpr int TC_BWARPS = 2;      // int8 collect pass: warps that write the row
 // the int8 collect pass has rows of two k-blocks in one stage less, beside its bias operands
 __host__ __device__ constexpr int scan_threads(int mode, bool i8) { return TC_THREADS + (mode == 1 && i8 ? 32 * TC_BWARPS : 0); }
 __host__ __device__ constexpr int scan_stages(int mode, bool i8, int kblk) { return mode == 1 && i8 && kblk == 2 ? TC_STAGES - 1 : TC_STAGES; }
-__host__ __device__ constexpr int scan_bias_bytes(int mode, bool i8, int nq) { return mode == 1 && i8 ? TC_STAGES * TC_ROWS * 32 + nq * 32 + nq * 4 : 0; }
+__host__ __device__ constexpr int scan_bias_bytes(int mode, bool i8, int nq) { return mode == 1 && i8 ? TC_STAGES * TC_ROWS * 32 + nq * 32 + nq * 4 + 16 : 0; }
 constexpr int QCAP = 64;          // per-warp queue of survivors (records of 16 bytes)
 constexpr int QFLUSH = 20;        // flush a warp's queue once it holds this many records
 
@@ -96,7 +96,8 @@ __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, uint32_t* r) {
 // reduced, so that x t is at most the smallest dot product whose score can reach the threshold.  A sum below zero is then no
 // hit, whatever its query, and 32 columns are tested by and-ing sign bits: no conversion, no scale, no group's smallest threshold.
 // c maps the 7/8 quantile of 1 / row scale (over 32 rows of the corpus) to x = 100; x ends at 127 and t at 4096, which only
-// lets more rows through to the second filter.
+// lets more rows through to the second filter.  A group with a query about which the bias can say nothing (bias_t < 0) goes to
+// the second filter as a whole.
 constexpr float BIAS_X = 100.0f;
 constexpr int BIAS_T_MAX = 4096;
 __device__ __forceinline__ int bias_x(float c, float row_scale) {
@@ -105,8 +106,9 @@ __device__ __forceinline__ int bias_x(float c, float row_scale) {
   return row_scale > 0.f ? (int)fminf(c * inv, 127.f) : 0;
 }
 __device__ __forceinline__ int bias_t(float c, float thr, float query_scale) {
-  // no statement about thresholds that are not positive (or close to the denormals), or where dot * scale may overflow
-  if (!(thr >= 1e-30f) || !(query_scale * 4194304.f < INFINITY) || !(c > 0.f)) return 0;
+  // no statement about thresholds that are not positive (or close to the denormals: sums below zero may reach them), or where
+  // dot * scale may overflow
+  if (!(thr >= 1e-30f) || !(query_scale * 4194304.f < INFINITY) || !(c > 0.f)) return -1;
   return (int)fminf(__fdiv_rn(__fdiv_rn(thr, query_scale), c) * 0.999f, (float)BIAS_T_MAX);
 }
 // The int32 accumulator of an int8 dot product as fp32 (exact: |dot| <= 128 * 128 * 256 = 2^22) times the query's scale;
@@ -157,6 +159,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   float* s_thr_min = s_us + 256;     // [8] smallest threshold of a group
   float* s_us_max = s_thr_min + 8;   // [8] largest query scale of a group
   int* s_t = reinterpret_cast<int*>(smem_raw + (bias_q + NQ * 32 - smem_u32(smem_raw)));   // BIAS: [NQ] t
+  int* s_open = s_t + NQ;            // BIAS: bit g: group g is not filtered by the bias
   float4* s_us2 = reinterpret_cast<float4*>(s_us_max + 8);   // [128] {scale, scale, -offset * scale, -offset * scale} of two queries
   uint4* s_queue = reinterpret_cast<uint4*>(smem_raw + (queue_smem - smem_u32(smem_raw)));
 
@@ -200,10 +203,12 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
       below += (o < s || (o == s && l < lane)) ? 1 : 0;
     }
     const uint32_t m = __ballot_sync(0xffffffffu, n_pos > 0 && below == n_pos / 8);
+    if (threadIdx.x == 0) *s_open = 0;
     if (m) bias_c = BIAS_X * __shfl_sync(0xffffffffu, s, __ffs(m) - 1);
     __syncthreads();                                 // thresholds and query scales are written
     for (int u = threadIdx.x; u < NQ; u += scan_threads(MODE, I8)) {
-      const int t = u < a.B ? bias_t(bias_c, s_thr[u], s_us[u]) : BIAS_T_MAX;
+      int t = u < a.B ? bias_t(bias_c, s_thr[u], s_us[u]) : BIAS_T_MAX;
+      if (t < 0) { atomicOr(s_open, 1 << (u / CH)); t = 0; }
       s_t[u] = t;
       const int each = t >> 5, more = t & 31;        // 32 bytes that sum to -t
       uint32_t w[8];
@@ -345,6 +350,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
       us_lane[c] = (I8 && lane < CH) ? s_us[part * CW + c * CH + lane] : 0.f;
       bt_lane[c] = (BIAS && lane < CH) ? s_t[part * CW + c * CH + lane] : 0;
     }
+    const int open = BIAS ? (a.scales_positive ? *s_open : -1) : 0;
     uint32_t it = 0;
     for (long long w = blockIdx.x; w < n_work; w += gridDim.x, ++it) {
       const long long tile = (MODE == 0) ? w * a.stride : w;
@@ -382,7 +388,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
             uint32_t sign = r[0] & r[1];
 #pragma unroll
             for (int k = 2; k < CH; k += 2) sign &= r[k] & r[k + 1];
-            pass = (int)sign >= 0 || !a.scales_positive;
+            pass = (int)sign >= 0 || ((open >> (u0 / CH)) & 1);
           } else {
             // the largest of the row's CH scores against the smallest of the CH thresholds
             float mx = max3(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]));
