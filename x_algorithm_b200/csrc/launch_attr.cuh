@@ -3,6 +3,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <stdlib.h>
+#include <string.h>
+
 #include <atomic>
 
 namespace phx {
@@ -27,6 +30,23 @@ class OncePerDevice {
  private:
   std::atomic<bool> done_[LAUNCH_MAX_DEVICES] = {};
 };
+
+// Launch of a kernel that waits (griddepcontrol.wait) before it touches memory: it may set up, and fill SMs as they come free,
+// while the kernel in front of it on the stream finishes.  PHX_PDL=0 keeps plain stream order.
+template <typename... P, typename... A>
+cudaError_t launch_programmatic(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A&... args) {
+  cudaLaunchConfig_t lc;
+  memset(&lc, 0, sizeof(lc));
+  lc.gridDim = grid; lc.blockDim = block; lc.dynamicSmemBytes = smem; lc.stream = stream;
+  cudaLaunchAttribute at[1];
+  static const bool pdl = !(getenv("PHX_PDL") && getenv("PHX_PDL")[0] == '0');
+  if (pdl) {
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at; lc.numAttrs = 1;
+  }
+  return cudaLaunchKernelEx(&lc, kern, static_cast<P>(args)...);
+}
 
 // A kernel's raised dynamic shared-memory limit: one static object per kernel and limit.
 class SmemLimit {

@@ -169,6 +169,9 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   const long long n_tiles = (a.rows + TC_ROWS - 1) / TC_ROWS;
   const long long n_work = (MODE == 0) ? (n_tiles + a.stride - 1) / a.stride : n_tiles;
 
+  // the kernels in front wrote the queries and thresholds; what follows may set up from here on
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     for (int x = 0; x < 2; ++x) { mbar_init(tfull_bar(x), 1); mbar_init(tempty_bar(x), 32 * TC_CWARPS); }
@@ -514,9 +517,9 @@ phx_status launch_scan_tc(const CUtensorMap& map_corpus, const CUtensorMap& map_
                           cudaStream_t stream, std::string& err) {
   const int kblk = a.row_bytes / 128;
   const size_t smem = (size_t)kblk * NQ * 128 + (size_t)scan_stages(MODE, I8, kblk) * kblk * TC_ROWS * 128 + scan_bias_bytes(MODE, I8, NQ) + 2 * 256 * 4 + 64 + 128 * 16 + TC_CWARPS * (QCAP * 16 + 128) + 256 + 1024;
-  PHX_CUDA_TRY(cudaFuncSetAttribute(scan_tc_kernel<MODE, I8, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), err);
-  scan_tc_kernel<MODE, I8, NQ><<<grid, scan_threads(MODE, I8), smem, stream>>>(map_corpus, map_users, a, err_flag);
-  PHX_CUDA_TRY(cudaGetLastError(), err);
+  static SmemLimit limit;
+  PHX_CUDA_TRY(limit.raise(scan_tc_kernel<MODE, I8, NQ>, 227 * 1024), err);
+  PHX_CUDA_TRY(launch_programmatic(scan_tc_kernel<MODE, I8, NQ>, grid, scan_threads(MODE, I8), smem, stream, map_corpus, map_users, a, err_flag), err);
   return PHX_OK;
 }
 template <int MODE, bool I8>
