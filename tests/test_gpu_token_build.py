@@ -60,3 +60,29 @@ def test_heads_with_and_without_staged_rows(D):
     eng.close()
     np.testing.assert_array_equal(some.log_probs, whole.log_probs[:296])
     np.testing.assert_array_equal(some.continuous, whole.continuous[:296])
+
+
+@pytest.mark.parametrize("C", [30, 700])                 # results in one copy; in row chunks
+def test_packed_results_are_laid_out_by_the_host(C):
+    """Packed calls bring back the valid rows alone: every slot without a candidate reads zero whatever the caller's arrays held, and
+    a request's results do not depend on the others' counts (none, one, all of its slots)."""
+    import x_algorithm_b200 as px
+    B, S = 41, 9
+    ocfg, w, rows_fn, eng = make_pair(max_batch=B, emb_size=128, num_layers=1, num_q_heads=2, num_kv_heads=2, key_size=64, history_len=S,
+                                      num_candidates=C, engine_kw=dict(pack_ragged=True))
+    eng.set_blend(px.blend_spec_from_weights(px.ValueModelWeights(w=dict(po.make_blend_weights(1).w)), px.HEAD_NAMES_19, ocfg.num_actions))
+    b = po.make_batch(ocfg, B, seed=5, ragged=True)
+    for q, n in ((0, 0), (1, 1), (2, C), (17, 0), (B - 1, 0)):
+        b.cand_post_ids[q, :], b.cand_author_ids[q, :] = 7, 9
+        b.cand_post_ids[q, n:], b.cand_author_ids[q, n:] = 0, 0
+    out = px.RankOutputs(np.full((B, C, ocfg.num_actions), np.nan, np.float32), np.full((B, C, ocfg.num_continuous), np.nan, np.float32),
+                         np.full((B, C), np.nan))
+    got = eng.rank(to_inputs(b), out)
+    names = ("hist_post_ids", "hist_author_ids", "hist_actions", "hist_surfaces", "cand_post_ids", "cand_author_ids")
+    for q in range(B):
+        one = eng.rank(to_inputs(type(b)(*[np.ascontiguousarray(getattr(b, f)[q:q + 1]) for f in names])))
+        n = int((b.cand_post_ids[q] != 0).sum())
+        for a, o in ((got.log_probs, one.log_probs), (got.continuous, one.continuous), (got.scores, one.scores)):
+            np.testing.assert_array_equal(a[q], o[0])
+            assert not np.any(a[q, n:])
+    eng.close()

@@ -72,6 +72,7 @@ struct phx_engine {
     long long M = 0, Mh = 0;      // packed rows in all, history rows
     int planned_batch = -1;       // batch size pos_rows / out_index were last planned for (full plan)
     bool ragged = false;
+    bool compact = false;         // results stay in packed row order (the host lays them out), no slot is zeroed on the device
   };
   phx_model_config cfg;
   int device = 0;
@@ -1076,7 +1077,9 @@ phx_status enqueue_forward(phx_engine* e, const phx_rank_batch* bd, const phx_ra
   if (e->split) { ha.x = e->x + (long long)B * e->S * e->D; ha.T = e->C; ha.S = 0; }   // the candidate block of the split layout
   if (pk) {   // packed rows: candidate rows back to back, scattered to their output slots; padded slots read zero
     ha.x = e->x + pk->Mh * e->D; ha.out_index = pk->out_index; ha.rows = pk->M - pk->Mh;
-    if (pk->ragged) {
+    if (pk->compact) {           // row r's results at place r: one request of so many candidates
+      ha.out_index = nullptr; ha.B = 1; ha.S = 0; ha.C = ha.T = (int)ha.rows;
+    } else if (pk->ragged) {
       const size_t rows = (size_t)B * e->C;
       if (od->log_probs) PHX_CUDA_TRY(cudaMemsetAsync(od->log_probs, 0, rows * e->V * 4, e->stream), e->err);
       if (od->continuous) PHX_CUDA_TRY(cudaMemsetAsync(od->continuous, 0, rows * e->NC * 4, e->stream), e->err);
@@ -1477,54 +1480,79 @@ phx_status phx_rank_forward(phx_engine* e, const phx_rank_batch* bh, const phx_r
     pk.hist_off_view = (const int*)put(ho, (B + 1) * 4);   // the plan reads its offsets from the staged block
     pk.cand_off_view = (const int*)put(co, (B + 1) * 4);
     pk.Mh = ho[B]; pk.M = (long long)ho[B] + co[B];
+    pk.compact = true;
     PHX_CUDA_TRY(cudaMemcpyAsync(dp, hp, off, cudaMemcpyHostToDevice, e->stream), e->err);
     e->pack_next = &pk;
   } else {
     PHX_CUDA_TRY(cudaMemcpyAsync(dp, hp, off, cudaMemcpyHostToDevice, e->stream), e->err);
   }
-  phx_rank_out od; od.log_probs = e->lp_dev; od.continuous = e->cont_dev; od.scores = e->score_dev;
-  const size_t rows = B * C;
+  // Packed calls bring back the valid rows alone, in packed order, and lay them out here; the other slots read zero.
+  // 48 ragged requests of up to 512 candidates: 580 us a call with the device zeroing and sending every slot, 524 this way.
+  const int* co = e->pack ? e->pack_host.data() + (B + 1) : nullptr;
+  const size_t rows = co ? (size_t)co[B] : B * C;
   // Small results (up to half a megabyte) lie back to back and come back in one copy, the flag right behind: in chunks the
   // twelve copies of one request, each a few kilobytes, took longer than their bytes.  Whole calls, chunks against one copy:
   // 44 KB 94 against 78 us, 484 KB 138 against 124, 704 KB 161 against 150, 1.4 MB 244 against 260.
   const OutLayout ol(rows, e->V, e->NC);
   const bool one_copy = ol.bytes <= (512u << 10);
-  if (one_copy) { od.log_probs = ol.lp(e->out_stage_dev); od.continuous = ol.cont(e->out_stage_dev); }
+  float* lp_dev = e->lp_dev; float* cont_dev = e->cont_dev;
+  float* lp_host = e->lp_host; float* cont_host = e->cont_host;
+  if (one_copy) {
+    lp_dev = ol.lp(e->out_stage_dev); cont_dev = ol.cont(e->out_stage_dev);
+    lp_host = ol.lp(e->out_stage_host); cont_host = ol.cont(e->out_stage_host);
+  }
+  const int V = e->V, NC = e->NC;
+  const bool want_scores = oh->scores && e->has_blend;
+  phx_rank_out od; od.log_probs = lp_dev; od.continuous = cont_dev; od.scores = e->score_dev;
   phx_status s = phx_rank_forward_device(e, &bd, &od);
   if (s) return s;
-  if (one_copy) {
-    PHX_CUDA_TRY(cudaMemcpyAsync(e->out_stage_host, e->out_stage_dev, ol.bytes, cudaMemcpyDeviceToHost, e->stream), e->err);
-    PHX_CUDA_TRY(cudaMemcpyAsync(e->flag_host, e->err_flag, sizeof(int), cudaMemcpyDeviceToHost, e->stream), e->err);
-    PHX_CUDA_TRY(cudaStreamSynchronize(e->stream), e->err);
-    if (oh->log_probs) memcpy(oh->log_probs, ol.lp(e->out_stage_host), rows * e->V * 4);
-    if (oh->continuous) memcpy(oh->continuous, ol.cont(e->out_stage_host), rows * e->NC * 4);
-    if (oh->scores && e->has_blend) memcpy(oh->scores, e->score_host, rows * 8);
-    return *e->flag_host ? check_err_flag(e) : PHX_OK;
-  }
+  if (one_copy && rows) PHX_CUDA_TRY(cudaMemcpyAsync(e->out_stage_host, e->out_stage_dev, ol.bytes, cudaMemcpyDeviceToHost, e->stream), e->err);
   // larger results come back in four row chunks: while the host copies chunk i out of the pinned staging block, chunk i+1
   // is still on the bus
   constexpr int NCH = 4;
   const size_t step = (rows + NCH - 1) / NCH;
-  for (int i = 0; i < NCH; ++i) {
+  for (int i = 0; i < NCH && !one_copy; ++i) {
     const size_t r0 = i * step, r1 = (r0 + step < rows) ? r0 + step : rows;
     if (r0 < r1) {
-      if (oh->log_probs) PHX_CUDA_TRY(cudaMemcpyAsync(e->lp_host + r0 * e->V, e->lp_dev + r0 * e->V, (r1 - r0) * e->V * 4, cudaMemcpyDeviceToHost, e->stream), e->err);
-      if (oh->continuous) PHX_CUDA_TRY(cudaMemcpyAsync(e->cont_host + r0 * e->NC, e->cont_dev + r0 * e->NC, (r1 - r0) * e->NC * 4, cudaMemcpyDeviceToHost, e->stream), e->err);
-      if (oh->scores && e->has_blend) PHX_CUDA_TRY(cudaMemcpyAsync(e->score_host + r0, e->score_dev + r0, (r1 - r0) * 8, cudaMemcpyDeviceToHost, e->stream), e->err);
+      if (oh->log_probs) PHX_CUDA_TRY(cudaMemcpyAsync(lp_host + r0 * V, lp_dev + r0 * V, (r1 - r0) * V * 4, cudaMemcpyDeviceToHost, e->stream), e->err);
+      if (oh->continuous) PHX_CUDA_TRY(cudaMemcpyAsync(cont_host + r0 * NC, cont_dev + r0 * NC, (r1 - r0) * NC * 4, cudaMemcpyDeviceToHost, e->stream), e->err);
+      if (want_scores) PHX_CUDA_TRY(cudaMemcpyAsync(e->score_host + r0, e->score_dev + r0, (r1 - r0) * 8, cudaMemcpyDeviceToHost, e->stream), e->err);
     }
     if (!e->ev_chunk[i]) PHX_CUDA_TRY(cudaEventCreateWithFlags(&e->ev_chunk[i], cudaEventDisableTiming), e->err);
     PHX_CUDA_TRY(cudaEventRecord(e->ev_chunk[i], e->stream), e->err);
   }
   PHX_CUDA_TRY(cudaMemcpyAsync(e->flag_host, e->err_flag, sizeof(int), cudaMemcpyDeviceToHost, e->stream), e->err);
-  for (int i = 0; i < NCH; ++i) {
+  // `n` rows from row r of the staging block to slot `slot` of the caller's arrays
+  auto place = [&](size_t slot, size_t r, size_t n) {
+    if (oh->log_probs) memcpy(oh->log_probs + slot * V, lp_host + r * V, n * V * 4);
+    if (oh->continuous) memcpy(oh->continuous + slot * NC, cont_host + r * NC, n * NC * 4);
+    if (want_scores) memcpy(oh->scores + slot, e->score_host + r, n * 8);
+  };
+  size_t placed = 0, q = 0;        // rows placed so far, and the request the next one belongs to
+  auto place_upto = [&](size_t r1) {
+    if (!co) { if (placed < r1) place(placed, placed, r1 - placed); placed = r1; return; }
+    while (placed < r1) {
+      while ((size_t)co[q + 1] <= placed) ++q;
+      const size_t end = (size_t)co[q + 1] < r1 ? (size_t)co[q + 1] : r1;
+      place(q * C + (placed - (size_t)co[q]), placed, end - placed);
+      placed = end;
+    }
+  };
+  if (co) {                        // the slots without a candidate, while the device works
+    for (size_t b = 0; b < B; ++b) {
+      const size_t slot = b * C + (size_t)(co[b + 1] - co[b]), n = (b + 1) * C - slot;
+      if (n == 0) continue;
+      if (oh->log_probs) memset(oh->log_probs + slot * V, 0, n * V * 4);
+      if (oh->continuous) memset(oh->continuous + slot * NC, 0, n * NC * 4);
+      if (want_scores) memset(oh->scores + slot, 0, n * 8);
+    }
+  }
+  for (int i = 0; i < NCH && !one_copy; ++i) {
     PHX_CUDA_TRY(cudaEventSynchronize(e->ev_chunk[i]), e->err);
-    const size_t r0 = i * step, r1 = (r0 + step < rows) ? r0 + step : rows;
-    if (r0 >= r1) continue;
-    if (oh->log_probs) memcpy(oh->log_probs + r0 * e->V, e->lp_host + r0 * e->V, (r1 - r0) * e->V * 4);
-    if (oh->continuous) memcpy(oh->continuous + r0 * e->NC, e->cont_host + r0 * e->NC, (r1 - r0) * e->NC * 4);
-    if (oh->scores && e->has_blend) memcpy(oh->scores + r0, e->score_host + r0, (r1 - r0) * 8);
+    place_upto((i + 1) * step < rows ? (i + 1) * step : rows);
   }
   PHX_CUDA_TRY(cudaStreamSynchronize(e->stream), e->err);
+  place_upto(rows);
   return *e->flag_host ? check_err_flag(e) : PHX_OK;
 }
 
