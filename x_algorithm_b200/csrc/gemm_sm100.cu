@@ -14,7 +14,7 @@
 // PAIR variant (cta_group::2): the two CTAs of a cluster work on one 256 x BN tile.  Each loads its own 128 rows of
 // A and its own half of the W tile, the even CTA issues one MMA (M=256) that reads both shared memories and
 // writes each CTA's 128 rows into that CTA's TMEM, and each CTA runs the epilogue on its own rows.  Operand bytes
-// per CTA per k-step fall from 128+BN to 128+BN/2 rows: the GEMM is bound by that shared-memory fill.
+// per CTA per k-step fall from 128+BN to 128+BN/2 rows: that fill, and the power it takes, is what a tile costs beside its MMAs.
 // Every mbarrier wait is bounded by wall time; on expiry the kernel raises *err_flag and unwinds.
 #include <stdlib.h>
 #include <string.h>
