@@ -47,10 +47,11 @@ def test_pooling_keeps_rows_where_they_fit(S, D, B):
     assert rel_l2(users.cpu().numpy()[ok], want[ok]) < TOL
 
 
-@pytest.mark.parametrize("D", [128, 1024])
-def test_heads_with_and_without_staged_rows(D):
+@pytest.mark.parametrize("D,actions", [(128, 19), (1024, 19), (1664, 30), (2048, 30)])    # the last: too wide for the rows to be staged
+def test_heads_with_and_without_staged_rows(D, actions):
     """296 strips of 16 candidates take eight warps a strip with its rows in shared memory, 297 a warp a strip: the same bits."""
-    kw = dict(emb_size=D, num_layers=1, num_q_heads=2, num_kv_heads=2, key_size=64, history_len=9, num_candidates=16)
+    kw = dict(emb_size=D, num_layers=1, num_q_heads=2, num_kv_heads=2, key_size=64, history_len=9, num_candidates=16, num_actions=actions,
+              widening_factor=1.0)
     ocfg, w, rows_fn, eng = make_pair(max_batch=297, **kw)
     b = po.make_batch(ocfg, 297, seed=5, ragged=True)
     whole = eng.rank(to_inputs(b))

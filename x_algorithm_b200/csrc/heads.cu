@@ -130,7 +130,7 @@ __device__ __forceinline__ void mma_bf16_16816_h(float (&c)[4], const uint32_t (
 // fetch the strip's rows into shared memory in one go, form the same sums and share the (row, output) items.  Same arithmetic,
 // same bits.  Kernel at 20 outputs, parameters not yet staged (one warp / eight): D = 512: 512 to 2048 rows 18.5 / 11.5 us, 4096
 // rows 18.7 / 14.9, 8192 rows 20.4 / 27.2; D = 1024: 512 rows 29.0 / 18.3, 4800 rows 28.3 / 38.3; D = 128: 128 rows 12.7 / 6.6.
-template <int NT, int WPS>
+template <int NT, int WPS, bool STAGED>
 __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_kernel(HeadsArgs a) {
   constexpr int WARPS = WPS == 1 ? HM_WARPS : WPS;      // warps per CTA
   extern __shared__ __align__(16) uint8_t hsm[];
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_ke
   float* sgain = reinterpret_cast<float*>(sw + NT * 8 * WLD);                // [D]
   float* sC_all = sgain + D;                                                 // per warp [16][NT*8] fp32 sums
   double* sD_all = reinterpret_cast<double*>(sC_all + WARPS * 16 * NT * 8);   // per strip [16][NT*8] blend inputs
-  bf16* sX = reinterpret_cast<bf16*>(sD_all + (WPS == 1 ? HM_WARPS : 1) * 16 * NT * 8);   // WPS > 1: [16][WLD] the strip's rows
+  bf16* sX = reinterpret_cast<bf16*>(sD_all + (WPS == 1 ? HM_WARPS : 1) * 16 * NT * 8);   // STAGED: [16][WLD] the strip's rows
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
 #pragma unroll 4
   for (int i = threadIdx.x; i < NT * 8 * (D / 8); i += WARPS * 32) {
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_ke
       const unsigned b = (unsigned)r / (unsigned)a.C, c = (unsigned)r - b * (unsigned)a.C;     // rows fit 31 bits
       return a.x + ((long long)b * a.T + a.S + c) * (long long)D;
     };
-    if (WPS == 1) {
+    if (!STAGED) {
 #pragma unroll
       for (int i = 0; i < 2; ++i) xr[i] = row_of(g + 8 * i) + 8 * t4;
     } else {
@@ -274,15 +274,21 @@ __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_ke
   }
 }
 
-template <int NT, int WPS>
+template <int NT, int WPS, bool STAGED>
+size_t heads_smem(int D) {
+  constexpr int WARPS = WPS == 1 ? HM_WARPS : WPS;
+  return (size_t)NT * 8 * (D + HM_WPAD) * sizeof(bf16) + (size_t)D * sizeof(float) +
+         (size_t)16 * NT * 8 * (WARPS * sizeof(float) + (WPS == 1 ? HM_WARPS : 1) * sizeof(double)) +
+         (STAGED ? (size_t)16 * (D + HM_WPAD) * sizeof(bf16) : 0);
+}
+constexpr size_t HEADS_SMEM_MAX = 200 * 1024;
+template <int NT, int WPS, bool STAGED>
 phx_status launch_heads_wps(const HeadsArgs& a, long long strips, cudaStream_t stream, std::string& err) {
   constexpr int WARPS = WPS == 1 ? HM_WARPS : WPS;
-  const size_t smem = (size_t)NT * 8 * (a.D + HM_WPAD) * sizeof(bf16) + (size_t)a.D * sizeof(float) +
-                      (size_t)16 * NT * 8 * (WARPS * sizeof(float) + (WPS == 1 ? HM_WARPS : 1) * sizeof(double)) +
-                      (WPS == 1 ? 0 : (size_t)16 * (a.D + HM_WPAD) * sizeof(bf16));
-  if (smem > 200 * 1024) { err = "heads: head matrix does not fit shared memory"; return PHX_E_CAPACITY; }
+  const size_t smem = heads_smem<NT, WPS, STAGED>(a.D);
+  if (smem > HEADS_SMEM_MAX) { err = "heads: head matrix does not fit shared memory"; return PHX_E_CAPACITY; }
   static SmemLimit limit;
-  PHX_CUDA_TRY(limit.raise(heads_mma_kernel<NT, WPS>, 200 * 1024), err);
+  PHX_CUDA_TRY(limit.raise(heads_mma_kernel<NT, WPS, STAGED>, (int)HEADS_SMEM_MAX), err);
   long long blocks = WPS == 1 ? (strips + HM_WARPS - 1) / HM_WARPS : strips;
   if (blocks > 148 * 3) blocks = 148 * 3;
   cudaLaunchConfig_t lc;
@@ -295,15 +301,18 @@ phx_status launch_heads_wps(const HeadsArgs& a, long long strips, cudaStream_t s
     at[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = at; lc.numAttrs = 1;
   }
-  PHX_CUDA_TRY(cudaLaunchKernelEx(&lc, heads_mma_kernel<NT, WPS>, a), err);
+  PHX_CUDA_TRY(cudaLaunchKernelEx(&lc, heads_mma_kernel<NT, WPS, STAGED>, a), err);
   return PHX_OK;
 }
 template <int NT>
 phx_status launch_heads_mma(const HeadsArgs& a, long long rows, cudaStream_t stream, std::string& err) {
   // up to two CTAs of a strip each per SM; a third round of them costs more than a warp a strip (measured beside the kernel)
   const long long strips = (rows + 15) / 16;
-  if (strips <= 2 * 148) return launch_heads_wps<NT, 8>(a, strips, stream, err);
-  return launch_heads_wps<NT, 1>(a, strips, stream, err);
+  if (strips <= 2 * 148) {
+    if (heads_smem<NT, 8, true>(a.D) <= HEADS_SMEM_MAX) return launch_heads_wps<NT, 8, true>(a, strips, stream, err);
+    return launch_heads_wps<NT, 4, false>(a, strips, stream, err);    // rows too wide to stand beside the head matrix
+  }
+  return launch_heads_wps<NT, 1, false>(a, strips, stream, err);
 }
 
 // users[b] = l2norm(mean over valid t of final_norm(x[b,t])), fp32; one CTA per user, one thread per column.  Two passes
