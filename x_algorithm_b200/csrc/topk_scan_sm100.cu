@@ -14,7 +14,7 @@
 // An int8 row of 128 columns is the byte image of a bf16 row of 64: tiles, swizzle, descriptors and tensor maps are the
 // same, only the instruction kind and what a consumer makes of an accumulator differ.
 // Measured (256 queries, k = 1000, one 12.5 M-row shard of 128 columns, whole top-k call): int8 rows 3.98 ms on mma.sync,
-// 1.49 ms when they moved here, 1.20 before their threshold went into the sum, 0.85 now (64 queries 0.68 -> 0.42); bf16 rows 1.28 ms with 8 consumer warps, 1.17 with 16, 0.96 now; one query over
+// 1.49 ms when they moved here, 1.20 before their threshold went into the sum, 0.85 now (64 queries 0.68 -> 0.42); bf16 rows 1.28 ms with 8 consumer warps, 1.17 with 16, 0.87 now; one query over
 // 1 M rows 227 -> 213 us with 64 query columns instead of 256.
 // All mbarrier waits are bounded; on expiry *err_flag is raised and the kernel unwinds.
 #include "common.cuh"
