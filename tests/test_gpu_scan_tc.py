@@ -173,3 +173,31 @@ def test_int8_threshold_in_the_sum(dim, kind):
     sh.close()
     np.testing.assert_array_equal(got_i, want_i)
     np.testing.assert_array_equal(got_s, want_s)
+
+
+def _int8_equals_the_oracle(N, dim, B, k, users, q8, scales):
+    from x_algorithm_b200.retrieval import CorpusShard
+    sh = CorpusShard(N, dim, max_queries=B, max_k=k)
+    sh.upload_int8(0, q8, scales)
+    sh.set_int8(True)
+    got_s, got_i = _topk(sh, users, k)
+    assert sh.exact_runs() == 0
+    want_s, want_i = po.top_k(po.int8_corpus_scores(users, q8, scales), k)
+    sh.close()
+    np.testing.assert_array_equal(got_i, want_i)
+    np.testing.assert_array_equal(got_s, want_s)
+
+
+@pytest.mark.parametrize("scales,shares", [
+    ((1e-39, 1.1e-38, 1.2e-38), (0.2, 0.4, 0.4)),       # below 2^-126 and just above it, in one corpus
+    ((1e-40, 9e-40), (0.5, 0.5)),                       # all of them below
+    ((1.2e-38, 1e-36), (0.5, 0.5)),                     # small, but none below
+    ((1e-44, 1e-30, 1e-3), (0.3, 0.3, 0.4))])
+@pytest.mark.parametrize("magnitude", [1e6, 1e14])
+def test_int8_row_scales_near_the_smallest(scales, shares, magnitude):
+    """Row scales down to the denormals, with queries large enough that their scores are ordinary numbers."""
+    N, B, dim, k = 40001, 3, 128, 25
+    r = np.random.default_rng(7)
+    s = r.choice(np.array(scales, np.float32), size=N, p=shares).astype(np.float32)
+    q8 = r.integers(-127, 128, size=(N, dim), dtype=np.int8)
+    _int8_equals_the_oracle(N, dim, B, k, (_users(B, dim, 3) * np.float32(magnitude)).astype(np.float32), q8, s)

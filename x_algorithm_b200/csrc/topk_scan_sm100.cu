@@ -21,6 +21,8 @@
 #include "sm100_ptx.cuh"
 #include "topk_scan.cuh"
 
+#include <float.h>
+
 namespace phx {
 namespace {
 
@@ -101,15 +103,19 @@ __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, uint32_t* r) {
 constexpr float BIAS_X = 100.0f;
 constexpr int BIAS_T_MAX = 4096;
 __device__ __forceinline__ int bias_x(float c, float row_scale) {
+  // no statement about a row whose scale is not an ordinary positive number: 1 / scale of a denormal one would come out infinite
+  if (!(row_scale >= FLT_MIN)) return 0;
   float inv;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(row_scale));   // 1 ulp, covered by the reduction of t
-  return row_scale > 0.f ? (int)fminf(c * inv, 127.f) : 0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(row_scale));   // 1 ulp, covered by the reduction of t; 0 for scales above 2^126
+  return (int)fminf(c * inv, 127.f);
 }
 __device__ __forceinline__ int bias_t(float c, float thr, float query_scale) {
-  // no statement about thresholds that are not positive (or close to the denormals: sums below zero may reach them), or where
-  // dot * scale may overflow
-  if (!(thr >= 1e-30f) || !(query_scale * 4194304.f < INFINITY) || !(c > 0.f)) return -1;
-  return (int)fminf(__fdiv_rn(__fdiv_rn(thr, query_scale), c) * 0.999f, (float)BIAS_T_MAX);
+  // no statement about thresholds that are not positive (or close to the denormals: sums below zero may reach them), where
+  // dot * scale may overflow, or where c or threshold / query scale is denormal (their rounding is not relative)
+  if (!(thr >= 1e-30f) || !(query_scale * 4194304.f < INFINITY) || !(c >= FLT_MIN)) return -1;
+  const float ratio = __fdiv_rn(thr, query_scale);
+  if (!(ratio >= FLT_MIN)) return -1;
+  return (int)fminf(__fdiv_rn(ratio, c) * 0.999f, (float)BIAS_T_MAX);
 }
 // The int32 accumulator of an int8 dot product as fp32 (exact: |dot| <= 128 * 128 * 256 = 2^22) times the query's scale;
 // the row's scale follows: (float(dot) * query scale) * row scale, in that order.
