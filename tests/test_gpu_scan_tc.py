@@ -201,3 +201,15 @@ def test_int8_row_scales_near_the_smallest(scales, shares, magnitude):
     s = r.choice(np.array(scales, np.float32), size=N, p=shares).astype(np.float32)
     q8 = r.integers(-127, 128, size=(N, dim), dtype=np.int8)
     _int8_equals_the_oracle(N, dim, B, k, (_users(B, dim, 3) * np.float32(magnitude)).astype(np.float32), q8, s)
+
+
+@pytest.mark.parametrize("scales,magnitude", [((1e36, 1.2e36), 1e-6), ((1e34, 5e37), 1e-5), ((2e38, 3e38), 1e-7), ((1e-3, 3e38), 1e-7)])
+def test_int8_row_scales_near_the_largest(scales, magnitude):
+    """Row scales so large that a threshold divided by the query's scale, or the reference of the rows' factors, is infinite."""
+    N, B, dim, k = 40001, 3, 128, 25
+    r = np.random.default_rng(7)
+    s = r.choice(np.array(scales, np.float32), size=N).astype(np.float32)
+    q8 = r.integers(-127, 128, size=(N, dim), dtype=np.int8)
+    users = (_users(B, dim, 3) * np.float32(magnitude)).astype(np.float32)
+    assert np.isfinite(po.int8_corpus_scores(users, q8, s)).all()
+    _int8_equals_the_oracle(N, dim, B, k, users, q8, s)

@@ -111,10 +111,10 @@ __device__ __forceinline__ int bias_x(float c, float row_scale) {
 }
 __device__ __forceinline__ int bias_t(float c, float thr, float query_scale) {
   // no statement about thresholds that are not positive (or close to the denormals: sums below zero may reach them), where
-  // dot * scale may overflow, or where c or threshold / query scale is denormal (their rounding is not relative)
-  if (!(thr >= 1e-30f) || !(query_scale * 4194304.f < INFINITY) || !(c >= FLT_MIN)) return -1;
+  // dot * scale may overflow, or where c or threshold / query scale is denormal (their rounding is not relative) or infinite
+  if (!(thr >= 1e-30f) || !(query_scale * 4194304.f < INFINITY) || !(c >= FLT_MIN && c < INFINITY)) return -1;
   const float ratio = __fdiv_rn(thr, query_scale);
-  if (!(ratio >= FLT_MIN)) return -1;
+  if (!(ratio >= FLT_MIN && ratio < INFINITY)) return -1;
   return (int)fminf(__fdiv_rn(ratio, c) * 0.999f, (float)BIAS_T_MAX);
 }
 // The int32 accumulator of an int8 dot product as fp32 (exact: |dot| <= 128 * 128 * 256 = 2^22) times the query's scale;
