@@ -213,3 +213,71 @@ def test_int8_row_scales_near_the_largest(scales, magnitude):
     users = (_users(B, dim, 3) * np.float32(magnitude)).astype(np.float32)
     assert np.isfinite(po.int8_corpus_scores(users, q8, s)).all()
     _int8_equals_the_oracle(N, dim, B, k, users, q8, s)
+
+
+@pytest.mark.parametrize("share", [0.15, 0.5, 0.85])
+@pytest.mark.parametrize("scale,where", [(1e-12, "end"), (1e-12, "mixed"), (0.0, "end"), (0.0, "mixed"), (-0.0, "mixed")])
+def test_int8_shard_with_empty_rows(share, scale, where):
+    """Rows of zeros, as the quantiser leaves them (scale 1e-12) or as an uploader marks them, at the end of a shard or all over it."""
+    N, B, dim, k = 40001, 70, 128, 25
+    r = np.random.default_rng(8)
+    q8 = r.integers(-127, 128, size=(N, dim), dtype=np.int8)
+    s = (r.random(N, dtype=np.float32) * np.float32(0.01) + np.float32(1e-3)).astype(np.float32)
+    empty = np.arange(N) >= int(N * (1 - share)) if where == "end" else r.random(N) < share
+    q8[empty] = 0
+    s[empty] = scale
+    _int8_equals_the_oracle(N, dim, B, k, _users(B, dim, 3), q8, s)
+
+
+def _median_us(sh, users, k, n=15):
+    import torch
+    B = users.shape[0]
+    u = torch.from_numpy(users).cuda()
+    sc = torch.empty((B, k), dtype=torch.float32, device="cuda"); ids = torch.empty((B, k), dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    t = []
+    for _ in range(n):
+        sh.topk_device(u, B, k, sc, ids)
+        sh.sync()
+        t.append(sh.last_device_ms() * 1e3)
+    return float(np.median(t[3:]))
+
+
+def _int8_shard(N, dim, B, k, change):
+    """A quantised synthetic shard with its scales (and empty rows) as `change` leaves them."""
+    import torch
+    from x_algorithm_b200.retrieval import CorpusShard
+    sh = CorpusShard(N, dim, max_queries=B, max_k=k)
+    sh.fill_synthetic(4)
+    sh.quantize_int8()
+    q = torch.empty((N, dim), dtype=torch.int8, device="cuda"); s = torch.empty(N, dtype=torch.float32, device="cuda")
+    sh.read_int8_device(0, N, q, s)
+    q8, scales = q.cpu().numpy(), s.cpu().numpy()
+    change(np.random.default_rng(1), q8, scales)
+    sh.upload_int8(0, q8, scales)
+    sh.set_int8(True)
+    return sh
+
+
+def _empty_tail(r, q8, scales):
+    n = int(0.85 * len(scales)); q8[n:] = 0; scales[n:] = 1e-12
+
+
+def _half_empty(r, q8, scales):
+    rows = r.random(len(scales)) < 0.5; q8[rows] = 0; scales[rows] = 1e-12
+
+
+@pytest.mark.parametrize("change", [_empty_tail, _half_empty])
+def test_int8_filter_serves_shards_that_are_not_full(change):
+    """Rows that hold nothing do not switch the filter inside the int8 sum off for the others: with it off such a shard takes 1.6 to 1.8
+    times as long as a full one, with it 1.0 to 1.1."""
+    N, dim, B, k = 4_000_000, 128, 256, 300
+    users = _users(B, dim, 3)
+    full = _int8_shard(N, dim, B, k, lambda *a: None)
+    t_full = _median_us(full, users, k)
+    full.close()
+    sh = _int8_shard(N, dim, B, k, change)
+    t = _median_us(sh, users, k)
+    assert sh.exact_runs() == 0
+    sh.close()
+    assert t < 1.35 * t_full, f"{t:.0f} us, a full shard {t_full:.0f} us"
