@@ -267,7 +267,11 @@ def _half_empty(r, q8, scales):
     rows = r.random(len(scales)) < 0.5; q8[rows] = 0; scales[rows] = 1e-12
 
 
-@pytest.mark.parametrize("change", [_empty_tail, _half_empty])
+def _zero_scales(r, q8, scales):
+    scales[r.random(len(scales)) < 0.15] = 0.0
+
+
+@pytest.mark.parametrize("change", [_empty_tail, _half_empty, _zero_scales])
 def test_int8_filter_serves_shards_that_are_not_full(change):
     """Rows that hold nothing do not switch the filter inside the int8 sum off for the others: with it off such a shard takes 1.6 to 1.8
     times as long as a full one, with it 1.0 to 1.1."""
@@ -277,7 +281,32 @@ def test_int8_filter_serves_shards_that_are_not_full(change):
     t_full = _median_us(full, users, k)
     full.close()
     sh = _int8_shard(N, dim, B, k, change)
+    # a negative scale that is overwritten leaves no trace
+    sh.upload_int8(N - 3, np.ones((1, dim), np.int8), np.full(1, -1.0, np.float32))
+    sh.upload_int8(N - 3, np.ones((1, dim), np.int8), np.full(1, 1e-3, np.float32))
     t = _median_us(sh, users, k)
     assert sh.exact_runs() == 0
     sh.close()
     assert t < 1.35 * t_full, f"{t:.0f} us, a full shard {t_full:.0f} us"
+
+
+def test_int8_negative_scales_come_and_go():
+    """A negative scale turns the order of its row round; uploaded anew with a positive one the row is like any other."""
+    from x_algorithm_b200.retrieval import CorpusShard
+    N, B, dim, k = 40001, 70, 128, 25
+    r = np.random.default_rng(9)
+    q8 = r.integers(-127, 128, size=(N, dim), dtype=np.int8)
+    s = (r.random(N, dtype=np.float32) * np.float32(0.01) + np.float32(1e-3)).astype(np.float32)
+    users = _users(B, dim, 3)
+    sh = CorpusShard(N, dim, max_queries=B, max_k=k)
+    sh.upload_int8(0, q8, s)
+    sh.set_int8(True)
+    for rows, sign in (((5, 900), -1.0), ((700, 39000), -1.0), ((5, 39000), 1.0)):
+        s[rows[0]:rows[1]] = np.abs(s[rows[0]:rows[1]]) * np.float32(sign)
+        sh.upload_int8(rows[0], q8[rows[0]:rows[1]], s[rows[0]:rows[1]])
+        got_s, got_i = _topk(sh, users, k)
+        want_s, want_i = po.top_k(po.int8_corpus_scores(users, q8, s), k)
+        np.testing.assert_array_equal(got_i, want_i)
+        np.testing.assert_array_equal(got_s, want_s)
+    assert sh.exact_runs() == 0
+    sh.close()

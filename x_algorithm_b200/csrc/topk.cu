@@ -507,7 +507,8 @@ struct phx_corpus {
   // int8 form of the corpus (phx_corpus_upload_int8 / phx_corpus_quantize_int8) and whether calls score with it
   signed char* q8 = nullptr;     // [rows, dim]
   float* row_scale = nullptr;    // [rows]
-  bool scales_positive = true;   // false once a scale that is not above zero was uploaded, until the rows are quantised anew
+  std::vector<bool> negative;    // rows whose scale is below zero, as uploaded last; empty until there is one
+  long long n_negative = 0;
   float* user_scale = nullptr;   // [256]
   bool int8 = false;
   CUtensorMap map_corpus, map_users;
@@ -752,8 +753,13 @@ phx_status phx_corpus_upload_int8(phx_corpus* c, int64_t row0, int64_t nrows, co
   phx_status s = ensure_int8_buffers(c);
   if (s) return s;
   PHX_CUDA_TRY(cudaMemcpy(c->q8 + row0 * c->dim, host_q8, (size_t)nrows * c->dim, cudaMemcpyHostToDevice), c->err);
-  for (int64_t i = 0; i < nrows; ++i)
-    if (!(host_scales[i] > 0.f)) { c->scales_positive = false; break; }
+  for (int64_t i = 0; i < nrows; ++i) {
+    const bool neg = host_scales[i] < 0.f;
+    if (neg && c->negative.empty()) c->negative.assign((size_t)c->rows, false);
+    if (c->negative.empty() || c->negative[row0 + i] == neg) continue;
+    c->negative[row0 + i] = neg;
+    c->n_negative += neg ? 1 : -1;
+  }
   PHX_CUDA_TRY(cudaMemcpy(c->row_scale + row0, host_scales, (size_t)nrows * 4, cudaMemcpyHostToDevice), c->err);
   return PHX_OK;
 }
@@ -763,7 +769,8 @@ phx_status phx_corpus_quantize_int8(phx_corpus* c) {
   cudaSetDevice(c->device);
   phx_status s = ensure_int8_buffers(c);
   if (s) return s;
-  c->scales_positive = true;      // the kernel's scales are at least 1e-12
+  std::vector<bool>().swap(c->negative);      // the kernel's scales are at least 1e-12
+  c->n_negative = 0;
   quantize_rows_int8_kernel<bf16><<<(unsigned)((c->rows + 7) / 8), 256, 0, c->stream>>>(c->data, c->rows, c->rows, c->dim, c->q8, c->row_scale, nullptr);
   PHX_CUDA_TRY(cudaGetLastError(), c->err);
   PHX_CUDA_TRY(cudaStreamSynchronize(c->stream), c->err);
@@ -900,7 +907,7 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
   a.i8 = c->int8 ? 1 : 0; a.user_scale = c->user_scale; a.row_scale = c->int8 ? c->row_scale + row_begin : nullptr;
   TcScanArgs ta;
   ta.mask = c->mask; ta.mask_row0 = row_begin;
-  if (c->int8) { ta.user_scale = c->user_scale; ta.row_scale = c->row_scale + row_begin; ta.scales_positive = c->scales_positive ? 1 : 0; }
+  if (c->int8) { ta.user_scale = c->user_scale; ta.row_scale = c->row_scale + row_begin; ta.scales_negative = c->n_negative > 0 ? 1 : 0; }
   ta.rows = rows; ta.row_offset = roff; ta.row_bytes = row_bytes; ta.B = B; ta.stride = 1; ta.gmax = c->gmax; ta.n_groups = 0;
   ta.pivot = c->pivot; ta.surv = c->surv; ta.counts = c->counts; ta.cap = c->cap;
   const long long n_tiles = (rows + tile_rows - 1) / tile_rows;

@@ -24,7 +24,7 @@ struct TcScanArgs {
   // null = bf16 corpus
   const float* user_scale = nullptr;   // [B]
   const float* row_scale = nullptr;    // [rows]
-  int scales_positive = 0;             // every row scale of the corpus is above zero
+  int scales_negative = 0;             // some row scale of the corpus is below zero
 };
 
 __device__ __forceinline__ bool row_eligible(const unsigned int* mask, long long mask_row0, long long row) {

@@ -103,8 +103,9 @@ __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, uint32_t* r) {
 constexpr float BIAS_X = 100.0f;
 constexpr int BIAS_T_MAX = 4096;
 __device__ __forceinline__ int bias_x(float c, float row_scale) {
-  // no statement about a row whose scale is not an ordinary positive number: 1 / scale of a denormal one would come out infinite
-  if (!(row_scale >= FLT_MIN)) return 0;
+  // No statement about a row whose scale is not an ordinary positive number: 1 / scale of a denormal one would come out infinite.  Zero
+  // scores are no hits where the bias says anything (thresholds are positive there): the largest x keeps such rows out.
+  if (!(row_scale >= FLT_MIN)) return row_scale == 0.f ? 127 : 0;
   float inv;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(row_scale));   // 1 ulp, covered by the reduction of t; 0 for scales above 2^126
   return (int)fminf(c * inv, 127.f);
@@ -215,7 +216,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
       const float o = __shfl_sync(0xffffffffu, s, l);
       below += (o < s || (o == s && l < lane)) ? 1 : 0;
     }
-    if (threadIdx.x == 0) *s_open = 0;
+    if (threadIdx.x == 0) *s_open = a.scales_negative ? ~0 : 0;   // scales below zero turn the order of the sums round
     const uint32_t up = __ballot_sync(0xffffffffu, n_pos > 0 && below == (n_pos > 1 ? n_pos - 2 : 0));
     if (up) {
       const float upper = __shfl_sync(0xffffffffu, s, __ffs(up) - 1);
@@ -368,7 +369,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
       us_lane[c] = (I8 && lane < CH) ? s_us[part * CW + c * CH + lane] : 0.f;
       bt_lane[c] = (BIAS && lane < CH) ? s_t[part * CW + c * CH + lane] : 0;
     }
-    const int open = BIAS ? (a.scales_positive ? *s_open : -1) : 0;
+    const int open = BIAS ? *s_open : 0;
     uint32_t it = 0;
     for (long long w = blockIdx.x; w < n_work; w += gridDim.x, ++it) {
       const long long tile = (MODE == 0) ? w * a.stride : w;
@@ -401,8 +402,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
           // per-column test below runs only for the rows that pass.
           bool pass;
           if (I8) {
-            // sums below zero are no hits (the threshold is part of the sum); a row scale that is not positive would turn the order
-            // round: no filter in a corpus that has one
+            // sums below zero are no hits (the threshold is part of the sum)
             uint32_t sign = r[0] & r[1];
 #pragma unroll
             for (int k = 2; k < CH; k += 2) sign &= r[k] & r[k + 1];
@@ -429,7 +429,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
             // offset's product off again.  Two roundings: the product's, at most 0.75 of the query scale, and the fma's, at
             // most 0.25 while |dot| < 2^22 (it is at most 128 * 127 * 256, which leaves 0.998 in all).  With the margin of one
             // scale the bound is not below the unrounded dot * scale, so the roundings of the tested value, which keep order,
-            // cannot put it above the bound's.
+            // cannot put it above the bound's.  A scale below zero (or no number) turns the order round: no filter then.
             float mx = -INFINITY;
 #pragma unroll
             for (int k = 0; k < CH; k += 2) {
@@ -439,7 +439,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
               const float2 v = __ffma2_rn(x, make_float2(s2.x, s2.y), make_float2(s2.z, s2.w));
               mx = max3(mx, v.x, v.y);
             }
-            pass = pass && (!(rs > 0.f) || !((mx + s_us_max[u0 / CH]) * rs < s_thr_min[u0 / CH]));
+            pass = pass && (!(rs >= 0.f) || !((mx + s_us_max[u0 / CH]) * rs < s_thr_min[u0 / CH]));
             rows_left = __ballot_sync(0xffffffffu, row_ok && pass);
           }
           // The few rows that pass, one at a time: the row's scores go through shared memory so that lane k holds column
