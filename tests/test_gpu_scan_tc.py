@@ -310,3 +310,21 @@ def test_int8_negative_scales_come_and_go():
         np.testing.assert_array_equal(got_s, want_s)
     assert sh.exact_runs() == 0
     sh.close()
+
+
+@pytest.mark.parametrize("B", [5, 70, 128, 200, 256])
+@pytest.mark.parametrize("negative", [False, True])
+@pytest.mark.parametrize("below", ["all", "some groups", "one query"])
+def test_int8_open_groups(B, negative, below):
+    """Queries whose scores are all below zero: throughout, in some groups of query columns, one alone; with and without a row whose scale is
+    negative.  The bias is left out, switched off by groups, or not there."""
+    N, dim, k = 40001, 128, 25
+    r = np.random.default_rng(B)
+    q8 = r.integers(20, 128, size=(N, dim), dtype=np.int8)
+    s = (r.random(N, dtype=np.float32) * np.float32(0.01) + np.float32(1e-3)).astype(np.float32)
+    if negative:
+        s[[0, 777, N - 1]] *= np.float32(-1)
+    users = np.abs(_users(B, dim, 3))
+    down = {"all": np.ones(B, bool), "some groups": np.arange(B) % 64 < 40, "one query": np.arange(B) == B // 2}[below]
+    users[down] *= -1
+    _int8_equals_the_oracle(N, dim, B, k, users, q8, s)

@@ -23,6 +23,8 @@
 
 #include <float.h>
 
+#include <type_traits>
+
 namespace phx {
 namespace {
 
@@ -34,10 +36,10 @@ constexpr int TC_CWARPS = 16;     // consumer warps: four per scheduler, what hi
 constexpr int TC_THREADS = 64 + 32 * TC_CWARPS;
 constexpr int TC_STAGES = 4;
 constexpr int TC_BWARPS = 2;      // int8 collect pass: warps that write the rows' side of the bias
-// the int8 collect pass has rows of two k-blocks in one stage less, beside its bias operands
-__host__ __device__ constexpr int scan_threads(int mode, bool i8) { return TC_THREADS + (mode == 1 && i8 ? 32 * TC_BWARPS : 0); }
-__host__ __device__ constexpr int scan_stages(int mode, bool i8, int kblk) { return mode == 1 && i8 && kblk == 2 ? TC_STAGES - 1 : TC_STAGES; }
-__host__ __device__ constexpr int scan_bias_bytes(int mode, bool i8, int nq) { return mode == 1 && i8 ? TC_STAGES * TC_ROWS * 32 + nq * 32 + nq * 4 + 16 : 0; }
+// the collect pass with the bias has rows of two k-blocks in one stage less, beside its bias operands
+__host__ __device__ constexpr int scan_threads(bool bias) { return TC_THREADS + (bias ? 32 * TC_BWARPS : 0); }
+__host__ __device__ constexpr int scan_stages(bool bias, int kblk) { return bias && kblk == 2 ? TC_STAGES - 1 : TC_STAGES; }
+__host__ __device__ constexpr int scan_bias_bytes(bool bias, int nq) { return bias ? TC_STAGES * TC_ROWS * 32 + nq * 32 + nq * 4 + 16 : 0; }
 constexpr int QCAP = 64;          // per-warp queue of survivors (records of 16 bytes)
 constexpr int QFLUSH = 20;        // flush a warp's queue once it holds this many records
 
@@ -99,7 +101,7 @@ __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, uint32_t* r) {
 // hit, whatever its query, and 32 columns are tested by and-ing sign bits: no conversion, no scale, no group's smallest threshold.
 // c maps one of the smaller scales among the rows that count (over 32 rows of the corpus) to x = 100; x ends at 127 and t at
 // 4096, which only lets more rows through to the second filter.  A group with a query about which the bias can say nothing (bias_t < 0) goes to
-// the second filter as a whole.
+// the second filter as a whole (it is open).
 constexpr float BIAS_X = 100.0f;
 constexpr int BIAS_T_MAX = 4096;
 __device__ __forceinline__ int bias_x(float c, float row_scale) {
@@ -132,13 +134,13 @@ template <int NQ> struct ScanCfg {
   static constexpr int GROUPS = NQ / CH;
 };
 
-template <int MODE, bool I8, int NQ>
-__global__ void __launch_bounds__(scan_threads(MODE, I8), 1)
+template <int MODE, bool I8, int NQ, bool BIAS>
+__global__ void __launch_bounds__(scan_threads(BIAS), 1)
 scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_constant__ CUtensorMap map_users,
                TcScanArgs a, int* err_flag) {
   using cfg = ScanCfg<NQ>;
   constexpr int CW = cfg::CW, CH = cfg::CH;
-  constexpr bool BIAS = MODE == 1 && I8;
+  static_assert(!BIAS || (MODE == 1 && I8), "the bias belongs to the int8 collect pass");
   extern __shared__ uint8_t smem_raw[];
   const int kblk = a.row_bytes / 128;                            // 128-byte k-blocks: 1 or 2
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -146,10 +148,10 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   const uint32_t users_bytes = (uint32_t)kblk * NQ * 128;
   const uint32_t stage_bytes = (uint32_t)kblk * TC_ROWS * 128;
   const uint32_t stage_base = users_smem + users_bytes;
-  const int stages = scan_stages(MODE, I8, kblk);
+  const int stages = scan_stages(BIAS, kblk);
   const uint32_t bias_smem = stage_base + stages * stage_bytes;    // BIAS: per stage [128 x 32 B] of x; [NQ x 32 B] of -t, [NQ] t
   const uint32_t bias_q = bias_smem + TC_STAGES * TC_ROWS * 32;
-  const uint32_t thr_smem = bias_smem + scan_bias_bytes(MODE, I8, NQ);  // [256] thresholds, [256] query scales, [8] + [8] per group, [128] query scale pairs
+  const uint32_t thr_smem = bias_smem + scan_bias_bytes(BIAS, NQ);  // [256] thresholds, [256] query scales, [8] + [8] per group, [128] query scale pairs
   const uint32_t queue_smem = thr_smem + 2 * 256 * 4 + 64 + 128 * 16;         // [consumer warps][QCAP] records
   const uint32_t rows_smem = queue_smem + TC_CWARPS * QCAP * 16;   // [consumer warps][32] scores of one corpus row
   const uint32_t bars = rows_smem + TC_CWARPS * 128;
@@ -186,7 +188,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
     mbar_init(users_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int u = threadIdx.x; u < NQ; u += scan_threads(MODE, I8)) {
+  for (int u = threadIdx.x; u < NQ; u += scan_threads(BIAS)) {
     if (MODE == 1) {
       // collect when the score >= thr, with thr a little below the midpoint under the pivot: a superset of
       // { bf16(score) >= pivot }; the exact selection happens later on the rounded scores
@@ -225,7 +227,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
       bias_c = BIAS_X * __shfl_sync(0xffffffffu, s, __ffs(m) - 1);
     }
     __syncthreads();                                 // thresholds and query scales are written
-    for (int u = threadIdx.x; u < NQ; u += scan_threads(MODE, I8)) {
+    for (int u = threadIdx.x; u < NQ; u += scan_threads(BIAS)) {
       int t = u < a.B ? bias_t(bias_c, s_thr[u], s_us[u]) : BIAS_T_MAX;
       if (t < 0) { atomicOr(s_open, 1 << (u / CH)); t = 0; }
       s_t[u] = t;
@@ -263,6 +265,9 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   }
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  // from 128 query columns on a call whose groups are all open leaves the bias out; the same in every thread
+  constexpr bool TWO_LOOPS = BIAS && NQ >= 128;
+  const bool biased = BIAS && !(TWO_LOOPS && (~*s_open & ((1 << cfg::GROUPS) - 1)) == 0);
 
   if (warp == 0) {
     if (elect_one()) {
@@ -300,7 +305,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
             else umma_bf16(tmem_base + acc * NQ, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (kb | k) != 0);
           }
         }
-        if (BIAS) {
+        if (biased) {
           if (!mbar_wait(xfull_bar(stage), phase, verr)) break;
           tc_fence_after();
           umma_s8(tmem_base + acc * NQ, make_smem_desc_32b(bias_smem + stage * TC_ROWS * 32), make_smem_desc_32b(bias_q), idesc, 1);
@@ -330,7 +335,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
     for (int d = 0; d < AHEAD; ++d) fetch(w_first + d * step, s[d]);
     int stage = first; uint32_t phase = 0;             // TC_BWARPS <= stages
     bool ok = true;
-    for (long long w0 = w_first; w0 < n_work && ok; w0 += AHEAD * step) {
+    for (long long w0 = biased ? w_first : n_work; w0 < n_work && ok; w0 += AHEAD * step) {
 #pragma unroll
       for (int d = 0; d < AHEAD; ++d) {
         const long long w = w0 + d * step;
@@ -353,168 +358,181 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
       }
     }
   } else {
-    const int ew = warp - 2;
-    const int part = ew >> 2;        // which quarter of the query columns
-    const int quad = warp & 3;       // TMEM lane quadrant
-    uint4* const queue = s_queue + ew * QCAP;
-    uint32_t* const s_row = reinterpret_cast<uint32_t*>(smem_raw + (rows_smem - smem_u32(smem_raw))) + ew * 32;
-    int nq = 0;                      // records in the queue (the same in every lane)
-    Flight flight;
-    // threshold and query scale of the column this lane tests in each group
-    float t_lane[CW / CH], us_lane[CW / CH];
-    int bt_lane[CW / CH];            // t of that column
+    // FOLDED: the thresholds are part of the sums.  128 and 256 columns have a loop without that as well, for calls whose scores are not
+    // above zero (12.5 M rows, all of them below, 256 / 100 queries: 10.25 / 6.35 ms before there was a bias, 10.65 / 6.62 with one loop,
+    // 9.84 / 6.11 with two), and of the two the one with the bias is compiled with fewer spilled registers (scores above zero: 813 -> 710 us,
+    // 502 -> 477).  64 columns: 310 us with one loop, 319 with two.
+    auto consume = [&](auto folded) {
+      constexpr bool FOLDED = decltype(folded)::value;
+      const int ew = warp - 2;
+      const int part = ew >> 2;        // which quarter of the query columns
+      const int quad = warp & 3;       // TMEM lane quadrant
+      uint4* const queue = s_queue + ew * QCAP;
+      uint32_t* const s_row = reinterpret_cast<uint32_t*>(smem_raw + (rows_smem - smem_u32(smem_raw))) + ew * 32;
+      int nq = 0;                      // records in the queue (the same in every lane)
+      Flight flight;
+      // threshold and query scale of the column this lane tests in each group
+      float t_lane[CW / CH], us_lane[CW / CH];
+      int bt_lane[CW / CH];            // t of that column
 #pragma unroll
-    for (int c = 0; c < CW / CH; ++c) {
-      t_lane[c] = (MODE == 1 && lane < CH) ? s_thr[part * CW + c * CH + lane] : INFINITY;
-      us_lane[c] = (I8 && lane < CH) ? s_us[part * CW + c * CH + lane] : 0.f;
-      bt_lane[c] = (BIAS && lane < CH) ? s_t[part * CW + c * CH + lane] : 0;
-    }
-    const int open = BIAS ? *s_open : 0;
-    uint32_t it = 0;
-    for (long long w = blockIdx.x; w < n_work; w += gridDim.x, ++it) {
-      const long long tile = (MODE == 0) ? w * a.stride : w;
-      const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-      const long long row = tile * TC_ROWS + quad * 32 + lane;
-      const bool row_ok = row < a.rows && row_eligible(a.mask, a.mask_row0, row);
-      // sample pass: the row's scale; collect pass: fetched only when a row passes the filter
-      float rs = (I8 && MODE == 0 && row < a.rows) ? __ldg(a.row_scale + row) : 0.f;
-      bool have_rs = false;
-      int x_row = 0;
-      bool ok = mbar_wait(tfull_bar(acc), acc_phase, verr);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t taddr = tmem_base + acc * NQ + ((uint32_t)(quad * 32) << 16) + part * CW;
-      if (MODE == 1) {
-        // the warp's whole slice of the tile (32 rows x CW queries) in one round trip to TMEM, then the accumulator
-        // goes straight back to the MMA warp: the filtering below works from registers
-        uint32_t rr[CW / CH][CH];
+      for (int c = 0; c < CW / CH; ++c) {
+        t_lane[c] = (MODE == 1 && lane < CH) ? s_thr[part * CW + c * CH + lane] : INFINITY;
+        us_lane[c] = (I8 && lane < CH) ? s_us[part * CW + c * CH + lane] : 0.f;
+        bt_lane[c] = (FOLDED && lane < CH) ? s_t[part * CW + c * CH + lane] : 0;
+      }
+      const int open = FOLDED ? *s_open : 0;
+      uint32_t it = 0;
+      for (long long w = blockIdx.x; w < n_work; w += gridDim.x, ++it) {
+        const long long tile = (MODE == 0) ? w * a.stride : w;
+        const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
+        const long long row = tile * TC_ROWS + quad * 32 + lane;
+        const bool row_ok = row < a.rows && row_eligible(a.mask, a.mask_row0, row);
+        // the row's scale; with the bias it is fetched only when a row passes the filter
+        float rs = (I8 && !FOLDED && row < a.rows) ? __ldg(a.row_scale + row) : 0.f;
+        bool have_rs = false;
+        int x_row = 0;
+        bool ok = mbar_wait(tfull_bar(acc), acc_phase, verr);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + acc * NQ + ((uint32_t)(quad * 32) << 16) + part * CW;
+        if (MODE == 1) {
+          // the warp's whole slice of the tile (32 rows x CW queries) in one round trip to TMEM, then the accumulator
+          // goes straight back to the MMA warp: the filtering below works from registers
+          uint32_t rr[CW / CH][CH];
 #pragma unroll
-        for (int c = 0; c < CW / CH; ++c) tmem_ld_chunk<CH>(taddr + c * CH, rr[c]);
-        tmem_ld_wait();
-        tc_fence_before();
-        mbar_arrive(tempty_bar(acc));
-#pragma unroll
-        for (int c = 0; c < CW / CH; ++c) {
-          uint32_t (&r)[CH] = rr[c];
-          const int u0 = part * CW + c * CH;
-          // First a filter.  Survivors are a few in 10^4 .. 10^5 elements, so for most groups the warp stops here; the exact
-          // per-column test below runs only for the rows that pass.
-          bool pass;
-          if (I8) {
-            // sums below zero are no hits (the threshold is part of the sum)
-            uint32_t sign = r[0] & r[1];
-#pragma unroll
-            for (int k = 2; k < CH; k += 2) sign &= r[k] & r[k + 1];
-            pass = (int)sign >= 0 || ((open >> (u0 / CH)) & 1);
-          } else {
-            // the largest of the row's CH scores against the smallest of the CH thresholds
-            float mx = max3(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]));
-#pragma unroll
-            for (int k = 3; k + 1 < CH; k += 2) mx = max3(mx, __uint_as_float(r[k]), __uint_as_float(r[k + 1]));
-            mx = fmaxf(mx, __uint_as_float(r[CH - 1]));
-            pass = mx >= s_thr_min[u0 / CH];
-          }
-          uint32_t rows_left = __ballot_sync(0xffffffffu, row_ok && pass);
-          if (BIAS && rows_left && !have_rs) {
-            rs = row < a.rows ? __ldg(a.row_scale + row) : 0.f;
-            x_row = bias_x(bias_c, rs);
-            have_rs = true;
-          }
-          if (BIAS && __popc(rows_left) > 4) {
-            // More rows than are worth testing one by one: the bias said nothing about some query (its threshold is not
-            // positive, or out of the bias' range), or the rows' scales lie too far apart.  The largest of the row's
-            // scores against the smallest threshold, then.  float(dot) * query scale without a conversion per element (those run
-            // at a fraction of the fp32 rate): 1.5 * 2^23 + dot is the integer sum of the bit patterns, and the fma takes the
-            // offset's product off again.  Two roundings: the product's, at most 0.75 of the query scale, and the fma's, at
-            // most 0.25 while |dot| < 2^22 (it is at most 128 * 127 * 256, which leaves 0.998 in all).  With the margin of one
-            // scale the bound is not below the unrounded dot * scale, so the roundings of the tested value, which keep order,
-            // cannot put it above the bound's.  A scale below zero (or no number) turns the order round: no filter then.
-            float mx = -INFINITY;
-#pragma unroll
-            for (int k = 0; k < CH; k += 2) {
-              const float4 s2 = s_us2[(u0 + k) >> 1];
-              const uint32_t d0 = r[k] + (uint32_t)(x_row * s_t[u0 + k]), d1 = r[k + 1] + (uint32_t)(x_row * s_t[u0 + k + 1]);
-              const float2 x = make_float2(__uint_as_float(d0 + S8_OFFSET_BITS), __uint_as_float(d1 + S8_OFFSET_BITS));
-              const float2 v = __ffma2_rn(x, make_float2(s2.x, s2.y), make_float2(s2.z, s2.w));
-              mx = max3(mx, v.x, v.y);
-            }
-            pass = pass && (!(rs >= 0.f) || !((mx + s_us_max[u0 / CH]) * rs < s_thr_min[u0 / CH]));
-            rows_left = __ballot_sync(0xffffffffu, row_ok && pass);
-          }
-          // The few rows that pass, one at a time: the row's scores go through shared memory so that lane k holds column
-          // k's, every lane compares with its own column's threshold, and the hits line up in the queue by ballot.  (Each
-          // lane testing its own row over all columns cost the warp 150 instructions per group and 90 per hit.)
-          while (rows_left) {
-            const int src = __ffs(rows_left) - 1;
-            rows_left &= rows_left - 1;
-            if (lane == src) {
-#pragma unroll
-              for (int k = 0; k < CH; k += 4) *reinterpret_cast<uint4*>(s_row + k) = make_uint4(r[k], r[k + 1], r[k + 2], r[k + 3]);
-            }
-            __syncwarp();
-            const uint32_t word = lane < CH ? s_row[lane] : 0u;
-            const int dot = I8 ? (int)word + __shfl_sync(0xffffffffu, x_row, src) * bt_lane[c] : 0;
-            const float v = I8 ? s8_value((uint32_t)dot, us_lane[c]) * __shfl_sync(0xffffffffu, rs, src) : __uint_as_float(word);
-            const bool hit = lane < CH && v >= t_lane[c];
-            const uint32_t hm = __ballot_sync(0xffffffffu, hit);
-            if (hm) {
-              const int n = __popc(hm);
-              if (nq + n > QCAP) { flush_queue(a, queue, nq, lane, flight); nq = 0; __syncwarp(); }
-              if (hit) {
-                const uint32_t grow = (uint32_t)(a.row_offset + row - lane + src);
-                queue[nq + __popc(hm & ((1u << lane) - 1u))] = make_uint4(0xFFFFFFFFu - grow, ord32(round_bf(v)), (uint32_t)(u0 + lane), 0u);
-              }
-              nq += n;
-            }
-            __syncwarp();
-          }
-        }
-      } else {
-#pragma unroll 1
-        for (int c = 0; c < CW / CH; ++c) {
-          uint32_t r[CH];
-          tmem_ld_chunk<CH>(taddr + c * CH, r);
+          for (int c = 0; c < CW / CH; ++c) tmem_ld_chunk<CH>(taddr + c * CH, rr[c]);
           tmem_ld_wait();
-          const int u0 = part * CW + c * CH;
-          const long long grp = w * 4 + quad;
-          float m[CH];
+          tc_fence_before();
+          mbar_arrive(tempty_bar(acc));
 #pragma unroll
-          for (int k = 0; k < CH; ++k) {
-            const float v = I8 ? s8_value(r[k], s_us[u0 + k]) * rs : __uint_as_float(r[k]);
-            m[k] = row_ok ? round_bf(v) : -INFINITY;
-          }
-          // Maximum over the 32 rows for every column: at each exchange a lane keeps the half of its columns that its lane
-          // bit names and hands over the other half, so lane k ends with column k's and one store writes the group
-          // (a warp-wide reduction and a store of its own per column took 3 times the instructions: 995 -> 964 us for the whole
-          // call on bf16 rows, 1262 -> 1202 on int8).
-          if (CH == 16) {
+          for (int c = 0; c < CW / CH; ++c) {
+            uint32_t (&r)[CH] = rr[c];
+            const int u0 = part * CW + c * CH;
+            // First a filter.  Survivors are a few in 10^4 .. 10^5 elements, so for most groups the warp stops here; the exact
+            // per-column test below runs only for the rows that pass.
+            bool pass = true;
+            if (FOLDED) {
+              // sums below zero are no hits (the threshold is part of the sum)
+              uint32_t sign = r[0] & r[1];
 #pragma unroll
-            for (int k = 0; k < CH; ++k) m[k] = fmaxf(m[k], __shfl_xor_sync(0xffffffffu, m[k], 16));
-          }
+              for (int k = 2; k < CH; k += 2) sign &= r[k] & r[k + 1];
+              pass = (int)sign >= 0 || ((open >> (u0 / CH)) & 1);
+            } else if (!I8) {
+              // the largest of the row's CH scores against the smallest of the CH thresholds
+              float mx = max3(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]));
 #pragma unroll
-          for (int o = CH / 2; o >= 1; o >>= 1) {
-            const bool upper = lane & o;
+              for (int k = 3; k + 1 < CH; k += 2) mx = max3(mx, __uint_as_float(r[k]), __uint_as_float(r[k + 1]));
+              mx = fmaxf(mx, __uint_as_float(r[CH - 1]));
+              pass = mx >= s_thr_min[u0 / CH];
+            }
+            uint32_t rows_left = __ballot_sync(0xffffffffu, row_ok && pass);
+            if (FOLDED && rows_left && !have_rs) {
+              rs = row < a.rows ? __ldg(a.row_scale + row) : 0.f;
+              x_row = bias_x(bias_c, rs);
+              have_rs = true;
+            }
+            if (FOLDED ? __popc(rows_left) > 4 : I8) {
+              // More rows than are worth testing one by one: the bias said nothing about some query (its threshold is not
+              // positive, or out of the bias' range), or the rows' scales lie too far apart.  Or there is no bias.  The largest of the row's
+              // scores against the smallest threshold, then.  float(dot) * query scale without a conversion per element (those run
+              // at a fraction of the fp32 rate): 1.5 * 2^23 + dot is the integer sum of the bit patterns, and the fma takes the
+              // offset's product off again.  Two roundings: the product's, at most 0.75 of the query scale, and the fma's, at
+              // most 0.25 while |dot| < 2^22 (it is at most 128 * 127 * 256, which leaves 0.998 in all).  With the margin of one
+              // scale the bound is not below the unrounded dot * scale, so the roundings of the tested value, which keep order,
+              // cannot put it above the bound's.  A scale below zero (or no number) turns the order round: no filter then.
+              float mx = -INFINITY;
 #pragma unroll
-            for (int k = 0; k < o; ++k) {
-              const float keep = upper ? m[k + o] : m[k], give = upper ? m[k] : m[k + o];
-              m[k] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, give, o));
+              for (int k = 0; k < CH; k += 2) {
+                const float4 s2 = s_us2[(u0 + k) >> 1];
+                uint32_t d0 = r[k], d1 = r[k + 1];
+                if (FOLDED) { d0 += (uint32_t)(x_row * s_t[u0 + k]); d1 += (uint32_t)(x_row * s_t[u0 + k + 1]); }
+                const float2 x = make_float2(__uint_as_float(d0 + S8_OFFSET_BITS), __uint_as_float(d1 + S8_OFFSET_BITS));
+                const float2 v = __ffma2_rn(x, make_float2(s2.x, s2.y), make_float2(s2.z, s2.w));
+                mx = max3(mx, v.x, v.y);
+              }
+              pass = pass && (!(rs >= 0.f) || !((mx + s_us_max[u0 / CH]) * rs < s_thr_min[u0 / CH]));
+              rows_left = __ballot_sync(0xffffffffu, row_ok && pass);
+            }
+            // The few rows that pass, one at a time: the row's scores go through shared memory so that lane k holds column
+            // k's, every lane compares with its own column's threshold, and the hits line up in the queue by ballot.  (Each
+            // lane testing its own row over all columns cost the warp 150 instructions per group and 90 per hit.)
+            while (rows_left) {
+              const int src = __ffs(rows_left) - 1;
+              rows_left &= rows_left - 1;
+              if (lane == src) {
+#pragma unroll
+                for (int k = 0; k < CH; k += 4) *reinterpret_cast<uint4*>(s_row + k) = make_uint4(r[k], r[k + 1], r[k + 2], r[k + 3]);
+              }
+              __syncwarp();
+              const uint32_t word = lane < CH ? s_row[lane] : 0u;
+              const int dot = (int)word + (FOLDED ? __shfl_sync(0xffffffffu, x_row, src) * bt_lane[c] : 0);
+              const float v = I8 ? s8_value((uint32_t)dot, us_lane[c]) * __shfl_sync(0xffffffffu, rs, src) : __uint_as_float(word);
+              const bool hit = lane < CH && v >= t_lane[c];
+              const uint32_t hm = __ballot_sync(0xffffffffu, hit);
+              if (hm) {
+                const int n = __popc(hm);
+                if (nq + n > QCAP) { flush_queue(a, queue, nq, lane, flight); nq = 0; __syncwarp(); }
+                if (hit) {
+                  const uint32_t grow = (uint32_t)(a.row_offset + row - lane + src);
+                  queue[nq + __popc(hm & ((1u << lane) - 1u))] = make_uint4(0xFFFFFFFFu - grow, ord32(round_bf(v)), (uint32_t)(u0 + lane), 0u);
+                }
+                nq += n;
+              }
+              __syncwarp();
             }
           }
-          if (lane < CH && u0 + lane < a.B) a.gmax[(size_t)(u0 + lane) * a.n_groups + grp] = m[0];
+        } else {
+#pragma unroll 1
+          for (int c = 0; c < CW / CH; ++c) {
+            uint32_t r[CH];
+            tmem_ld_chunk<CH>(taddr + c * CH, r);
+            tmem_ld_wait();
+            const int u0 = part * CW + c * CH;
+            const long long grp = w * 4 + quad;
+            float m[CH];
+#pragma unroll
+            for (int k = 0; k < CH; ++k) {
+              const float v = I8 ? s8_value(r[k], s_us[u0 + k]) * rs : __uint_as_float(r[k]);
+              m[k] = row_ok ? round_bf(v) : -INFINITY;
+            }
+            // Maximum over the 32 rows for every column: at each exchange a lane keeps the half of its columns that its lane
+            // bit names and hands over the other half, so lane k ends with column k's and one store writes the group
+            // (a warp-wide reduction and a store of its own per column took 3 times the instructions: 995 -> 964 us for the whole
+            // call on bf16 rows, 1262 -> 1202 on int8).
+            if (CH == 16) {
+#pragma unroll
+              for (int k = 0; k < CH; ++k) m[k] = fmaxf(m[k], __shfl_xor_sync(0xffffffffu, m[k], 16));
+            }
+#pragma unroll
+            for (int o = CH / 2; o >= 1; o >>= 1) {
+              const bool upper = lane & o;
+#pragma unroll
+              for (int k = 0; k < o; ++k) {
+                const float keep = upper ? m[k + o] : m[k], give = upper ? m[k] : m[k + o];
+                m[k] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, give, o));
+              }
+            }
+            if (lane < CH && u0 + lane < a.B) a.gmax[(size_t)(u0 + lane) * a.n_groups + grp] = m[0];
+          }
+          tc_fence_before();
+          mbar_arrive(tempty_bar(acc));
         }
-        tc_fence_before();
-        mbar_arrive(tempty_bar(acc));
+        if (MODE == 1 && nq >= QFLUSH) {
+          flush_queue(a, queue, nq, lane, flight);
+          nq = 0;
+          __syncwarp();
+        }
       }
-      if (MODE == 1 && nq >= QFLUSH) {
+      if (MODE == 1) {   // what is left
         flush_queue(a, queue, nq, lane, flight);
-        nq = 0;
-        __syncwarp();
+        flight.land(a);
       }
-    }
-    if (MODE == 1) {   // what is left
-      flush_queue(a, queue, nq, lane, flight);
-      flight.land(a);
+    };
+    if constexpr (TWO_LOOPS) {
+      if (biased) consume(std::true_type()); else consume(std::false_type());
+    } else {
+      consume(std::integral_constant<bool, BIAS>());
     }
   }
 
@@ -527,23 +545,23 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   }
 }
 
-template <int MODE, bool I8, int NQ>
+template <int MODE, bool I8, int NQ, bool BIAS>
 phx_status launch_scan_tc(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, int grid, int* err_flag,
                           cudaStream_t stream, std::string& err) {
   const int kblk = a.row_bytes / 128;
-  const size_t smem = (size_t)kblk * NQ * 128 + (size_t)scan_stages(MODE, I8, kblk) * kblk * TC_ROWS * 128 + scan_bias_bytes(MODE, I8, NQ) + 2 * 256 * 4 + 64 + 128 * 16 + TC_CWARPS * (QCAP * 16 + 128) + 256 + 1024;
+  const size_t smem = (size_t)kblk * NQ * 128 + (size_t)scan_stages(BIAS, kblk) * kblk * TC_ROWS * 128 + scan_bias_bytes(BIAS, NQ) + 2 * 256 * 4 + 64 + 128 * 16 + TC_CWARPS * (QCAP * 16 + 128) + 256 + 1024;
   static SmemLimit limit;
-  PHX_CUDA_TRY(limit.raise(scan_tc_kernel<MODE, I8, NQ>, 227 * 1024), err);
-  PHX_CUDA_TRY(launch_programmatic(scan_tc_kernel<MODE, I8, NQ>, grid, scan_threads(MODE, I8), smem, stream, map_corpus, map_users, a, err_flag), err);
+  PHX_CUDA_TRY(limit.raise(scan_tc_kernel<MODE, I8, NQ, BIAS>, 227 * 1024), err);
+  PHX_CUDA_TRY(launch_programmatic(scan_tc_kernel<MODE, I8, NQ, BIAS>, grid, scan_threads(BIAS), smem, stream, map_corpus, map_users, a, err_flag), err);
   return PHX_OK;
 }
-template <int MODE, bool I8>
+template <int MODE, bool I8, bool BIAS>
 phx_status launch_scan_nq(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, int grid, int* err_flag,
                           cudaStream_t stream, std::string& err) {
   // query columns: the multiple of 64 that holds the batch (the tensor core and the consumers work on all NQ of them)
-  if (a.B <= 64) return launch_scan_tc<MODE, I8, 64>(map_corpus, map_users, a, grid, err_flag, stream, err);
-  if (a.B <= 128) return launch_scan_tc<MODE, I8, 128>(map_corpus, map_users, a, grid, err_flag, stream, err);
-  return launch_scan_tc<MODE, I8, 256>(map_corpus, map_users, a, grid, err_flag, stream, err);
+  if (a.B <= 64) return launch_scan_tc<MODE, I8, 64, BIAS>(map_corpus, map_users, a, grid, err_flag, stream, err);
+  if (a.B <= 128) return launch_scan_tc<MODE, I8, 128, BIAS>(map_corpus, map_users, a, grid, err_flag, stream, err);
+  return launch_scan_tc<MODE, I8, 256, BIAS>(map_corpus, map_users, a, grid, err_flag, stream, err);
 }
 
 }  // namespace
@@ -566,10 +584,13 @@ phx_status tc_scan_launch(const CUtensorMap& map_corpus, const CUtensorMap& map_
   if (grid <= 0) return PHX_OK;
   const bool i8 = a.row_scale != nullptr;
   if (mode == 0)
-    return i8 ? launch_scan_nq<0, true>(map_corpus, map_users, a, grid, err_flag, stream, err)
-              : launch_scan_nq<0, false>(map_corpus, map_users, a, grid, err_flag, stream, err);
-  return i8 ? launch_scan_nq<1, true>(map_corpus, map_users, a, grid, err_flag, stream, err)
-            : launch_scan_nq<1, false>(map_corpus, map_users, a, grid, err_flag, stream, err);
+    return i8 ? launch_scan_nq<0, true, false>(map_corpus, map_users, a, grid, err_flag, stream, err)
+              : launch_scan_nq<0, false, false>(map_corpus, map_users, a, grid, err_flag, stream, err);
+  if (!i8) return launch_scan_nq<1, false, false>(map_corpus, map_users, a, grid, err_flag, stream, err);
+  // Scales below zero turn the order of the sums round, and the sign of a sum says nothing in a corpus that has one: every group is
+  // open, or the bias is left out (one such row, 12.5 M rows, device us open / without: 256 queries 1545 / 1103, 100 847 / 690, one 539 / 589)
+  return a.scales_negative && a.B > 64 ? launch_scan_nq<1, true, false>(map_corpus, map_users, a, grid, err_flag, stream, err)
+                           : launch_scan_nq<1, true, true>(map_corpus, map_users, a, grid, err_flag, stream, err);
 }
 
 }  // namespace phx
