@@ -328,3 +328,33 @@ def test_int8_open_groups(B, negative, below):
     down = {"all": np.ones(B, bool), "some groups": np.arange(B) % 64 < 40, "one query": np.arange(B) == B // 2}[below]
     users[down] *= -1
     _int8_equals_the_oracle(N, dim, B, k, users, q8, s)
+
+
+@pytest.mark.parametrize("L", [20_000, 33_000, 36_000, 40_000, 90_000])
+@pytest.mark.parametrize("masked", [False, True])
+def test_short_list_with_its_rows_in_one_block(L, masked):
+    """The rows that matter stand together - a topic's posts uploaded in a row, or a mask that leaves one range: more of them than
+    the survivor buffer holds (32768), fewer than a sparse sample would notice.  The pivot still falls among them."""
+    from helpers import check_topk_against_scores
+    from x_algorithm_b200.retrieval import CorpusShard
+    N, dim, k, first = 1_200_000, 64, 10, 500_001
+    r = np.random.default_rng(L)
+    base = r.standard_normal(dim).astype(np.float32); base /= np.linalg.norm(base)
+    x = r.standard_normal((N, dim), dtype=np.float32) * np.float32(0.02)
+    if not masked:
+        x[first:first + L] = base + r.standard_normal((L, dim), dtype=np.float32) * np.float32(0.02)
+    bits = (x.view(np.uint32) >> 16).astype(np.uint16)
+    rows = (bits.astype(np.uint32) << 16).view(np.float32)
+    sh = CorpusShard(N, dim, max_queries=1, max_k=k)
+    sh.upload(0, bits)
+    eligible = np.ones(N, bool)
+    if masked:
+        eligible[:] = False
+        eligible[first:first + L] = True
+        sh.set_mask(eligible)
+    users = po.bf16_round((base + np.float32(0.05) * r.standard_normal(dim).astype(np.float32))[None]).astype(np.float32)
+    got_s, got_i = _topk(sh, users, k)
+    assert sh.exact_runs() == 0
+    scores = np.where(eligible[None], users @ rows.T, np.float32(-100))
+    check_topk_against_scores(scores, got_s, got_i, k)
+    sh.close()

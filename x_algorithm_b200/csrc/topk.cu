@@ -917,10 +917,13 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
     // Rows wanted at or above the pivot: 3k, and for short lists as many as keep the sample small.  Every stride-th tile is sampled
     // so that about 48 of them fall into the sample: with 3k alone a list of 10 had every tile scored twice.  A wanted row
     // costs about 0.14 ns a query in the collect pass and the select, a sampled tile as much as a collected one: the sum is
-    // smallest at sqrt(17.5 rows / queries).  Whole calls, 3k rows / this rule: 256 queries, 12.5 M rows, k = 10 1393 -> 739 us,
-    // k = 100 911 -> 752; one query 1170 -> 542; 3 M rows, k = 10 574 -> 262; 700 k rows, 16 queries 160 -> 125.
+    // smallest at sqrt(17.5 rows / queries).  Where the good rows stand together - a topic uploaded in a row, a mask that leaves one
+    // range - a block of L rows shows in L / (group_rows * stride) groups of the sample, and with fewer of them than the 48 the pivot
+    // falls below the block.  So short lists sample densely enough that a block as long as the survivor buffer has half as many again.
+    // Whole calls, us, 3k rows / up to 3000 / this rule: k = 10: 12.5 M rows, 256 queries 1435 / 738 / 755, one query 1139 / 498 / 531, 3 M rows 342 /
+    // 167 / 174, 700 k rows, 16 queries 142 / 86 / 86; k = 100, 256 queries 987 / 755 / 802; 1.2 M rows with one block of 40 k 168 / 1337 / 126.
     const double balanced = sqrt(17.5 * (double)rows / (double)B);
-    const double want = fmax(3.0 * k_real, fmin(3000.0, balanced));
+    const double want = fmax(3.0 * k_real, fmin((double)c->cap / (1.5 * group_rows), balanced));
     long long stride = (long long)(want / 48.0);
     if (stride < 1) stride = 1;
     long long sampled_tiles = (n_tiles + stride - 1) / stride;
