@@ -358,3 +358,36 @@ def test_short_list_with_its_rows_in_one_block(L, masked):
     scores = np.where(eligible[None], users @ rows.T, np.float32(-100))
     check_topk_against_scores(scores, got_s, got_i, k)
     sh.close()
+
+
+@pytest.mark.parametrize("through", ["sync", "communicator"])
+def test_short_list_among_rows_a_bf16_step_apart(through):
+    """A quarter of the corpus scores within a few bf16 steps of each other: a pivot for some hundred rows lets more of them through than the
+    survivor buffer holds, one for three times the list does not.  The call is done again with that one, not by the exact passes."""
+    import torch
+    from helpers import check_topk_against_scores
+    from x_algorithm_b200.retrieval import CorpusShard
+    N, dim, k, L = 1_200_000, 64, 10, 300_000
+    r = np.random.default_rng(2)
+    base = r.standard_normal(dim).astype(np.float32)
+    x = r.standard_normal((N, dim), dtype=np.float32) * np.float32(0.05)
+    x[500_001:500_001 + L] = base + r.standard_normal((L, dim), dtype=np.float32) * np.float32(0.02)
+    bits = (x.view(np.uint32) >> 16).astype(np.uint16)
+    rows = (bits.astype(np.uint32) << 16).view(np.float32)
+    sh = CorpusShard(N, dim, max_queries=1, max_k=k)
+    sh.upload(0, bits)
+    users = po.bf16_round((base + np.float32(0.1) * r.standard_normal(dim).astype(np.float32))[None]).astype(np.float32)
+    if through == "sync":
+        got_s, got_i = _topk(sh, users, k)
+    else:
+        from x_algorithm_b200 import comm as pc
+        cm = pc.Communicator(pc.unique_id(), 0, 1, 0)
+        u = torch.from_numpy(users).cuda()
+        sc = torch.empty((1, k), dtype=torch.float32, device="cuda"); ids = torch.empty((1, k), dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        cm.retrieve_topk(sh, u, 1, k, sc, ids)
+        got_s, got_i = sc.cpu().numpy(), ids.cpu().numpy()
+        cm.close()
+    assert sh.exact_runs() == 0
+    check_topk_against_scores(users @ rows.T, got_s, got_i, k, slack=1e-4)
+    sh.close()

@@ -526,12 +526,14 @@ struct phx_corpus {
   unsigned long long* keys_out = nullptr;   // set for one call by phx_corpus_topk_keys_device
   // exact passes (the sampled pivot missed, or phx_corpus_set_exact): per-user threshold keys found by bisection
   bool exact = false;
+  bool dense = false;            // set for one call: the sample is drawn for 3k rows whatever the list's length
   unsigned long long* thr = nullptr;        // device [256]
   long long exact_runs = 0;                 // calls completed through the exact passes
-  int reran = 0;                            // set by a sync that had to redo the last call exactly
-  // the last top-k call, kept so that phx_corpus_sync can redo it exactly when its status says the pivot missed
+  int reran = 0;                            // set by a sync that had to redo the last call
+  // the last top-k call, kept so that phx_corpus_sync can redo it when its status says the pivot missed
   struct LastCall {
     bool valid = false; const float* users = nullptr; int B = 0, k = 0; long long row_begin = 0, row_end = 0;
+    bool sparse = false;         // its sample was drawn for more than 3k rows
     float* scores = nullptr; long long* ids = nullptr; unsigned long long* keys = nullptr;
   } last;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -875,6 +877,7 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
   };
   c->last.valid = true; c->last.users = users_dev; c->last.B = B; c->last.k = k; c->last.row_begin = row_begin;
   c->last.row_end = row_end; c->last.scores = scores_dev; c->last.ids = (long long*)ids_dev; c->last.keys = c->keys_out;
+  c->last.sparse = false;
   c->state_fresh = false;
   PHX_CUDA_TRY(cudaEventRecord(c->ev0, c->stream), c->err);
   if (c->exact) {
@@ -923,7 +926,8 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
     // Whole calls, us, 3k rows / up to 3000 / this rule: k = 10: 12.5 M rows, 256 queries 1435 / 738 / 755, one query 1139 / 498 / 531, 3 M rows 342 /
     // 167 / 174, 700 k rows, 16 queries 142 / 86 / 86; k = 100, 256 queries 987 / 755 / 802; 1.2 M rows with one block of 40 k 168 / 1337 / 126.
     const double balanced = sqrt(17.5 * (double)rows / (double)B);
-    const double want = fmax(3.0 * k_real, fmin((double)c->cap / (1.5 * group_rows), balanced));
+    const double want = fmax(3.0 * k_real, c->dense ? 0.0 : fmin((double)c->cap / (1.5 * group_rows), balanced));
+    c->last.sparse = want > 3.0 * k_real;
     long long stride = (long long)(want / 48.0);
     if (stride < 1) stride = 1;
     long long sampled_tiles = (n_tiles + stride - 1) / stride;
@@ -1016,7 +1020,7 @@ phx_status phx_retrieve_topk(phx_comm* cm, phx_corpus* c, const float* users_dev
   cudaStream_t st = (cudaStream_t)stream;
   cudaStream_t saved = c->stream;
   c->stream = st;
-  struct Restore { phx_corpus* c; cudaStream_t s; ~Restore() { c->stream = s; c->keys_out = nullptr; c->exact = false; c->state_fresh = false; } } restore{c, saved};
+  struct Restore { phx_corpus* c; cudaStream_t s; ~Restore() { c->stream = s; c->keys_out = nullptr; c->exact = c->dense = false; c->state_fresh = false; } } restore{c, saved};
   int* my_word = cm->status_all + PHX_MAX_SHARDS;
   auto shard_list = [&]() -> phx_status {
     c->keys_out = cm->keys_local;
@@ -1039,29 +1043,28 @@ phx_status phx_retrieve_topk(phx_comm* cm, phx_corpus* c, const float* users_dev
   };
   phx_status s;
   if ((s = shard_list())) { cm->err = c->err; return s; }
-  if ((s = gather_and_merge())) return s;
-  int any = 0;
-  for (int r = 0; r < W; ++r) any |= cm->status_host[r];
-  if (any & 0x100) {
-    cudaMemsetAsync(c->err_flag, 0, sizeof(int), st);
-    c->err = cm->err = "phx_retrieve_topk: a bounded device-side wait ran out on some rank (scan pipeline)";
-    return PHX_E_TIMEOUT;
-  }
-  if (any & 3) {
-    // the sampled pivot missed on some shard: that shard takes the exact passes, every rank gathers and merges again
-    // (all ranks hold the same status words, so all take this branch together)
+  // Where the sampled pivot missed on some shard, that shard takes its list again - a short list first with a pivot for 3k rows, then by the
+  // exact passes - and every rank gathers and merges again (all ranks hold the same status words, so all take the same turns together)
+  const bool sparse = c->last.sparse;
+  for (int turn = 0;; ++turn) {
+    if ((s = gather_and_merge())) return s;
+    int any = 0;
+    for (int r = 0; r < W; ++r) any |= cm->status_host[r];
+    if (any & 0x100) {
+      cudaMemsetAsync(c->err_flag, 0, sizeof(int), st);
+      c->err = cm->err = "phx_retrieve_topk: a bounded device-side wait ran out on some rank (scan pipeline)";
+      return PHX_E_TIMEOUT;
+    }
+    if (!(any & 3)) return PHX_OK;
+    if (turn == 2) { c->err = cm->err = "phx_retrieve_topk: a shard's exact passes left a status behind"; return PHX_E_CAPACITY; }
     if (cm->status_host[cm->rank] & 3) {
       PHX_CUDA_TRY(cudaMemsetAsync(c->status, 0, sizeof(int), st), cm->err);
-      c->exact = true;
+      (turn == 0 && sparse ? c->dense : c->exact) = true;
       s = shard_list();
-      c->exact = false;
+      c->exact = c->dense = false;
       if (s) { cm->err = c->err; return s; }
     }
-    if ((s = gather_and_merge())) return s;
-    for (int r = 0; r < W; ++r)
-      if (cm->status_host[r] & 3) { c->err = cm->err = "phx_retrieve_topk: a shard's exact passes left a status behind"; return PHX_E_CAPACITY; }
   }
-  return PHX_OK;
 }
 
 phx_status phx_corpus_set_stream(phx_corpus* c, void* stream, int32_t use_own) {
@@ -1192,11 +1195,12 @@ phx_status phx_corpus_sync(phx_corpus* c) {
   c->state_fresh = false;
   const int ef = state[0];
   int st = state[2];
-  if (ef != 0) {
+  auto wait_ran_out = [&]() {
     cudaMemset(c->err_flag, 0, 4);
     c->err = "topk: a bounded device-side wait ran out (scan pipeline)";
     return PHX_E_TIMEOUT;
-  }
+  };
+  if (ef != 0) return wait_ran_out();
   if (st & 4) {
     cudaMemset(c->status, 0, 4);
     c->err = "topk merge: an id does not fit 32 bits; the entry was left out";
@@ -1204,19 +1208,25 @@ phx_status phx_corpus_sync(phx_corpus* c) {
   }
   if (st != 0 && c->last.valid && !c->exact) {
     // The sampled pivot missed for some query (fewer than k rows, or more than the survivor buffer holds, reached it):
-    // the call is done again with exact thresholds, into the same output buffers, before this sync returns.  The
-    // queries must still be where the call read them.
-    cudaMemset(c->status, 0, 4);
-    c->exact = true;
-    c->keys_out = c->last.keys;
-    const phx_status xs = phx_corpus_topk_window_device(c, c->last.users, c->last.B, c->last.k, c->last.row_begin, c->last.row_end,
-                                                        c->last.scores, (int64_t*)c->last.ids);
-    c->keys_out = nullptr;
-    c->exact = false;
-    c->state_fresh = false;
-    if (xs) return xs;
-    c->reran = 1;
-    PHX_CUDA_TRY(cudaMemcpy(&st, c->status, 4, cudaMemcpyDeviceToHost), c->err);
+    // the call is done again into the same output buffers before this sync returns, a short list first with a pivot for 3k rows (many
+    // rows a few bf16 steps apart, 300 k of them in 1.2 M rows, k = 10: 1512 us a call by the exact passes, 294 so), then with exact
+    // thresholds.  The queries must still be where the call read them.
+    const phx_corpus::LastCall call = c->last;
+    for (int exact = call.sparse ? 0 : 1; exact < 2 && st != 0; ++exact) {
+      PHX_CUDA_TRY(cudaMemsetAsync(c->status, 0, 4, c->stream), c->err);
+      (exact ? c->exact : c->dense) = true;
+      c->keys_out = call.keys;
+      const phx_status xs = phx_corpus_topk_window_device(c, call.users, call.B, call.k, call.row_begin, call.row_end, call.scores,
+                                                          (int64_t*)call.ids);
+      c->keys_out = nullptr;
+      c->exact = c->dense = false;
+      c->state_fresh = false;
+      if (xs) return xs;
+      c->reran = 1;
+      PHX_CUDA_TRY(cudaEventSynchronize(c->ev1), c->err);      // behind the re-run's last kernel and its state (close_call)
+      if (c->state_host[0]) return wait_ran_out();
+      st = c->state_host[2];
+    }
   }
   if (st != 0) {
     cudaMemset(c->status, 0, 4);

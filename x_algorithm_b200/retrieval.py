@@ -112,8 +112,8 @@ class CorpusShard:
         self._check(lib.phx_corpus_sync(self._h))
 
     def finish(self) -> bool:
-        """Wait for the shard's work; True when the last top-k had to be done again with exact thresholds (its output
-        buffers then hold the exact answer)."""
+        """Wait for the shard's work; True when the last top-k had to be done again (its output buffers then hold the
+        exhaustive answer)."""
         r = C.c_int32()
         self._check(lib.phx_corpus_finish(self._h, C.byref(r)))
         return bool(r.value)
