@@ -502,6 +502,7 @@ struct phx_corpus {
   int* status = nullptr;
   int* state_host = nullptr;     // pinned: flag and status as the last call left them (close_call)
   bool state_fresh = false;      // ... and nothing has changed them since
+  bool state_wanted = true;      // false inside phx_retrieve_topk, which gathers the ranks' status words itself
   bool use_tc = false;           // tcgen05 scan of the bf16 rows (dim 64 / 128), else the mma.sync scan
   bool use_tc_i8 = false;        // the same of the int8 rows (dim 128 / 256)
   // int8 form of the corpus (phx_corpus_upload_int8 / phx_corpus_quantize_int8) and whether calls score with it
@@ -590,9 +591,9 @@ phx_status convert_users(phx_corpus* c, const float* users_dev, int B, int Bpad)
 // The end of a call: flag and status follow its kernels into pinned memory, so that the wait for the call is all a check needs
 // (with two blocking copies of four bytes behind it one query over 1 M rows took 131 us, 106 without).
 phx_status close_call(phx_corpus* c) {
-  PHX_CUDA_TRY(cudaMemcpyAsync(c->state_host, c->err_flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->stream), c->err);
+  if (c->state_wanted) PHX_CUDA_TRY(cudaMemcpyAsync(c->state_host, c->err_flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->stream), c->err);
   PHX_CUDA_TRY(cudaEventRecord(c->ev1, c->stream), c->err);
-  c->state_fresh = true;
+  c->state_fresh = c->state_wanted;
   return PHX_OK;
 }
 
@@ -1020,7 +1021,11 @@ phx_status phx_retrieve_topk(phx_comm* cm, phx_corpus* c, const float* users_dev
   cudaStream_t st = (cudaStream_t)stream;
   cudaStream_t saved = c->stream;
   c->stream = st;
-  struct Restore { phx_corpus* c; cudaStream_t s; ~Restore() { c->stream = s; c->keys_out = nullptr; c->exact = c->dense = false; c->state_fresh = false; } } restore{c, saved};
+  c->state_wanted = false;
+  struct Restore {
+    phx_corpus* c; cudaStream_t s;
+    ~Restore() { c->stream = s; c->keys_out = nullptr; c->exact = c->dense = c->state_fresh = false; c->state_wanted = true; }
+  } restore{c, saved};
   int* my_word = cm->status_all + PHX_MAX_SHARDS;
   auto shard_list = [&]() -> phx_status {
     c->keys_out = cm->keys_local;
