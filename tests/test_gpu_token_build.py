@@ -87,3 +87,21 @@ def test_packed_results_are_laid_out_by_the_host(C):
             np.testing.assert_array_equal(a[q], o[0])
             assert not np.any(a[q, n:])
     eng.close()
+
+
+@pytest.mark.parametrize("D,actions", [(1024, 29), (1280, 19), (1536, 19)])
+def test_heads_at_one_and_two_strips_an_sm(D, actions):
+    """Wide rows: their strips in shared memory while one CTA an SM holds them all (148 strips of 16), four warps a strip up to
+    twice that, a warp a strip beyond: the same bits."""
+    kw = dict(emb_size=D, num_layers=1, num_q_heads=2, num_kv_heads=2, key_size=64, history_len=9, num_candidates=16, num_actions=actions,
+              widening_factor=1.0)
+    ocfg, w, rows_fn, eng = make_pair(max_batch=297, **kw)
+    b = po.make_batch(ocfg, 297, seed=5, ragged=True)
+    whole = eng.rank(to_inputs(b))
+    for n in (148, 149, 296):
+        part = type(b)(*[np.ascontiguousarray(a[:n]) for a in (b.hist_post_ids, b.hist_author_ids, b.hist_actions, b.hist_surfaces,
+                                                               b.cand_post_ids, b.cand_author_ids)])
+        some = eng.rank(to_inputs(part))
+        np.testing.assert_array_equal(some.log_probs, whole.log_probs[:n])
+        np.testing.assert_array_equal(some.continuous, whole.continuous[:n])
+    eng.close()

@@ -282,6 +282,7 @@ size_t heads_smem(int D) {
          (STAGED ? (size_t)16 * (D + HM_WPAD) * sizeof(bf16) : 0);
 }
 constexpr size_t HEADS_SMEM_MAX = 200 * 1024;
+constexpr size_t HEADS_SMEM_SM = 228 * 1024;    // an SM's, 1 KB of it taken by each CTA
 template <int NT, int WPS, bool STAGED>
 phx_status launch_heads_wps(const HeadsArgs& a, long long strips, cudaStream_t stream, std::string& err) {
   constexpr int WARPS = WPS == 1 ? HM_WARPS : WPS;
@@ -306,11 +307,17 @@ phx_status launch_heads_wps(const HeadsArgs& a, long long strips, cudaStream_t s
 }
 template <int NT>
 phx_status launch_heads_mma(const HeadsArgs& a, long long rows, cudaStream_t stream, std::string& err) {
-  // up to two CTAs of a strip each per SM; a third round of them costs more than a warp a strip (measured beside the kernel)
+  // Up to two CTAs of a strip each per SM; a third round of them costs more than a warp a strip (measured beside the kernel).  Staged
+  // rows and the sums of eight warps take half an SM or more from about D = 1024 on: where staged CTAs would need a second round
+  // and four-warp ones, whose rows stay in global memory, would not, those run (150 / 296 strips, us, staged / four warps: D = 1024, 30 outputs
+  // 31.2 / 27.1, 33.3 / 29.2; D = 1280, 20 outputs 35.3 / 27.1, 39.4 / 31.2; D = 1536 41.5 / 33.2, 47.6 / 37.4; two of either an SM: D = 1024, 18
+  // outputs 25.1 / 25.1, 27.1 / 26.9; one of either: D = 1664, 30 outputs 47.6 / 53.7, 53.7 / 62.0).
   const long long strips = (rows + 15) / 16;
   if (strips <= 2 * 148) {
-    if (heads_smem<NT, 8, true>(a.D) <= HEADS_SMEM_MAX) return launch_heads_wps<NT, 8, true>(a, strips, stream, err);
-    return launch_heads_wps<NT, 4, false>(a, strips, stream, err);    // rows too wide to stand beside the head matrix
+    const size_t staged = heads_smem<NT, 8, true>(a.D), plain = heads_smem<NT, 4, false>(a.D);
+    auto one_round = [&](size_t smem) { return strips <= 148 || 2 * (smem + 1024) <= HEADS_SMEM_SM; };
+    if (staged <= HEADS_SMEM_MAX && (one_round(staged) || !one_round(plain))) return launch_heads_wps<NT, 8, true>(a, strips, stream, err);
+    return launch_heads_wps<NT, 4, false>(a, strips, stream, err);
   }
   return launch_heads_wps<NT, 1, false>(a, strips, stream, err);
 }
