@@ -32,7 +32,7 @@ def test_tokens_a_warp(monkeypatch, B, S, C, D, H, pack):
     np.testing.assert_array_equal(got.continuous, want.continuous)
 
 
-@pytest.mark.parametrize("S,D,B", [(140, 256, 3), (144, 256, 3), (33, 128, 5), (200, 256, 2)])   # 72 KB of rows and statistics: 143 x 256
+@pytest.mark.parametrize("S,D,B", [(140, 256, 3), (144, 256, 3), (33, 128, 5), (200, 256, 2)])   # 72 KB of rows and statistics: 142 x 256
 def test_pooling_keeps_rows_where_they_fit(S, D, B):
     import torch
     ocfg, w, rows_fn, eng = make_pair(max_batch=B, emb_size=D, num_candidates=0, history_len=S, num_layers=1)
@@ -105,3 +105,71 @@ def test_heads_at_one_and_two_strips_an_sm(D, actions):
         np.testing.assert_array_equal(some.log_probs, whole.log_probs[:n])
         np.testing.assert_array_equal(some.continuous, whole.continuous[:n])
     eng.close()
+
+
+@pytest.mark.parametrize("compute,S,D", [("bf16", 142, 256), ("fp32", 71, 256)])     # the most rows of 512 / 1024 bytes that fit
+def test_pooling_bits_with_rows_in_shared_memory_and_without(compute, S, D):
+    """One history slot more moves the pooling from rows in shared memory to rows in global memory: users whose last slots are padding
+    come out the same to the bit from both."""
+    import torch
+    B, n = 3, S - 2
+    users = []
+    for slots in (S, S + 1):
+        ocfg, w, rows_fn, eng = make_pair(max_batch=B, emb_size=D, num_q_heads=2, num_kv_heads=2, key_size=32, num_candidates=0,
+                                          history_len=slots, num_layers=1, compute=compute)
+        b = po.make_batch(po.ModelConfig(history_len=n, num_candidates=1), B, seed=5, ragged=True)
+        dev = []
+        for a in (b.hist_post_ids, b.hist_author_ids, b.hist_actions, b.hist_surfaces):
+            wide = np.zeros((B, slots), a.dtype)
+            wide[:, :n] = a
+            dev.append(torch.from_numpy(wide).cuda())
+        out = torch.empty((B, D), dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        eng.user_tower_device(B, *dev, out)
+        eng.sync()
+        eng.close()
+        users.append(out.cpu().numpy())
+    assert np.isfinite(users[0]).all() and np.abs(users[0]).max() > 0
+    np.testing.assert_array_equal(users[0], users[1])
+
+
+@pytest.mark.parametrize("S,D", [(9, 256), (71, 256), (72, 256)])
+def test_pooling_of_fp32_rows(S, D):
+    """The full-precision tower against the oracle's: fp32 sums in another order through one layer, bound of the fp32 parity tests."""
+    import torch
+    B = 3
+    ocfg, w, rows_fn, eng = make_pair(max_batch=B, emb_size=D, num_candidates=0, history_len=S, num_layers=1, compute="fp32")
+    b = po.make_batch(po.ModelConfig(history_len=S, num_candidates=1), B, seed=5, ragged=True)
+    want = po.user_tower(ocfg, w, rows_fn, b)
+    users = torch.empty((B, D), dtype=torch.float32, device="cuda")
+    dev = [torch.from_numpy(a).cuda() for a in (b.hist_post_ids, b.hist_author_ids, b.hist_actions, b.hist_surfaces)]
+    eng.user_tower_device(B, *dev, users)
+    eng.sync()
+    eng.close()
+    ok = b.hist_post_ids[:, 0] != 0
+    assert rel_l2(users.cpu().numpy()[ok], want[ok]) < 1e-5
+
+
+@pytest.mark.parametrize("C", [30, 700])
+def test_packed_batch_without_any_candidate(C):
+    """No request has a candidate: nothing comes back, every slot reads zero, and the engine's next call is an ordinary one."""
+    import x_algorithm_b200 as px
+    B, S = 3, 9
+    ocfg, w, rows_fn, eng = make_pair(max_batch=B, emb_size=128, num_layers=2, num_q_heads=2, num_kv_heads=2, key_size=64, history_len=S,
+                                      num_candidates=C, engine_kw=dict(pack_ragged=True))
+    eng.set_blend(px.blend_spec_from_weights(px.ValueModelWeights(w=dict(po.make_blend_weights(1).w)), px.HEAD_NAMES_19, ocfg.num_actions))
+    b = po.make_batch(ocfg, B, seed=5, ragged=True)
+    want = eng.rank(to_inputs(b))
+    want_lp, want_s = want.log_probs.copy(), want.scores.copy()
+    posts, authors = b.cand_post_ids.copy(), b.cand_author_ids.copy()
+    b.cand_post_ids[:], b.cand_author_ids[:] = 0, 0
+    out = px.RankOutputs(np.full((B, C, ocfg.num_actions), np.nan, np.float32), np.full((B, C, ocfg.num_continuous), np.nan, np.float32),
+                         np.full((B, C), np.nan))
+    got = eng.rank(to_inputs(b), out)
+    assert not got.log_probs.any() and not got.continuous.any() and not got.scores.any()
+    b.cand_post_ids[:], b.cand_author_ids[:] = posts, authors
+    again = eng.rank(to_inputs(b))
+    eng.close()
+    assert np.any(want_lp)
+    np.testing.assert_array_equal(again.log_probs, want_lp)
+    np.testing.assert_array_equal(again.scores, want_s)
