@@ -226,9 +226,9 @@ __global__ void __launch_bounds__(256, 3) build_tokens_kernel(TokenBuildArgs a) 
 // instructions on the hash of one token - 64-bit multiplications and remainders on 2H lanes while the others wait - and
 // on its prologue.  Here a warp takes TPW tokens: lane l hashes slot l % SL of token l / SL (SL = 2H rounded up to a power of
 // two), then the warp walks over (token, 256 columns) pairs, the rows of two pairs in flight.  Same order of additions and
-// roundings: the same bits.  Kernel,
-// one token a warp / this one: 640 tokens of 512 columns 7.7 / 5.6 us, 10240: 19.9 / 13.7, 81920: 103.5 / 56.9 (419 MB of
-// rows, ids and results: HBM); 32768 of 256 columns 35.8 / 22.1; a ragged batch of 48 packed requests 44.6 / 20.9.
+// roundings: the same bits.  The kernel above without its options, as it stood here before / this one with the tokens a warp that the
+// launcher chooses: 640 tokens of 512 columns 7.7 / 5.6 us, 10240: 19.9 / 13.7, 81920: 103.5 / 56.9 (419 MB of rows, ids and
+// results, part of them from L2); 32768 of 256 columns 35.8 / 22.1; a ragged batch of 48 packed requests 44.6 / 20.9.
 template <int SL, int TPW>
 __global__ void __launch_bounds__(256, SL == 8 ? 2 : 3) build_tokens_bulk_kernel(TokenBuildArgs a) {
   static_assert(SL * TPW <= 32, "a lane per hash");
@@ -594,7 +594,7 @@ __global__ void corpus_fill_kernel(bf16* rows_ptr, long long global_row0, long l
 
 namespace {
 // Tokens a warp of the plain build takes.  Few tokens want a warp each (every warp is one round trip for ids and one for rows), many
-// want the hash shared.  1 / 2 / 4 / 8 tokens, us (2 hashes): D = 512: 2560 tokens 6.0 / 6.7 / 8.3 / 12.4, 5120: 8.8 / 8.4 / 9.5 /
+// want the hash shared.  The bulk kernel with 1 / 2 / 4 / 8 tokens, us (2 hashes): D = 512: 2560 tokens 6.0 / 6.7 / 8.3 / 12.4, 5120: 8.8 / 8.4 / 9.5 /
 // 13.6, 10240: 15.5 / 14.4 / 13.9 / 18.4, 20480: 25.9 / 21.3 / 21.3 / 21.8, 81920: 88 / 70 / 61 / 57; D = 256: 2048: 4.7 / 4.7 / 6.0 /
 // 8.3, 8192: 11.0 / 9.8 / 7.7 / 9.3, 32768: 36.7 / 25.8 / 22.3 / 21.9; D = 1024: 8688: 21.1 / 21.3 / 19.8 / 28.0.
 inline int tokens_per_warp(long long toks) { return toks < 4096 ? 1 : toks < 8192 ? 2 : toks < 32768 ? 4 : 8; }

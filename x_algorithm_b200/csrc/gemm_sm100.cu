@@ -360,7 +360,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const bool d64 = ROPE && !D128 && rope.dh == 64;
       // A thread is a row.  With one table row per position every lane of a load touched a cache line of its own, 32 tag
       // look-ups an instruction and 5.5 k cycles a 256-column tile, which is what the tile waited for; with positions
-      // as the fast index a load touches four lines at most.  User tower (32768 rows, K = 256, four layers) 517 -> 489 us,
+      // as the fast index a load touches four or five lines (more where a warp's rows cross a request).  User tower (32768 rows, K = 256, four layers) 517 -> 489 us,
       // two layers of 8 x 1086 rows with heads of 128 455 -> 449 us; full batches (K = 512) gain no more than runs differ.
       float4 ang[8];
       const float4* ang_col = nullptr;

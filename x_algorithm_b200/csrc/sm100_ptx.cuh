@@ -20,16 +20,15 @@ constexpr int ERR_FLAG_INTS = 2;
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // One lane of a converged warp, always the same one.  A role that one thread plays - issuing TMA copies, MMAs, commits - runs
-// under this predicate and not under `lane == 0`: those instructions take uniform registers, and only from elect.sync does the
-// compiler know that a single lane is active; under any other condition each of them gets a loop over the lanes that might
-// hold different operands.  Measured, one producer thread copying 16 KB tiles into a ring (wait, expect, copy a round): 294 cycles
-// a round under lane == 0, 176 here; 32 KB in two copies 442 against 264, which is the copies' own rate (124 bytes a cycle).
+// under this predicate and not under `lane == 0`, which is slower by measurement: one producer thread copying 16 KB tiles into a ring
+// (wait, expect, copy a round) takes 294 cycles a round under lane == 0, 176 here; 32 KB in two copies 442 against 264, which is the copies'
+// own rate (124 bytes a cycle).
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
   return p != 0;
 }
-// warp of the CTA this thread is in, in a form the compiler knows to be the same in all of its lanes
+// warp of the CTA this thread is in, taken from one lane
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {

@@ -61,9 +61,10 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// The kernels of one call form a chain of short launches; each is launched with launch_programmatic, lets the next one start its
-// set-up as soon as it runs itself, and waits for the one in front before it touches memory.  One query over 1 M rows
-// 136 -> 131 us a call, 16 queries over 50 k rows 99 -> 90.
+// The kernels of one call form a chain of short launches: the conversion of the queries, the tcgen05 scans and the pivot are launched with
+// launch_programmatic, let the next one start its set-up as soon as they run themselves, and wait for the one in front before they touch
+// memory (the select, the masked rows' padding and the mma.sync scans follow in plain stream order).  One query over 1 M rows 136 -> 131 us
+// a call, 16 queries over 50 k rows 99 -> 90.
 __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

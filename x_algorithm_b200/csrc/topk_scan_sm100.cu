@@ -2,20 +2,19 @@
 // phoenix/xrex/models/recsys_two_tower_model.py:2455-2456; its int8 form 2518-2533): the score tile of 128 corpus rows x NQ
 // queries is formed in TMEM and consumed there, so the only HBM traffic is the corpus itself, read once.
 //
-// Persistent kernel, one CTA per SM, 576 threads:
+// Persistent kernel, one CTA per SM, 576 threads (640 in the int8 collect pass with the threshold bias):
 //   warp 0      TMA producer: the query matrix once (stays in shared memory), then one corpus tile of 128 rows per
 //               stage (128-byte swizzle, 128-byte boxes: 64 bf16 or 128 int8 columns)
 //   warp 1      MMA issuer: tcgen05.mma M=128 (corpus rows) x N=NQ (queries), 32 bytes of a row per instruction
 //               (kind::f16: 16 bf16, fp32 sums; kind::i8: 32 int8, int32 sums), into one of two TMEM accumulators
-//   (int8 collect pass: warps 18, 19 write the rows' side of the threshold bias, see bias_x)
+//   (with the bias: warps 18, 19 write the rows' side of it, see bias_x)
 //   warps 2-17  consumers: each warp reads its 32-row lane quadrant and a quarter of the query columns with
 //               tcgen05.ld and either appends rows whose score reaches the query's threshold to the survivor list
 //               (collect pass) or reduces the 32-row maximum per query (sample pass)
 // An int8 row of 128 columns is the byte image of a bf16 row of 64: tiles, swizzle, descriptors and tensor maps are the
 // same, only the instruction kind and what a consumer makes of an accumulator differ.
-// Measured (256 queries, k = 1000, one 12.5 M-row shard of 128 columns, whole top-k call): int8 rows 3.98 ms on mma.sync,
-// 1.49 ms when they moved here, 1.20 before their threshold went into the sum, 0.85 now (64 queries 0.68 -> 0.42); bf16 rows 1.28 ms with 8 consumer warps, 1.17 with 16, 0.87 now; one query over
-// 1 M rows 227 -> 213 us with 64 query columns instead of 256.
+// Measured (256 queries, k = 1000, one 12.5 M-row shard of 128 columns, whole top-k call, each pair on one box): int8 rows 1198 -> 840 us
+// when their thresholds went into the sum, 835 -> 772 with the consumers' loop compiled twice; bf16 rows 910 us.
 // All mbarrier waits are bounded; on expiry *err_flag is raised and the kernel unwinds.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
