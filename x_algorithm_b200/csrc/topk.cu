@@ -919,18 +919,26 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
   int j = 0;
   // a window whose eligible rows all fit the survivor buffer needs no pivot: every eligible row is collected
   if (rows > c->cap && !(c->mask && c->elig_count <= c->cap)) {
-    // Rows wanted at or above the pivot: 3k, and for short lists as many as keep the sample small.  Every stride-th tile is sampled
-    // so that about 48 of them fall into the sample: with 3k alone a list of 10 had every tile scored twice.  A wanted row
-    // costs about 0.14 ns a query in the collect pass and the select, a sampled tile as much as a collected one: the sum is
-    // smallest at sqrt(17.5 rows / queries).  Where the good rows stand together - a topic uploaded in a row, a mask that leaves one
-    // range - a block of L rows shows in L / (group_rows * stride) groups of the sample, and with fewer of them than the 48 the pivot
-    // falls below the block.  So short lists sample densely enough that a block as long as the survivor buffer has half as many again.
-    // Whole calls, us, 3k rows / up to 3000 / this rule: k = 10: 12.5 M rows, 256 queries 1435 / 738 / 755, one query 1139 / 498 / 531, 3 M rows 342 /
-    // 167 / 174, 700 k rows, 16 queries 142 / 86 / 86; k = 100, 256 queries 987 / 755 / 802; 1.2 M rows with one block of 40 k 168 / 1337 / 126.
-    const double balanced = sqrt(17.5 * (double)rows / (double)B);
-    const double want = fmax(3.0 * k_real, c->dense ? 0.0 : fmin((double)c->cap / (1.5 * group_rows), balanced));
+    // Rows wanted at or above the pivot, and how many of them (`picks`) the sample is to hold: every (want / picks)-th tile is scored for
+    // it.  3k and 48 serve every list; a list of 10 has every tile scored twice that way.  A short list may want more rows: a wanted row costs
+    // about 0.14 ns a query in the collect pass and the select, a sampled tile as much as a collected one, and the more rows a list
+    // has to spare the fewer picks keep it from running short: with want = r k and j picks that is the chance of a sum of j exponential
+    // variables below j / r, at most exp(-j (1 / r - 1 + ln r)) (Chernoff), here e^-14 a query, and a call that missed is done again.
+    // Where the good rows stand together - a topic uploaded in a row, a mask that leaves one range - a block of L rows shows in
+    // L picks / (group_rows want) groups of the sample, and with fewer of them than the picks the pivot falls below the block: want is
+    // bounded so that a block as long as the survivor buffer has half as many again.
+    // Whole calls, us, 3k rows and 48 picks / up to 3000 rows and 48 picks / this rule: k = 10: 12.5 M rows, 256 queries 1466 / 726 / 680, one query
+    // 1139 / 497 / 504, 3 M rows 336 / 162 / 162, 700 k rows, 16 queries 143 / 86 / 79; k = 100, 256 queries 983 / 765 / 683; k = 200, 10 queries
+    // 572 / 519 / 523; 1.2 M rows with one block of 40 k 168 / 1337 / 81.
+    const double limit = c->dense ? 0.0 : (double)c->cap / (1.5 * group_rows), unit = 17.5 * (double)rows / (double)B;
+    double want = 3.0 * k_real, picks = 48.0, cost = want + unit / want;
+    for (double w = want; w < limit;) {
+      w = fmin(1.25 * w, limit);
+      const double r = w / k_real, j = fmin(48.0, fmax(16.0, 14.0 / (1.0 / r - 1.0 + log(r)))), t = w + unit * (j / 48.0) / w;
+      if (t < cost) { want = w; picks = j; cost = t; }
+    }
     c->last.sparse = want > 3.0 * k_real;
-    long long stride = (long long)(want / 48.0);
+    long long stride = (long long)(want / picks);
     if (stride < 1) stride = 1;
     long long sampled_tiles = (n_tiles + stride - 1) / stride;
     while (sampled_tiles * 4 * (long long)B > c->gmax_elems) { stride *= 2; sampled_tiles = (n_tiles + stride - 1) / stride; }
