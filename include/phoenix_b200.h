@@ -526,7 +526,7 @@ phx_status phx_topk_merge_static_status(int32_t device, void* stream, int32_t* s
 /* Wait for the shard's work and report what went wrong in it.  The fast top-k keeps the rows at or above a pivot
  * estimated from a sample of the corpus; when a query's pivot turns out too high (fewer than k rows reach it) or too low
  * (more rows than the survivor buffer holds: long runs of equal scores, clustered rows), the sync does that call again
- * into the same output buffers - a short list first with a pivot from a denser sample, then with exact thresholds:
+ * into the same output buffers - a short list first with the pivot of a longer one's sample, then with exact thresholds:
  * bisection on the 64-bit (score, row) key with one counting scan per step - so a top-k call followed by a sync always
  * yields the exhaustive answer, as the reference's top_k does
  * (cuda/top_k_by_key/__init__.py:56-94).  The query buffer of the call must still hold the queries.
@@ -561,7 +561,7 @@ phx_status phx_comm_barrier(phx_comm* c, void* stream);
  * queries): this rank's shard is scanned for its top-k, the per-shard lists travel in one NCCL all-gather (one 64-bit
  * key per entry) together with every shard's status word, every rank merges them by (score desc, row asc) into
  * scores_dev f32 [B,k] / ids_dev int64 [B,k] (global rows), and the call returns when the result is ready.  If the
- * sampled pivot missed on any shard, that shard repeats its scan with exact thresholds and all ranks gather and merge
+ * sampled pivot missed on any shard, that shard repeats its scan as phx_corpus_sync does and all ranks gather and merge
  * again, so the answer is always the exhaustive top-k.  Replaces compute_top_k under shard_map: shard-local top-k,
  * all_gather, top_k (recsys_two_tower_model.py:2455-2516, 193-221).  `stream`: a cudaStream_t of the shard's device the
  * work is ordered on (NULL = default stream). */

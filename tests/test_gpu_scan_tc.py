@@ -391,3 +391,22 @@ def test_short_list_among_rows_a_bf16_step_apart(through):
     assert sh.exact_runs() == 0
     check_topk_against_scores(users @ rows.T, got_s, got_i, k, slack=1e-4)
     sh.close()
+
+
+@pytest.mark.parametrize("k", [1, 10, 60, 150, 220, 300])
+def test_short_lists_do_not_run_short(k):
+    """However few rows the sample holds for a short list, the pivot leaves enough of them: over 1024 queries (4 calls of 256, where want is
+    smallest) no call is done again.  The bound per query is e^-14."""
+    import torch
+    from x_algorithm_b200.retrieval import CorpusShard
+    N, B = 1_000_000, 256
+    sh = CorpusShard(N, 64, max_queries=B, max_k=k)
+    sh.fill_synthetic(5)
+    sc = torch.empty((B, k), dtype=torch.float32, device="cuda"); ids = torch.empty((B, k), dtype=torch.int64, device="cuda")
+    for seed in range(4):
+        u = torch.from_numpy(_users(B, 64, seed)).cuda()
+        torch.cuda.synchronize()
+        sh.topk_device(u, B, k, sc, ids)
+        assert not sh.finish()
+        assert (ids.sort(dim=1).values.diff(dim=1) > 0).all() and (sc.diff(dim=1) <= 0).all()
+    sh.close()
