@@ -1,0 +1,44 @@
+"""The streaming attention kernel at the edges of its key blocks and query tiles, and with every kind of row in every place, against a
+plain fp32 reference: candidates whose tile is half padding, rows that attend to themselves inside the history, no history at all."""
+import math
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(q, k, v, seg, S, scale):
+    import torch
+    q, k, v = q.float(), k.float(), v.float()
+    g = q.shape[2] // k.shape[2]
+    k, v = k.repeat_interleave(g, 2), v.repeat_interleave(g, 2)
+    s = torch.einsum("bqhd,bkhd->bhqk", q, k[:, :S]) * scale
+    s = s.masked_fill((seg[:, None, None, :S] != 1), -math.inf)
+    own = ((q * k).sum(-1) * scale).permute(0, 2, 1)[..., None].masked_fill((seg != -1)[:, None, :, None], -math.inf)
+    p = torch.nan_to_num(torch.softmax(torch.cat((s, own), -1), -1))
+    o = torch.einsum("bhqk,bkhd->bqhd", p[..., :S], v[:, :S]) + p[..., S:].permute(0, 2, 1, 3) * v
+    return o * (seg != 0)[:, :, None, None]
+
+
+@pytest.mark.parametrize("dh,H,Hk", [(128, 4, 2), (64, 4, 4)])
+@pytest.mark.parametrize("S,C", [(0, 5), (0, 129), (1, 1), (63, 64), (64, 65), (65, 127), (127, 129), (129, 63), (192, 200), (193, 1), (257, 0), (1025, 130)])
+def test_streaming_edges(monkeypatch, dh, H, Hk, S, C):
+    import torch
+    from x_algorithm_b200.engine import dispatch_counts, ranker_attention
+    monkeypatch.setenv("PHX_ATTN", "tcgen05")
+    B, T = 3, S + C
+    g = torch.Generator(device="cuda").manual_seed(S * 131 + C)
+    q, k, v = (torch.randn(B, T, h, dh, device="cuda", generator=g).to(torch.bfloat16) for h in (H, Hk, Hk))
+    seg = torch.ones((B, T), dtype=torch.int32, device="cuda")
+    seg[:, S:] = -1
+    seg[1, S + C // 2:] = 0                       # half of the candidates are padding: whole halves of a tile without a self key
+    seg[1, : S // 3] = 0
+    seg[2, S // 2: S: 7] = -1                     # rows of the history that are no keys and attend to themselves
+    before = dispatch_counts()["attn.tcgen05"]
+    got, _ = ranker_attention(q, k, v, seg, S, 1.0 / math.sqrt(dh))
+    assert dispatch_counts()["attn.tcgen05"] == before + 1
+    want = reference(q, k, v, seg, S, 1.0 / math.sqrt(dh))
+    assert bool((got[seg == 0] == 0).all())
+    # P and the output are rounded to bf16 (2^-9 each, at most a row's largest |v| in all), scores are fp32 sums of exact products
+    assert (got.float() - want).abs().max() <= 2.0 ** -7 * v.float().abs().max()
+    assert torch.linalg.norm(got.float() - want) <= 2.0 ** -8 * torch.linalg.norm(want)

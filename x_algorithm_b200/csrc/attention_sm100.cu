@@ -2,15 +2,22 @@
 // attention.cu (mask: phoenix/xrex/pallas/ranker_attention_utils.py:16-56; softmax and P rounding:
 // phoenix/xrex/pallas/ranker_attention_v2.py:113-148, 183).
 //
-// One CTA = 128 query rows of one (batch, head), 192 threads:
-//   warp 0      TMA producer: the Q tile once, then per key block the K tile and the V tile (3-D tensor maps over
+// Streaming kernel: one CTA = 128 query rows of one (batch, head), 192 threads, two CTAs an SM:
+//   warp 0      TMA producer: the Q tile once, then per key block the K tile and the V tile, then - if any of the tile's
+//               queries attends to itself - the tile's own K and V rows as blocks more (3-D tensor maps over
 //               [batch][token][column]: rows past the request's last token are zero-filled, never the next request's)
-//   warp 1      MMA issuer: S = Q K^T into TMEM (M=128, N=keys of the block), later O += P V with P read from shared
-//               memory (K-major) and V as an MN-major operand straight from its row-major tile
+//   warp 1      MMA issuer: S = Q K^T into TMEM (M=128, N=keys of the block), later O += P V with P read from tensor
+//               memory and V as an MN-major operand straight from its row-major tile
 //   warps 2-5   softmax: thread = query row; S row from TMEM, mask / max / exp2 / row sum in registers, P rounded to
-//               bf16 into swizzled shared memory, O rescaled in TMEM when the running max moved; at the end the
-//               candidate's self key is folded in with a per-row dot product, O is normalised, staged in shared
-//               memory and written with TMA stores
+//               bf16 back into tensor memory over the S columns, O rescaled there when the row's reference moved; at the end
+//               the candidate's self key is folded in with a per-row dot product over the rows in shared memory, O is
+//               normalised, staged in shared memory and written with TMA stores
+// What bounds it: the 1000 W cap (SM clock 1.5-1.7 GHz) and, per block of keys, the softmax warps' chain.  Before a row's own K and V came
+// by TMA, every thread fetched them with plain loads, 13-19 of a CTA's 45 thousand cycles; with that, keys' validity read eight words a round
+// trip, exponentials packed chunk by chunk and no wait for the output's last write (device us, 16 heads of 128, before / now): 32 x (1024 + 1024
+// rows) 628-670 / 565, 4 x (1024 + 2048) 149 / 126, 4 x (128 + 2048) 80 / 45, 8 x (1022 + 64), 4 kv heads 91-98 / 88; heads of 64, 4 x (1024 +
+// 512) 70-77 / 63.  Tried in its place: blocks of 128 keys with one S buffer (600; 4096 keys 751 against 682), that as two persistent CTAs an SM
+// (597), a quarter or a third of the exponentials as polynomials on the fma pipe (a twentieth slower: power, not the special-function unit).
 // Only history keys are ever multiplied: the candidate x candidate block does not exist in this kernel.
 // Waits are bounded; when one runs out the flag is raised and every later wait returns at once, so all roles
 // drain through the same control flow (no thread is left at a barrier) and the host reports PHX_E_TIMEOUT.
@@ -32,7 +39,9 @@ using namespace sm100;
 constexpr int QT = 128;            // query rows per CTA
 constexpr int A_THREADS = 192;
 constexpr int SLAB = QT * 128;     // bytes of one [128 rows x 64 bf16] swizzled tile
-constexpr int TC_MAX_BLOCKS = 256; // key blocks whose validity words fit the CTA's table
+// keys per block of the streaming kernel: its Q, K and V tiles take 96 or 64 KB, two CTAs an SM
+__host__ __device__ constexpr int key_block(int dh) { return dh == 64 ? 128 : 64; }
+constexpr int TC_MAX_KEYS = 16384; // history keys whose validity bits fit the CTA's table
 
 __device__ __forceinline__ float ex2f(float x) {
   float y;
@@ -55,6 +64,12 @@ __device__ __forceinline__ void st_shared_16(uint32_t addr, uint4 v) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
+__device__ __forceinline__ uint4 ld_shared_16(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
 struct AttnTcArgs {
   const bf16* q; const bf16* k; const bf16* v;          // for the per-row self term (plain loads)
   bf16* out;                                            // [B*T][Hq][dh], for kernels that store rows directly
@@ -73,8 +88,8 @@ struct AttnTcArgs {
 __device__ __forceinline__ int q_column(int h, int head_stride, int group, int group_stride) {
   return group <= 1 ? h * head_stride : (h / group) * group_stride + (h % group) * head_stride;
 }
-// the tensor maps of a streaming launch: Q / out over the history block and over the candidate block, K / V over history
-struct TcMaps { CUtensorMap qh, qc, k, v, oh, oc; };
+// the tensor maps of a streaming launch: Q / out, K and V over the history block and over the candidate block
+struct TcMaps { CUtensorMap qh, qc, k, v, kc, vc, oh, oc; };
 
 // D[tmem] (+)= A[tmem] * B[smem desc]: the A operand (bf16 pairs, one row per lane) comes from tensor memory
 __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
@@ -120,26 +135,28 @@ __device__ __forceinline__ void tmem_ld_wait_on(float (&r)[32]) {
 template <int DH, bool CAP>
 __global__ void __launch_bounds__(A_THREADS, 2)
 ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
-  constexpr int KBLK = (DH == 64) ? 128 : 64;   // keys per block (keeps shared memory at 80 KB: two CTAs per SM)
   constexpr int DCH = DH / 64;                  // 64-column chunks of the head dim
-  // S is double-buffered in TMEM (and K in shared memory): S of block j+1 is computed while the softmax warps are
-  // still on block j, so the tensor pipe and the softmax overlap inside one CTA.  KBLK <= 64 or two S buffers of
-  // 128 columns would not fit next to O in the CTA's 256 columns; at head dim 64 (KBLK 128) S stays single.
+  constexpr int KBLK = key_block(DH);
+  // S is double-buffered in TMEM (and K in shared memory) where two buffers fit next to O in the CTA's 256 columns: S of block
+  // j + 1 is computed while the softmax warps are still on block j.  At head dim 64 (KBLK 128) S stays single.
   constexpr int NSB = (KBLK <= 64) ? 2 : 1;     // S buffers (TMEM) = K buffers (shared memory)
+  constexpr int OWN = QT / KBLK;                // blocks that the tile's own K or V rows make
+  constexpr uint32_t TILE = DCH * SLAB;         // bytes of 128 rows of one head
+  constexpr uint32_t BLK = DCH * KBLK * 128;    // bytes of a block of keys
   constexpr uint32_t TM_S = 0, TM_O = 128;      // TMEM columns of S (NSB x KBLK) and O
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sQ = base;                               // DCH x [128 x 128 B]; reused to stage the output
-  const uint32_t sK = sQ + DCH * SLAB;                    // NSB x DCH x [KBLK x 128 B]
-  const uint32_t sV = sK + NSB * DCH * KBLK * 128;        // 2 x DCH x [KBLK x 128 B]
-  const uint32_t sMask = sV + 2 * DCH * KBLK * 128;       // [TC_MAX_BLOCKS][4] key-validity words
-  const uint32_t bars = sMask + TC_MAX_BLOCKS * 16;
-  const uint32_t q_full = bars, p_ready = bars + 24, o_done = bars + 32, tmem_slot = bars + 88;
-  auto v_full = [&](int i) { return bars + (i ? 96u : 8u); };
-  auto v_empty = [&](int i) { return bars + (i ? 104u : 16u); };
+  const uint32_t sK = sQ + TILE;                          // NSB blocks
+  const uint32_t sV = sK + NSB * BLK;                     // 2 blocks
+  const uint32_t sMask = sV + 2 * BLK;                    // one validity bit per key
+  const uint32_t bars = sMask + TC_MAX_KEYS / 8;
+  const uint32_t q_full = bars, p_half = bars + 8, p_ready = bars + 16, o_done = bars + 24, tmem_slot = bars + 32;
   auto k_full = [&](int i) { return bars + 40u + 8u * i; };
   auto k_empty = [&](int i) { return bars + 56u + 8u * i; };
   auto s_full = [&](int i) { return bars + 72u + 8u * i; };
+  auto v_full = [&](int i) { return bars + 88u + 8u * i; };
+  auto v_empty = [&](int i) { return bars + 104u + 8u * i; };
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
   uint32_t* mask_words = reinterpret_cast<uint32_t*>(smem_raw + (sMask - smem_u32(smem_raw)));
 
@@ -149,13 +166,17 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
   const int q0 = ((int)blockIdx.x - (cand_tile ? a.hist_tiles : 0)) * QT;
   const int hk = h / (a.Hq / a.Hkv);
   const int qcol = q_column(h, a.q_head_stride, a.q_group, a.q_group_stride);
+  const int kcol = hk * a.k_head_stride, vcol = hk * a.v_head_stride;
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_hist = a.n_hist;
   const int n_blocks = (n_hist + KBLK - 1) / KBLK;
+  const long long hist0 = a.hist_row0 + (long long)b * a.hist_req_rows;
+  const long long tok0 = (cand_tile ? a.cand_row0 + (long long)b * a.cand_req_rows : hist0) + q0;   // token row of the tile's first query
+  const int rows_in = (cand_tile ? a.n_cand : n_hist) - q0;                                         // queries from there on
   volatile int* verr = a.err_flag;
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1); mbar_init(p_ready, 128); mbar_init(o_done, 1);
+    mbar_init(q_full, 1); mbar_init(p_half, 128); mbar_init(p_ready, 128); mbar_init(o_done, 1);
     for (int i = 0; i < 2; ++i) { mbar_init(k_full(i), 1); mbar_init(k_empty(i), 1); mbar_init(s_full(i), 1); mbar_init(v_full(i), 1); mbar_init(v_empty(i), 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -171,39 +192,61 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
+    int seg_own[4];                       // does any query of the tile attend to itself?
+#pragma unroll
+    for (int i = 0; i < 4; ++i) seg_own[i] = (i * 32 + lane < rows_in) ? a.seg[tok0 + i * 32 + lane] : 0;
+    auto load_k = [&](const CUtensorMap* m, int j, int row) {   // block j: the buffer is free once S of block j - NSB has been computed
+      const int kb = j % NSB;
+      mbar_wait(k_empty(kb), (uint32_t)((j / NSB) & 1) ^ 1u, verr);
+      mbar_expect_tx(k_full(kb), BLK);
+      for (int c = 0; c < DCH; ++c) tma_load_3d(sK + kb * BLK + c * KBLK * 128, m, k_full(kb), kcol + c * 64, row, b);
+    };
+    auto load_v = [&](const CUtensorMap* m, int j, int row) {   // V is double-buffered: block j + 1 arrives under P V of block j
+      const int vb = j & 1;
+      mbar_wait(v_empty(vb), (uint32_t)((j >> 1) & 1) ^ 1u, verr);
+      mbar_expect_tx(v_full(vb), BLK);
+      for (int c = 0; c < DCH; ++c) tma_load_3d(sV + vb * BLK + c * KBLK * 128, m, v_full(vb), vcol + c * 64, row, b);
+    };
     if (elect_one()) {
-      mbar_expect_tx(q_full, DCH * SLAB);
+      mbar_expect_tx(q_full, TILE);
       for (int c = 0; c < DCH; ++c) tma_load_3d(sQ + c * SLAB, cand_tile ? &maps.qc : &maps.qh, q_full, qcol + c * 64, q0, b);
-      auto load_k = [&](int j) {   // K block j into buffer j % NSB, once S of block j - NSB has been computed
-        const int kb = j % NSB; const uint32_t use = (uint32_t)(j / NSB);
-        mbar_wait(k_empty(kb), (use & 1) ^ 1, verr);
-        mbar_expect_tx(k_full(kb), DCH * KBLK * 128);
-        for (int c = 0; c < DCH; ++c)
-          tma_load_3d(sK + (kb * DCH + c) * KBLK * 128, &maps.k, k_full(kb), hk * a.k_head_stride + c * 64, j * KBLK, b);
-      };
-      for (int j = 0; j < NSB - 1 && j < n_blocks; ++j) load_k(j);
-      for (int j = 0; j < n_blocks; ++j) {
-        if (j + NSB - 1 < n_blocks) load_k(j + NSB - 1);
-        const int vb = j & 1;                           // V is double-buffered: block j + 1 arrives under P V of block j
-        mbar_wait(v_empty(vb), (uint32_t)((j >> 1) & 1) ^ 1u, verr);
-        mbar_expect_tx(v_full(vb), DCH * KBLK * 128);
-        for (int c = 0; c < DCH; ++c)
-          tma_load_3d(sV + (vb * DCH + c) * KBLK * 128, &maps.v, v_full(vb), hk * a.v_head_stride + c * 64, j * KBLK, b);
+      for (int j = 0; j < NSB && j < n_blocks; ++j) load_k(&maps.k, j, j * KBLK);
+      if (n_blocks > 0) load_v(&maps.v, 0, 0);
+    }
+    __syncwarp();
+    const bool self = __any_sync(0xffffffffu, seg_own[0] == -1 || seg_own[1] == -1 || seg_own[2] == -1 || seg_own[3] == -1);
+    if (elect_one()) {
+      // behind the blocks of keys come the tile's own K and V rows, as OWN blocks more
+      const int n_all = n_blocks + (self ? OWN : 0);
+      const CUtensorMap* const ko = cand_tile ? &maps.kc : &maps.k;
+      const CUtensorMap* const vo = cand_tile ? &maps.vc : &maps.v;
+      auto next_k = [&](int j) { if (j < n_blocks) load_k(&maps.k, j, j * KBLK); else if (j < n_all) load_k(ko, j, q0 + (j - n_blocks) * KBLK); };
+      auto next_v = [&](int j) { if (j < n_blocks) load_v(&maps.v, j, j * KBLK); else if (j < n_all) load_v(vo, j, q0 + (j - n_blocks) * KBLK); };
+      for (int j = n_blocks; j < NSB; ++j) next_k(j);         // fewer blocks of keys than buffers
+      for (int j = (n_blocks > 0 ? 1 : 0); j < n_all; ++j) {
+        const int jk = j - 1 + NSB;                           // K runs NSB - 1 blocks ahead of V
+        if (jk >= NSB) next_k(jk);
+        next_v(j);
+      }
+      for (int j = n_blocks; j < n_all; ++j) {                // rows that nobody attends to as themselves are waited for by nobody else
+        mbar_wait(k_full(j % NSB), (uint32_t)((j / NSB) & 1), verr);
+        mbar_wait(v_full(j & 1), (uint32_t)((j >> 1) & 1), verr);
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
-      constexpr uint32_t idesc_s = make_idesc(QT, KBLK);
       constexpr uint32_t idesc_o = make_idesc_b_mn(QT, DH);
       mbar_wait(q_full, 0, verr);
+      auto short_block = [&](int j) { return NSB == 1 && n_hist - j * KBLK <= KBLK / 2; };   // a last block of at most 64 of 128 keys
       auto issue_s = [&](int j) {   // S(j) = Q K(j)^T into S buffer j % NSB
-        const int kb = j % NSB; const uint32_t use = (uint32_t)(j / NSB);
-        mbar_wait(k_full(kb), use & 1, verr);
+        const int kb = j % NSB;
+        const uint32_t idesc_s = short_block(j) ? make_idesc(QT, KBLK / 2) : make_idesc(QT, KBLK);
+        mbar_wait(k_full(kb), (uint32_t)((j / NSB) & 1), verr);
         tc_fence_after();
 #pragma unroll
         for (int c = 0; c < DCH; ++c) {
-          const uint64_t qd = make_smem_desc(sQ + c * SLAB), kd = make_smem_desc(sK + (kb * DCH + c) * KBLK * 128);
+          const uint64_t qd = make_smem_desc(sQ + c * SLAB), kd = make_smem_desc(sK + kb * BLK + c * KBLK * 128);
 #pragma unroll
           for (int k = 0; k < 4; ++k) umma_bf16(tmem + TM_S + kb * KBLK, qd + (uint64_t)(k * 2), kd + (uint64_t)(k * 2), idesc_s, (c | k) != 0);
         }
@@ -215,15 +258,20 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
         const uint32_t ph = (uint32_t)(j & 1);
         // the S buffer of block j + NSB - 1 was last read by the softmax of block j - 1, whose P has been awaited below
         if (j + NSB - 1 < n_blocks) issue_s(j + NSB - 1);
+        // P sits in tensor memory, as bf16 pairs over the first half of its S buffer (16 keys = 8 columns per step).  Where S is
+        // single, the product's first half runs under the exponentials of the second.
         const int vb = j & 1;
-        mbar_wait(p_ready, ph, verr);
         mbar_wait(v_full(vb), (uint32_t)((j >> 1) & 1), verr);
+        mbar_wait(NSB == 1 ? p_half : p_ready, ph, verr);
         tc_fence_after();
-        // P sits in tensor memory, as bf16 pairs over the first KBLK / 2 columns of the S buffer it was computed from
-        // (16 keys = 8 columns per step); that buffer is overwritten by S of block j + NSB, issued after this product
 #pragma unroll
         for (int kk = 0; kk < KBLK / 16; ++kk) {
-          const uint64_t vd = make_smem_desc_mn(sV + vb * DCH * KBLK * 128 + kk * 16 * 128, KBLK * 128, 1024);
+          if (NSB == 1 && kk == KBLK / 32) {
+            if (short_block(j)) break;
+            mbar_wait(p_ready, ph, verr);
+            tc_fence_after();
+          }
+          const uint64_t vd = make_smem_desc_mn(sV + vb * BLK + kk * 16 * 128, KBLK * 128, 1024);
           umma_bf16_ts(tmem + TM_O, tmem + TM_S + (j % NSB) * KBLK + kk * 8, vd, idesc_o, (j | kk) != 0);
         }
         umma_commit(v_empty(vb));
@@ -235,54 +283,53 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
     const int quad = warp & 3;
     const int r = quad * 32 + lane;
     const int sw = r & 7;
-    // token row of this thread's query, and of the request's first history key
-    const bool in = q0 + r < (cand_tile ? a.n_cand : n_hist);
-    const long long hist0 = a.hist_row0 + (long long)b * a.hist_req_rows;
-    const long long tok = (cand_tile ? a.cand_row0 + (long long)b * a.cand_req_rows : hist0) + q0 + r;
-    const int segq = in ? a.seg[tok] : 0;
+    const int segq = r < rows_in ? a.seg[tok0 + r] : 0;
     const uint32_t lane_base = ((uint32_t)(quad * 32) << 16);
     const float csc = CAP ? 1.0f : a.sm_scale * 1.4426950408889634f;
     float m = -INFINITY, l = 0.f;
 
-    // validity of every history key, once per CTA (thread r looks at key r of each block; the loads of all blocks are
-    // in flight together instead of one exposed round trip per block)
-    for (int j = 0; j < n_blocks; ++j) {
-      const int key = j * KBLK + r;
-      const bool ok = (r < KBLK) && (key < n_hist) && (a.seg[hist0 + key] == 1);
-      const uint32_t word = __ballot_sync(0xffffffffu, ok);
-      if (lane == 0) mask_words[j * 4 + quad] = word;
+    // validity of every history key, once per CTA, 1024 keys a round trip
+    for (int k0 = 0; k0 < n_blocks * KBLK; k0 += 8 * QT) {
+      int sg[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sg[i] = k0 + i * QT + r < n_hist ? a.seg[hist0 + k0 + i * QT + r] : 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t word = __ballot_sync(0xffffffffu, sg[i] == 1);
+        if (lane == 0) mask_words[((k0 + i * QT) >> 5) + quad] = word;
+      }
     }
     bar_sync_128();
 
     for (int j = 0; j < n_blocks; ++j) {
       const uint32_t ph = (uint32_t)(j & 1);
-      uint32_t kmask[4];
-#pragma unroll
-      for (int w = 0; w < 4; ++w) kmask[w] = mask_words[j * 4 + w];
-      bool all_ok = true;
-#pragma unroll
-      for (int w = 0; w < KBLK / 32; ++w) all_ok = all_ok && (kmask[w] == 0xffffffffu);
-
+      const uint32_t s_col = tmem + TM_S + (j % NSB) * KBLK + lane_base;
+      const bool half = NSB == 1 && n_hist - j * KBLK <= KBLK / 2;
       mbar_wait(s_full(j % NSB), (uint32_t)((j / NSB) & 1), verr);
       tc_fence_after();
       float s[KBLK];
 #pragma unroll
-      for (int c = 0; c < KBLK / 32; ++c) tmem_ld32_nowait(tmem + TM_S + (j % NSB) * KBLK + lane_base + c * 32, reinterpret_cast<uint32_t*>(s) + c * 32);
+      for (int c = 0; c < KBLK / 32; ++c)
+        if (c < KBLK / 64 || !half) tmem_ld32_nowait(s_col + c * 32, reinterpret_cast<uint32_t*>(s) + c * 32);
       tmem_ld_wait();
       if (CAP) {
 #pragma unroll
         for (int k = 0; k < KBLK; ++k) s[k] = capped_log2(s[k], a.sm_scale, a.cap, a.cap_method);
       }
-      if (!all_ok) {
 #pragma unroll
-        for (int k = 0; k < KBLK; ++k)
-          if (!((kmask[k >> 5] >> (k & 31)) & 1u)) s[k] = -INFINITY;
+      for (int c = 0; c < KBLK / 32; ++c) {
+        const uint32_t kmask = mask_words[j * (KBLK / 32) + c];
+        if (kmask != 0xffffffffu) {
+#pragma unroll
+          for (int k = 0; k < 32; ++k)
+            if (!((kmask >> k) & 1u)) s[c * 32 + k] = -INFINITY;
+        }
       }
       float bm;
       {
         float b4[4] = {s[0], s[1], s[2], s[3]};   // four chains of three-input max
 #pragma unroll
-        for (int k = 4; k + 7 < KBLK + 4 && k + 7 < KBLK; k += 8) {
+        for (int k = 4; k + 7 < KBLK; k += 8) {
           b4[0] = max3f(b4[0], s[k], s[k + 1]); b4[1] = max3f(b4[1], s[k + 2], s[k + 3]);
           b4[2] = max3f(b4[2], s[k + 4], s[k + 5]); b4[3] = max3f(b4[3], s[k + 6], s[k + 7]);
         }
@@ -300,103 +347,110 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
       const float mns = (m_new == -INFINITY) ? 0.f : m_new;   // finite stand-in while nothing is allowed yet
       const float alpha = ex2f(m - mns);                      // -inf - finite -> 0; unmoved: 1
       m = m_new;
-      float ls;
-      {
-        const float2 c2 = make_float2(csc, csc), n2 = make_float2(-mns, -mns);
-        float2 acc2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-        for (int k = 0; k < KBLK; k += 2) {   // packed fp32: two columns per instruction; masked: 2^-inf = 0
-          const float2 e = __ffma2_rn(make_float2(s[k], s[k + 1]), c2, n2);
-          s[k] = ex2f(e.x); s[k + 1] = ex2f(e.y);
-          acc2[(k >> 1) & 1] = __fadd2_rn(acc2[(k >> 1) & 1], make_float2(s[k], s[k + 1]));
-        }
-        ls = (acc2[0].x + acc2[0].y) + (acc2[1].x + acc2[1].y);
-      }
-      l = l * alpha + ls;
-
-      if (j > 0) {
-        // O of the previous blocks must be complete (and P's previous contents consumed) before it is rescaled
+      if (j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+        // O of the blocks before must be complete before it is rescaled
         mbar_wait(o_done, ph ^ 1, verr);
         tc_fence_after();
-        const bool need = __any_sync(0xffffffffu, alpha != 1.0f);
-        if (need) {
 #pragma unroll
-          for (int c = 0; c < DH / 32; ++c) {
-            uint32_t o[32];
-            tmem_ld32(tmem + TM_O + lane_base + c * 32, o);
+        for (int c = 0; c < DH / 16; ++c) {
+          uint32_t o[16];
+          tmem_ld16_nowait(tmem + TM_O + lane_base + c * 16, o);
+          tmem_ld_wait();
 #pragma unroll
-            for (int k = 0; k < 32; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * alpha);
-            tmem_st32(tmem + TM_O + lane_base + c * 32, o);
-          }
+          for (int k = 0; k < 16; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * alpha);
+          tmem_st16_nowait(tmem + TM_O + lane_base + c * 16, o);
         }
       }
-      // P (bf16 pairs) back into tensor memory, over the first KBLK / 2 columns of this block's S buffer (the whole
-      // row of S is in registers by now): the second MMA takes its A operand from there
-      {
-        uint32_t pw[KBLK / 2];
+      // P (bf16 pairs) goes back into tensor memory over the first half of the S columns (the whole row of S is in registers by
+      // now): the second MMA takes its A operand from there, and may start once the first half has been written
+      const float2 c2 = make_float2(csc, csc), n2 = make_float2(-mns, -mns);
+      float2 acc2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-        for (int k = 0; k < KBLK / 2; ++k) pw[k] = pack_bf2(s[2 * k], s[2 * k + 1]);
+      for (int c = 0; c < KBLK / 32; ++c) {
+        if (c == KBLK / 64 && half) break;
+        uint32_t pw[16];
 #pragma unroll
-        for (int c = 0; c < KBLK / 64; ++c) tmem_st32_nowait(tmem + TM_S + (j % NSB) * KBLK + lane_base + c * 32, pw + c * 32);
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        for (int k = 0; k < 16; ++k) {   // packed fp32: two columns per instruction; masked: 2^-inf = 0
+          const float2 e = __ffma2_rn(make_float2(s[c * 32 + 2 * k], s[c * 32 + 2 * k + 1]), c2, n2);
+          const float2 x = make_float2(ex2f(e.x), ex2f(e.y));
+          acc2[k & 1] = __fadd2_rn(acc2[k & 1], x);
+          pw[k] = pack_bf2(x.x, x.y);
+        }
+        tmem_st16_nowait(s_col + c * 16, pw);
+        if ((NSB == 1 && c == KBLK / 64 - 1) || c == KBLK / 32 - 1) {
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          tc_fence_before();
+          // where S of this block did not wait for P V of the one before: its barrier must not run two phases ahead of the issuer
+          if (NSB > 1 && j > 0) mbar_wait(o_done, ph ^ 1, verr);
+          mbar_arrive(c == KBLK / 32 - 1 ? p_ready : p_half);
+        }
       }
-      tc_fence_before();
-      mbar_arrive(p_ready);
+      l = l * alpha + ((acc2[0].x + acc2[0].y) + (acc2[1].x + acc2[1].y));
     }
 
-    // ---- epilogue: O row, self key of a candidate, normalise, stage, TMA store --------------------------------
-    float o[DH];
-    if (n_blocks > 0) {
-      mbar_wait(o_done, (uint32_t)((n_blocks - 1) & 1), verr);
-      tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < DH / 32; ++c) tmem_ld32(tmem + TM_O + lane_base + c * 32, reinterpret_cast<uint32_t*>(o) + c * 32);
-    } else {
-#pragma unroll
-      for (int k = 0; k < DH; ++k) o[k] = 0.f;
-    }
+    // ---- epilogue: self key of a candidate, O row, normalise, stage, TMA store --------------------------------
+    float scale = 1.0f, pr = 0.f;          // of O, of the row's own V
+    const int own = n_blocks + r / KBLK, own_row = (r % KBLK) * 128;     // block and place of the row's own K and V
     if (segq == -1) {
-      const uint4* qp = reinterpret_cast<const uint4*>(a.q + tok * a.q_tok_stride + qcol);
-      const uint4* kp = reinterpret_cast<const uint4*>(a.k + tok * a.k_tok_stride + (long long)hk * a.k_head_stride);
-      const uint4* vp = reinterpret_cast<const uint4*>(a.v + tok * a.v_tok_stride + (long long)hk * a.v_head_stride);
+      mbar_wait(q_full, 0, verr);
+      mbar_wait(k_full(own % NSB), (uint32_t)((own / NSB) & 1), verr);
       float dot = 0.f;
 #pragma unroll
       for (int c = 0; c < DH / 8; ++c) {
-        const uint4 qa = __ldg(qp + c), ka = __ldg(kp + c);
+        const uint32_t at = (uint32_t)((c & 7) ^ sw) << 4;
+        const uint4 qa = ld_shared_16(sQ + (c >> 3) * SLAB + r * 128 + at), ka = ld_shared_16(sK + (own % NSB) * BLK + (c >> 3) * KBLK * 128 + own_row + at);
         const float2 q0f = unpack_bf2(qa.x), q1f = unpack_bf2(qa.y), q2f = unpack_bf2(qa.z), q3f = unpack_bf2(qa.w);
         const float2 k0f = unpack_bf2(ka.x), k1f = unpack_bf2(ka.y), k2f = unpack_bf2(ka.z), k3f = unpack_bf2(ka.w);
         dot += q0f.x * k0f.x + q0f.y * k0f.y + q1f.x * k1f.x + q1f.y * k1f.y + q2f.x * k2f.x + q2f.y * k2f.y + q3f.x * k3f.x + q3f.y * k3f.y;
       }
       const float sv = CAP ? capped_log2(dot, a.sm_scale, a.cap, a.cap_method) : dot * csc;
       const float mn = fmaxf(m, sv);
-      const float alpha = ex2f(m - mn);           // no history: 2^-inf = 0
+      scale = ex2f(m - mn);                // no history: 2^-inf = 0
       const float p = ex2f(sv - mn);
-      const float pr = round_bf(p);
-      l = l * alpha + p;
-#pragma unroll
-      for (int c = 0; c < DH / 8; ++c) {
-        const uint4 va = __ldg(vp + c);
-        const float2 v0 = unpack_bf2(va.x), v1 = unpack_bf2(va.y), v2 = unpack_bf2(va.z), v3 = unpack_bf2(va.w);
-        o[c * 8 + 0] = o[c * 8 + 0] * alpha + pr * v0.x; o[c * 8 + 1] = o[c * 8 + 1] * alpha + pr * v0.y;
-        o[c * 8 + 2] = o[c * 8 + 2] * alpha + pr * v1.x; o[c * 8 + 3] = o[c * 8 + 3] * alpha + pr * v1.y;
-        o[c * 8 + 4] = o[c * 8 + 4] * alpha + pr * v2.x; o[c * 8 + 5] = o[c * 8 + 5] * alpha + pr * v2.y;
-        o[c * 8 + 6] = o[c * 8 + 6] * alpha + pr * v3.x; o[c * 8 + 7] = o[c * 8 + 7] * alpha + pr * v3.y;
-      }
+      pr = round_bf(p);
+      l = l * scale + p;
     }
     const float inv = (l == 0.f || segq == 0) ? 0.f : 1.0f / l;   // padded rows, rows with no allowed key -> zeros
+    if (n_blocks > 0) {
+      mbar_wait(o_done, (uint32_t)((n_blocks - 1) & 1), verr);
+      tc_fence_after();
+    }
+    if (segq == -1) mbar_wait(v_full(own & 1), (uint32_t)((own >> 1) & 1), verr);
+    __syncwarp();
 #pragma unroll
-    for (int c = 0; c < DH / 8; ++c) {
-      uint4 w;
-      w.x = pack_bf2(o[c * 8 + 0] * inv, o[c * 8 + 1] * inv); w.y = pack_bf2(o[c * 8 + 2] * inv, o[c * 8 + 3] * inv);
-      w.z = pack_bf2(o[c * 8 + 4] * inv, o[c * 8 + 5] * inv); w.w = pack_bf2(o[c * 8 + 6] * inv, o[c * 8 + 7] * inv);
-      st_shared_16(sQ + (c >> 3) * SLAB + r * 128 + ((uint32_t)((c & 7) ^ sw) << 4), w);   // Q is no longer needed
+    for (int c = 0; c < DH / 32; ++c) {
+      float o[32];
+      __syncwarp();
+      if (n_blocks > 0) {
+        tmem_ld32(tmem + TM_O + lane_base + c * 32, reinterpret_cast<uint32_t*>(o));
+      } else {
+#pragma unroll
+        for (int k = 0; k < 32; ++k) o[k] = 0.f;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t at = (uint32_t)(((c & 1) * 4 + i) ^ sw) << 4;
+        float* const x = o + i * 8;
+        if (segq == -1) {
+          const uint4 va = ld_shared_16(sV + (own & 1) * BLK + (c >> 1) * KBLK * 128 + own_row + at);
+          const float2 v0 = unpack_bf2(va.x), v1 = unpack_bf2(va.y), v2 = unpack_bf2(va.z), v3 = unpack_bf2(va.w);
+          x[0] = x[0] * scale + pr * v0.x; x[1] = x[1] * scale + pr * v0.y;
+          x[2] = x[2] * scale + pr * v1.x; x[3] = x[3] * scale + pr * v1.y;
+          x[4] = x[4] * scale + pr * v2.x; x[5] = x[5] * scale + pr * v2.y;
+          x[6] = x[6] * scale + pr * v3.x; x[7] = x[7] * scale + pr * v3.y;
+        }
+        uint4 w;
+        w.x = pack_bf2(x[0] * inv, x[1] * inv); w.y = pack_bf2(x[2] * inv, x[3] * inv);
+        w.z = pack_bf2(x[4] * inv, x[5] * inv); w.w = pack_bf2(x[6] * inv, x[7] * inv);
+        st_shared_16(sQ + (c >> 1) * SLAB + r * 128 + at, w);   // Q is no longer needed: its products are done, and the row's own thread has read it
+      }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     bar_sync_128();
     if (warp == 2 && elect_one()) {
       for (int c = 0; c < DCH; ++c) tma_store_3d(cand_tile ? &maps.oc : &maps.oh, sQ + c * SLAB, h * DH + c * 64, q0, b);
       asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the writes land before the grid counts as done
     }
   }
 
@@ -1154,10 +1208,9 @@ phx_status launch_pingpong(const AttnArgs& a, int* err_flag, int num_sms, cudaSt
 
 template <int DH, bool CAP>
 phx_status launch_tc(const AttnArgs& a, int* err_flag, cudaStream_t stream, std::string& err) {
-  constexpr int KBLK = (DH == 64) ? 128 : 64;
   constexpr int DCH = DH / 64;
-  constexpr int NSB = (KBLK <= 64) ? 2 : 1;   // K buffers, as in the kernel
-  const size_t smem = (size_t)DCH * SLAB + (NSB + 2) * (size_t)DCH * KBLK * 128 + TC_MAX_BLOCKS * 16 + 128 + 1024;
+  constexpr int KBLK = key_block(DH), NSB = KBLK <= 64 ? 2 : 1;   // K buffers, as in the kernel
+  const size_t smem = (size_t)DCH * SLAB + (NSB + 2) * (size_t)DCH * KBLK * 128 + TC_MAX_KEYS / 8 + 128 + 1024;
   static SmemLimit limit;
   PHX_CUDA_TRY(limit.raise(ranker_attention_tc_kernel<DH, CAP>, (int)smem), err);
   AttnTcArgs t;
@@ -1188,6 +1241,8 @@ phx_status launch_tc(const AttnArgs& a, int* err_flag, cudaStream_t stream, std:
   if ((s = cached_map3d(&m.qc, a.q + c0 * a.q_tok_stride, qcols, crows, creq, a.B, a.q_tok_stride, QT, err))) return s;
   if ((s = cached_map3d(&m.k, a.k + h0 * a.k_tok_stride, kcols, hrows, hreq, a.B, a.k_tok_stride, KBLK, err))) return s;
   if ((s = cached_map3d(&m.v, a.v + h0 * a.v_tok_stride, vcols, hrows, hreq, a.B, a.v_tok_stride, KBLK, err))) return s;
+  if ((s = cached_map3d(&m.kc, a.k + c0 * a.k_tok_stride, kcols, crows, creq, a.B, a.k_tok_stride, KBLK, err))) return s;
+  if ((s = cached_map3d(&m.vc, a.v + c0 * a.v_tok_stride, vcols, crows, creq, a.B, a.v_tok_stride, KBLK, err))) return s;
   if ((s = cached_map3d(&m.oh, a.out + h0 * ocols, ocols, hrows, hreq, a.B, ocols, QT, err))) return s;
   if ((s = cached_map3d(&m.oc, a.out + c0 * ocols, ocols, crows, creq, a.B, ocols, QT, err))) return s;
   dim3 grid(t.hist_tiles + cand_tiles, a.Hq, a.B);
@@ -1246,7 +1301,7 @@ bool ranker_attention_tc_supported(const AttnArgs& a) {
   if (a.pack.hist_off || (a.q_start != 0 && a.q_start != (a.hist_len < a.T ? a.hist_len : a.T))) return false;
   {
     const int n_hist = a.hist_len < a.T ? a.hist_len : a.T;
-    if ((n_hist + 63) / 64 > TC_MAX_BLOCKS) return false;   // validity table of the CTA
+    if (n_hist > TC_MAX_KEYS) return false;   // validity table of the CTA
   }
   // TMA: 16-byte aligned bases and strides, head offsets that are multiples of 8 elements
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
