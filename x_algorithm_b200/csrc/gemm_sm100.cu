@@ -57,9 +57,9 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t sr
                ::"l"(map), "r"(src), "r"(c0), "r"(c1) : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // named barrier `id` over the 128 threads of one epilogue group, AND-reducing a per-thread flag: every thread
 // always arrives, so a thread that gave up on a bounded wait can never leave the others parked here
@@ -587,20 +587,20 @@ phx_status launch_e(const GemmPlan& p, int epilogue, const GemmRope& rp, const G
 //   64-column slab g >> 1 (RoPE: the column pairs of pass g & 1)
 // Measured: a forward of one request (640 rows, 8 layers) 492 -> 431 us, 16 small requests through two layers 155 -> 143 us.
 // The arithmetic per element, the order of the row statistics included, is the pair kernel's: results are the same bits.
-template <int BN>
+template <int BN, bool DEEP>
 struct SmallCfg {
   static constexpr int NG = BN / 32;
   static constexpr int THREADS = 64 + NG * 128;
   static constexpr int STAGE_BYTES = (BM + BN) * BK * 2;
-  static constexpr int STAGES = 98304 / STAGE_BYTES;          // 96 KB of ring: 4 (BN = 64) or 3 (BN = 128) k-steps
+  static constexpr int STAGES = (DEEP ? 196608 : 98304) / STAGE_BYTES;   // ring: 4 (BN = 64) or 3 (BN = 128) k-steps, deep 8 or 6
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + (BN / 64) * BM * 4 + 128 + 1024;   // + partial row sums, barriers, alignment
 };
 
-template <int BN, int EPI>
-__global__ void __launch_bounds__(SmallCfg<BN>::THREADS, 1)
+template <int BN, int EPI, bool DEEP>
+__global__ void __launch_bounds__(SmallCfg<BN, DEEP>::THREADS, 1)
 gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, bf16* C, const bf16* R,
                   GemmRope rope, GemmNorm norm, long long M, int N, int K, int early_w, int* err_flag) {
-  using cfg = SmallCfg<BN>;
+  using cfg = SmallCfg<BN, DEEP>;
   constexpr bool RES = (EPI == EPI_RESIDUAL);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -794,11 +794,11 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   }
 }
 
-template <int BN, int EPI>
-phx_status launch_small_t(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C, const bf16* R, const GemmRope& rope,
+template <int BN, int EPI, bool DEEP>
+phx_status launch_small_d(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C, const bf16* R, const GemmRope& rope,
                           const GemmNorm& norm, int64_t M, int* err_flag, cudaStream_t stream, std::string& err) {
-  using cfg = SmallCfg<BN>;
-  auto kern = gemm_small_kernel<BN, EPI>;
+  using cfg = SmallCfg<BN, DEEP>;
+  auto kern = gemm_small_kernel<BN, EPI, DEEP>;
   static SmemLimit limit;
   PHX_CUDA_TRY(limit.raise(kern, cfg::SMEM_BYTES), err);
   cudaLaunchConfig_t lc;
@@ -819,14 +819,28 @@ phx_status launch_small_t(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C
   PHX_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, p.map_a, map_b64, C, R, rope, norm, Mll, N, K, early, err_flag), err);
   return PHX_OK;
 }
+// A deep ring has its SM for itself; a shallow one leaves room for a CTA of the kernel behind.  Deep from K = 1024 on, and from 512 where the
+// kernel behind finds SMs free anyway or has few CTAs.  Forwards of 1 to 16 requests on the device, us, shallow / deep from K = 1024 / from 512 /
+// as here: eight layers of D = 512 and 106 rows a request, one 248 / 222 / 216 / 216, three 242 / 219 / 213 / 213, 118 rows, 16 requests 383 / 336 /
+// 324 / 324; 640 rows, one request 276 / 251 / 254 / 250; D = 1024, two layers of 275 rows, six requests 210 / 168.
+bool deep_ring(int K, int epilogue, long long tiles, int num_sms) {
+  return K >= 1024 || (K >= 512 && (epilogue == EPI_RESIDUAL || 3 * tiles <= 2 * num_sms));
+}
+template <int BN, int EPI>
+phx_status launch_small_t(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C, const bf16* R, const GemmRope& rope,
+                          const GemmNorm& norm, int64_t M, int num_sms, int* err_flag, cudaStream_t stream, std::string& err) {
+  const long long tiles = ((M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
+  return deep_ring(p.K, EPI, tiles, num_sms) ? launch_small_d<BN, EPI, true>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err)
+                                             : launch_small_d<BN, EPI, false>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err);
+}
 template <int BN>
 phx_status launch_small(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C, const bf16* R, int epilogue, const GemmRope& rp,
-                        const GemmNorm& nm, int64_t M, int* err_flag, cudaStream_t stream, std::string& err) {
+                        const GemmNorm& nm, int64_t M, int num_sms, int* err_flag, cudaStream_t stream, std::string& err) {
   switch (epilogue) {
-    case EPI_STORE: return launch_small_t<BN, EPI_STORE>(p, map_b64, C, R, rp, nm, M, err_flag, stream, err);
-    case EPI_RESIDUAL: return launch_small_t<BN, EPI_RESIDUAL>(p, map_b64, C, R, rp, nm, M, err_flag, stream, err);
-    case EPI_GELU: return launch_small_t<BN, EPI_GELU>(p, map_b64, C, R, rp, nm, M, err_flag, stream, err);
-    case EPI_ROPE: return launch_small_t<BN, EPI_ROPE>(p, map_b64, C, R, rp, nm, M, err_flag, stream, err);
+    case EPI_STORE: return launch_small_t<BN, EPI_STORE>(p, map_b64, C, R, rp, nm, M, num_sms, err_flag, stream, err);
+    case EPI_RESIDUAL: return launch_small_t<BN, EPI_RESIDUAL>(p, map_b64, C, R, rp, nm, M, num_sms, err_flag, stream, err);
+    case EPI_GELU: return launch_small_t<BN, EPI_GELU>(p, map_b64, C, R, rp, nm, M, num_sms, err_flag, stream, err);
+    case EPI_ROPE: return launch_small_t<BN, EPI_ROPE>(p, map_b64, C, R, rp, nm, M, num_sms, err_flag, stream, err);
   }
   err = "gemm: unknown epilogue";
   return PHX_E_ARG;
@@ -936,8 +950,8 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
     // forwards: D = 512, 640 rows a request 1.31 with one, 1.04 with four, 0.99 with eight (only the last layer's narrow ones are few).
     const CUtensorMap& map_b64 = p.BN == 256 ? p.map_b_narrow : p.map_b;   // boxes of 64 W rows, either way
     const long long mt = (M + BM - 1) / BM, t64 = mt * ((p.N + 63) / 64), t128 = mt * ((p.N + 127) / 128);
-    if (t64 <= num_sms && !(epilogue == EPI_ROPE && rp.dh == 128)) { dispatch_note(DK_GEMM_SMALL); return launch_small<64>(p, map_b64, C, R, epilogue, rp, nm, M, err_flag, stream, err); }
-    if (t128 <= num_sms) { dispatch_note(DK_GEMM_SMALL); return launch_small<128>(p, map_b64, C, R, epilogue, rp, nm, M, err_flag, stream, err); }
+    if (t64 <= num_sms && !(epilogue == EPI_ROPE && rp.dh == 128)) { dispatch_note(DK_GEMM_SMALL); return launch_small<64>(p, map_b64, C, R, epilogue, rp, nm, M, num_sms, err_flag, stream, err); }
+    if (t128 <= num_sms) { dispatch_note(DK_GEMM_SMALL); return launch_small<128>(p, map_b64, C, R, epilogue, rp, nm, M, num_sms, err_flag, stream, err); }
   }
   if (p.BN == 256) {
     if (!p.pair) {
