@@ -116,9 +116,16 @@ __global__ void __launch_bounds__(ATT_THREADS) ranker_attention_kernel(AttnArgs 
       cp16((uint32_t)__cvta_generic_to_shared(dk + kr * LD + dc), kbase + tok * a.k_tok_stride + dc, ok);
       cp16((uint32_t)__cvta_generic_to_shared(dv + kr * LD + dc), vbase + tok * a.v_tok_stride + dc, ok);
     }
-    if (threadIdx.x < KB) {  // warps 0 and 1
-      const int key = blk * KB + threadIdx.x;
-      const int ok = (key < n_hist) && (a.seg[trow(key)] == 1);
+  };
+  // validity of the keys of `n` blocks from blk on, two warps a block.  The load goes out before the copies and is looked at behind
+  // them: looked at in between, it kept the second block's copies back by a round trip.
+  auto load_key = [&](int blk, int n) {
+    const int key = blk * KB + threadIdx.x;
+    return (threadIdx.x < n * KB && key < n_hist) ? a.seg[trow(key)] : 0;
+  };
+  auto mark_keys = [&](int seg_key, int buf, int n) {
+    if (threadIdx.x < n * KB) {
+      const int ok = seg_key == 1;
       skey_ok[buf * KB + threadIdx.x] = ok;
       const int all32 = __all_sync(0xffffffffu, ok);
       if ((threadIdx.x & 31) == 0) sall_ok[buf * 2 + (threadIdx.x >> 5)] = all32;
@@ -126,6 +133,11 @@ __global__ void __launch_bounds__(ATT_THREADS) ranker_attention_kernel(AttnArgs 
   };
 
   // ---- prologue: Q tile, own K/V rows, key blocks 0 and 1 --------------------------------------------
+  const int rq[2] = {q0 + warp * 16 + g, q0 + warp * 16 + g + 8};
+  int segq[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) segq[i] = (rq[i] < T) ? a.seg[trow(rq[i])] : 0;
+  const int seg_key = load_key(0, 2);
   for (int c = threadIdx.x; c < QROWS * CH; c += ATT_THREADS) {
     const int r = c / CH, dc = (c % CH) * 8;
     const bool ok = (q0 + r) < T;
@@ -140,11 +152,7 @@ __global__ void __launch_bounds__(ATT_THREADS) ranker_attention_kernel(AttnArgs 
   cp_commit();
   if (n_blocks > 1) load_block(1, 1);
   cp_commit();
-
-  const int rq[2] = {q0 + warp * 16 + g, q0 + warp * 16 + g + 8};
-  int segq[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) segq[i] = (rq[i] < T) ? a.seg[trow(rq[i])] : 0;
+  mark_keys(seg_key, 0, 2);
 
   cp_wait<1>();
   __syncthreads();
@@ -257,8 +265,10 @@ __global__ void __launch_bounds__(ATT_THREADS) ranker_attention_kernel(AttnArgs 
     // refill this buffer with block blk+2
     if (blk + 2 < n_blocks) {
       __syncthreads();
+      const int next_key = load_key(blk + 2, 1);
       load_block(blk + 2, buf);
       cp_commit();
+      mark_keys(next_key, buf, 1);
     }
   }
 

@@ -175,7 +175,9 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
   const int rows_in = (cand_tile ? a.n_cand : n_hist) - q0;                                         // queries from there on
   volatile int* verr = a.err_flag;
 
+  if (warp == 0 && lane < 8) prefetch_map(&maps.qh + lane);
   if (threadIdx.x == 0) {
+    *gave_up() = 0;
     mbar_init(q_full, 1); mbar_init(p_half, 128); mbar_init(p_ready, 128); mbar_init(o_done, 1);
     for (int i = 0; i < 2; ++i) { mbar_init(k_full(i), 1); mbar_init(k_empty(i), 1); mbar_init(s_full(i), 1); mbar_init(v_full(i), 1); mbar_init(v_empty(i), 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -454,9 +456,7 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
     }
   }
 
-  if (*verr != 0) __nanosleep(1000000);  // error path: let in-flight bulk copies land before the CTA retires
-  tc_fence_before();
-  __syncthreads();
+  settle();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, 256);
@@ -498,6 +498,7 @@ ranker_attention_resident_kernel(const __grid_constant__ CUtensorMap map_q, cons
   volatile int* verr = a.err_flag;
 
   if (threadIdx.x == 0) {
+    *gave_up() = 0;
     // a Q buffer is free once S has been computed from it (commit) and the 128 softmax threads have read their rows
     for (int i = 0; i < 2; ++i) { mbar_init(q_full(i), 1); mbar_init(q_free(i), 129); }
     mbar_init(kv_full, 1); mbar_init(s_full, 1); mbar_init(p_ready, 128); mbar_init(o_done, 1);
@@ -718,9 +719,7 @@ ranker_attention_resident_kernel(const __grid_constant__ CUtensorMap map_q, cons
     }
   }
 
-  if (*verr != 0) __nanosleep(1000000);
-  tc_fence_before();
-  __syncthreads();
+  settle();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, 256);
@@ -803,7 +802,9 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
   auto item_at = [&](int li) { return li < rounds ? (int)blockIdx.x + li * (int)gridDim.x : rounds * (int)gridDim.x + ri0 + (li - rounds); };
   auto first_tile = [&](int li) { return li == rounds ? rt0 : 0; };
 
+  if (warp == 0 && lane < 8) prefetch_map(&maps.qh + lane);
   if (threadIdx.x == 0) {
+    *gave_up() = 0;
     for (int i = 0; i < 2; ++i) {
       mbar_init(kv_full(i), 1); mbar_init(kv_free(i), 1); mbar_init(s_full(i), 1); mbar_init(p_ready(i), 128);
       mbar_init(o_done(i), 1); mbar_init(o_staged(i), 128);
@@ -914,7 +915,6 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         mbar_arrive(q_free(st));
       }
-      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
   } else {
     // ---------------- softmax / epilogue: warpgroup w takes the tiles g = w, w + 2, ... ----------------
@@ -1108,9 +1108,7 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
     }
   }
 
-  if (*verr != 0) __nanosleep(1000000);   // error path: let in-flight bulk copies land before the CTA retires
-  tc_fence_before();
-  __syncthreads();
+  settle();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);

@@ -57,7 +57,6 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t sr
                ::"l"(map), "r"(src), "r"(c0), "r"(c1) : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -163,6 +162,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   volatile int* verr = err_flag;
 
   if (threadIdx.x == 0) {
+    *gave_up() = 0;
+    prefetch_map(&map_a); prefetch_map(&map_b); prefetch_map(&map_c);
+    if (EPI == EPI_RESIDUAL) prefetch_map(&map_r);
     for (int s = 0; s < cfg::STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     // a pair's accumulators are drained by the epilogue threads of both CTAs, counted on the issuing CTA
     for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), DRAIN_THREADS); }
@@ -476,13 +478,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         bulk_commit();
       }
     }
-    if (issuer_warp && elect_one()) bulk_wait_all();
+    if (issuer_warp && elect_one()) bulk_wait_read<0>();   // the slabs have been read; their writes land before the grid counts as done
   }
 
   // ---------------- teardown ----------------
-  if (*verr != 0) __nanosleep(1000000);  // error path: let in-flight bulk copies land before the CTA retires
-  tc_fence_before();
-  __syncthreads();
+  settle();
   if (PAIR) cluster_sync_all();   // neither CTA retires (or frees tensor memory) while the other may still signal or read it
   if (warp == 1) {
     tc_fence_after();
@@ -619,6 +619,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   volatile int* verr = err_flag;
 
   if (threadIdx.x == 0) {
+    *gave_up() = 0;
+    prefetch_map(&map_a); prefetch_map(&map_b);
     for (int s = 0; s < cfg::STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     mbar_init(tfull_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -785,9 +787,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   }
 
   // ---------------- teardown ----------------
-  if (*verr != 0) __nanosleep(1000000);  // error path: let in-flight bulk copies land before the CTA retires
-  tc_fence_before();
-  __syncthreads();
+  settle();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_d, BN);
@@ -823,6 +823,7 @@ phx_status launch_small_d(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C
 // kernel behind finds SMs free anyway or has few CTAs.  Forwards of 1 to 16 requests on the device, us, shallow / deep from K = 1024 / from 512 /
 // as here: eight layers of D = 512 and 106 rows a request, one 248 / 222 / 216 / 216, three 242 / 219 / 213 / 213, 118 rows, 16 requests 383 / 336 /
 // 324 / 324; 640 rows, one request 276 / 251 / 254 / 250; D = 1024, two layers of 275 rows, six requests 210 / 168.
+// (Each kernel ends without a look at the error flag in all but the first figure of each.)
 bool deep_ring(int K, int epilogue, long long tiles, int num_sms) {
   return K >= 1024 || (K >= 512 && (epilogue == EPI_RESIDUAL || 3 * tiles <= 2 * num_sms));
 }

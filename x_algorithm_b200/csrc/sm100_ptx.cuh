@@ -45,6 +45,19 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
+// Whether a wait of this CTA gave up: one word of shared memory that a kernel clears before its first wait.  A CTA whose waits all
+// returned has no copies in flight when it is done; one that gave up lingers for what may still land in its memory.  (Each CTA read the
+// error flag itself for that, a round trip to L2 as its last act: 0.5 us of every kernel, which a forward of one request has 42 of.)
+__device__ __forceinline__ volatile int* gave_up() {
+  __shared__ int word;
+  return &word;
+}
+// The CTA's last barrier; behind it tensor memory may be freed.
+__device__ __forceinline__ void settle() {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (*gave_up()) __nanosleep(1000000);
+}
 // Bounded wait.  Returns false when the limit ran out or another role already raised the flag.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* err_flag) {
   unsigned long long t0 = 0;
@@ -57,18 +70,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         : "memory");
     if (done) return true;
     if ((it & 0x3FF) == 0x3FF) {
-      if (*err_flag != 0) return false;
+      if (*err_flag != 0) { *gave_up() = 1; return false; }
       unsigned long long now = globaltimer_ns();
       if (t0 == 0) t0 = now;
       else {
         const unsigned int us = (unsigned int)err_flag[1];
         const unsigned long long limit = us ? 1000ull * us : WAIT_LIMIT_NS;
-        if (now - t0 > limit) { *err_flag = 1; __threadfence(); return false; }
+        if (now - t0 > limit) { *err_flag = 1; __threadfence(); *gave_up() = 1; return false; }
       }
     }
   }
 }
 
+// A tensor map on its way before the first copy that needs it: 0.2-0.5 us of that copy's latency otherwise
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"

@@ -181,6 +181,8 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
+    *gave_up() = 0;
+    prefetch_map(&map_corpus); prefetch_map(&map_users);
     for (int s = 0; s < TC_STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     for (int x = 0; x < 2; ++x) { mbar_init(tfull_bar(x), 1); mbar_init(tempty_bar(x), 32 * TC_CWARPS); }
     for (int s = 0; s < TC_STAGES; ++s) mbar_init(xfull_bar(s), 1);
@@ -535,9 +537,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
     }
   }
 
-  if (*verr != 0) __nanosleep(1000000);  // error path: let in-flight bulk copies land before the CTA retires
-  tc_fence_before();
-  __syncthreads();
+  settle();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 2 * NQ);
@@ -550,7 +550,7 @@ phx_status launch_scan_tc(const CUtensorMap& map_corpus, const CUtensorMap& map_
   const int kblk = a.row_bytes / 128;
   const size_t smem = (size_t)kblk * NQ * 128 + (size_t)scan_stages(BIAS, kblk) * kblk * TC_ROWS * 128 + scan_bias_bytes(BIAS, NQ) + 2 * 256 * 4 + 64 + 128 * 16 + TC_CWARPS * (QCAP * 16 + 128) + 256 + 1024;
   static SmemLimit limit;
-  PHX_CUDA_TRY(limit.raise(scan_tc_kernel<MODE, I8, NQ, BIAS>, 227 * 1024), err);
+  PHX_CUDA_TRY(limit.raise(scan_tc_kernel<MODE, I8, NQ, BIAS>, 226 * 1024), err);
   PHX_CUDA_TRY(launch_programmatic(scan_tc_kernel<MODE, I8, NQ, BIAS>, grid, scan_threads(BIAS), smem, stream, map_corpus, map_users, a, err_flag), err);
   return PHX_OK;
 }
