@@ -398,11 +398,13 @@ __global__ void __launch_bounds__(256) finish_tokens_kernel(const bf16* __restri
 }
 
 // Packed rows: the position of every packed row (RoPE) and, for the candidate rows, the slot of the [B, C] output
-// arrays each one answers.  One thread per (request, slot).
-__global__ void pack_plan_kernel(PackMap pk, int B, int S, int C, int* __restrict__ pos_rows, int* __restrict__ out_index) {
+// arrays each one answers.  One thread per (request, slot).  Offsets in host memory are copied on the way (T >= 2: threads enough).
+__global__ void pack_plan_kernel(PackMap pk, int B, int S, int C, int* __restrict__ pos_rows, int* __restrict__ out_index,
+                                 int* __restrict__ hist_copy, int* __restrict__ cand_copy) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int T = S + C;
   if (i >= (long long)B * T) return;
+  if (hist_copy && i <= B) { hist_copy[i] = pk.hist_off[i]; cand_copy[i] = pk.cand_off[i]; }
   const int b = (int)(i / T), t = (int)(i % T);
   if (t < S) {
     if (t < pk.hist_cnt(b)) pos_rows[pk.hist_off[b] + t] = t;
@@ -625,11 +627,11 @@ phx_status build_tokens_launch(const TokenBuildArgs& a, cudaStream_t stream, std
   return PHX_OK;
 }
 
-phx_status pack_plan_launch(const PackMap& pk, int B, int S, int C, int* pos_rows, int* out_index, cudaStream_t stream,
-                            std::string& err) {
+phx_status pack_plan_launch(const PackMap& pk, int B, int S, int C, int* pos_rows, int* out_index, int* hist_copy, int* cand_copy,
+                            cudaStream_t stream, std::string& err) {
   const long long n = (long long)B * (S + C);
   if (n == 0) return PHX_OK;
-  pack_plan_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(pk, B, S, C, pos_rows, out_index);
+  pack_plan_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(pk, B, S, C, pos_rows, out_index, hist_copy, cand_copy);
   PHX_CUDA_TRY(cudaGetLastError(), err);
   return PHX_OK;
 }

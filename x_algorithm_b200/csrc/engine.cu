@@ -69,6 +69,7 @@ struct phx_engine {
   struct PackState {
     int *hist_off = nullptr, *cand_off = nullptr, *pos_rows = nullptr, *out_index = nullptr;   // device, owned
     const int *hist_off_view = nullptr, *cand_off_view = nullptr;   // offsets living in a staging block instead
+    const int* host_off = nullptr;   // both in pinned memory, B + 1 entries each: the plan brings them into the owned arrays
     long long M = 0, Mh = 0;      // packed rows in all, history rows
     int planned_batch = -1;       // batch size pos_rows / out_index were last planned for (full plan)
     bool ragged = false;
@@ -148,7 +149,7 @@ struct phx_engine {
   bool fused_norm = false;   // RMSNorm folded into the GEMMs (no primer norm, no qk-norm-before-fusion issue, tcgen05 path)
   bool folded_dirty = true;
   int* hashes = nullptr;
-  int* err_flag = nullptr;
+  int* err_flag = nullptr;   // pinned
   // staging for the host-buffer entry point
   void* in_stage_dev = nullptr;
   void* in_stage_host = nullptr;
@@ -157,7 +158,6 @@ struct phx_engine {
   void* out_stage_host = nullptr;
   float* lp_dev = nullptr; float* cont_dev = nullptr; double* score_dev = nullptr;      // inside out_stage_dev / _host
   float* lp_host = nullptr; float* cont_host = nullptr; double* score_host = nullptr;
-  int* flag_host = nullptr;   // pinned: err_flag[0] comes back with a call's results
 
   // token prefetch (phx_rank_prefetch_device): tokens of the next batch are built on a side stream into the
   // alternate residual buffer while the current forward runs
@@ -242,6 +242,12 @@ phx_status dev_alloc(phx_engine* e, Tp** p, size_t count) {
 }
 
 // Results of `rows` candidates as one block: f64 scores, log-probabilities, continuous values, each on a 256-byte boundary
+// Up to this size a host-buffer call has the device write its results straight to pinned memory.  A copy costs its bytes and, behind
+// or in front of a kernel, 5 to 10 us of hand-over between the engines; larger results are worth copying in chunks, so that the
+// host can take one while the next is on the bus.  Inputs are read from pinned memory at every size.  Whole calls, us, copies both ways /
+// results direct / inputs too: 11 KB in, 44 KB out 322 / 281 / 274; 14 KB, 11 KB 91 / 82 / 75; 112 KB, 450 KB 165 / 158 / 145; 270 KB,
+// 1.1 MB 302 / 282 / 268; 606 KB, 2.3 MB 503 / 523 / - (inputs alone 485); inputs alone, 1.4 MB 1054 -> 1018, 2.9 MB 1986 -> 1924.
+constexpr size_t DIRECT_OUT_BYTES = 1280u << 10;
 struct OutLayout {
   size_t lp_off, cont_off, bytes;
   OutLayout(size_t rows, int V, int NC) {
@@ -651,11 +657,11 @@ phx_status build_tokens(phx_engine* e, const phx_rank_batch* bd, int B, int Cc, 
   return build_tokens_launch(ta, e->stream, e->err);
 }
 
+// the stream (or the event behind the call in question) has been waited for
 phx_status check_err_flag(phx_engine* e) {
-  int flag = 0;
-  PHX_CUDA_TRY(cudaMemcpy(&flag, e->err_flag, sizeof(int), cudaMemcpyDeviceToHost), e->err);
-  if (flag != 0) {
-    cudaMemset(e->err_flag, 0, sizeof(int));
+  volatile int* const flag = e->err_flag;
+  if (*flag != 0) {
+    *flag = 0;
     e->err = "a bounded device-side wait ran out (GEMM / attention pipeline)";
     return PHX_E_TIMEOUT;
   }
@@ -788,8 +794,10 @@ phx_status phx_engine_create(const phx_model_config* cfg, int32_t device, phx_en
     TRY(dev_alloc(e, &e->tokens, (size_t)M * e->D));
     TRY(dev_alloc(e, &e->hashes, (size_t)M * 2 * cfg->item.num_hashes));
   }
-  TRY(dev_alloc(e, &e->err_flag, 2));   // [0] raised by a wait that ran out, [1] the wait limit in microseconds (0 = default)
-  CU(cudaMemset(e->err_flag, 0, 2 * sizeof(int)));
+  // [0] raised by a wait that ran out, [1] the wait limit in microseconds (0 = default).  In pinned memory: kernels look at it only
+  // when a wait has been long or has run out, and the host needs no copy to see it (a copy behind each call: 6-10 us of it).
+  CU(cudaMallocHost(reinterpret_cast<void**>(&e->err_flag), 2 * sizeof(int)));
+  e->err_flag[0] = e->err_flag[1] = 0;
   // RoPE tables: angle = pos * base^(-2j/dh), positions 0..S (layers.py:52-60)
   {
     const int half = e->dh / 2, npos = e->S + 1;
@@ -868,7 +876,6 @@ phx_status phx_engine_create(const phx_model_config* cfg, int32_t device, phx_en
     CU(cudaMallocHost(&e->out_stage_host, ol.bytes));
     e->score_dev = (double*)e->out_stage_dev; e->lp_dev = ol.lp(e->out_stage_dev); e->cont_dev = ol.cont(e->out_stage_dev);
     e->score_host = (double*)e->out_stage_host; e->lp_host = ol.lp(e->out_stage_host); e->cont_host = ol.cont(e->out_stage_host);
-    CU(cudaMallocHost(reinterpret_cast<void**>(&e->flag_host), sizeof(int)));
   }
   // the memsets above ran on the default stream; every later launch uses the engine's own non-blocking stream, which
   // does not order itself behind them
@@ -909,10 +916,10 @@ void phx_engine_destroy(phx_engine* e) {
   fr(e->proj_hist_t); fr(e->proj_cand_t); fr(e->cat_hist); fr(e->cat_cand); fr(e->tok_proj); fr(e->proj_user_t); fr(e->cat_user);
   for (int i = 0; i < PHX_MAX_HIST_CONT; ++i) { fr(e->cont_w1[i]); fr(e->cont_w2[i]); }
   fr(e->x32); fr(e->h32); fr(e->qkv32); fr(e->attn32); fr(e->ffn32); fr(e->tmp32); fr(e->hist32);
-  fr(e->x_alt); fr(e->seg_alt); fr(e->rowss_a_alt); fr(e->rowss_a); fr(e->rowss_f); fr(e->seg); fr(e->hashes); fr(e->err_flag); fr(e->in_stage_dev); fr(e->out_stage_dev);
+  fr(e->x_alt); fr(e->seg_alt); fr(e->rowss_a_alt); fr(e->rowss_a); fr(e->rowss_f); fr(e->seg); fr(e->hashes); fr(e->in_stage_dev); fr(e->out_stage_dev);
   if (e->in_stage_host) cudaFreeHost(e->in_stage_host);
   if (e->out_stage_host) cudaFreeHost(e->out_stage_host);
-  if (e->flag_host) cudaFreeHost(e->flag_host);
+  if (e->err_flag) cudaFreeHost(e->err_flag);
   if (e->ev0) cudaEventDestroy(e->ev0);
   if (e->ev1) cudaEventDestroy(e->ev1);
   for (auto& pe : e->prof_events) { cudaEventDestroy(pe.second.first); cudaEventDestroy(pe.second.second); }
@@ -1065,7 +1072,10 @@ phx_status enqueue_forward(phx_engine* e, const phx_rank_batch* bd, const phx_ra
     // positions of the packed rows and the output slot of every candidate row (the full plan only when B changed)
     if (!pk->ragged) { pk->Mh = (long long)B * e->S; pk->M = (long long)B * e->T; }
     e->last_launches++;
-    if ((s = pack_plan_launch(pack_map(pk), B, e->S, e->C, pk->pos_rows, pk->out_index, e->stream, e->err))) return s;
+    PackMap from = pack_map(pk);
+    if (pk->host_off) { from.hist_off = pk->host_off; from.cand_off = pk->host_off + B + 1; }
+    if ((s = pack_plan_launch(from, B, e->S, e->C, pk->pos_rows, pk->out_index, pk->host_off ? pk->hist_off : nullptr,
+                              pk->host_off ? pk->cand_off : nullptr, e->stream, e->err))) return s;
     pk->planned_batch = pk->ragged ? -1 : B;
   }
   if (!tokens_ready && (s = build_tokens(e, bd, B, e->C, nullptr, nullptr, nullptr, nullptr, nullptr, landing, pos, hb))) return s;
@@ -1228,7 +1238,7 @@ phx_status phx_rank_forward_packed_device(phx_engine* e, const phx_rank_batch* b
     return PHX_E_ARG;
   }
   phx_engine::PackState& pk = e->pack_device;
-  pk.hist_off_view = hist_off_dev; pk.cand_off_view = cand_off_dev;
+  pk.hist_off_view = hist_off_dev; pk.cand_off_view = cand_off_dev; pk.host_off = nullptr;
   pk.pos_rows = e->pack_ragged.pos_rows; pk.out_index = e->pack_ragged.out_index;
   pk.Mh = hist_rows; pk.M = hist_rows + cand_rows;
   pk.ragged = true;
@@ -1459,59 +1469,59 @@ phx_status phx_rank_forward(phx_engine* e, const phx_rank_batch* bh, const phx_r
   cudaSetDevice(e->device);
   const size_t B = bh->batch, S = e->S, C = e->C;
   if (B == 0) return PHX_OK;
-  // pack the six input arrays into one pinned block -> one H2D copy
+  // The six input arrays go into one pinned block, which the tokens are built from.  A packed batch's valid slots are all that is
+  // staged: nothing reads the rest.
+  int* const ho = e->pack ? e->pack_host.data() : nullptr;
+  const int* const co = e->pack ? e->pack_host.data() + (B + 1) : nullptr;
+  if (e->pack) plan_ragged(bh, B, S, C, ho, ho + (B + 1));
   uint8_t* hp = (uint8_t*)e->in_stage_host;
-  uint8_t* dp = (uint8_t*)e->in_stage_dev;
   size_t off = 0;
   phx_rank_batch bd; bd.batch = bh->batch; bd._pad = 0;
-  auto put = [&](const void* src, size_t bytes) { memcpy(hp + off, src, bytes); const void* d = dp + off; off += bytes; return d; };
-  bd.hist_post_ids = (const int64_t*)put(bh->hist_post_ids, B * S * 8);
-  bd.hist_author_ids = (const int64_t*)put(bh->hist_author_ids, B * S * 8);
-  bd.cand_post_ids = (const int64_t*)put(bh->cand_post_ids, B * C * 8);
-  bd.cand_author_ids = (const int64_t*)put(bh->cand_author_ids, B * C * 8);
-  bd.hist_actions = (const int32_t*)put(bh->hist_actions, B * S * 4);
-  bd.hist_surfaces = (const int32_t*)put(bh->hist_surfaces, B * S * 4);
+  auto put = [&](const void* src, size_t bytes) { memcpy(hp + off, src, bytes); const void* d = hp + off; off += bytes; return d; };
+  auto put_rows = [&](const void* src, size_t slots, size_t bytes, const int* first) {   // [B][slots] values, of a packed batch the valid ones
+    if (!first) return put(src, B * slots * bytes);
+    for (size_t b = 0; b < B; ++b)
+      memcpy(hp + off + b * slots * bytes, (const uint8_t*)src + b * slots * bytes, (size_t)(first[b + 1] - first[b]) * bytes);
+    const void* d = hp + off;
+    off += B * slots * bytes;
+    return d;
+  };
+  bd.hist_post_ids = (const int64_t*)put_rows(bh->hist_post_ids, S, 8, ho);
+  bd.hist_author_ids = (const int64_t*)put_rows(bh->hist_author_ids, S, 8, ho);
+  bd.cand_post_ids = (const int64_t*)put_rows(bh->cand_post_ids, C, 8, co);
+  bd.cand_author_ids = (const int64_t*)put_rows(bh->cand_author_ids, C, 8, co);
+  bd.hist_actions = (const int32_t*)put_rows(bh->hist_actions, S, 4, ho);
+  bd.hist_surfaces = (const int32_t*)put_rows(bh->hist_surfaces, S, 4, ho);
   if (e->pack) {
-    int* ho = e->pack_host.data();
-    int* co = ho + (B + 1);
-    plan_ragged(bh, B, S, C, ho, co);
     off = (off + 15) & ~(size_t)15;
     phx_engine::PackState& pk = e->pack_ragged;
-    pk.hist_off_view = (const int*)put(ho, (B + 1) * 4);   // the plan reads its offsets from the staged block
-    pk.cand_off_view = (const int*)put(co, (B + 1) * 4);
+    pk.host_off = (const int*)put(ho, 2 * (B + 1) * 4);   // the plan brings them in: every layer's attention reads them
+    pk.hist_off_view = pk.cand_off_view = nullptr;
     pk.Mh = ho[B]; pk.M = (long long)ho[B] + co[B];
     pk.compact = true;
-    PHX_CUDA_TRY(cudaMemcpyAsync(dp, hp, off, cudaMemcpyHostToDevice, e->stream), e->err);
     e->pack_next = &pk;
-  } else {
-    PHX_CUDA_TRY(cudaMemcpyAsync(dp, hp, off, cudaMemcpyHostToDevice, e->stream), e->err);
   }
   // Packed calls bring back the valid rows alone, in packed order, and lay them out here; the other slots read zero.
   // 48 ragged requests of up to 512 candidates: 580 us a call with the device zeroing and sending every slot, 524 this way.
-  const int* co = e->pack ? e->pack_host.data() + (B + 1) : nullptr;
   const size_t rows = co ? (size_t)co[B] : B * C;
-  // Small results (up to half a megabyte) lie back to back and come back in one copy, the flag right behind: in chunks the
-  // twelve copies of one request, each a few kilobytes, took longer than their bytes.  Whole calls, chunks against one copy:
-  // 44 KB 94 against 78 us, 484 KB 138 against 124, 704 KB 161 against 150, 1.4 MB 244 against 260.
   const OutLayout ol(rows, e->V, e->NC);
-  const bool one_copy = ol.bytes <= (512u << 10);
-  float* lp_dev = e->lp_dev; float* cont_dev = e->cont_dev;
+  const bool direct_out = ol.bytes <= DIRECT_OUT_BYTES;
+  float* lp_dev = e->lp_dev; float* cont_dev = e->cont_dev; double* score_dev = e->score_dev;
   float* lp_host = e->lp_host; float* cont_host = e->cont_host;
-  if (one_copy) {
-    lp_dev = ol.lp(e->out_stage_dev); cont_dev = ol.cont(e->out_stage_dev);
-    lp_host = ol.lp(e->out_stage_host); cont_host = ol.cont(e->out_stage_host);
+  if (direct_out) {
+    lp_dev = lp_host = ol.lp(e->out_stage_host); cont_dev = cont_host = ol.cont(e->out_stage_host);
+    score_dev = e->score_host;
   }
   const int V = e->V, NC = e->NC;
   const bool want_scores = oh->scores && e->has_blend;
-  phx_rank_out od; od.log_probs = lp_dev; od.continuous = cont_dev; od.scores = e->score_dev;
+  phx_rank_out od; od.log_probs = lp_dev; od.continuous = cont_dev; od.scores = score_dev;
   phx_status s = phx_rank_forward_device(e, &bd, &od);
   if (s) return s;
-  if (one_copy && rows) PHX_CUDA_TRY(cudaMemcpyAsync(e->out_stage_host, e->out_stage_dev, ol.bytes, cudaMemcpyDeviceToHost, e->stream), e->err);
   // larger results come back in four row chunks: while the host copies chunk i out of the pinned staging block, chunk i+1
   // is still on the bus
   constexpr int NCH = 4;
   const size_t step = (rows + NCH - 1) / NCH;
-  for (int i = 0; i < NCH && !one_copy; ++i) {
+  for (int i = 0; i < NCH && !direct_out; ++i) {
     const size_t r0 = i * step, r1 = (r0 + step < rows) ? r0 + step : rows;
     if (r0 < r1) {
       if (oh->log_probs) PHX_CUDA_TRY(cudaMemcpyAsync(lp_host + r0 * V, lp_dev + r0 * V, (r1 - r0) * V * 4, cudaMemcpyDeviceToHost, e->stream), e->err);
@@ -1521,7 +1531,6 @@ phx_status phx_rank_forward(phx_engine* e, const phx_rank_batch* bh, const phx_r
     if (!e->ev_chunk[i]) PHX_CUDA_TRY(cudaEventCreateWithFlags(&e->ev_chunk[i], cudaEventDisableTiming), e->err);
     PHX_CUDA_TRY(cudaEventRecord(e->ev_chunk[i], e->stream), e->err);
   }
-  PHX_CUDA_TRY(cudaMemcpyAsync(e->flag_host, e->err_flag, sizeof(int), cudaMemcpyDeviceToHost, e->stream), e->err);
   // `n` rows from row r of the staging block to slot `slot` of the caller's arrays
   auto place = [&](size_t slot, size_t r, size_t n) {
     if (oh->log_probs) memcpy(oh->log_probs + slot * V, lp_host + r * V, n * V * 4);
@@ -1547,13 +1556,13 @@ phx_status phx_rank_forward(phx_engine* e, const phx_rank_batch* bh, const phx_r
       if (want_scores) memset(oh->scores + slot, 0, n * 8);
     }
   }
-  for (int i = 0; i < NCH && !one_copy; ++i) {
+  for (int i = 0; i < NCH && !direct_out; ++i) {
     PHX_CUDA_TRY(cudaEventSynchronize(e->ev_chunk[i]), e->err);
     place_upto((i + 1) * step < rows ? (i + 1) * step : rows);
   }
   PHX_CUDA_TRY(cudaStreamSynchronize(e->stream), e->err);
   place_upto(rows);
-  return *e->flag_host ? check_err_flag(e) : PHX_OK;
+  return check_err_flag(e);
 }
 
 // ---- pipelined host-buffer requests ------------------------------------------------------------------------------
@@ -1672,8 +1681,7 @@ phx_status phx_set_wait_limit_us(phx_engine* e, uint32_t microseconds) {
   if (!e) return PHX_E_ARG;
   cudaSetDevice(e->device);
   PHX_CUDA_TRY(cudaStreamSynchronize(e->stream), e->err);
-  const int v = (int)(microseconds > 0x7FFFFFFFu ? 0x7FFFFFFFu : microseconds);
-  PHX_CUDA_TRY(cudaMemcpy(e->err_flag + 1, &v, sizeof(int), cudaMemcpyHostToDevice), e->err);
+  e->err_flag[1] = (int)(microseconds > 0x7FFFFFFFu ? 0x7FFFFFFFu : microseconds);
   return PHX_OK;
 }
 
@@ -1868,23 +1876,20 @@ phx_status phx_user_tower_device(phx_engine* e, const phx_rank_batch* bd, float*
 }
 
 namespace {
-// What a stand-alone operator call needs beside its operands: the kernels' error flag block, a pinned word it is read into
-// and two events.  Kept between calls (allocating and freeing them took longer than a small operator: cudaFree waits for the
+// What a stand-alone operator call needs beside its operands: the kernels' error flag block and two events.  Kept between calls (allocating and freeing them took longer than a small operator: cudaFree waits for the
 // device), one set per call in flight; at most eight idle ones are held, the rest and any set whose call failed are freed.
 struct OpScratch {
   int device = -1;
-  int* flag = nullptr;        // device, zero between calls
-  int* flag_host = nullptr;   // pinned
+  int* flag = nullptr;        // pinned, zero between calls
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   bool create(int dev) {
     device = dev;
-    return cudaMalloc(reinterpret_cast<void**>(&flag), 2 * sizeof(int)) == cudaSuccess && cudaMemset(flag, 0, 2 * sizeof(int)) == cudaSuccess &&
-           cudaMallocHost(reinterpret_cast<void**>(&flag_host), sizeof(int)) == cudaSuccess && cudaEventCreate(&e0) == cudaSuccess &&
-           cudaEventCreate(&e1) == cudaSuccess;
+    if (cudaMallocHost(reinterpret_cast<void**>(&flag), 2 * sizeof(int)) != cudaSuccess) return false;
+    flag[0] = flag[1] = 0;
+    return cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess;
   }
   void destroy() {
-    if (flag) cudaFree(flag);
-    if (flag_host) cudaFreeHost(flag_host);
+    if (flag) cudaFreeHost(flag);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     *this = OpScratch();
@@ -1914,11 +1919,10 @@ void op_release(OpScratch* s, bool clean) {
 // The end of a call whose launch returned `s`: wait, read the flag and the time, hand the scratch back.
 phx_status op_finish(OpScratch* sc, phx_status s, const char* what, float* device_ms, std::string& err) {
   cudaError_t ce = cudaEventRecord(sc->e1, 0);
-  if (ce == cudaSuccess) ce = cudaMemcpyAsync(sc->flag_host, sc->flag, sizeof(int), cudaMemcpyDeviceToHost, 0);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(0);
   if (s == PHX_OK && ce != cudaSuccess) { err = cudaGetErrorString(ce); s = PHX_E_CUDA; }
   if (s == PHX_OK && device_ms) cudaEventElapsedTime(device_ms, sc->e0, sc->e1);
-  const bool raised = ce == cudaSuccess && *sc->flag_host != 0;
+  const bool raised = ce == cudaSuccess && *static_cast<volatile int*>(sc->flag) != 0;
   if (s == PHX_OK && raised) { err = std::string("a bounded device-side wait ran out (") + what + " pipeline)"; s = PHX_E_TIMEOUT; }
   op_release(sc, ce == cudaSuccess && !raised);
   return s;

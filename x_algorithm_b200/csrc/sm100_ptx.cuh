@@ -76,7 +76,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
       else {
         const unsigned int us = (unsigned int)err_flag[1];
         const unsigned long long limit = us ? 1000ull * us : WAIT_LIMIT_NS;
-        if (now - t0 > limit) { *err_flag = 1; __threadfence(); *gave_up() = 1; return false; }
+        if (now - t0 > limit) { *err_flag = 1; __threadfence_system(); *gave_up() = 1; return false; }
       }
     }
   }
