@@ -138,6 +138,7 @@ struct GemmNorm {
 // are encoded once for (pointer, rows_max) and reused for every M <= rows_max.
 struct GemmPlan {
   CUtensorMap map_a;
+  CUtensorMap map_a_low;      // A in boxes of 64 rows, for the low tiles of small calls
   CUtensorMap map_b;
   CUtensorMap map_b_narrow;   // BN = 256: W map for narrower tiles, used when a call has too few wide tiles to fill the device
   CUtensorMap map_c;   // output map, re-encoded when the output pointer or M changes

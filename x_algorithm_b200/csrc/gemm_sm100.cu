@@ -587,25 +587,27 @@ phx_status launch_e(const GemmPlan& p, int epilogue, const GemmRope& rp, const G
 //   64-column slab g >> 1 (RoPE: the column pairs of pass g & 1)
 // Measured: a forward of one request (640 rows, 8 layers) 492 -> 431 us, 16 small requests through two layers 155 -> 143 us.
 // The arithmetic per element, the order of the row statistics included, is the pair kernel's: results are the same bits.
-template <int BN, bool DEEP>
+template <int TM, int BN, bool DEEP>
 struct SmallCfg {
   static constexpr int NG = BN / 32;
   static constexpr int THREADS = 64 + NG * 128;
-  static constexpr int STAGE_BYTES = (BM + BN) * BK * 2;
-  static constexpr int STAGES = (DEEP ? 196608 : 98304) / STAGE_BYTES;   // ring: 4 (BN = 64) or 3 (BN = 128) k-steps, deep 8 or 6
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + (BN / 64) * BM * 4 + 128 + 1024;   // + partial row sums, barriers, alignment
+  static constexpr int A_BYTES = TM * BK * 2;
+  static constexpr int STAGE_BYTES = A_BYTES + BN * BK * 2;
+  static constexpr int STAGES = (DEEP ? 196608 : 98304) / STAGE_BYTES;   // ring: 4 (BN = 64) or 3 (BN = 128) k-steps, deep 8 or 6, of low tiles 12
+  static constexpr int BAR_BYTES = (2 * STAGES + 2) * 8;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + (BN / 64) * TM * 4 + BAR_BYTES + 1024;   // + partial row sums, barriers, alignment
 };
 
-template <int BN, int EPI, bool DEEP>
-__global__ void __launch_bounds__(SmallCfg<BN, DEEP>::THREADS, 1)
+template <int TM, int BN, int EPI, bool DEEP>
+__global__ void __launch_bounds__(SmallCfg<TM, BN, DEEP>::THREADS, 1)
 gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, bf16* C, const bf16* R,
                   GemmRope rope, GemmNorm norm, long long M, int N, int K, int early_w, int* err_flag) {
-  using cfg = SmallCfg<BN, DEEP>;
+  using cfg = SmallCfg<TM, BN, DEEP>;
   constexpr bool RES = (EPI == EPI_RESIDUAL);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t ss_base = smem_base + cfg::STAGES * cfg::STAGE_BYTES;     // [slab][128] first halves of the row sums
-  const uint32_t bars = ss_base + (BN / 64) * BM * 4;
+  const uint32_t bars = ss_base + (BN / 64) * TM * 4;
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (cfg::STAGES + s); };
   const uint32_t tfull_bar = bars + 8u * (2 * cfg::STAGES);
@@ -614,7 +616,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_tiles = (N + BN - 1) / BN;
   const int n0 = ((int)blockIdx.x % n_tiles) * BN;
-  const long long m0 = (long long)((int)blockIdx.x / n_tiles) * BM;
+  const long long m0 = (long long)((int)blockIdx.x / n_tiles) * TM;
   const int k_blocks = (K + BK - 1) / BK;
   volatile int* verr = err_flag;
 
@@ -632,7 +634,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const uint32_t tmem_d = *tmem_slot_ptr;
 
   auto load_w = [&](int kb, int stage) {
-    const uint32_t dst = smem_base + stage * cfg::STAGE_BYTES + BM * BK * 2;
+    const uint32_t dst = smem_base + stage * cfg::STAGE_BYTES + cfg::A_BYTES;
     for (int c = 0; c < BN / 64; ++c) tma_load_2d(dst + c * 64 * BK * 2, &map_b, full_bar(stage), kb * BK, n0 + c * 64);
   };
   const int ahead = k_blocks < cfg::STAGES ? k_blocks : cfg::STAGES;
@@ -658,14 +660,14 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = make_idesc(BM, BN);
+      constexpr uint32_t idesc = make_idesc(TM, BN);
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       for (int kb = 0; kb < k_blocks; ++kb) {
         if (!mbar_wait(full_bar(stage), phase, verr)) { ok = false; break; }
         tc_fence_after();
         const uint64_t adesc = make_smem_desc(smem_base + stage * cfg::STAGE_BYTES);
-        const uint64_t bdesc = make_smem_desc(smem_base + stage * cfg::STAGE_BYTES + BM * BK * 2);
+        const uint64_t bdesc = make_smem_desc(smem_base + stage * cfg::STAGE_BYTES + cfg::A_BYTES);
 #pragma unroll
         for (int k = 0; k < 4; ++k) umma_bf16(tmem_d, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (kb | k) != 0);
         umma_commit(empty_bar(stage));
@@ -678,9 +680,11 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const bool d128 = EPI == EPI_ROPE && BN == 128 && rope.dh == 128;
     const int gidx = (warp - 2) >> 2, slab = d128 ? 0 : gidx >> 1, p = d128 ? gidx : gidx & 1;
     const int quad = warp & 3;
-    const int r = quad * 32 + lane;
+    // a tile of 64 rows lies in the first 16 lanes of each quadrant of tensor memory
+    const bool has_row = TM == 128 || lane < 16;
+    const int r = quad * (TM / 4) + (TM == 128 ? lane : lane & 15);
     const long long row = m0 + r;
-    const bool in = row < M;
+    const bool in = has_row && row < M;
     const int c0 = n0 + slab * 64;                       // first column of the slab
     // two runs of 16 columns: neighbours, or (RoPE) the halves of a head that are rotated against each other
     const bool d64 = EPI == EPI_ROPE && rope.dh == 64;
@@ -766,12 +770,12 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       if (RES && norm.ss_out != nullptr) {
         // statistics of the fp32 sums, one chain over the slab's 64 columns: the second half's thread goes on from where
         // the first half's stopped
-        const uint32_t slot = ss_base + (slab * BM + r) * 4;
+        const uint32_t slot = ss_base + (slab * TM + r) * 4;
         float ss = 0.f;
         if (p == 0) {
 #pragma unroll
           for (int k = 0; k < (RES ? 16 : 1); ++k) { ss += v[k].x * v[k].x; ss += v[k].y * v[k].y; }
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot), "f"(ss) : "memory");
+          if (has_row) asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot), "f"(ss) : "memory");
         }
         asm volatile("bar.sync %0, 256;" ::"r"(1 + slab) : "memory");
         if (p == 1) {
@@ -794,11 +798,11 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   }
 }
 
-template <int BN, int EPI, bool DEEP>
+template <int TM, int BN, int EPI, bool DEEP>
 phx_status launch_small_d(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C, const bf16* R, const GemmRope& rope,
                           const GemmNorm& norm, int64_t M, int* err_flag, cudaStream_t stream, std::string& err) {
-  using cfg = SmallCfg<BN, DEEP>;
-  auto kern = gemm_small_kernel<BN, EPI, DEEP>;
+  using cfg = SmallCfg<TM, BN, DEEP>;
+  auto kern = gemm_small_kernel<TM, BN, EPI, DEEP>;
   static SmemLimit limit;
   PHX_CUDA_TRY(limit.raise(kern, cfg::SMEM_BYTES), err);
   cudaLaunchConfig_t lc;
@@ -810,13 +814,13 @@ phx_status launch_small_d(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr; lc.numAttrs = 1;
   }
-  lc.gridDim = dim3((unsigned)(((M + BM - 1) / BM) * ((p.N + BN - 1) / BN)));
+  lc.gridDim = dim3((unsigned)(((M + TM - 1) / TM) * ((p.N + BN - 1) / BN)));
   lc.blockDim = dim3(cfg::THREADS);
   lc.dynamicSmemBytes = cfg::SMEM_BYTES;
   lc.stream = stream;
   long long Mll = M;
   int N = p.N, K = p.K, early = p.w_stable ? 1 : 0;
-  PHX_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, p.map_a, map_b64, C, R, rope, norm, Mll, N, K, early, err_flag), err);
+  PHX_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, TM == 64 ? p.map_a_low : p.map_a, map_b64, C, R, rope, norm, Mll, N, K, early, err_flag), err);
   return PHX_OK;
 }
 // A deep ring has its SM for itself; a shallow one leaves room for a CTA of the kernel behind.  Deep from K = 1024 on, and from 512 where the
@@ -827,12 +831,17 @@ phx_status launch_small_d(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C
 bool deep_ring(int K, int epilogue, long long tiles, int num_sms) {
   return K >= 1024 || (K >= 512 && (epilogue == EPI_RESIDUAL || 3 * tiles <= 2 * num_sms));
 }
+// Tiles of 64 rows where those find an SM each: a k-step is paced by the rows its copies bring in (1.6 to 1.9 cycles a row of 128 bytes,
+// however deep the ring), 128 in place of 192.  The forwards above: one request of 172 rows 216 -> 203 us, three of 106 213 -> 197, one of 640
+// 250 -> 240 (from K = 1024 on alone: 213, 206, 244).
+bool low_tiles(int64_t M, int N, int K, int num_sms) { return K >= 512 && ((M + 63) / 64) * ((N + 63) / 64) <= num_sms; }
 template <int BN, int EPI>
 phx_status launch_small_t(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C, const bf16* R, const GemmRope& rope,
                           const GemmNorm& norm, int64_t M, int num_sms, int* err_flag, cudaStream_t stream, std::string& err) {
+  if (BN == 64 && low_tiles(M, p.N, p.K, num_sms)) return launch_small_d<64, 64, EPI, true>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err);
   const long long tiles = ((M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
-  return deep_ring(p.K, EPI, tiles, num_sms) ? launch_small_d<BN, EPI, true>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err)
-                                             : launch_small_d<BN, EPI, false>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err);
+  return deep_ring(p.K, EPI, tiles, num_sms) ? launch_small_d<BM, BN, EPI, true>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err)
+                                             : launch_small_d<BM, BN, EPI, false>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err);
 }
 template <int BN>
 phx_status launch_small(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C, const bf16* R, int epilogue, const GemmRope& rp,
@@ -897,6 +906,7 @@ phx_status gemm_plan_create(GemmPlan* plan, const bf16* A, const bf16* Wt, int64
   if (plan->pair && !(getenv("PHX_GEMM_TILES") && strcmp(getenv("PHX_GEMM_TILES"), "narrow") == 0)) narrow_tiles = false;
   plan->BN = (N % 256 == 0 && !narrow_tiles) ? 256 : 128;
   phx_status s = make_map(&plan->map_a, A, rows_max, K, BM, err);
+  if (s == PHX_OK) s = make_map(&plan->map_a_low, A, rows_max, K, 64, err);
   if (s != PHX_OK) return s;
   s = make_map(&plan->map_b, Wt, N, K, plan->pair ? plan->BN / 2 : plan->BN, err);
   if (s != PHX_OK) return s;
@@ -922,6 +932,7 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
     // the activation buffer moved (double-buffered residual stream, or a block of rows inside it): re-encode its
     // map over exactly the M rows of this call, so that no tile reads past them
     phx_status s = make_map(&p.map_a, A, M, p.K, BM, err);
+    if (s == PHX_OK) s = make_map(&p.map_a_low, A, M, p.K, 64, err);
     if (s != PHX_OK) return s;
     p.A = A; p.a_rows = M;
   }
