@@ -126,18 +126,25 @@ __device__ __forceinline__ float s8_value(uint32_t acc, float query_scale) { ret
 constexpr float S8_OFFSET = 12582912.0f;            // 1.5 * 2^23: its bit pattern plus an integer below 2^22 in size is the float of their sum
 constexpr uint32_t S8_OFFSET_BITS = 0x4B400000u;
 
-// Columns per group of the collect filter: the group's threshold is the smallest of its queries'.
-template <int NQ> struct ScanCfg {
-  static constexpr int CW = NQ / 4;                  // query columns per consumer warp
-  static constexpr int CH = CW < 32 ? CW : 32;       // columns per group
+// How the consumer warps share the tiles: all sixteen on every tile, a quarter of the columns each, or (SPLIT: the collect pass with 64
+// columns) eight on every other tile, half of the columns each.  A warp that has rows to test is late for its next tile, and an
+// accumulator goes back to the MMA warp when the last of its warps has read it: split, fewer warps wait for one another, each has two
+// tiles' time, and what a tile costs beside its columns (wait, vote, release) is paid half as often.  12.5 M int8 rows, 64 queries, us, k = 1 /
+// 1000: 320 / 369 -> 311 / 330.  With 128 columns it takes as much from short lists as it gives long ones (396 / 477 -> 414 / 460); with 256 a
+// warp's half would take two turns, and rows to test in the first would hold the accumulator (581 / 710 -> 726 / 918).
+template <int MODE, int NQ> struct ScanCfg {
+  static constexpr bool SPLIT = MODE == 1 && NQ == 64;
+  static constexpr int CW = SPLIT ? NQ / 2 : NQ / 4; // query columns per consumer warp
+  static constexpr int CH = CW < 32 ? CW : 32;       // columns per group; the collect filter's threshold is the smallest of the group's
   static constexpr int GROUPS = NQ / CH;
+  static constexpr int DRAIN = (SPLIT ? TC_CWARPS / 2 : TC_CWARPS) * 32;   // threads that release an accumulator
 };
 
 template <int MODE, bool I8, int NQ, bool BIAS>
 __global__ void __launch_bounds__(scan_threads(BIAS), 1)
 scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_constant__ CUtensorMap map_users,
                TcScanArgs a, int* err_flag) {
-  using cfg = ScanCfg<NQ>;
+  using cfg = ScanCfg<MODE, NQ>;
   constexpr int CW = cfg::CW, CH = cfg::CH;
   static_assert(!BIAS || (MODE == 1 && I8), "the bias belongs to the int8 collect pass");
   extern __shared__ uint8_t smem_raw[];
@@ -184,7 +191,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
     *gave_up() = 0;
     prefetch_map(&map_corpus); prefetch_map(&map_users);
     for (int s = 0; s < TC_STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-    for (int x = 0; x < 2; ++x) { mbar_init(tfull_bar(x), 1); mbar_init(tempty_bar(x), 32 * TC_CWARPS); }
+    for (int x = 0; x < 2; ++x) { mbar_init(tfull_bar(x), 1); mbar_init(tempty_bar(x), cfg::DRAIN); }
     for (int s = 0; s < TC_STAGES; ++s) mbar_init(xfull_bar(s), 1);
     mbar_init(users_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -366,7 +373,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
     auto consume = [&](auto folded) {
       constexpr bool FOLDED = decltype(folded)::value;
       const int ew = warp - 2;
-      const int part = ew >> 2;        // which quarter of the query columns
+      const int part = cfg::SPLIT ? (ew >> 2) & 1 : ew >> 2;   // which half or quarter of the query columns
       const int quad = warp & 3;       // TMEM lane quadrant
       uint4* const queue = s_queue + ew * QCAP;
       uint32_t* const s_row = reinterpret_cast<uint32_t*>(smem_raw + (rows_smem - smem_u32(smem_raw))) + ew * 32;
@@ -382,12 +389,13 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
         bt_lane[c] = (FOLDED && lane < CH) ? s_t[part * CW + c * CH + lane] : 0;
       }
       const int open = FOLDED ? *s_open : 0;
-      uint32_t it = 0;
-      for (long long w = blockIdx.x; w < n_work; w += gridDim.x, ++it) {
+      constexpr int EACH = cfg::SPLIT ? 2 : 1;                 // a warp's tiles: every one, or every other one
+      uint32_t it = cfg::SPLIT ? ew >> 3 : 0;
+      for (long long w = blockIdx.x + (long long)it * gridDim.x; w < n_work; w += (long long)EACH * gridDim.x, it += EACH) {
         const long long tile = (MODE == 0) ? w * a.stride : w;
         const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
         const long long row = tile * TC_ROWS + quad * 32 + lane;
-        const bool row_ok = row < a.rows && row_eligible(a.mask, a.mask_row0, row);
+        const bool row_ok = MODE == 1 || (row < a.rows && row_eligible(a.mask, a.mask_row0, row));   // collect pass: asked of rows that pass
         // the row's scale; with the bias it is fetched only when a row passes the filter
         float rs = (I8 && !FOLDED && row < a.rows) ? __ldg(a.row_scale + row) : 0.f;
         bool have_rs = false;
@@ -427,7 +435,8 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
               mx = fmaxf(mx, __uint_as_float(r[CH - 1]));
               pass = mx >= s_thr_min[u0 / CH];
             }
-            uint32_t rows_left = __ballot_sync(0xffffffffu, row_ok && pass);
+            uint32_t rows_left = __ballot_sync(0xffffffffu, pass);
+            if (rows_left) rows_left &= __ballot_sync(0xffffffffu, row < a.rows && row_eligible(a.mask, a.mask_row0, row));
             if (FOLDED && rows_left && !have_rs) {
               rs = row < a.rows ? __ldg(a.row_scale + row) : 0.f;
               x_row = bias_x(bias_c, rs);
@@ -453,7 +462,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
                 mx = max3(mx, v.x, v.y);
               }
               pass = pass && (!(rs >= 0.f) || !((mx + s_us_max[u0 / CH]) * rs < s_thr_min[u0 / CH]));
-              rows_left = __ballot_sync(0xffffffffu, row_ok && pass);
+              rows_left &= __ballot_sync(0xffffffffu, pass);
             }
             // The few rows that pass, one at a time: the row's scores go through shared memory so that lane k holds column
             // k's, every lane compares with its own column's threshold, and the hits line up in the queue by ballot.  (Each
