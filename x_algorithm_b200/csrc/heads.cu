@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(256) heads_kernel(HeadsArgs a) {
 
 
 // ---- tensor-core variant (D a multiple of 32) -----------------------------------------------------------------------
-// One warp = 16 candidate rows.  The head matrix product runs on mma.sync m16n8k16: within every group of 32 columns
+// A strip = 16 candidate rows.  The head matrix product runs on mma.sync m16n8k16: within every group of 32 columns
 // the k index is permuted so that a thread's A fragments for two k-steps are one 16-byte load of its row (columns
 // 8*t4 .. 8*t4+7 of the group) and its B fragments one 16-byte read of the head matrix row in shared memory.  Rows are
 // normalised exactly like the scalar kernel (x * rstd * gain rounded to bf16) on their way into the fragments; the
@@ -125,12 +125,131 @@ __device__ __forceinline__ void mma_bf16_16816_h(float (&c)[4], const uint32_t (
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// NT: n-tiles of 8 outputs, V + NC <= 8 * NT.  WPS: warps per strip.  With enough strips every warp has its own (1); a small call
-// is one strip's chain of latencies - round trips to its rows, then rounds of logarithms and f64 exponentials - so eight warps
-// fetch the strip's rows into shared memory in one go, form the same sums and share the (row, output) items.  Same arithmetic,
-// same bits.  Kernel at 20 outputs, parameters not yet staged (one warp / eight): D = 512: 512 to 2048 rows 18.5 / 11.5 us, 4096
-// rows 18.7 / 14.9, 8192 rows 20.4 / 27.2; D = 1024: 512 rows 29.0 / 18.3, 4800 rows 28.3 / 38.3; D = 128: 128 rows 12.7 / 6.6.
-template <int NT, int WPS, bool STAGED>
+// Row r of the call: candidate r % C of request r / C, or (packed) the r-th candidate row.  Rows fit 31 bits.
+__device__ __forceinline__ const bf16* head_row(const HeadsArgs& a, long long r, long long nrows) {
+  if (r >= nrows) r = nrows - 1;
+  if (a.out_index) return a.x + r * (long long)a.D;
+  const unsigned b = (unsigned)r / (unsigned)a.C, c = (unsigned)r - b * (unsigned)a.C;
+  return a.x + ((long long)b * a.T + a.S + c) * (long long)a.D;
+}
+// One (row, output) pair: the result, and its value for the blend.
+__device__ __forceinline__ double head_item(const HeadsArgs& a, float mine, long long r, long long nrows, int oo) {
+  const long long orow = (a.out_index && r < nrows) ? a.out_index[r] : r;   // packed rows: the output slot this row answers
+  if (oo < a.V) {
+    float lg = round_bf(round_bf(mine) * a.output_scale);
+    if (a.final_logit_cap > 0.f) lg = round_bf(a.final_logit_cap * tanhf(lg / a.final_logit_cap));
+    const float logp = fminf(lg, 0.f) - log1pf(expf(-fabsf(lg)));  // log_sigmoid in fp32
+    if (a.log_probs && r < nrows) a.log_probs[orow * a.V + oo] = logp;
+    return a.has_blend ? exp((double)logp) : 0.0;   // exp(ln p as f32 -> f64) like the client side
+  }
+  const float cl = round_bf(mine);
+  const float sg = round_bf(1.0f / (1.0f + expf(-cl)));
+  const float value = round_bf(sg * a.dwell_norm_scale);
+  if (a.continuous && r < nrows) a.continuous[orow * a.NC + (oo - a.V)] = value;
+  return (double)value;
+}
+__device__ __forceinline__ void head_blend(const HeadsArgs& a, const double* cols, long long r) {
+  double s = 0.0;   // terms summed left to right in f64
+#pragma unroll 4
+  for (int i = 0; i < a.blend.num_terms; ++i) s = s + cols[a.blend.src[i]] * a.blend.weight[i];
+  double out;
+  if (a.blend.total_sum == 0.0) out = s > 0.0 ? s : 0.0;
+  else if (s < 0.0) out = (s + a.blend.negative_sum) / a.blend.total_sum * 0.001;
+  else out = s + 0.001;
+  a.scores[a.out_index ? a.out_index[r] : r] = out;
+}
+__device__ __forceinline__ float square_sum(uint4 u) {
+  const float2 p0 = unpack_bf2(u.x), p1 = unpack_bf2(u.y), p2 = unpack_bf2(u.z), p3 = unpack_bf2(u.w);
+  return (p0.x * p0.x + p0.y * p0.y) + (p1.x * p1.x + p1.y * p1.y) + (p2.x * p2.x + p2.y * p2.y) + (p3.x * p3.x + p3.y * p3.y);
+}
+// the head matrix and the norm's gain, staged while the last GEMM of the trunk drains
+template <int NT>
+__device__ __forceinline__ void stage_parameters(const HeadsArgs& a, bf16* sw, float* sgain) {
+  const int D = a.D, NO = a.V + a.NC, WLD = D + HM_WPAD;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < NT * 8 * (D / 8); i += blockDim.x) {
+    const int n = i / (D / 8), ch = i % (D / 8);
+    uint4 w = make_uint4(0u, 0u, 0u, 0u);
+    if (n < NO) w = *reinterpret_cast<const uint4*>(a.unembed_t + (long long)n * D + ch * 8);
+    *reinterpret_cast<uint4*>(sw + n * WLD + ch * 8) = w;
+  }
+  for (int i = threadIdx.x; i < D; i += blockDim.x) sgain[i] = a.final_gain[i];
+}
+
+// NT: n-tiles of 8 outputs, V + NC <= 8 * NT.  A strip of 16 rows is a chain of latencies - a round trip to its rows, sums of squares in a
+// fixed order, products, logarithms and f64 exponentials, the blend.  In a small call sixteen warps take it together: the rows arrive in
+// shared memory by one round of copies, two warps form the sums of squares (a quad a row), all of them normalise, a warp per n-tile
+// multiplies, and every (row, output) pair has a thread.  Where eight warps each went through the whole strip, 512 rows of 512 columns with 20
+// outputs took 2.1 us for the rows, 1.2 + 2.6 for sums and products, 1.1 and 0.7 for the rest.
+constexpr int HS_WARPS = 16;
+template <int NT>
+__global__ void __launch_bounds__(HS_WARPS * 32, 3) heads_strip_kernel(HeadsArgs a) {
+  extern __shared__ __align__(16) uint8_t hsm[];
+  const int D = a.D, NO = a.V + a.NC, WLD = D + HM_WPAD, per_row = D / 8, groups = D / 32;
+  bf16* sw = reinterpret_cast<bf16*>(hsm);                                   // [NT*8][WLD], rows >= NO are zero
+  float* sgain = reinterpret_cast<float*>(sw + NT * 8 * WLD);                // [D]
+  float* sC = sgain + D;                                                     // [16][NT*8] fp32 sums
+  double* sD = reinterpret_cast<double*>(sC + 16 * NT * 8);                  // [16][NT*8] blend inputs
+  float* srstd = reinterpret_cast<float*>(sD + 16 * NT * 8);                 // [16]
+  bf16* sX = reinterpret_cast<bf16*>(srstd + 16);                            // [16][WLD] the strip's rows, normalised in place
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const long long nrows = a.out_index ? a.rows : (long long)a.B * a.C, r0 = (long long)blockIdx.x * 16;
+  stage_parameters<NT>(a, sw, sgain);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  for (int i = threadIdx.x; i < 16 * per_row; i += HS_WARPS * 32) {
+    const int rr = i / per_row, ch = i - rr * per_row;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(sX + rr * WLD + ch * 8);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(head_row(a, r0 + rr, nrows) + ch * 8) : "memory");
+  }
+  asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  if (warp < 2) {    // sums of squares: a row's 32-column groups are spread over the 4 lanes of its quad
+    const bf16* xr = sX + (warp * 8 + g) * WLD + 8 * t4;
+    float ss = 0.f;
+#pragma unroll 8
+    for (int gr = 0; gr < groups; ++gr) ss += square_sum(*reinterpret_cast<const uint4*>(xr + gr * 32));
+    ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+    if (t4 == 0) srstd[warp * 8 + g] = rsqrtf(ss / (float)D + a.eps);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 16 * per_row; i += HS_WARPS * 32) {   // the normed row is bf16
+    const int rr = i / per_row, ch = i - rr * per_row;
+    uint4* const at = reinterpret_cast<uint4*>(sX + rr * WLD + ch * 8);
+    const float4 ga = *reinterpret_cast<const float4*>(sgain + ch * 8), gb = *reinterpret_cast<const float4*>(sgain + ch * 8 + 4);
+    const float rstd = srstd[rr];
+    const uint4 u = *at;
+    const float2 p0 = unpack_bf2(u.x), p1 = unpack_bf2(u.y), p2 = unpack_bf2(u.z), p3 = unpack_bf2(u.w);
+    *at = make_uint4(pack_bf2(p0.x * rstd * ga.x, p0.y * rstd * ga.y), pack_bf2(p1.x * rstd * ga.z, p1.y * rstd * ga.w),
+                     pack_bf2(p2.x * rstd * gb.x, p2.y * rstd * gb.y), pack_bf2(p3.x * rstd * gb.z, p3.y * rstd * gb.w));
+  }
+  __syncthreads();
+  if (warp < NT) {
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int gr = 0; gr < groups; ++gr) {
+      // k-step 0 uses pairs 0, 1 of each row's 8 columns, k-step 1 pairs 2, 3: fragment order [g][lo], [g+8][lo], [g][hi], [g+8][hi]
+      const uint4 lo = *reinterpret_cast<const uint4*>(sX + g * WLD + gr * 32 + 8 * t4), hi = *reinterpret_cast<const uint4*>(sX + (g + 8) * WLD + gr * 32 + 8 * t4);
+      const uint4 w = *reinterpret_cast<const uint4*>(sw + (warp * 8 + g) * WLD + gr * 32 + 8 * t4);
+      const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
+      mma_bf16_16816_h(acc, a0, w.x, w.y);
+      mma_bf16_16816_h(acc, a1, w.z, w.w);
+    }
+    *reinterpret_cast<float2*>(sC + g * (NT * 8) + warp * 8 + 2 * t4) = make_float2(acc[0], acc[1]);
+    *reinterpret_cast<float2*>(sC + (g + 8) * (NT * 8) + warp * 8 + 2 * t4) = make_float2(acc[2], acc[3]);
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < 16 * NO; idx += HS_WARPS * 32) {
+    const int rr = idx / NO, oo = idx - rr * NO;
+    sD[rr * (NT * 8) + oo] = head_item(a, sC[rr * (NT * 8) + oo], r0 + rr, nrows, oo);
+  }
+  __syncthreads();
+  if (a.has_blend && a.scores && threadIdx.x < 16 && r0 + threadIdx.x < nrows) head_blend(a, sD + threadIdx.x * (NT * 8), r0 + threadIdx.x);
+}
+
+// Many strips: every warp has its own (WPS = 1) and reads its rows where they are, once for the sums of squares, once for the products; the
+// same arithmetic, the same bits.  Four warps share one in small calls of rows too wide to stand beside the head matrix in shared memory.
+template <int NT, int WPS>
 __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_kernel(HeadsArgs a) {
   constexpr int WARPS = WPS == 1 ? HM_WARPS : WPS;      // warps per CTA
   extern __shared__ __align__(16) uint8_t hsm[];
@@ -139,16 +258,8 @@ __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_ke
   float* sgain = reinterpret_cast<float*>(sw + NT * 8 * WLD);                // [D]
   float* sC_all = sgain + D;                                                 // per warp [16][NT*8] fp32 sums
   double* sD_all = reinterpret_cast<double*>(sC_all + WARPS * 16 * NT * 8);   // per strip [16][NT*8] blend inputs
-  bf16* sX = reinterpret_cast<bf16*>(sD_all + (WPS == 1 ? HM_WARPS : 1) * 16 * NT * 8);   // STAGED: [16][WLD] the strip's rows
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < NT * 8 * (D / 8); i += WARPS * 32) {
-    const int n = i / (D / 8), ch = i % (D / 8);
-    uint4 w = make_uint4(0u, 0u, 0u, 0u);
-    if (n < NO) w = *reinterpret_cast<const uint4*>(a.unembed_t + (long long)n * D + ch * 8);
-    *reinterpret_cast<uint4*>(sw + n * WLD + ch * 8) = w;
-  }
-  for (int i = threadIdx.x; i < D; i += blockDim.x) sgain[i] = a.final_gain[i];
+  stage_parameters<NT>(a, sw, sgain);
   // programmatic dependent launch: the parameters above are staged while the last GEMM of the trunk drains; its
   // output is read only from here on
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -163,38 +274,14 @@ __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_ke
   for (long long strip = (long long)blockIdx.x * CTA_STRIPS + (WPS == 1 ? warp : 0); strip < n_strips; strip += (long long)gridDim.x * CTA_STRIPS) {
     const long long r0 = strip * 16;
     const bf16* xr[2];
-    auto row_of = [&](int i) {
-      long long r = r0 + i;
-      if (r >= nrows) r = nrows - 1;
-      if (a.out_index) return a.x + r * (long long)D;
-      const unsigned b = (unsigned)r / (unsigned)a.C, c = (unsigned)r - b * (unsigned)a.C;     // rows fit 31 bits
-      return a.x + ((long long)b * a.T + a.S + c) * (long long)D;
-    };
-    if (!STAGED) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) xr[i] = row_of(g + 8 * i) + 8 * t4;
-    } else {
-      // one round trip for the whole strip instead of one per 32 columns and pass
-      const int per_row = D / 8;
-#pragma unroll 8
-      for (int i = threadIdx.x; i < 16 * per_row; i += WARPS * 32) {
-        const int rr = i / per_row, ch = i - rr * per_row;
-        *reinterpret_cast<uint4*>(sX + rr * WLD + ch * 8) = *reinterpret_cast<const uint4*>(row_of(rr) + ch * 8);
-      }
-      __syncthreads();
-#pragma unroll
-      for (int i = 0; i < 2; ++i) xr[i] = sX + (g + 8 * i) * WLD + 8 * t4;
-    }
+    for (int i = 0; i < 2; ++i) xr[i] = head_row(a, r0 + g + 8 * i, nrows) + 8 * t4;
     // pass 1: sums of squares (a row's 32-column groups are spread over the 4 lanes of its quad)
     float ss[2] = {0.f, 0.f};
 #pragma unroll 8
     for (int gr = 0; gr < groups; ++gr) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const uint4 u = *reinterpret_cast<const uint4*>(xr[i] + gr * 32);
-        const float2 p0 = unpack_bf2(u.x), p1 = unpack_bf2(u.y), p2 = unpack_bf2(u.z), p3 = unpack_bf2(u.w);
-        ss[i] += (p0.x * p0.x + p0.y * p0.y) + (p1.x * p1.x + p1.y * p1.y) + (p2.x * p2.x + p2.y * p2.y) + (p3.x * p3.x + p3.y * p3.y);
-      }
+      for (int i = 0; i < 2; ++i) ss[i] += square_sum(*reinterpret_cast<const uint4*>(xr[i] + gr * 32));
     }
     float rstd[2];
 #pragma unroll
@@ -240,86 +327,40 @@ __global__ void __launch_bounds__((WPS == 1 ? HM_WARPS : WPS) * 32) heads_mma_ke
     __syncwarp();
     for (int idx = lane + 32 * part; idx < 16 * NO; idx += 32 * WPS) {
       const int rr = idx / NO, oo = idx % NO;
-      const long long r = r0 + rr;
-      const long long orow = (a.out_index && r < nrows) ? a.out_index[r] : r;   // packed rows: the output slot this row answers
-      const float mine = sC[rr * (NT * 8) + oo];
-      double col;
-      if (oo < a.V) {
-        float lg = round_bf(round_bf(mine) * a.output_scale);
-        if (a.final_logit_cap > 0.f) lg = round_bf(a.final_logit_cap * tanhf(lg / a.final_logit_cap));
-        const float logp = fminf(lg, 0.f) - log1pf(expf(-fabsf(lg)));  // log_sigmoid in fp32
-        if (a.log_probs && r < nrows) a.log_probs[orow * a.V + oo] = logp;
-        col = a.has_blend ? exp((double)logp) : 0.0;   // exp(ln p as f32 -> f64) like the client side
-      } else {
-        const float cl = round_bf(mine);
-        const float sg = round_bf(1.0f / (1.0f + expf(-cl)));
-        const float value = round_bf(sg * a.dwell_norm_scale);
-        if (a.continuous && r < nrows) a.continuous[orow * a.NC + (oo - a.V)] = value;
-        col = (double)value;
-      }
-      sD[rr * (NT * 8) + oo] = col;
+      sD[rr * (NT * 8) + oo] = head_item(a, sC[rr * (NT * 8) + oo], r0 + rr, nrows, oo);
     }
     if (WPS == 1) __syncwarp(); else __syncthreads();
-    if (a.has_blend && a.scores && part == 0 && lane < 16 && r0 + lane < nrows) {
-      double s = 0.0;   // terms summed left to right in f64
-#pragma unroll 4
-      for (int i = 0; i < a.blend.num_terms; ++i) s = s + sD[lane * (NT * 8) + a.blend.src[i]] * a.blend.weight[i];
-      double out;
-      if (a.blend.total_sum == 0.0) out = s > 0.0 ? s : 0.0;
-      else if (s < 0.0) out = (s + a.blend.negative_sum) / a.blend.total_sum * 0.001;
-      else out = s + 0.001;
-      a.scores[a.out_index ? a.out_index[r0 + lane] : r0 + lane] = out;
-    }
+    if (a.has_blend && a.scores && part == 0 && lane < 16 && r0 + lane < nrows) head_blend(a, sD + lane * (NT * 8), r0 + lane);
     if (WPS == 1) __syncwarp(); else __syncthreads();
   }
 }
 
-template <int NT, int WPS, bool STAGED>
-size_t heads_smem(int D) {
-  constexpr int WARPS = WPS == 1 ? HM_WARPS : WPS;
-  return (size_t)NT * 8 * (D + HM_WPAD) * sizeof(bf16) + (size_t)D * sizeof(float) +
-         (size_t)16 * NT * 8 * (WARPS * sizeof(float) + (WPS == 1 ? HM_WARPS : 1) * sizeof(double)) +
-         (STAGED ? (size_t)16 * (D + HM_WPAD) * sizeof(bf16) : 0);
-}
 constexpr size_t HEADS_SMEM_MAX = 200 * 1024;
-constexpr size_t HEADS_SMEM_SM = 228 * 1024;    // an SM's, 1 KB of it taken by each CTA
-template <int NT, int WPS, bool STAGED>
-phx_status launch_heads_wps(const HeadsArgs& a, long long strips, cudaStream_t stream, std::string& err) {
-  constexpr int WARPS = WPS == 1 ? HM_WARPS : WPS;
-  const size_t smem = heads_smem<NT, WPS, STAGED>(a.D);
+// Launched programmatically: the kernel stages its parameters while the one in front drains, and waits before it reads the residual stream.
+template <typename Kernel>
+phx_status launch_heads(Kernel kern, SmemLimit& limit, const HeadsArgs& a, long long blocks, int threads, size_t smem, cudaStream_t stream, std::string& err) {
   if (smem > HEADS_SMEM_MAX) { err = "heads: head matrix does not fit shared memory"; return PHX_E_CAPACITY; }
-  static SmemLimit limit;
-  PHX_CUDA_TRY(limit.raise(heads_mma_kernel<NT, WPS, STAGED>, (int)HEADS_SMEM_MAX), err);
-  long long blocks = WPS == 1 ? (strips + HM_WARPS - 1) / HM_WARPS : strips;
-  if (blocks > 148 * 3) blocks = 148 * 3;
-  cudaLaunchConfig_t lc;
-  memset(&lc, 0, sizeof(lc));
-  lc.gridDim = dim3((unsigned)blocks); lc.blockDim = dim3(WARPS * 32); lc.dynamicSmemBytes = smem; lc.stream = stream;
-  cudaLaunchAttribute at[1];
-  static const bool pdl = !(getenv("PHX_PDL") && getenv("PHX_PDL")[0] == '0');
-  if (pdl) {   // start while the kernel in front drains; the kernel waits before it reads the residual stream
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    lc.attrs = at; lc.numAttrs = 1;
-  }
-  PHX_CUDA_TRY(cudaLaunchKernelEx(&lc, heads_mma_kernel<NT, WPS, STAGED>, a), err);
+  PHX_CUDA_TRY(limit.raise(kern, (int)HEADS_SMEM_MAX), err);
+  PHX_CUDA_TRY(launch_programmatic(kern, dim3((unsigned)blocks), dim3(threads), smem, stream, a), err);
   return PHX_OK;
 }
 template <int NT>
 phx_status launch_heads_mma(const HeadsArgs& a, long long rows, cudaStream_t stream, std::string& err) {
-  // Up to two CTAs of a strip each per SM; a third round of them costs more than a warp a strip (measured beside the kernel).  Staged
-  // rows and the sums of eight warps take half an SM or more from about D = 1024 on: where staged CTAs would need a second round
-  // and four-warp ones, whose rows stay in global memory, would not, those run (150 / 296 strips, us, staged / four warps: D = 1024, 30 outputs
-  // 31.2 / 27.1, 33.3 / 29.2; D = 1280, 20 outputs 35.3 / 27.1, 39.4 / 31.2; D = 1536 41.5 / 33.2, 47.6 / 37.4; two of either an SM: D = 1024, 18
-  // outputs 25.1 / 25.1, 27.1 / 26.9; one of either: D = 1664, 30 outputs 47.6 / 53.7, 53.7 / 62.0).
   const long long strips = (rows + 15) / 16;
-  if (strips <= 2 * 148) {
-    const size_t staged = heads_smem<NT, 8, true>(a.D), plain = heads_smem<NT, 4, false>(a.D);
-    auto one_round = [&](size_t smem) { return strips <= 148 || 2 * (smem + 1024) <= HEADS_SMEM_SM; };
-    if (staged <= HEADS_SMEM_MAX && (one_round(staged) || !one_round(plain))) return launch_heads_wps<NT, 8, true>(a, strips, stream, err);
-    return launch_heads_wps<NT, 4, false>(a, strips, stream, err);
-  }
-  return launch_heads_wps<NT, 1, false>(a, strips, stream, err);
+  const size_t params = (size_t)NT * 8 * (a.D + HM_WPAD) * sizeof(bf16) + (size_t)a.D * sizeof(float);
+  const size_t strip_smem = params + (size_t)16 * NT * 8 * (sizeof(float) + sizeof(double)) + 64 + (size_t)16 * (a.D + HM_WPAD) * sizeof(bf16);
+  // Three CTAs of a strip each fit an SM's registers (one or two its shared memory from D = 768 on); about two rounds of them and a warp a strip
+  // are level.  Kernel at 20 outputs, us, eight warps a strip up to 296 strips and then one / this: D = 512: 32 strips 14.7 / 10.7, 288: 18.7 / 14.7;
+  // beyond the line 768: 22.9 / 22.8, 2048: 27.0 / 45.4, 8192: 92 / 164; D = 1024: 32 strips 20.7 / 14.7, 300: 31.1 / 24.9; D = 128: 8 strips
+  // 10.6 / 10.5, beyond 3750: 29.0 / 39.3.
+  static SmemLimit limit16, limit4, limit1;
+  if (strips <= 3 * 148 && strip_smem <= HEADS_SMEM_MAX)
+    return launch_heads(heads_strip_kernel<NT>, limit16, a, strips, HS_WARPS * 32, strip_smem, stream, err);
+  if (strips <= 2 * 148)
+    return launch_heads(heads_mma_kernel<NT, 4>, limit4, a, strips, 4 * 32, params + (size_t)16 * NT * 8 * (4 * sizeof(float) + sizeof(double)), stream, err);
+  const long long blocks = (strips + HM_WARPS - 1) / HM_WARPS;
+  return launch_heads(heads_mma_kernel<NT, 1>, limit1, a, blocks < 148 * 3 ? blocks : 148 * 3, HM_WARPS * 32,
+                      params + (size_t)16 * NT * 8 * HM_WARPS * (sizeof(float) + sizeof(double)), stream, err);
 }
 
 // users[b] = l2norm(mean over valid t of final_norm(x[b,t])), fp32; one CTA per user, one thread per column.  Two passes
