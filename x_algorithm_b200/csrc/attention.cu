@@ -362,7 +362,8 @@ phx_status launch_dh(const AttnArgs& a, cudaStream_t stream, std::string& err) {
 // CTA walks over all query tiles of the request.  Each warp owns a 16-row strip per tile and runs its own cp.async
 // pipeline: the strip's Q rows for tile i+1 are requested right after tile i's Q fragments are in registers, its
 // own K/V rows (for the candidates' self key) right after tile i's self term, so every load has a whole tile of
-// tensor work to hide behind and, after the prologue, no CTA-wide barrier is needed.  Rows are 128 bytes with the
+// tensor work to hide behind and, after the prologue, no CTA-wide barrier is needed.  In packed batches an item's tiles may be shared
+// between a few CTAs (launch_strip).  Rows are 128 bytes with the
 // 16-byte chunk index XOR-ed with (row & 7): conflict-free ldmatrix without padding, 96 KB per CTA, two CTAs per SM.
 constexpr int STRIP_HIST = 128;
 constexpr int STRIP_SMEM = 2 * STRIP_HIST * 64 * 2 + ATT_WARPS * 4 * 16 * 64 * 2 + (STRIP_HIST + 4) * (int)sizeof(int);
@@ -405,7 +406,11 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) ranker_attention_strip_kernel(
   else { hrow0 = (int)token_row(a.split, a.B, hist_len, T, b, 0); crow0 = (int)token_row(a.split, a.B, hist_len, T, b, n_hist) - n_hist; }
   auto trow = [&](int t) -> long long { return (long long)((t < n_hist ? hrow0 : crow0) + t); };
   const int n_blocks = (n_hist + KB - 1) / KB;
-  const int n_tiles = (T + QROWS - 1) / QROWS;
+  // this CTA's share of the request's query tiles (blockIdx.z of gridDim.z)
+  const int first = q_start / QROWS;   // candidate-only layer: query tiles in front of q_start are not wanted
+  const int all = (T + QROWS - 1) / QROWS - first;
+  const int tile0 = first + all * (int)blockIdx.z / (int)gridDim.z, n_tiles = first + all * ((int)blockIdx.z + 1) / (int)gridDim.z;
+  if (tile0 >= n_tiles) return;
   const bf16* qbase = a.q + a.q_col(h);
   const bf16* kbase = a.k + (long long)hk * a.k_head_stride;
   const bf16* vbase = a.v + (long long)hk * a.v_head_stride;
@@ -437,6 +442,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) ranker_attention_strip_kernel(
   };
 
   // ---- prologue: history K/V for the CTA, strip 0 for each warp ----------------------------------------
+  const int seg_key = (threadIdx.x < STRIP_HIST && (int)threadIdx.x < n_hist) ? a.seg[trow(threadIdx.x)] : 0;   // looked at behind the copies
   for (int c = threadIdx.x; c < STRIP_HIST * CH; c += ATT_THREADS) {
     const int kr = c >> 3, ch = c & 7;
     const bool ok = kr < n_hist;
@@ -444,17 +450,15 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) ranker_attention_strip_kernel(
     cp16((uint32_t)__cvta_generic_to_shared(hk_s + swz(kr, ch)), kbase + tok * a.k_tok_stride + ch * 8, ok);
     cp16((uint32_t)__cvta_generic_to_shared(hv_s + swz(kr, ch)), vbase + tok * a.v_tok_stride + ch * 8, ok);
   }
-  if (threadIdx.x < STRIP_HIST) {   // warps 0..3
-    const int key = threadIdx.x;
-    const int ok = (key < n_hist) && (a.seg[trow(key)] == 1);
-    skey_ok[key] = ok;
-    const int all32 = __all_sync(0xffffffffu, ok);
-    if (lane == 0) sall_ok[key >> 5] = all32;
-  }
-  const int tile0 = q_start / QROWS;   // candidate-only layer: query tiles in front of q_start are not wanted
   load_q(tile0, wq(tile0));
   if (strip_has_cand(tile0)) load_own_kv(tile0);
   cp_commit();
+  if (threadIdx.x < STRIP_HIST) {   // warps 0..3
+    const int ok = seg_key == 1;
+    skey_ok[threadIdx.x] = ok;
+    const int all32 = __all_sync(0xffffffffu, ok);
+    if (lane == 0) sall_ok[threadIdx.x >> 5] = all32;
+  }
   cp_wait<0>();
   __syncthreads();
 
@@ -661,7 +665,12 @@ template <bool CAP>
 phx_status launch_strip(const AttnArgs& a, cudaStream_t stream, std::string& err) {
   static SmemLimit limit;
   PHX_CUDA_TRY(limit.raise(ranker_attention_strip_kernel<CAP>, STRIP_SMEM), err);
-  dim3 grid(a.Hq, a.B);
+  // Packed requests are of uneven lengths: up to eight CTAs an SM in all share them out, else the kernel ends with the longest ones alone.
+  // Two layers of a batch with 1 .. 128 history and 1 .. 512 candidate rows, 8 heads, us, a CTA an item / two / three / five: 24 requests
+  // 58 / 50 / 50 / 42, 48: 81 / 70 / 66 / 66, 200: 204 / 218 / 232 / 243; 100 of up to 64 + 100 rows 46 / 50 / 52 / 58.
+  const long long items = (long long)a.Hq * a.B, tiles = (a.T + QROWS - 1) / QROWS, room = 8 * 148 / items;
+  const int parts = (int)(!a.pack.hist_off || room < 1 ? 1 : room < tiles ? room : tiles);
+  dim3 grid(a.Hq, a.B, parts);
   PHX_CUDA_TRY(launch_overlapped(ranker_attention_strip_kernel<CAP>, grid, ATT_THREADS, STRIP_SMEM, stream, a), err);
   return PHX_OK;
 }
