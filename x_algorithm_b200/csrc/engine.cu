@@ -247,7 +247,8 @@ phx_status dev_alloc(phx_engine* e, Tp** p, size_t count) {
 // host can take one while the next is on the bus.  Inputs are read from pinned memory at every size.  Whole calls, us, copies both ways /
 // results direct / inputs too: 11 KB in, 44 KB out 322 / 281 / 274; 14 KB, 11 KB 91 / 82 / 75; 112 KB, 450 KB 165 / 158 / 145; 270 KB,
 // 1.1 MB 302 / 282 / 268; 606 KB, 2.3 MB 503 / 523 / - (inputs alone 485); inputs alone, 1.4 MB 1054 -> 1018, 2.9 MB 1986 -> 1924.
-constexpr size_t DIRECT_OUT_BYTES = 1280u << 10;
+// Packed results are laid out request by request: from half a megabyte on that is worth overlapping (1.1 MB: 500 direct, 491 copied).
+constexpr size_t DIRECT_OUT_BYTES = 1280u << 10, DIRECT_OUT_PACKED_BYTES = 512u << 10;
 struct OutLayout {
   size_t lp_off, cont_off, bytes;
   OutLayout(size_t rows, int V, int NC) {
@@ -1505,7 +1506,7 @@ phx_status phx_rank_forward(phx_engine* e, const phx_rank_batch* bh, const phx_r
   // 48 ragged requests of up to 512 candidates: 580 us a call with the device zeroing and sending every slot, 524 this way.
   const size_t rows = co ? (size_t)co[B] : B * C;
   const OutLayout ol(rows, e->V, e->NC);
-  const bool direct_out = ol.bytes <= DIRECT_OUT_BYTES;
+  const bool direct_out = ol.bytes <= (co ? DIRECT_OUT_PACKED_BYTES : DIRECT_OUT_BYTES);
   float* lp_dev = e->lp_dev; float* cont_dev = e->cont_dev; double* score_dev = e->score_dev;
   float* lp_host = e->lp_host; float* cont_host = e->cont_host;
   if (direct_out) {
