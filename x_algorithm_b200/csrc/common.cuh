@@ -94,6 +94,10 @@ struct GemmRope {
   // split_rows = 0: plain layout.
   long long row_offset = 0, split_rows = 0;
   const int* pos_rows = nullptr;   // packed rows: position of every token row (overrides the rule above)
+  // The q columns of the first kv_rows rows are read by nobody (history rows of a candidate-only layer): tiles that hold nothing else
+  // may be left out.  Of every kv_per column tiles the first kv_skip, in the first kv_m_tiles row tiles (set by gemm_launch).
+  long long kv_rows = 0;
+  int kv_m_tiles = 0, kv_per = 1, kv_skip = 0;
 };
 
 // Token rows of a [B, S + C] batch.  Plain layout: row = b * T + t.  Split layout (engines with candidate-only tail

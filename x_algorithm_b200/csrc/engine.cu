@@ -563,6 +563,7 @@ phx_status run_trunk(phx_engine* e, int B, int Tt, int pos_cap, int hist_len, bo
       gr.g = e->Hq / e->Hkv; gr.group = gr.g + 2;
       if (split) { gr.T = hist_len; gr.split_rows = (long long)B * hist_len; }
       if (pk) gr.pos_rows = pk->pos_rows;
+      gr.kv_rows = off;
       if ((s = do_gemm(e, pq, a_in, e->qkv, nullptr, M, EPI_ROPE, &gr, fused ? &n_attn_in : nullptr))) return s;
     } else {
       if ((s = do_gemm(e, pq, a_in, e->qkv, nullptr, M, EPI_STORE, nullptr, fused ? &n_attn_in : nullptr))) return s;
