@@ -5,8 +5,8 @@
 //
 // The candidate x candidate block is never formed: only the history keys stream through shared memory
 // (64 keys per step, two cp.async buffers) and a candidate's single self key is folded in as one extra
-// online-softmax step computed as a per-row dot product.  One CTA = 128 query rows of one
-// (batch, head): 8 warps x 16 rows.  Everything a CTA needs at the start (Q tile, the tile's own K/V rows
+// online-softmax step computed as a per-row dot product.  One CTA = 128 (small calls: 64) query rows
+// of one (batch, head), 16 rows a warp.  Everything a CTA needs at the start (Q tile, the tile's own K/V rows
 // for the self term, the first two key blocks) is requested up front with cp.async, so a history of
 // <= 128 keys costs a single round trip to L2/HBM.  S = Q K^T and O += P V run on mma.sync m16n8k16
 // bf16 with fp32 accumulation, fragments come from padded shared memory through ldmatrix, P is rounded
@@ -61,17 +61,18 @@ __device__ __forceinline__ float scaled_logit(float s, float sm_scale, float cap
 }
 
 // CAP = false: logits stay raw accumulators and the scale sm_scale * log2(e) is folded into the exponent's FMA
-template <int DH, bool CAP>
-__global__ void __launch_bounds__(ATT_THREADS) ranker_attention_kernel(AttnArgs a) {
+template <int DH, bool CAP, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) ranker_attention_kernel(AttnArgs a) {
+  constexpr int ROWS = 16 * WARPS, THREADS = 32 * WARPS;
   constexpr int LD = DH + 8;          // padded row (elements): conflict-free ldmatrix
   constexpr int KSTEPS = DH / 16;     // k-steps of Q K^T
   constexpr int DT = DH / 8;          // output n-tiles
   constexpr int CH = DH / 8;          // 16-byte chunks per row
   extern __shared__ __align__(128) uint8_t asm_raw[];
-  bf16* sq = reinterpret_cast<bf16*>(asm_raw);     // [QROWS][LD]  Q tile, later the output tile
-  bf16* sks = sq + QROWS * LD;                     // [QROWS][LD]  K rows of the tile's own tokens
-  bf16* svs = sks + QROWS * LD;                    // [QROWS][LD]  V rows of the tile's own tokens
-  bf16* skv = svs + QROWS * LD;                    // [2][2][KB][LD]  key-block ring: (buffer, K|V)
+  bf16* sq = reinterpret_cast<bf16*>(asm_raw);     // [ROWS][LD]  Q tile, later the output tile
+  bf16* sks = sq + ROWS * LD;                     // [ROWS][LD]  K rows of the tile's own tokens
+  bf16* svs = sks + ROWS * LD;                    // [ROWS][LD]  V rows of the tile's own tokens
+  bf16* skv = svs + ROWS * LD;                    // [2][2][KB][LD]  key-block ring: (buffer, K|V)
   int* skey_ok = reinterpret_cast<int*>(skv + 4 * KB * LD);  // [2][KB]
   int* sall_ok = skey_ok + 2 * KB;                           // [2][2] per buffer and 32-key half: all keys valid history
   const float csc = CAP ? 1.0f : a.sm_scale * 1.4426950408889634f;
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(ATT_THREADS) ranker_attention_kernel(AttnArgs 
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-  const int b = blockIdx.z, h = blockIdx.y, q0 = blockIdx.x * QROWS;
+  const int b = blockIdx.z, h = blockIdx.y, q0 = blockIdx.x * ROWS;
   // rows of this request: the batch's common shape, or its own counts when the rows are packed
   int T = a.T, hist_len = a.hist_len, q_start = a.q_start;
   if (a.pack.on()) {
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(ATT_THREADS) ranker_attention_kernel(AttnArgs 
     T = hist_len + a.pack.cand_cnt(b);
     if (q_start > 0) q_start = hist_len;
   }
-  if (q0 >= T || q0 + QROWS <= q_start) return;   // past the request's rows, or history queries of a candidate-only layer
+  if (q0 >= T || q0 + ROWS <= q_start) return;   // past the request's rows, or history queries of a candidate-only layer
   const int hk = h / (a.Hq / a.Hkv);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t4 = lane & 3;
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(ATT_THREADS) ranker_attention_kernel(AttnArgs 
   else { hrow0 = (int)token_row(a.split, a.B, hist_len, T, b, 0); crow0 = (int)token_row(a.split, a.B, hist_len, T, b, n_hist) - n_hist; }
   auto trow = [&](int t) -> long long { return (long long)((t < n_hist ? hrow0 : crow0) + t); };
   const int n_blocks = (n_hist + KB - 1) / KB;
-  const bool has_cand = (q0 + QROWS > n_hist);     // rows at or past hist_len may be candidates
+  const bool has_cand = (q0 + ROWS > n_hist);     // rows at or past hist_len may be candidates
 
   const bf16* kbase = a.k + (long long)hk * a.k_head_stride;
   const bf16* vbase = a.v + (long long)hk * a.v_head_stride;
@@ -108,7 +109,7 @@ __global__ void __launch_bounds__(ATT_THREADS) ranker_attention_kernel(AttnArgs 
   auto load_block = [&](int blk, int buf) {
     bf16* dk = skv + (size_t)(buf * 2 + 0) * KB * LD;
     bf16* dv = skv + (size_t)(buf * 2 + 1) * KB * LD;
-    for (int c = threadIdx.x; c < KB * CH; c += ATT_THREADS) {
+    for (int c = threadIdx.x; c < KB * CH; c += THREADS) {
       const int kr = c / CH, dc = (c % CH) * 8;
       const int key = blk * KB + kr;
       const bool ok = key < n_hist;
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(ATT_THREADS) ranker_attention_kernel(AttnArgs 
 #pragma unroll
   for (int i = 0; i < 2; ++i) segq[i] = (rq[i] < T) ? a.seg[trow(rq[i])] : 0;
   const int seg_key = load_key(0, 2);
-  for (int c = threadIdx.x; c < QROWS * CH; c += ATT_THREADS) {
+  for (int c = threadIdx.x; c < ROWS * CH; c += THREADS) {
     const int r = c / CH, dc = (c % CH) * 8;
     const bool ok = (q0 + r) < T;
     const long long tok = trow(ok ? q0 + r : 0);
@@ -345,15 +346,22 @@ cudaError_t launch_overlapped(Kern kern, dim3 grid, int threads, size_t smem, cu
   return cudaLaunchKernelEx(&lc, kern, a);
 }
 
+template <int DH, bool CAP, int WARPS>
+phx_status launch_rows(const AttnArgs& a, cudaStream_t stream, std::string& err) {
+  constexpr int LD = DH + 8, ROWS = 16 * WARPS;
+  const size_t smem = (size_t)(3 * ROWS + 4 * KB) * LD * 2 + (2 * KB + 4) * sizeof(int);
+  static SmemLimit limit;
+  PHX_CUDA_TRY(limit.raise(ranker_attention_kernel<DH, CAP, WARPS>, (int)smem), err);
+  dim3 grid((a.T + ROWS - 1) / ROWS, a.Hq, a.B);
+  PHX_CUDA_TRY(launch_overlapped(ranker_attention_kernel<DH, CAP, WARPS>, grid, 32 * WARPS, smem, stream, a), err);
+  return PHX_OK;
+}
+// Tiles of 64 rows while two of them fit every SM: a small call's time is one tile's, and eight warps of a tile share the tensor cores
+// that four of it would have to themselves (eight layers, device us: one request of 640 rows 238 -> 231, of 172 rows 203 -> 193, 16 of 118 322 -> 313).
 template <int DH, bool CAP>
 phx_status launch_dh(const AttnArgs& a, cudaStream_t stream, std::string& err) {
-  constexpr int LD = DH + 8;
-  const size_t smem = (size_t)(3 * QROWS + 4 * KB) * LD * 2 + (2 * KB + 4) * sizeof(int);
-  static SmemLimit limit;
-  PHX_CUDA_TRY(limit.raise(ranker_attention_kernel<DH, CAP>, (int)smem), err);
-  dim3 grid((a.T + QROWS - 1) / QROWS, a.Hq, a.B);
-  PHX_CUDA_TRY(launch_overlapped(ranker_attention_kernel<DH, CAP>, grid, ATT_THREADS, smem, stream, a), err);
-  return PHX_OK;
+  const long long low = (long long)((a.T + 63) / 64) * a.Hq * a.B;
+  return low <= 2 * 148 ? launch_rows<DH, CAP, 4>(a, stream, err) : launch_rows<DH, CAP, ATT_WARPS>(a, stream, err);
 }
 
 
