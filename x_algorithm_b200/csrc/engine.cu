@@ -100,6 +100,7 @@ struct phx_engine {
   bool taps_plain = false;
   bool taps_of_rank = false;       // the last forward ranked candidates (the tower's rows are plain as they are)
   bool history_done = false;       // its history rows have been taken through the last layer
+  bool history_q_done = false;     // ... and have their queries of that layer, which the forward may have left out
   // packed rows (cfg.pack_ragged): every forward addresses its token rows through a PackMap; `full` covers all slots
   // of every request (device-pointer entry points, batches that are not front-filled), `ragged` the counts the
   // host-buffer call found in its batch
@@ -529,6 +530,48 @@ phx_status layer_update(phx_engine* e, Layer& L, long long off, long long Mu) {
   return PHX_OK;
 }
 
+// QKV projection of one layer over the first M rows, with RoPE and the norm in front of it; of the first kv_rows rows nobody reads q
+phx_status layer_qkv(phx_engine* e, Layer& L, int B, int Tt, int pos_cap, int hist_len, bool split, const phx_engine::PackState* pk,
+                     long long M, long long kv_rows) {
+  const phx_model_config& c = e->cfg;
+  const bool fused = e->fused_norm;
+  const int slots = e->D / 64;
+  phx_status s;
+  GemmNorm n_attn_in = {e->rowss_a, nullptr, slots, 1.0f / (float)e->D, c.rms_eps};   // consume stats of x -> QKV
+  if (!fused) {
+    { ProfScope ps(e, KC_NORM);
+    if ((s = rmsnorm_launch(e->x, L.pre_attn_norm, e->hbuf, nullptr, M, e->D, c.rms_eps, e->stream, e->err))) return s; }
+    e->last_launches++;
+  }
+  GemmPlan& pq = fused ? L.p_qkv_f : L.p_qkv;
+  const bf16* a_in = fused ? e->x : e->hbuf;
+  // RoPE rides in the QKV epilogue unless qk-norm has to run first (heads of 128 through a pass of their own: 522 us for a
+  // two-layer forward of 8 x 1086 rows, 465 us in the epilogue)
+  const bool fuse_rope = c.rotary && !c.qk_norm && !e->use_simt_gemm;
+  if (fuse_rope) {
+    GemmRope gr;
+    gr.angles = e->angles; gr.n_pos = e->S + 1; gr.T = Tt; gr.pos_cap = pos_cap; gr.dh = e->dh;
+    gr.g = e->Hq / e->Hkv; gr.group = gr.g + 2;
+    if (split) { gr.T = hist_len; gr.split_rows = (long long)B * hist_len; }
+    if (pk) gr.pos_rows = pk->pos_rows;
+    gr.kv_rows = kv_rows;
+    if ((s = do_gemm(e, pq, a_in, e->qkv, nullptr, M, EPI_ROPE, &gr, fused ? &n_attn_in : nullptr))) return s;
+  } else {
+    if ((s = do_gemm(e, pq, a_in, e->qkv, nullptr, M, EPI_STORE, nullptr, fused ? &n_attn_in : nullptr))) return s;
+  }
+  if (!fuse_rope && (c.rotary || c.qk_norm)) {
+    QkNormRopeArgs qa;
+    qa.qkv = e->qkv; qa.M = M; qa.T = Tt; qa.Hq = e->Hq; qa.Hkv = e->Hkv; qa.dh = e->dh; qa.pos_cap = pos_cap;
+    qa.rotary = c.rotary; qa.qk_norm = c.qk_norm; qa.q_gain = L.q_norm; qa.k_gain = L.k_norm;
+    qa.cos_tab = e->cos_tab; qa.sin_tab = e->sin_tab;
+    if (split) { qa.T = hist_len; qa.split_rows = (long long)B * hist_len; }
+    if (pk) qa.pos_rows = pk->pos_rows;
+    { ProfScope ps(e, KC_ROPE); if ((s = qknorm_rope_launch(qa, e->stream, e->err))) return s; }
+    e->last_launches++;
+  }
+  return PHX_OK;
+}
+
 // trunk over `Tt` tokens per request (history + candidates, or history only for the tower).
 // split: the rows are in split layout (token_row); the last `n_tail` layers then update the candidate rows only
 // (transformer.py:789-871): their QKV projection still covers every row - the history keys / values of a tail layer
@@ -542,42 +585,9 @@ phx_status run_trunk(phx_engine* e, int B, int Tt, int pos_cap, int hist_len, bo
   phx_status s;
   for (int l = 0; l < c.num_layers; ++l) {
     Layer& L = e->layers[l];
-    const bool fused = e->fused_norm;
-    const int slots = e->D / 64;
     const bool tail = (split || pk) && l >= c.num_layers - n_tail;
     const long long off = tail ? (pk ? pk->Mh : (long long)B * hist_len) : 0;   // first row the out-projection and FFN update
-    GemmNorm n_attn_in = {e->rowss_a, nullptr, slots, 1.0f / (float)e->D, c.rms_eps};   // consume stats of x -> QKV
-    if (!fused) {
-      { ProfScope ps(e, KC_NORM);
-      if ((s = rmsnorm_launch(e->x, L.pre_attn_norm, e->hbuf, nullptr, M, e->D, c.rms_eps, e->stream, e->err))) return s; }
-      e->last_launches++;
-    }
-    GemmPlan& pq = fused ? L.p_qkv_f : L.p_qkv;
-    const bf16* a_in = fused ? e->x : e->hbuf;
-    // RoPE rides in the QKV epilogue unless qk-norm has to run first (heads of 128 through a pass of their own: 522 us for a
-    // two-layer forward of 8 x 1086 rows, 465 us in the epilogue)
-    const bool fuse_rope = c.rotary && !c.qk_norm && !e->use_simt_gemm;
-    if (fuse_rope) {
-      GemmRope gr;
-      gr.angles = e->angles; gr.n_pos = e->S + 1; gr.T = Tt; gr.pos_cap = pos_cap; gr.dh = e->dh;
-      gr.g = e->Hq / e->Hkv; gr.group = gr.g + 2;
-      if (split) { gr.T = hist_len; gr.split_rows = (long long)B * hist_len; }
-      if (pk) gr.pos_rows = pk->pos_rows;
-      gr.kv_rows = off;
-      if ((s = do_gemm(e, pq, a_in, e->qkv, nullptr, M, EPI_ROPE, &gr, fused ? &n_attn_in : nullptr))) return s;
-    } else {
-      if ((s = do_gemm(e, pq, a_in, e->qkv, nullptr, M, EPI_STORE, nullptr, fused ? &n_attn_in : nullptr))) return s;
-    }
-    if (!fuse_rope && (c.rotary || c.qk_norm)) {
-      QkNormRopeArgs qa;
-      qa.qkv = e->qkv; qa.M = M; qa.T = Tt; qa.Hq = e->Hq; qa.Hkv = e->Hkv; qa.dh = e->dh; qa.pos_cap = pos_cap;
-      qa.rotary = c.rotary; qa.qk_norm = c.qk_norm; qa.q_gain = L.q_norm; qa.k_gain = L.k_norm;
-      qa.cos_tab = e->cos_tab; qa.sin_tab = e->sin_tab;
-      if (split) { qa.T = hist_len; qa.split_rows = (long long)B * hist_len; }
-      if (pk) qa.pos_rows = pk->pos_rows;
-      { ProfScope ps(e, KC_ROPE); if ((s = qknorm_rope_launch(qa, e->stream, e->err))) return s; }
-      e->last_launches++;
-    }
+    if ((s = layer_qkv(e, L, B, Tt, pos_cap, hist_len, split, pk, M, off))) return s;
     if ((s = layer_attention(e, B, Tt, hist_len, split, tail ? hist_len : 0, pk))) return s;
     if ((s = layer_update(e, L, off, M - off))) return s;
   }
@@ -1138,7 +1148,7 @@ phx_status phx_rank_forward_device(phx_engine* e, const phx_rank_batch* bd, cons
   if (!params_complete(e, true) || !shards_complete(e)) return PHX_E_STATE;
   cudaSetDevice(e->device);
   const int B = bd->batch;
-  e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = true; e->history_done = false;
+  e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = true; e->history_done = e->history_q_done = false;
   e->cur_pack = e->pack ? (planned ? planned : &e->pack_full) : nullptr;
   if (B == 0) return PHX_OK;
   PHX_CUDA_TRY(cudaEventRecord(e->ev0, e->stream), e->err);
@@ -1268,7 +1278,7 @@ phx_status phx_rank_forward_rows_device(phx_engine* e, const phx_rank_batch* bd,
   if (!params_complete(e, true)) return PHX_E_STATE;
   cudaSetDevice(e->device);
   const int B = bd->batch;
-  e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = true; e->history_done = false;
+  e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = true; e->history_done = e->history_q_done = false;
   e->prefetch_valid = false;
   e->graph_key_valid = false;
   e->cur_pack = e->pack ? &e->pack_full : nullptr;
@@ -1286,7 +1296,7 @@ namespace {
 phx_status forward_hashed_core(phx_engine* e, const HashedIn& in, int B, const phx_rank_out* od) {
   if (!params_complete(e, true) || !shards_complete(e)) return PHX_E_STATE;
   cudaSetDevice(e->device);
-  e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = true; e->history_done = false;
+  e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = true; e->history_done = e->history_q_done = false;
   e->prefetch_valid = false;
   e->graph_key_valid = false;   // plain launches: the graph cache is keyed on id batches
   e->cur_pack = e->pack ? &e->pack_full : nullptr;
@@ -1806,8 +1816,20 @@ phx_status phx_debug_read(phx_engine* e, const char* what, void* host, size_t nb
   else if (w == "hashes" && e->debug_taps) { src = e->hashes; avail = M * 2 * e->cfg.item.num_hashes * 4; }
   else { e->err = "phx_debug_read: unknown tap (tokens / hashes need PHX_DEBUG_TAPS=1): " + w; return PHX_E_ARG; }
   if (nbytes > avail) { e->err = "phx_debug_read: more bytes requested than the tap holds"; return PHX_E_ARG; }
+  if (e->dh == 128 && !e->fp32 && e->n_tail > 0 && e->taps_of_rank && !e->history_q_done && e->last_batch > 0 && nbytes > 0 &&
+      (w == "qkv" || (plain && (w == "hidden" || w == "attn")))) {
+    // the queries of the history rows: the rows stand where the layer found them
+    const int launches = e->last_launches;
+    const size_t profiled = e->prof_used;
+    const phx_engine::PackState* pk = e->split ? nullptr : e->cur_pack;
+    phx_status s = layer_qkv(e, e->layers.back(), e->last_batch, e->T, e->S, e->S, e->split, pk,
+                             pk ? pk->Mh : (long long)e->last_batch * e->S, 0);
+    e->last_launches = launches; e->prof_used = profiled;
+    if (s) return s;
+    e->history_q_done = true;
+  }
   if (plain && !e->history_done && nbytes > 0 && (w == "hidden" || w == "attn")) {
-    // the history rows' share of the last layer: q, k and v are there, the rows stand where the layer found them
+    // the history rows' share of the last layer: q, k and v are there, the rows stand where it found them
     const int launches = e->last_launches;
     const size_t profiled = e->prof_used;
     phx_status s = layer_attention(e, e->last_batch, e->T, e->S, true, 0, nullptr);
