@@ -168,7 +168,7 @@ phx_status gemm_plan_create(GemmPlan* plan, const bf16* A, const bf16* Wt, int64
                             bool narrow_tiles, std::string& err, int pair = -1);
 // pair: 1 = CTA pairs share 256-row tiles (cta_group::2), 0 = one CTA per 128-row tile, -1 = pairs unless the
 // environment says PHX_GEMM=cta1
-// Launch on `stream`.  `R` is the residual (EPI_RESIDUAL) or null.  `err_flag` is a device int the
+// Launch on `stream`.  `R` is the residual (EPI_RESIDUAL) or null.  `err_flag` is an int in device or pinned memory the
 // kernel sets to 1 when a bounded wait ran out.
 phx_status gemm_launch(GemmPlan& plan, const bf16* A, bf16* C, const bf16* R, int64_t M, int epilogue,
                        const GemmRope* rope, const GemmNorm* norm, int* err_flag, int num_sms, cudaStream_t stream,
@@ -317,7 +317,7 @@ struct AttnArgs {
   int B, T, Hq, Hkv, dh, hist_len;
   float sm_scale, cap;
   int cap_method;
-  int* err_flag;         // device int raised by a bounded wait that ran out (tcgen05 path); null = mma.sync path only
+  int* err_flag;         // int in device or pinned memory, raised by a bounded wait that ran out (tcgen05 path); null = mma.sync path only
   // Split token layout (token_row): q / k / v / out / seg rows are the B * hist_len history rows followed by the
   // candidate rows.  q_start > 0: query rows below it are not computed (candidate-only layers).
   int split = 0, q_start = 0;

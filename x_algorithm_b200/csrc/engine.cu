@@ -151,7 +151,7 @@ struct phx_engine {
   bool folded_dirty = true;
   int* hashes = nullptr;
   int* err_flag = nullptr;   // pinned
-  // staging for the host-buffer entry point
+  // staging of the host-buffer entry points: the ids form is read where it lies in in_stage_host, the others are copied to in_stage_dev
   void* in_stage_dev = nullptr;
   void* in_stage_host = nullptr;
   size_t in_stage_bytes = 0;
@@ -882,7 +882,7 @@ phx_status phx_engine_create(const phx_model_config* cfg, int32_t device, phx_en
     CU(cudaMallocHost(&e->in_stage_host, e->in_stage_bytes));
     const size_t rows = B * (size_t)(e->C > 0 ? e->C : 1);
     // one block each side: scores, log-probabilities, continuous values of max_batch requests; a small call lays its own
-    // rows out in front of it, back to back, and fetches them with one copy
+    // rows out in front of the host's, back to back, and the heads kernel writes them there
     const OutLayout ol(rows, e->V, e->NC);
     CU(cudaMalloc(&e->out_stage_dev, ol.bytes));
     CU(cudaMallocHost(&e->out_stage_host, ol.bytes));

@@ -8,7 +8,7 @@
 //   warp 1      MMA issuer: tcgen05.mma M=128 (corpus rows) x N=NQ (queries), 32 bytes of a row per instruction
 //               (kind::f16: 16 bf16, fp32 sums; kind::i8: 32 int8, int32 sums), into one of two TMEM accumulators
 //   (with the bias: warps 18, 19 write the rows' side of it, see bias_x)
-//   warps 2-17  consumers: each warp reads its 32-row lane quadrant and a quarter of the query columns with
+//   warps 2-17  consumers: each warp reads its 32-row lane quadrant and a quarter (ScanCfg::SPLIT: half) of the query columns with
 //               tcgen05.ld and either appends rows whose score reaches the query's threshold to the survivor list
 //               (collect pass) or reduces the 32-row maximum per query (sample pass)
 // An int8 row of 128 columns is the byte image of a bf16 row of 64: tiles, swizzle, descriptors and tensor maps are the
