@@ -82,3 +82,26 @@ def test_merge_of_lists_with_empty_slots():
         np.testing.assert_array_equal(out_i[b].cpu().numpy(), want_i)
         np.testing.assert_array_equal(out_s[b].cpu().numpy(), want_s)
     sh.close()
+
+
+@pytest.mark.parametrize("P,k", [(2, 5), (3, 37), (5, 256)])
+def test_merge_of_lists_that_share_entries(P, k):
+    """An entry that several lists hold is there as often in the result."""
+    import torch
+    from x_algorithm_b200.retrieval import CorpusShard
+    B = 2
+    rng = np.random.default_rng(P)
+    one = -np.sort(-rng.uniform(0.5, 0.9, (B, k)).astype(np.float32), axis=1)
+    sc = np.ascontiguousarray(np.broadcast_to(one, (P, B, k)))
+    ids = np.ascontiguousarray(np.broadcast_to(rng.permutation(B * k).reshape(B, k), (P, B, k))).astype(np.int64)
+    sh = CorpusShard(64, 64, max_queries=B, max_k=k)
+    out_s = torch.full((B, k), 7.0, dtype=torch.float32, device="cuda")
+    out_i = torch.full((B, k), 7, dtype=torch.int64, device="cuda")
+    sh.merge_device(torch.from_numpy(sc).cuda(), torch.from_numpy(ids).cuda(), P, B, k, out_s, out_i)
+    sh.sync()
+    for b in range(B):
+        s, i = sc[:, b].ravel(), ids[:, b].ravel()
+        order = np.lexsort((i, -s))[:k]
+        np.testing.assert_array_equal(out_i[b].cpu().numpy(), i[order])
+        np.testing.assert_array_equal(out_s[b].cpu().numpy(), s[order])
+    sh.close()

@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(SEL_THREADS) select_kernel(const unsigned long
   }
   const unsigned long long* ku = keys + (size_t)u * cap;
   // One histogram of the codes below the largest finds the k-th entry's code.  Grouped by code the keys from there on are all but sorted: a
-  // key's place is its code's first one plus the number of larger keys of the same code.  Every key is fetched once, up to four a thread.
+  // key's place is its code's first one plus the number of larger keys of the same code (and of equal ones in front of it).  Every key is fetched once, up to four a thread.
   // Lists that reach further down or have many keys of one code take the digits and a sort, as every list did (kernel, us: one query, k = 500
   // 16.3 -> 4.9, 256 queries, k = 1000 39.7 -> 12.1).
   constexpr int KEEP = 4, BIN_MAX = 256;
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(SEL_THREADS) select_kernel(const unsigned long
       const unsigned long long v = s_keys[i];
       const int bin = top_bin(top, (uint32_t)(v >> 32)), lo = s_first[bin], hi = lo + s_hist[bin];
       int place = lo;
-      for (int x = lo; x < hi; ++x) place += s_keys[x] > v ? 1 : 0;
+      for (int x = lo; x < hi; ++x) place += s_keys[x] > v || (s_keys[x] == v && x < i) ? 1 : 0;   // (lists to merge may share entries)
       if (place >= k) continue;
       if (out_keys) out_keys[ob + place] = v;
       else {
