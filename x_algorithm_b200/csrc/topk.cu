@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(SEL_THREADS) select_kernel(const unsigned long
   // One histogram of the codes below the largest finds the k-th entry's code.  Grouped by code the keys from there on are all but sorted: a
   // key's place is its code's first one plus the number of larger keys of the same code (and of equal ones in front of it).  Every key is fetched once, up to four a thread.
   // Lists that reach further down or have many keys of one code take the digits and a sort, as every list did (kernel, us: one query, k = 500
-  // 16.3 -> 4.9, 256 queries, k = 1000 39.7 -> 12.1).
+  // 16.3 -> 4.9, 256 queries, k = 1000 39.7 -> 12.1 to 16.4).
   constexpr int KEEP = 4, BIN_MAX = 256;
   unsigned long long mine[KEEP];
   uint32_t top = 0;
