@@ -42,3 +42,26 @@ def test_streaming_edges(monkeypatch, dh, H, Hk, S, C):
     # P and the output are rounded to bf16 (2^-9 each, at most a row's largest |v| in all), scores are fp32 sums of exact products
     assert (got.float() - want).abs().max() <= 2.0 ** -7 * v.float().abs().max()
     assert torch.linalg.norm(got.float() - want) <= 2.0 ** -8 * torch.linalg.norm(want)
+
+
+@pytest.mark.parametrize("dh,H,Hk", [(128, 8, 2), (64, 8, 8)])
+@pytest.mark.parametrize("C", [128, 300, 520])
+def test_no_history_rows_without_a_key_are_zero(monkeypatch, dh, H, Hk, C):
+    """Without a history nothing but the staging itself waits for a tile's queries to land: whole tiles and warps of rows that are padding, or
+    that have no key to attend to, read zero, never what their queries' copy leaves behind."""
+    import torch
+    from x_algorithm_b200.engine import dispatch_counts, ranker_attention
+    monkeypatch.setenv("PHX_ATTN", "tcgen05")
+    B = 64
+    g = torch.Generator(device="cuda").manual_seed(C + dh)
+    q, k, v = (torch.randn(B, C, h, dh, device="cuda", generator=g).to(torch.bfloat16) for h in (H, Hk, Hk))
+    seg = torch.zeros((B, C), dtype=torch.int32, device="cuda")            # requests 0, 4, ...: padding alone
+    seg[1::4] = 1                                                          # no key, and not their own
+    seg[2::4, : C // 3] = -1                                               # then padding, from within a warp's rows on
+    seg[3::4, 96:97] = -1                                                  # one row of one warp
+    before = dispatch_counts()["attn.tcgen05"]
+    for _ in range(5):
+        got, _ = ranker_attention(q, k, v, seg, 0, 1.0 / math.sqrt(dh))
+        own = v.repeat_interleave(H // Hk, 2) * (seg == -1)[:, :, None, None]      # a row that sees itself alone is its own v
+        assert torch.equal(got, own)
+    assert dispatch_counts()["attn.tcgen05"] == before + 5

@@ -416,6 +416,8 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
     if (n_blocks > 0) {
       mbar_wait(o_done, (uint32_t)((n_blocks - 1) & 1), verr);
       tc_fence_after();
+    } else {
+      mbar_wait(q_full, 0, verr);   // no product has waited for Q: the output must not be staged under its copy
     }
     if (segq == -1) mbar_wait(v_full(own & 1), (uint32_t)((own >> 1) & 1), verr);
     __syncwarp();
@@ -444,7 +446,7 @@ ranker_attention_tc_kernel(const __grid_constant__ TcMaps maps, AttnTcArgs a) {
         uint4 w;
         w.x = pack_bf2(x[0] * inv, x[1] * inv); w.y = pack_bf2(x[2] * inv, x[3] * inv);
         w.z = pack_bf2(x[4] * inv, x[5] * inv); w.w = pack_bf2(x[6] * inv, x[7] * inv);
-        st_shared_16(sQ + (c >> 1) * SLAB + r * 128 + at, w);   // Q is no longer needed: its products are done, and the row's own thread has read it
+        st_shared_16(sQ + (c >> 1) * SLAB + r * 128 + at, w);   // Q is no longer needed: it has landed, its products are done, and the row's own thread has read it
       }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
