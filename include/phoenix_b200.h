@@ -319,14 +319,18 @@ phx_status phx_rank_prefetch_device(phx_engine* e, const phx_rank_batch* batch_d
 phx_status phx_sync(phx_engine* e);
 /* Failure detection on the device.  Every wait inside the tcgen05 kernels (on an mbarrier that a TMA copy, an MMA
  * commit or another warp role signals) is bounded: when the limit passes, the waiting thread raises the engine's error
- * flag, every role drains, the kernel returns, and the next blocking call (phx_rank_forward, phx_rank_collect, phx_sync)
- * reports PHX_E_TIMEOUT once and clears the flag; the context stays usable.  phx_set_wait_limit_us sets the limit
+ * flag, every role drains and the kernel returns; the context stays usable.  Kernels behind it give their own long waits
+ * up until the flag is cleared, so every call whose kernels ran from there on reports PHX_E_TIMEOUT, once: a host-buffer call
+ * (phx_rank_forward and its other forms) when it returns, a pipelined request when it is collected - its own forward's outcome,
+ * whatever the other slot's was - and all device-buffer calls since the last phx_sync together at the next one.  The first of
+ * them to report clears the flag, once the engine's stream is idle.  phx_set_wait_limit_us sets the limit
  * (microseconds; 0 = the default of 2 s; synchronises the engine's stream).  phx_wait_selftest launches a one-thread
  * kernel that waits on a barrier nothing signals and returns what phx_sync returns after it: PHX_E_TIMEOUT after
- * about one limit when the mechanism works.  The reference leaves hangs to its serving shell (per-request deadlines,
+ * about one limit when the mechanism works; phx_wait_selftest_async returns behind the launch, like a device-buffer call.  The reference leaves hangs to its serving shell (per-request deadlines,
  * xai-recsys-engine/src/request_queue.rs:10-27); a kernel of its own that waits for ever holds the GPU. */
 phx_status phx_set_wait_limit_us(phx_engine* e, uint32_t microseconds);
 phx_status phx_wait_selftest(phx_engine* e);
+phx_status phx_wait_selftest_async(phx_engine* e);
 /* Which kernel variants the library's launches took, counted over the life of the process: out[i] for i < n receives the
  * count of variant i, the return value is the number of variants; phx_dispatch_name(i) names them ("attn.strip",
  * "attn.stream", "attn.tcgen05", "attn.resident", "gemm.pair256", "gemm.pair128", "gemm.cta256", "gemm.cta128",

@@ -129,6 +129,7 @@ SIGNATURES = {
     "phx_sync": (C.c_int32, [_P]),
     "phx_set_wait_limit_us": (C.c_int32, [_P, C.c_uint32]),
     "phx_wait_selftest": (C.c_int32, [_P]),
+    "phx_wait_selftest_async": (C.c_int32, [_P]),
     "phx_dispatch_counts": (C.c_int32, [_P, C.c_int32]),
     "phx_dispatch_name": (C.c_char_p, [C.c_int32]),
     "phx_last_device_ms": (C.c_int32, [_P, C.POINTER(C.c_float)]),

@@ -15,6 +15,7 @@
 
 #include "comm.cuh"
 #include "common.cuh"
+#include "launch_attr.cuh"
 
 namespace phx {
 
@@ -151,6 +152,8 @@ struct phx_engine {
   bool folded_dirty = true;
   int* hashes = nullptr;
   int* err_flag = nullptr;   // pinned
+  bool device_calls = false;    // device-buffer calls since the last phx_sync, which answers for them
+  bool device_failed = false;   // ... and a flag that another call found, and cleared, behind one of them
   // staging of the host-buffer entry points: the ids form is read where it lies in in_stage_host, the others are copied to in_stage_dev
   void* in_stage_dev = nullptr;
   void* in_stage_host = nullptr;
@@ -173,6 +176,7 @@ struct phx_engine {
     float* lp_host = nullptr; float* cont_host = nullptr; double* score_host = nullptr;
     cudaEvent_t in_ready = nullptr, fwd_done = nullptr, out_done = nullptr;
     cudaEvent_t chunk[4] = {nullptr, nullptr, nullptr, nullptr};
+    int* raised = nullptr;          // pinned: the error flag as the request's own forward left it (publish_flag_kernel)
     bool busy = false;
     int batch = 0;
     PackState pack;                 // packed rows of the request in this slot (offset arrays inside the slot's block)
@@ -669,15 +673,34 @@ phx_status build_tokens(phx_engine* e, const phx_rank_batch* bd, int B, int Cc, 
   return build_tokens_launch(ta, e->stream, e->err);
 }
 
-// the stream (or the event behind the call in question) has been waited for
-phx_status check_err_flag(phx_engine* e) {
+// The flag is one word for all of an engine's kernels, and stays up for those behind the one that raised it: their waits may give up too.
+// So it is cleared only when the stream has been waited for, and whoever has not been answered by then keeps word of it: a request of
+// the two-deep pipeline in its own slot, device-buffer calls in device_failed.
+bool take_err_flag(phx_engine* e) {
   volatile int* const flag = e->err_flag;
-  if (*flag != 0) {
-    *flag = 0;
-    e->err = "a bounded device-side wait ran out (GEMM / attention pipeline)";
-    return PHX_E_TIMEOUT;
-  }
-  return PHX_OK;
+  if (*flag == 0) return false;
+  *flag = 0;
+  if (e->device_calls) e->device_failed = true;
+  return true;
+}
+phx_status wait_ran_out(phx_engine* e) {
+  e->err = "a bounded device-side wait ran out (GEMM / attention pipeline)";
+  return PHX_E_TIMEOUT;
+}
+// the end of a host-buffer call; the stream has been waited for
+phx_status check_err_flag(phx_engine* e) { return take_err_flag(e) ? wait_ran_out(e) : PHX_OK; }
+// A host-buffer call goes through the device-buffer form, but answers for it itself
+template <typename F>
+phx_status own_forward(phx_engine* e, F call) {
+  const bool others = e->device_calls;
+  const phx_status s = call();
+  e->device_calls = others;
+  return s;
+}
+// the end of a pipelined request's forward: the flag as it is now, in stream order
+__global__ void publish_flag_kernel(const volatile int* flag, volatile int* raised) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  *raised = *flag;
 }
 
 }  // namespace
@@ -912,6 +935,7 @@ void phx_engine_destroy(phx_engine* e) {
     if (sl.lp_host) cudaFreeHost(sl.lp_host);
     if (sl.cont_host) cudaFreeHost(sl.cont_host);
     if (sl.score_host) cudaFreeHost(sl.score_host);
+    if (sl.raised) cudaFreeHost(sl.raised);
     if (sl.in_ready) cudaEventDestroy(sl.in_ready);
     if (sl.fwd_done) cudaEventDestroy(sl.fwd_done);
     if (sl.out_done) cudaEventDestroy(sl.out_done);
@@ -1149,6 +1173,7 @@ phx_status phx_rank_forward_device(phx_engine* e, const phx_rank_batch* bd, cons
   cudaSetDevice(e->device);
   const int B = bd->batch;
   e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = true; e->history_done = e->history_q_done = false;
+  e->device_calls = true;
   e->cur_pack = e->pack ? (planned ? planned : &e->pack_full) : nullptr;
   if (B == 0) return PHX_OK;
   PHX_CUDA_TRY(cudaEventRecord(e->ev0, e->stream), e->err);
@@ -1279,6 +1304,7 @@ phx_status phx_rank_forward_rows_device(phx_engine* e, const phx_rank_batch* bd,
   cudaSetDevice(e->device);
   const int B = bd->batch;
   e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = true; e->history_done = e->history_q_done = false;
+  e->device_calls = true;
   e->prefetch_valid = false;
   e->graph_key_valid = false;
   e->cur_pack = e->pack ? &e->pack_full : nullptr;
@@ -1297,6 +1323,7 @@ phx_status forward_hashed_core(phx_engine* e, const HashedIn& in, int B, const p
   if (!params_complete(e, true) || !shards_complete(e)) return PHX_E_STATE;
   cudaSetDevice(e->device);
   e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = true; e->history_done = e->history_q_done = false;
+  e->device_calls = true;
   e->prefetch_valid = false;
   e->graph_key_valid = false;   // plain launches: the graph cache is keyed on id batches
   e->cur_pack = e->pack ? &e->pack_full : nullptr;
@@ -1390,7 +1417,7 @@ phx_status phx_rank_forward_hashed(phx_engine* e, const phx_rank_batch_hashed* b
   bd.hist_surfaces = put(bh->hist_surfaces, B * S * 4);
   PHX_CUDA_TRY(cudaMemcpyAsync(dp, hp, off, cudaMemcpyHostToDevice, e->stream), e->err);
   phx_rank_out od; od.log_probs = e->lp_dev; od.continuous = e->cont_dev; od.scores = e->score_dev;
-  phx_status s = phx_rank_forward_hashed_device(e, &bd, &od);
+  phx_status s = own_forward(e, [&] { return phx_rank_forward_hashed_device(e, &bd, &od); });
   if (s) return s;
   return fetch_outputs(e, B, oh);
 }
@@ -1439,7 +1466,7 @@ phx_status phx_rank_forward_prep(phx_engine* e, const phx_rank_batch_prep* bh, c
   if (!fits) { e->err = "phx_rank_forward_prep: staging block too small"; return PHX_E_CAPACITY; }
   PHX_CUDA_TRY(cudaMemcpyAsync(dp, hp, off, cudaMemcpyHostToDevice, e->stream), e->err);
   phx_rank_out od; od.log_probs = e->lp_dev; od.continuous = e->cont_dev; od.scores = e->score_dev;
-  phx_status s = phx_rank_forward_prep_device(e, &bd, &od);
+  phx_status s = own_forward(e, [&] { return phx_rank_forward_prep_device(e, &bd, &od); });
   if (s) return s;
   return fetch_outputs(e, B, oh);
 }
@@ -1527,7 +1554,7 @@ phx_status phx_rank_forward(phx_engine* e, const phx_rank_batch* bh, const phx_r
   const int V = e->V, NC = e->NC;
   const bool want_scores = oh->scores && e->has_blend;
   phx_rank_out od; od.log_probs = lp_dev; od.continuous = cont_dev; od.scores = score_dev;
-  phx_status s = phx_rank_forward_device(e, &bd, &od);
+  phx_status s = own_forward(e, [&] { return phx_rank_forward_device(e, &bd, &od); });
   if (s) return s;
   // larger results come back in four row chunks: while the host copies chunk i out of the pinned staging block, chunk i+1
   // is still on the bus
@@ -1592,6 +1619,7 @@ phx_status slots_init(phx_engine* e) {
     PHX_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&sl.lp_host), rows * (e->V > 0 ? e->V : 1) * 4), e->err);
     PHX_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&sl.cont_host), rows * (e->NC > 0 ? e->NC : 1) * 4), e->err);
     PHX_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&sl.score_host), rows * 8), e->err);
+    PHX_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&sl.raised), sizeof(int)), e->err);
     PHX_CUDA_TRY(cudaEventCreateWithFlags(&sl.in_ready, cudaEventDisableTiming), e->err);
     PHX_CUDA_TRY(cudaEventCreateWithFlags(&sl.fwd_done, cudaEventDisableTiming), e->err);
     PHX_CUDA_TRY(cudaEventCreateWithFlags(&sl.out_done, cudaEventDisableTiming), e->err);
@@ -1644,7 +1672,8 @@ phx_status phx_rank_submit(phx_engine* e, const phx_rank_batch* bh, int32_t slot
   PHX_CUDA_TRY(cudaStreamWaitEvent(e->stream, sl.in_ready, 0), e->err);
   PHX_CUDA_TRY(cudaStreamWaitEvent(e->stream, sl.out_done, 0), e->err);
   phx_rank_out od; od.log_probs = sl.lp_dev; od.continuous = sl.cont_dev; od.scores = sl.score_dev;
-  if ((s = phx_rank_forward_device(e, &bd, &od))) return s;
+  if ((s = own_forward(e, [&] { return phx_rank_forward_device(e, &bd, &od); }))) return s;
+  PHX_CUDA_TRY(launch_programmatic(publish_flag_kernel, dim3(1), dim3(1), 0, e->stream, (const volatile int*)e->err_flag, (volatile int*)sl.raised), e->err);
   PHX_CUDA_TRY(cudaEventRecord(sl.fwd_done, e->stream), e->err);
   // results: back on the copy stream, in row chunks
   PHX_CUDA_TRY(cudaStreamWaitEvent(e->copy_stream, sl.fwd_done, 0), e->err);
@@ -1679,14 +1708,20 @@ phx_status phx_rank_collect(phx_engine* e, int32_t slot, const phx_rank_out* oh)
     if (oh->scores && e->has_blend) memcpy(oh->scores + r0, sl.score_host + r0, (r1 - r0) * 8);
   }
   sl.busy = false;
-  return check_err_flag(e);
+  if (*static_cast<volatile int*>(sl.raised) == 0) return PHX_OK;
+  // what was enqueued behind this request ran with the flag up: it ends, and its own word says so, before the flag is cleared
+  PHX_CUDA_TRY(cudaStreamSynchronize(e->stream), e->err);
+  take_err_flag(e);
+  return wait_ran_out(e);
 }
 
 phx_status phx_sync(phx_engine* e) {
   if (!e) return PHX_E_ARG;
   cudaSetDevice(e->device);
   PHX_CUDA_TRY(cudaStreamSynchronize(e->stream), e->err);
-  return check_err_flag(e);
+  const bool raised = take_err_flag(e) || e->device_failed;
+  e->device_calls = e->device_failed = false;
+  return raised ? wait_ran_out(e) : PHX_OK;
 }
 
 phx_status phx_set_wait_limit_us(phx_engine* e, uint32_t microseconds) {
@@ -1697,12 +1732,16 @@ phx_status phx_set_wait_limit_us(phx_engine* e, uint32_t microseconds) {
   return PHX_OK;
 }
 
-phx_status phx_wait_selftest(phx_engine* e) {
+phx_status phx_wait_selftest_async(phx_engine* e) {
   if (!e) return PHX_E_ARG;
   cudaSetDevice(e->device);
-  phx_status s = wait_selftest_launch(e->err_flag, e->stream, e->err);
-  if (s) return s;
-  return phx_sync(e);
+  e->device_calls = true;
+  return wait_selftest_launch(e->err_flag, e->stream, e->err);
+}
+
+phx_status phx_wait_selftest(phx_engine* e) {
+  const phx_status s = phx_wait_selftest_async(e);
+  return s ? s : phx_sync(e);
 }
 
 int32_t phx_dispatch_counts(int64_t* out, int32_t n) {
@@ -1885,6 +1924,7 @@ phx_status phx_user_tower_device(phx_engine* e, const phx_rank_batch* bd, float*
   cudaSetDevice(e->device);
   const int B = bd->batch;
   e->last_batch = B; e->last_launches = 0; e->prof_used = 0; e->taps_of_rank = false;
+  e->device_calls = true;
   if (B == 0) return PHX_OK;
   PHX_CUDA_TRY(cudaEventRecord(e->ev0, e->stream), e->err);
   phx_status s;

@@ -289,6 +289,10 @@ class PhoenixEngine:
         """Let one device-side wait run out: raises PhoenixError(PHX_E_TIMEOUT) when the mechanism works."""
         self._check(lib.phx_wait_selftest(self._h))
 
+    def wait_selftest_async(self):
+        """The same without waiting for it: the next sync() reports it."""
+        self._check(lib.phx_wait_selftest_async(self._h))
+
     def last_device_ms(self) -> float:
         ms = C.c_float()
         self._check(lib.phx_last_device_ms(self._h, C.byref(ms)))
