@@ -1,4 +1,4 @@
-"""The streaming attention kernel at the edges of its key blocks and query tiles, and with every kind of row in every place, against a
+"""The streaming attention kernels at the edges of their key blocks and query tiles, and with every kind of row in every place, against a
 plain fp32 reference: candidates whose tile is half padding, rows that attend to themselves inside the history, no history at all."""
 import math
 
@@ -65,3 +65,38 @@ def test_no_history_rows_without_a_key_are_zero(monkeypatch, dh, H, Hk, C):
         own = v.repeat_interleave(H // Hk, 2) * (seg == -1)[:, :, None, None]      # a row that sees itself alone is its own v
         assert torch.equal(got, own)
     assert dispatch_counts()["attn.tcgen05"] == before + 5
+
+
+# tiles of 64 / 128 rows on 148 SMs: heads of 128 have one CTA an SM at either height, heads of 64 two
+@pytest.mark.parametrize("dh,H,Hk,B,S,C,low", [
+    (128, 16, 4, 1, 512, 64, True),      # 144 / 80: one round of either
+    (128, 16, 4, 1, 512, 65, False),     # 160 / 80: two rounds against one
+    (128, 16, 4, 1, 1022, 64, False),    # 272 / 144
+    (128, 8, 2, 5, 300, 148, True),      # 280 / 160: two rounds of either
+    (128, 8, 2, 5, 300, 213, False),     # 360 / 200: more than two for every SM
+    (64, 8, 8, 1, 257, 2111, True),      # 296 / 152: two low tiles an SM
+    (64, 8, 8, 1, 257, 2112, False),     # 304 / 152
+    (32, 4, 4, 2, 70, 2223, True)])      # 288 / 144
+def test_rows_of_a_tile_follow_the_rounds(monkeypatch, dh, H, Hk, B, S, C, low):
+    """The mma.sync kernel's tile height, on both sides of the rule that picks it."""
+    import torch
+    from x_algorithm_b200.engine import dispatch_counts, ranker_attention
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the tile counts are for 148 SMs")
+    monkeypatch.setenv("PHX_ATTN", "mma")
+    T = S + C
+    g = torch.Generator(device="cuda").manual_seed(T)
+    q, k, v = (torch.randn(B, T, h, dh, device="cuda", generator=g).to(torch.bfloat16) for h in (H, Hk, Hk))
+    seg = torch.ones((B, T), dtype=torch.int32, device="cuda")
+    seg[:, S:] = -1
+    seg[:, S - 5: S] = 0
+    seg[0, S + C // 2:] = 0
+    before = dispatch_counts()
+    got, _ = ranker_attention(q, k, v, seg, S, 1.0 / math.sqrt(dh))
+    after = dispatch_counts()
+    assert after["attn.stream"] == before["attn.stream"] + 1
+    assert after["form.attn_low"] == before["form.attn_low"] + (1 if low else 0)
+    want = reference(q, k, v, seg, S, 1.0 / math.sqrt(dh))
+    assert bool((got[seg == 0] == 0).all())
+    assert (got.float() - want).abs().max() <= 2.0 ** -7 * v.float().abs().max()          # as above
+    assert torch.linalg.norm(got.float() - want) <= 2.0 ** -8 * torch.linalg.norm(want)

@@ -346,22 +346,32 @@ cudaError_t launch_overlapped(Kern kern, dim3 grid, int threads, size_t smem, cu
   return cudaLaunchKernelEx(&lc, kern, a);
 }
 
+constexpr int stream_smem(int dh, int rows) { return (3 * rows + 4 * KB) * (dh + 8) * 2 + (2 * KB + 4) * (int)sizeof(int); }
 template <int DH, bool CAP, int WARPS>
 phx_status launch_rows(const AttnArgs& a, cudaStream_t stream, std::string& err) {
-  constexpr int LD = DH + 8, ROWS = 16 * WARPS;
-  const size_t smem = (size_t)(3 * ROWS + 4 * KB) * LD * 2 + (2 * KB + 4) * sizeof(int);
+  constexpr int ROWS = 16 * WARPS;
+  const size_t smem = stream_smem(DH, ROWS);
   static SmemLimit limit;
   PHX_CUDA_TRY(limit.raise(ranker_attention_kernel<DH, CAP, WARPS>, (int)smem), err);
   dim3 grid((a.T + ROWS - 1) / ROWS, a.Hq, a.B);
   PHX_CUDA_TRY(launch_overlapped(ranker_attention_kernel<DH, CAP, WARPS>, grid, 32 * WARPS, smem, stream, a), err);
   return PHX_OK;
 }
-// Tiles of 64 rows while two of them fit every SM: a small call's time is one tile's, and eight warps of a tile share the tensor cores
-// that four of it would have to themselves (eight layers, device us: one request of 640 rows 238 -> 231, of 172 rows 203 -> 193, 16 of 118 322 -> 313).
+// Tiles of 64 rows, up to two for every SM, where they take no more rounds than tiles of 128: a small call's time is its rounds of tiles, and
+// eight warps of a tile share the tensor cores that four of it would have to themselves (heads of 64, eight layers, device us: one request of 640 rows
+// 238 -> 231, of 172 rows 203 -> 193, 16 of 118 322 -> 313).  Heads of 128 leave room for one CTA an SM at either height, so that from 149 low
+// tiles on the tall ones win until they need a second round too (16 heads, one launch, us, 128 rows / 64): 80 / 144 tiles 27.2 / 23.1,
+// 80 / 160 29.2 / 43.5, 144 / 272 45.9 / 70.2, 144 / 288 13.4 / 19.1, 160 / 288 47.6 / 41.5; two-layer packed forwards, 80 / 144 149.1 / 142.8,
+// 96 / 176 160.1 / 171.7, 144 / 272 203.4 / 220.7, 160 / 288 197.8 / 189.2.
 template <int DH, bool CAP>
 phx_status launch_dh(const AttnArgs& a, cudaStream_t stream, std::string& err) {
-  const long long low = (long long)((a.T + 63) / 64) * a.Hq * a.B;
-  return low <= 2 * 148 ? launch_rows<DH, CAP, 4>(a, stream, err) : launch_rows<DH, CAP, ATT_WARPS>(a, stream, err);
+  constexpr int SM_SMEM = 228 * 1024;    // an SM's, 1 KB of it taken by each CTA
+  constexpr int FIT_LOW = 2 * (stream_smem(DH, 64) + 1024) <= SM_SMEM ? 2 : 1, FIT_HIGH = 2 * (stream_smem(DH, QROWS) + 1024) <= SM_SMEM ? 2 : 1;
+  const long long sms = device_sms(), low = (long long)((a.T + 63) / 64) * a.Hq * a.B, high = (long long)((a.T + QROWS - 1) / QROWS) * a.Hq * a.B;
+  auto rounds = [&](long long tiles, int fit) { return (tiles + fit * sms - 1) / (fit * sms); };
+  if (low > 2 * sms || rounds(low, FIT_LOW) > rounds(high, FIT_HIGH)) return launch_rows<DH, CAP, ATT_WARPS>(a, stream, err);
+  dispatch_note(DK_FORM_ATTN_LOW);
+  return launch_rows<DH, CAP, 4>(a, stream, err);
 }
 
 
@@ -676,7 +686,7 @@ phx_status launch_strip(const AttnArgs& a, cudaStream_t stream, std::string& err
   // Packed requests are of uneven lengths: up to eight CTAs an SM in all share them out, else the kernel ends with the longest ones alone.
   // Two layers of a batch with 1 .. 128 history and 1 .. 512 candidate rows, 8 heads, us, a CTA an item / two / three / five: 24 requests
   // 58 / 50 / 50 / 42, 48: 81 / 70 / 66 / 66, 200: 204 / 218 / 232 / 243; 100 of up to 64 + 100 rows 46 / 50 / 52 / 58.
-  const long long items = (long long)a.Hq * a.B, tiles = (a.T + QROWS - 1) / QROWS, room = 8 * 148 / items;
+  const long long items = (long long)a.Hq * a.B, tiles = (a.T + QROWS - 1) / QROWS, room = 8LL * device_sms() / (items > 0 ? items : 1);
   const int parts = (int)(!a.pack.hist_off || room < 1 ? 1 : room < tiles ? room : tiles);
   dim3 grid(a.Hq, a.B, parts);
   PHX_CUDA_TRY(launch_overlapped(ranker_attention_strip_kernel<CAP>, grid, ATT_THREADS, STRIP_SMEM, stream, a), err);

@@ -47,7 +47,9 @@ enum DispatchKind {
   DK_GEMM_SMALL = 13,    // tcgen05 GEMM, one tile per CTA (few tiles)
   DK_GATHER = 14,        // stand-alone gather-sum, a lane group per id
   DK_GATHER_BULK = 15,   // ... many ids per warp
-  DK_COUNT = 16
+  // forms of a kernel, counted beside it
+  DK_FORM_ATTN_LOW = 16,   // streaming mma.sync kernel, tiles of 64 rows
+  DK_COUNT = 17
 };
 void dispatch_note(int kind);
 

@@ -48,6 +48,18 @@ cudaError_t launch_programmatic(void (*kern)(P...), dim3 grid, dim3 block, size_
   return cudaLaunchKernelEx(&lc, kern, static_cast<P>(args)...);
 }
 
+// SMs of the current device
+inline int device_sms() {
+  static std::atomic<int> known[LAUNCH_MAX_DEVICES] = {};
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  const bool kept = dev >= 0 && dev < LAUNCH_MAX_DEVICES;
+  if (kept && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+  if (kept) known[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 // A kernel's raised dynamic shared-memory limit: one static object per kernel and limit.
 class SmemLimit {
  public:
