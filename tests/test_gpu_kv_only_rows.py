@@ -15,13 +15,18 @@ pytestmark = pytest.mark.gpu
 def test_unread_query_tiles_change_nothing(monkeypatch, hq, hkv, B, S, C, tail, pack):
     kw = dict(max_batch=B, emb_size=256, num_layers=2, num_q_heads=hq, num_kv_heads=hkv, key_size=128, history_len=S, num_candidates=C,
               num_candidate_only_layers=tail, engine_kw=dict(pack_ragged=pack))
+    from x_algorithm_b200.engine import dispatch_counts
     out = []
     for mode in (None, "cta1"):                       # the single-CTA kernel works on every tile
         if mode:
             monkeypatch.setenv("PHX_GEMM", mode)
         ocfg, w, rows_fn, eng = make_pair(**kw)
+        before = dispatch_counts()["form.gemm_kv_only"]
         for seed in (8, 9):                           # the second call meets the buffers of the first
             got = eng.rank(to_inputs(po.make_batch(ocfg, B, seed=seed, ragged=True)))
+        # a key head's own query head (4, 4) is half a column tile: nothing to leave out
+        left_out = 0 if mode or hq == hkv else 2 * max(tail, 1)
+        assert dispatch_counts()["form.gemm_kv_only"] == before + left_out
         out.append(got)
         eng.close()
     assert np.isfinite(out[0].log_probs).all()

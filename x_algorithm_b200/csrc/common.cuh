@@ -49,7 +49,10 @@ enum DispatchKind {
   DK_GATHER_BULK = 15,   // ... many ids per warp
   // forms of a kernel, counted beside it
   DK_FORM_ATTN_LOW = 16,   // streaming mma.sync kernel, tiles of 64 rows
-  DK_COUNT = 17
+  DK_FORM_GEMM_LOW = 17,    // one tile per CTA: tiles of 64 rows
+  DK_FORM_GEMM_DEEP = 18,   // ... of 128 rows with the deep ring
+  DK_FORM_GEMM_KV = 19,     // QKV projection without the query tiles that nobody reads
+  DK_COUNT = 20
 };
 void dispatch_note(int kind);
 

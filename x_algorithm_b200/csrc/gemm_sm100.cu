@@ -855,10 +855,14 @@ bool low_tiles(int64_t M, int N, int K, int num_sms) { return K >= 512 && ((M + 
 template <int BN, int EPI>
 phx_status launch_small_t(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C, const bf16* R, const GemmRope& rope,
                           const GemmNorm& norm, int64_t M, int num_sms, int* err_flag, cudaStream_t stream, std::string& err) {
-  if (BN == 64 && low_tiles(M, p.N, p.K, num_sms)) return launch_small_d<64, 64, EPI, true>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err);
+  if (BN == 64 && low_tiles(M, p.N, p.K, num_sms)) {
+    dispatch_note(DK_FORM_GEMM_LOW);
+    return launch_small_d<64, 64, EPI, true>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err);
+  }
   const long long tiles = ((M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
-  return deep_ring(p.K, EPI, tiles, num_sms) ? launch_small_d<BM, BN, EPI, true>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err)
-                                             : launch_small_d<BM, BN, EPI, false>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err);
+  if (!deep_ring(p.K, EPI, tiles, num_sms)) return launch_small_d<BM, BN, EPI, false>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err);
+  dispatch_note(DK_FORM_GEMM_DEEP);
+  return launch_small_d<BM, BN, EPI, true>(p, map_b64, C, R, rope, norm, M, err_flag, stream, err);
 }
 template <int BN>
 phx_status launch_small(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C, const bf16* R, int epilogue, const GemmRope& rp,
@@ -1004,6 +1008,7 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
       }
     }
     dispatch_note(p.pair ? DK_GEMM_PAIR256 : DK_GEMM_CTA256);
+    if (rp.kv_m_tiles > 0) dispatch_note(DK_FORM_GEMM_KV);
     return p.pair ? launch_e<256, true>(p, epilogue, rp, nm, M, err_flag, num_sms, stream, err)
                   : launch_e<256, false>(p, epilogue, rp, nm, M, err_flag, num_sms, stream, err);
   }
