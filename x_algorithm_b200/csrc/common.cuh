@@ -99,10 +99,6 @@ struct GemmRope {
   // split_rows = 0: plain layout.
   long long row_offset = 0, split_rows = 0;
   const int* pos_rows = nullptr;   // packed rows: position of every token row (overrides the rule above)
-  // The q columns of the first kv_rows rows are read by nobody (history rows of a candidate-only layer): tiles that hold nothing else
-  // may be left out.  Of every kv_per column tiles the first kv_skip, in the first kv_m_tiles row tiles (set by gemm_launch).
-  long long kv_rows = 0;
-  int kv_m_tiles = 0, kv_per = 1, kv_skip = 0;
 };
 
 // Token rows of a [B, S + C] batch.  Plain layout: row = b * T + t.  Split layout (engines with candidate-only tail
@@ -174,10 +170,11 @@ phx_status gemm_plan_create(GemmPlan* plan, const bf16* A, const bf16* Wt, int64
 // pair: 1 = CTA pairs share 256-row tiles (cta_group::2), 0 = one CTA per 128-row tile, -1 = pairs unless the
 // environment says PHX_GEMM=cta1
 // Launch on `stream`.  `R` is the residual (EPI_RESIDUAL) or null.  `err_flag` is an int in device or pinned memory the
-// kernel sets to 1 when a bounded wait ran out.
+// kernel sets to 1 when a bounded wait ran out.  kv_rows: the q columns of the first so many rows are read by nobody (history
+// rows of a candidate-only layer): tiles that hold nothing else may be left out.
 phx_status gemm_launch(GemmPlan& plan, const bf16* A, bf16* C, const bf16* R, int64_t M, int epilogue,
                        const GemmRope* rope, const GemmNorm* norm, int* err_flag, int num_sms, cudaStream_t stream,
-                       std::string& err);
+                       std::string& err, int64_t kv_rows = 0);
 // Plain SIMT GEMM with the same epilogues (debug / cross-check path, selected by PHX_GEMM=simt).
 phx_status gemm_simt_launch(const bf16* A, const bf16* Wt, bf16* C, const bf16* R, int64_t M, int N, int K,
                             int epilogue, cudaStream_t stream, std::string& err);

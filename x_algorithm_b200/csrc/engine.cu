@@ -375,11 +375,11 @@ phx_status upload_bf16(phx_engine* e, bf16** dst, const float* host, int64_t row
 }
 
 phx_status do_gemm(phx_engine* e, GemmPlan& p, const bf16* A, bf16* Cc, const bf16* R, int64_t M, int epi,
-                   const GemmRope* rope = nullptr, const GemmNorm* norm = nullptr) {
+                   const GemmRope* rope = nullptr, const GemmNorm* norm = nullptr, int64_t kv_rows = 0) {
   ProfScope ps(e, KC_GEMM | ((epi + 1) << 8));   // sub-class = epilogue, for the optional per-GEMM breakdown
   e->last_launches++;
   if (e->use_simt_gemm) return gemm_simt_launch(A, p.Wt, Cc, R, M, p.N, p.K, epi, e->stream, e->err);
-  return gemm_launch(p, A, Cc, R, M, epi, rope, norm, e->err_flag, e->num_sms, e->stream, e->err);
+  return gemm_launch(p, A, Cc, R, M, epi, rope, norm, e->err_flag, e->num_sms, e->stream, e->err, kv_rows);
 }
 
 // fold the norm gains into the weights of the GEMMs that consume the normed rows (after any parameter reload)
@@ -558,8 +558,7 @@ phx_status layer_qkv(phx_engine* e, Layer& L, int B, int Tt, int pos_cap, int hi
     gr.g = e->Hq / e->Hkv; gr.group = gr.g + 2;
     if (split) { gr.T = hist_len; gr.split_rows = (long long)B * hist_len; }
     if (pk) gr.pos_rows = pk->pos_rows;
-    gr.kv_rows = kv_rows;
-    if ((s = do_gemm(e, pq, a_in, e->qkv, nullptr, M, EPI_ROPE, &gr, fused ? &n_attn_in : nullptr))) return s;
+    if ((s = do_gemm(e, pq, a_in, e->qkv, nullptr, M, EPI_ROPE, &gr, fused ? &n_attn_in : nullptr, kv_rows))) return s;
   } else {
     if ((s = do_gemm(e, pq, a_in, e->qkv, nullptr, M, EPI_STORE, nullptr, fused ? &n_attn_in : nullptr))) return s;
   }

@@ -121,12 +121,19 @@ __device__ __forceinline__ int rope_pos(const GemmRope& rope, long long row, boo
   return t < rope.pos_cap ? t : rope.pos_cap;
 }
 
+// Column tiles of a QKV projection that nobody reads: of every `per` the first `skip`, in the first `m_tiles` row tiles.  Not part of GemmRope, which
+// the kernels for few tiles take as well: with 24 bytes more in it (416 bytes of parameters in place of 392) each of their launches took
+// 0.35 us longer on the host, the small tower's 22-launch forward 64 us in place of 58 (and 97.6 us on the device in place of 95.6).
+struct GemmLeftOut { int m_tiles = 0, per = 1, skip = 0; };
+static_assert(sizeof(GemmRope) <= 56 && sizeof(GemmNorm) <= 32, "parameters of gemm_small_kernel: measure the host time of a small call");
+__host__ __device__ constexpr bool leaves_out(int bn, int epi, bool pair) { return epi == EPI_ROPE128 && pair && bn == 256; }
+
 template <int BN, int EPI, bool PAIR, int NG>
 __global__ void __launch_bounds__(gemm_threads(NG), 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_r,
                     GemmRope rope, GemmNorm norm, long long M, int N, int K, int* err_flag,
-                    unsigned long long* counters) {
+                    unsigned long long* counters, GemmLeftOut out) {
   // C and R may be the same buffer (in-place residual update): a slab is fetched before it is written back,
   // and no other CTA touches the tile.
   using cfg = Cfg<BN, PAIR, NG>;
@@ -158,17 +165,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const int n_tiles = (N + BN - 1) / BN;
   const long long m_tiles = (M + TILE_M - 1) / TILE_M;
   // work list: the row tiles whose q columns nobody reads, their other column tiles; then every column tile of the other rows
-  constexpr bool KV = EPI == EPI_ROPE128 && PAIR && BN == 256;
-  const int kv_keep = rope.kv_per - rope.kv_skip, kv_n = KV ? n_tiles / rope.kv_per * kv_keep : 0;
-  const long long kv_tiles = KV ? (long long)rope.kv_m_tiles * kv_n : 0;
-  const long long total_tiles = KV ? kv_tiles + (m_tiles - rope.kv_m_tiles) * n_tiles : m_tiles * n_tiles;
+  constexpr bool KV = leaves_out(BN, EPI, PAIR);
+  const int kept = out.per - out.skip, kv_n = KV ? n_tiles / out.per * kept : 1;      // column tiles of such a row tile
+  const long long kv_tiles = KV ? (long long)out.m_tiles * kv_n : 0;
+  const long long total_tiles = KV ? kv_tiles + (m_tiles - out.m_tiles) * n_tiles : m_tiles * n_tiles;
   auto place = [&](long long tile, long long& m_blk, int& n_blk) {
-    if (KV && tile < kv_tiles) {
-      const int j = (int)(tile % kv_n);
-      m_blk = tile / kv_n; n_blk = j / kv_keep * rope.kv_per + rope.kv_skip + j % kv_keep;
+    if constexpr (KV) {
+      if (tile < kv_tiles) {
+        const int j = (int)(tile % kv_n);
+        m_blk = tile / kv_n; n_blk = j / kept * out.per + out.skip + j % kept;
+      } else {
+        tile -= kv_tiles;
+        m_blk = out.m_tiles + tile / n_tiles; n_blk = (int)(tile % n_tiles);
+      }
     } else {
-      const long long t = KV ? tile - kv_tiles : tile;
-      m_blk = (KV ? rope.kv_m_tiles : 0) + t / n_tiles; n_blk = (int)(t % n_tiles);
+      m_blk = tile / n_tiles; n_blk = (int)(tile % n_tiles);
     }
   };
   const int k_blocks = (K + BK - 1) / BK;
@@ -509,7 +520,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
 template <int BN, int EPI, bool PAIR>
 phx_status launch_t(const GemmPlan& p, const GemmRope& rope, const GemmNorm& norm, int64_t M, int* err_flag, int num_sms,
-                    cudaStream_t stream, std::string& err) {
+                    cudaStream_t stream, std::string& err, const GemmLeftOut& out = {}) {
   // the residual epilogues are fed by TMA prefetch and keep up with two groups; the others (RoPE, GELU, norm
   // scaling) are bound by the latency of each thread's instruction stream and get four groups where a pair's
   // smaller stages leave room for the slab buffers
@@ -562,7 +573,7 @@ phx_status launch_t(const GemmPlan& p, const GemmRope& rope, const GemmNorm& nor
   constexpr int TILE_M = PAIR ? 2 * BM : BM;
   const int n_tiles = (p.N + BN - 1) / BN;
   long long tiles = (M + TILE_M - 1) / TILE_M * n_tiles;
-  if (EPI == EPI_ROPE128 && PAIR && BN == 256) tiles -= (long long)rope.kv_m_tiles * (n_tiles / rope.kv_per * rope.kv_skip);
+  if (leaves_out(BN, EPI, PAIR)) tiles -= (long long)out.m_tiles * (n_tiles / out.per * out.skip);
   const int slots = PAIR ? max_pairs : num_sms;
   const int units = (int)(tiles < slots ? tiles : slots);
   if (units <= 0) return PHX_OK;
@@ -571,20 +582,20 @@ phx_status launch_t(const GemmPlan& p, const GemmRope& rope, const GemmNorm& nor
   long long Mll = M;
   int N = p.N, K = p.K;
   unsigned long long* counters = p.counters;
-  PHX_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, p.map_a, p.map_b, p.map_c, mr, rope, norm, Mll, N, K, err_flag, counters), err);
+  PHX_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, p.map_a, p.map_b, p.map_c, mr, rope, norm, Mll, N, K, err_flag, counters, out), err);
   return PHX_OK;
 }
 
 template <int BN, bool PAIR>
 phx_status launch_e(const GemmPlan& p, int epilogue, const GemmRope& rp, const GemmNorm& nm, int64_t M, int* err_flag,
-                    int num_sms, cudaStream_t stream, std::string& err) {
+                    int num_sms, cudaStream_t stream, std::string& err, const GemmLeftOut& out = {}) {
   switch (epilogue) {
     case EPI_STORE: return launch_t<BN, EPI_STORE, PAIR>(p, rp, nm, M, err_flag, num_sms, stream, err);
     case EPI_RESIDUAL: return launch_t<BN, EPI_RESIDUAL, PAIR>(p, rp, nm, M, err_flag, num_sms, stream, err);
     case EPI_GELU: return launch_t<BN, EPI_GELU, PAIR>(p, rp, nm, M, err_flag, num_sms, stream, err);
     case EPI_ROPE:
       if (rp.dh == 128) {   // a single CTA's 256-column tiles leave no room for the item buffers: gemm_launch takes narrow ones
-        if constexpr (PAIR || BN == 128) return launch_t<BN, EPI_ROPE128, PAIR>(p, rp, nm, M, err_flag, num_sms, stream, err);
+        if constexpr (PAIR || BN == 128) return launch_t<BN, EPI_ROPE128, PAIR>(p, rp, nm, M, err_flag, num_sms, stream, err, out);
         break;
       }
       return launch_t<BN, EPI_ROPE, PAIR>(p, rp, nm, M, err_flag, num_sms, stream, err);
@@ -940,10 +951,11 @@ phx_status gemm_plan_create(GemmPlan* plan, const bf16* A, const bf16* Wt, int64
 }
 
 phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64_t M, int epilogue, const GemmRope* rope,
-                       const GemmNorm* norm, int* err_flag, int num_sms, cudaStream_t stream, std::string& err) {
+                       const GemmNorm* norm, int* err_flag, int num_sms, cudaStream_t stream, std::string& err, int64_t kv_rows) {
   if (!p.ready || M > p.rows_max) { err = "gemm: plan not ready or M exceeds plan rows"; return PHX_E_ARG; }
   if (epilogue == EPI_RESIDUAL && R == nullptr) { err = "gemm: residual epilogue needs R"; return PHX_E_ARG; }
   GemmRope rp;
+  GemmLeftOut out;
   memset(&rp, 0, sizeof(rp));
   GemmNorm nm;
   memset(&nm, 0, sizeof(nm));
@@ -963,12 +975,11 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
       return PHX_E_ARG;
     }
     rp = *rope;
-    rp.kv_m_tiles = 0; rp.kv_per = 1; rp.kv_skip = 0;
     // pairs of CTAs on 256 columns and heads of 128: the q heads of a group that fill whole tiles (where four share a key head, four of the
     // twelve column tiles of 16 heads are left: 8 x (1022 + 64) rows 42.4 -> 23.1 us)
     const int width = rp.group * rp.dh, q_tiles = rp.g * rp.dh / 256;
-    if (rp.dh == 128 && p.pair && p.BN == 256 && rp.kv_rows > 0 && width % 256 == 0 && p.N % width == 0 && q_tiles > 0) {
-      rp.kv_m_tiles = (int)(rp.kv_rows / (2 * BM)); rp.kv_per = width / 256; rp.kv_skip = q_tiles;
+    if (rp.dh == 128 && p.pair && p.BN == 256 && kv_rows > 0 && width % 256 == 0 && p.N % width == 0 && q_tiles > 0) {
+      out.m_tiles = (int)(kv_rows / (2 * BM)); out.per = width / 256; out.skip = q_tiles;
     }
   }
   // output / residual maps are [M, N] with 128 x 64 boxes; rows past M are clipped by the TMA unit
@@ -1008,8 +1019,8 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
       }
     }
     dispatch_note(p.pair ? DK_GEMM_PAIR256 : DK_GEMM_CTA256);
-    if (rp.kv_m_tiles > 0) dispatch_note(DK_FORM_GEMM_KV);
-    return p.pair ? launch_e<256, true>(p, epilogue, rp, nm, M, err_flag, num_sms, stream, err)
+    if (out.m_tiles > 0) dispatch_note(DK_FORM_GEMM_KV);
+    return p.pair ? launch_e<256, true>(p, epilogue, rp, nm, M, err_flag, num_sms, stream, err, out)
                   : launch_e<256, false>(p, epilogue, rp, nm, M, err_flag, num_sms, stream, err);
   }
   dispatch_note(p.pair ? DK_GEMM_PAIR128 : DK_GEMM_CTA128);
