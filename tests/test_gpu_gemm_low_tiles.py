@@ -70,3 +70,42 @@ def test_low_tiles_in_the_engine(monkeypatch, B, S, C, D):
         eng.close()
     np.testing.assert_array_equal(out[0].log_probs, out[1].log_probs)
     np.testing.assert_array_equal(out[0].continuous, out[1].continuous)
+
+
+def test_low_tiles_follow_the_rows_and_the_buffers():
+    """Calls of several sizes on one engine, some from the buffers that a prefetch has filled: the 64-row tiles read the rows of the call."""
+    import numpy as np
+    import torch
+    from helpers import make_pair
+    from oracle import phoenix_oracle as po
+    from x_algorithm_b200.engine import dispatch_counts
+    C, dev = 43, {}
+    ocfg, w, rows_fn, eng = make_pair(max_batch=4, emb_size=512, num_layers=2, num_q_heads=8, num_kv_heads=8, key_size=64, history_len=20,
+                                      num_candidates=C)
+    _, _, _, plain = make_pair(max_batch=4, emb_size=512, num_layers=2, num_q_heads=8, num_kv_heads=8, key_size=64, history_len=20,
+                               num_candidates=C)
+    for B in (1, 3, 4):
+        b = po.make_batch(ocfg, B, seed=B, ragged=True)
+        dev[B] = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in
+                  (b.hist_post_ids, b.hist_author_ids, b.hist_actions, b.hist_surfaces, b.cand_post_ids, b.cand_author_ids)]
+
+    def forward(e, B):
+        lp, co = torch.empty((B, C, ocfg.num_actions), device="cuda"), torch.empty((B, C, ocfg.num_continuous), device="cuda")
+        e.rank_device(B, *dev[B], lp, co)
+        return lp, co
+
+    sizes = (4, 1, 3, 3, 1, 4)
+    before = dispatch_counts()
+    got = []
+    for i, B in enumerate(sizes):
+        got.append(forward(eng, B))
+        if i + 1 < len(sizes) and i % 2 == 0:
+            eng.rank_prefetch_device(sizes[i + 1], *dev[sizes[i + 1]])
+    eng.sync()
+    assert forms_since(before)[1] >= len(sizes)
+    for B, (lp, co) in zip(sizes, got):
+        want = forward(plain, B)
+        plain.sync()
+        assert torch.equal(lp, want[0]) and torch.equal(co, want[1])
+    eng.close()
+    plain.close()

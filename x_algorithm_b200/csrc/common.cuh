@@ -143,7 +143,7 @@ struct GemmNorm {
 // are encoded once for (pointer, rows_max) and reused for every M <= rows_max.
 struct GemmPlan {
   CUtensorMap map_a;
-  CUtensorMap map_a_low;      // A in boxes of 64 rows, for the low tiles of small calls
+  CUtensorMap map_a_low;      // A in boxes of 64 rows, for the low tiles of small calls; encoded by the first call that takes them
   CUtensorMap map_b;
   CUtensorMap map_b_narrow;   // BN = 256: W map for narrower tiles, used when a call has too few wide tiles to fill the device
   CUtensorMap map_c;   // output map, re-encoded when the output pointer or M changes
@@ -154,6 +154,7 @@ struct GemmPlan {
   const bf16* Wt = nullptr;
   int64_t rows_max = 0;
   int64_t a_rows = 0;   // rows the A map was encoded over (rows_max, or the M of the call that moved A)
+  const bf16* low_A = nullptr; int64_t low_rows = -1;   // what map_a_low was encoded over
   int N = 0, K = 0, BN = 0;
   bool pair = false;   // two CTAs of a cluster share each 256-row tile (tcgen05 cta_group::2)
   bool small_ok = false;   // calls of few tiles take one tile per CTA (gemm_small_kernel)

@@ -937,8 +937,8 @@ phx_status gemm_plan_create(GemmPlan* plan, const bf16* A, const bf16* Wt, int64
   // (out-projection, N = K = 512: 0.100 ms wide against 0.146 ms narrow)
   if (plan->pair && !(getenv("PHX_GEMM_TILES") && strcmp(getenv("PHX_GEMM_TILES"), "narrow") == 0)) narrow_tiles = false;
   plan->BN = (N % 256 == 0 && !narrow_tiles) ? 256 : 128;
+  plan->low_A = nullptr;
   phx_status s = make_map(&plan->map_a, A, rows_max, K, BM, err);
-  if (s == PHX_OK) s = make_map(&plan->map_a_low, A, rows_max, K, 64, err);
   if (s != PHX_OK) return s;
   s = make_map(&plan->map_b, Wt, N, K, plan->pair ? plan->BN / 2 : plan->BN, err);
   if (s != PHX_OK) return s;
@@ -965,7 +965,6 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
     // the activation buffer moved (double-buffered residual stream, or a block of rows inside it): re-encode its
     // map over exactly the M rows of this call, so that no tile reads past them
     phx_status s = make_map(&p.map_a, A, M, p.K, BM, err);
-    if (s == PHX_OK) s = make_map(&p.map_a_low, A, M, p.K, 64, err);
     if (s != PHX_OK) return s;
     p.A = A; p.a_rows = M;
   }
@@ -1001,7 +1000,15 @@ phx_status gemm_launch(GemmPlan& p, const bf16* A, bf16* C, const bf16* R, int64
     // forwards: D = 512, 640 rows a request 1.31 with one, 1.04 with four, 0.99 with eight (only the last layer's narrow ones are few).
     const CUtensorMap& map_b64 = p.BN == 256 ? p.map_b_narrow : p.map_b;   // boxes of 64 W rows, either way
     const long long mt = (M + BM - 1) / BM, t64 = mt * ((p.N + 63) / 64), t128 = mt * ((p.N + 127) / 128);
-    if (t64 <= num_sms && !(epilogue == EPI_ROPE && rp.dh == 128)) { dispatch_note(DK_GEMM_SMALL); return launch_small<64>(p, map_b64, C, R, epilogue, rp, nm, M, num_sms, err_flag, stream, err); }
+    if (t64 <= num_sms && !(epilogue == EPI_ROPE && rp.dh == 128)) {
+      if (low_tiles(M, p.N, p.K, num_sms) && (p.low_A != p.A || p.low_rows != p.a_rows)) {
+        phx_status s = make_map(&p.map_a_low, A, p.a_rows, p.K, 64, err);
+        if (s != PHX_OK) return s;
+        p.low_A = p.A; p.low_rows = p.a_rows;
+      }
+      dispatch_note(DK_GEMM_SMALL);
+      return launch_small<64>(p, map_b64, C, R, epilogue, rp, nm, M, num_sms, err_flag, stream, err);
+    }
     if (t128 <= num_sms) { dispatch_note(DK_GEMM_SMALL); return launch_small<128>(p, map_b64, C, R, epilogue, rp, nm, M, num_sms, err_flag, stream, err); }
   }
   if (p.BN == 256) {
