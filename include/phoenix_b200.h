@@ -335,7 +335,7 @@ phx_status phx_wait_selftest_async(phx_engine* e);
  * count of variant i, the return value is the number of variants; phx_dispatch_name(i) names them ("attn.strip",
  * "attn.stream", "attn.tcgen05", "attn.resident", "gemm.pair256", "gemm.pair128", "gemm.cta256", "gemm.cta128",
  * "gemm.simt", "scan.tcgen05", "scan.mma", "topk.exact", "attn.pingpong", "gemm.small", "gather", "gather.bulk"; forms of
- * them, counted beside them: "form.attn_low", "form.gemm_low", "form.gemm_deep", "form.gemm_kv_only").  A forward replayed from its CUDA graph counts nothing.  Lets a
+ * them, counted beside them: "form.attn_low", "form.gemm_low", "form.gemm_deep", "form.gemm_kv_only", "form.scan_split").  A forward replayed from its CUDA graph counts nothing.  Lets a
  * test or a monitor assert that a workload runs on the kernels meant for it.  The reference's counterpart is its
  * attention-implementation switch being logged at start-up (phoenix/xrex/models/recsys_attention.py:18-242). */
 int32_t phx_dispatch_counts(int64_t* out, int32_t n);

@@ -410,3 +410,33 @@ def test_short_lists_do_not_run_short(k):
         assert not sh.finish()
         assert (ids.sort(dim=1).values.diff(dim=1) > 0).all() and (sc.diff(dim=1) <= 0).all()
     sh.close()
+
+
+# 200000 rows: 1563 tiles; 10 picks for 17 queries expect five rows of a tile to pass, 1000 more than 30
+@pytest.mark.parametrize("int8,N,B,k,split", [(True, 3001, 16, 40, True), (True, 3001, 17, 40, False), (True, 200_000, 17, 10, True),
+                                              (True, 200_000, 17, 1000, False), (True, 200_000, 16, 1000, True), (True, 200_000, 65, 10, False),
+                                              (False, 3001, 16, 40, True), (False, 200_000, 16, 1000, True), (False, 200_000, 17, 10, False)])
+def test_scan_shares_its_tiles_by_the_rows_expected_to_pass(int8, N, B, k, split):
+    """Both forms of the collect pass, on both sides of the rule that picks them: int8 lists are the exact passes' (whole sums), bf16 lists the other
+    form's, to the bit."""
+    from x_algorithm_b200.engine import dispatch_counts
+    from x_algorithm_b200.retrieval import CorpusShard
+    sh = CorpusShard(N, 128, max_queries=max(B, 17), max_k=k)
+    sh.fill_synthetic(4)
+    if int8:
+        sh.quantize_int8()
+        sh.set_int8(True)
+    before = dispatch_counts()
+    got = _topk(sh, _users(B, 128, 9), k)
+    after = dispatch_counts()
+    assert after["scan.tcgen05"] > before["scan.tcgen05"] and after["topk.exact"] == before["topk.exact"]
+    assert (after["form.scan_split"] > before["form.scan_split"]) == split
+    if int8:
+        sh.set_exact(True)
+        want = _topk(sh, _users(B, 128, 9), k)
+    else:
+        want = _topk(sh, _users(33 - B, 128, 9), k)             # 16 and 17: the first 16 queries are the same
+        assert (dispatch_counts()["form.scan_split"] > after["form.scan_split"]) != split
+    for g, w in zip(got, want):
+        np.testing.assert_array_equal(g[:16] if not int8 else g, w[:16] if not int8 else w)
+    sh.close()

@@ -52,7 +52,8 @@ enum DispatchKind {
   DK_FORM_GEMM_LOW = 17,    // one tile per CTA: tiles of 64 rows
   DK_FORM_GEMM_DEEP = 18,   // ... of 128 rows with the deep ring
   DK_FORM_GEMM_KV = 19,     // QKV projection without the query tiles that nobody reads
-  DK_COUNT = 20
+  DK_FORM_SCAN_SPLIT = 20,  // tcgen05 corpus scan, collect pass with the tiles shared between two sets of warps
+  DK_COUNT = 21
 };
 void dispatch_note(int kind);
 

@@ -1751,7 +1751,7 @@ int32_t phx_dispatch_counts(int64_t* out, int32_t n) {
 const char* phx_dispatch_name(int32_t kind) {
   static const char* names[DK_COUNT] = {"attn.strip", "attn.stream", "attn.tcgen05", "attn.resident", "gemm.pair256", "gemm.pair128",
                                         "gemm.cta256", "gemm.cta128", "gemm.simt", "scan.tcgen05", "scan.mma", "topk.exact", "attn.pingpong",
-                                        "gemm.small", "gather", "gather.bulk", "form.attn_low", "form.gemm_low", "form.gemm_deep", "form.gemm_kv_only"};
+                                        "gemm.small", "gather", "gather.bulk", "form.attn_low", "form.gemm_low", "form.gemm_deep", "form.gemm_kv_only", "form.scan_split"};
   return (kind >= 0 && kind < DK_COUNT) ? names[kind] : "";
 }
 

@@ -1035,6 +1035,7 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
   ta.pivot = c->pivot; ta.surv = c->surv; ta.counts = c->counts; ta.cap = c->cap;
   const long long n_tiles = (rows + tile_rows - 1) / tile_rows;
   int j = 0;
+  double expected = c->mask ? (double)c->elig_count : (double)rows;    // rows of a query's list before the select
   // a window whose eligible rows all fit the survivor buffer needs no pivot: every eligible row is collected
   if (rows > c->cap && !(c->mask && c->elig_count <= c->cap)) {
     // Rows wanted at or above the pivot, and how many of them (`picks`) the sample is to hold: every (want / picks)-th tile is scored for
@@ -1056,6 +1057,7 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
       if (t < cost) { want = w; picks = j; cost = t; }
     }
     c->last.sparse = want > 3.0 * k_real;
+    expected = want;
     long long stride = (long long)(want / picks);
     if (stride < 1) stride = 1;
     long long sampled_tiles = (n_tiles + stride - 1) / stride;
@@ -1069,7 +1071,7 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
     if (j < 1) j = 1;
     phx_status s;
     dispatch_note(tc ? DK_SCAN_TC : DK_SCAN_MMA);
-    if (tc) s = tc_scan_launch(*map_corpus, map_users, ta, 0, c->num_sms, c->err_flag, c->stream, c->err);
+    if (tc) s = tc_scan_launch(*map_corpus, map_users, ta, 0, expected, c->num_sms, c->err_flag, c->stream, c->err);
     else s = run_scan(c, a, 0, (int)(sampled_tiles < c->num_sms * 2 ? sampled_tiles : c->num_sms * 2));
     if (s) return s;
   }
@@ -1077,13 +1079,13 @@ phx_status phx_corpus_topk_window_device(phx_corpus* c, const float* users_dev, 
   {
     phx_status s;
     dispatch_note(tc ? DK_SCAN_TC : DK_SCAN_MMA);
-    if (tc) s = tc_scan_launch(*map_corpus, map_users, ta, 1, c->num_sms, c->err_flag, c->stream, c->err);
+    if (tc) s = tc_scan_launch(*map_corpus, map_users, ta, 1, expected, c->num_sms, c->err_flag, c->stream, c->err);
     else s = run_scan(c, a, 1, (int)(n_tiles < c->num_sms * 2 ? n_tiles : c->num_sms * 2));
     if (s) return s;
   }
   const int kp2 = next_pow2(k_real);
   // In plain stream order: a CTA that comes up beside the scan's is left with the L1 that the scan's shared memory leaves over, and
-  // reads its list eight times (30 k rows, all of them survivors: 164 us a call instead of 142).
+  // reads a long list up to eight times (30 k rows, all of them survivors, the digits alone: 164 us a call instead of 142).
   select_kernel<<<B, SEL_THREADS, (size_t)sel_room(kp2) * 8, c->stream>>>(c->surv, c->counts, 0, c->cap, k_real, kp2, scores_dev,
                                                                (long long*)ids_dev, c->status, c->keys_out, k);
   PHX_CUDA_TRY(cudaGetLastError(), c->err);

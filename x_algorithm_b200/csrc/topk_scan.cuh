@@ -38,8 +38,8 @@ bool tc_scan_supported(int row_bytes);
 // `queries`: [256][row_bytes], in the corpus' type
 phx_status tc_scan_make_maps(CUtensorMap* map_corpus, CUtensorMap* map_users, const void* corpus, long long rows, int row_bytes,
                              const void* queries, std::string& err);
-// mode 0 = sample pass (group maxima), 1 = collect pass (survivors)
-phx_status tc_scan_launch(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, int mode,
+// mode 0 = sample pass (group maxima), 1 = collect pass (survivors).  expected: rows that the pivot is to let through for a query
+phx_status tc_scan_launch(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, int mode, double expected,
                           int num_sms, int* err_flag, cudaStream_t stream, std::string& err);
 
 }  // namespace phx

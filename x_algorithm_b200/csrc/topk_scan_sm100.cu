@@ -126,25 +126,25 @@ __device__ __forceinline__ float s8_value(uint32_t acc, float query_scale) { ret
 constexpr float S8_OFFSET = 12582912.0f;            // 1.5 * 2^23: its bit pattern plus an integer below 2^22 in size is the float of their sum
 constexpr uint32_t S8_OFFSET_BITS = 0x4B400000u;
 
-// How the consumer warps share the tiles: all sixteen on every tile, a quarter of the columns each, or (SPLIT: the collect pass with 64
-// columns) eight on every other tile, half of the columns each.  A warp that has rows to test is late for its next tile, and an
+// How the consumer warps share the tiles: all sixteen on every tile, a quarter of the columns each, or (SPLIT: some collect passes with 64
+// columns, split_tiles) eight on every other tile, half of the columns each.  A warp that has rows to test is late for its next tile, and an
 // accumulator goes back to the MMA warp when the last of its warps has read it: split, fewer warps wait for one another, each has two
-// tiles' time, and what a tile costs beside its columns (wait, vote, release) is paid half as often.  12.5 M int8 rows, 64 queries, us, k = 1 /
-// 1000: 320 / 369 -> 311 / 330.  With 128 columns it takes as much from short lists as it gives long ones (396 / 477 -> 414 / 460); with 256 a
-// warp's half would take two turns, and rows to test in the first would hold the accumulator (581 / 710 -> 726 / 918).
-template <int MODE, int NQ> struct ScanCfg {
-  static constexpr bool SPLIT = MODE == 1 && NQ == 64;
+// tiles' time, and what a tile costs beside its columns (wait, vote, release) is paid half as often; but twice the columns share one
+// smallest threshold, and a group's rows are tested by one warp instead of two.  With 128 columns it takes as much from short lists as it gives long
+// ones (12.5 M int8 rows, us, k = 1 / 1000: 396 / 477 -> 414 / 460); with 256 a warp's half would take two turns, and rows to test in the first would
+// hold the accumulator (581 / 710 -> 726 / 918).
+template <int NQ, bool SPLIT> struct ScanCfg {
   static constexpr int CW = SPLIT ? NQ / 2 : NQ / 4; // query columns per consumer warp
   static constexpr int CH = CW < 32 ? CW : 32;       // columns per group; the collect filter's threshold is the smallest of the group's
   static constexpr int GROUPS = NQ / CH;
   static constexpr int DRAIN = (SPLIT ? TC_CWARPS / 2 : TC_CWARPS) * 32;   // threads that release an accumulator
 };
 
-template <int MODE, bool I8, int NQ, bool BIAS>
+template <int MODE, bool I8, int NQ, bool BIAS, bool SPLIT>
 __global__ void __launch_bounds__(scan_threads(BIAS), 1)
 scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_constant__ CUtensorMap map_users,
                TcScanArgs a, int* err_flag) {
-  using cfg = ScanCfg<MODE, NQ>;
+  using cfg = ScanCfg<NQ, SPLIT>;
   constexpr int CW = cfg::CW, CH = cfg::CH;
   static_assert(!BIAS || (MODE == 1 && I8), "the bias belongs to the int8 collect pass");
   extern __shared__ uint8_t smem_raw[];
@@ -373,7 +373,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
     auto consume = [&](auto folded) {
       constexpr bool FOLDED = decltype(folded)::value;
       const int ew = warp - 2;
-      const int part = cfg::SPLIT ? (ew >> 2) & 1 : ew >> 2;   // which half or quarter of the query columns
+      const int part = SPLIT ? (ew >> 2) & 1 : ew >> 2;   // which half or quarter of the query columns
       const int quad = warp & 3;       // TMEM lane quadrant
       uint4* const queue = s_queue + ew * QCAP;
       uint32_t* const s_row = reinterpret_cast<uint32_t*>(smem_raw + (rows_smem - smem_u32(smem_raw))) + ew * 32;
@@ -389,8 +389,8 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
         bt_lane[c] = (FOLDED && lane < CH) ? s_t[part * CW + c * CH + lane] : 0;
       }
       const int open = FOLDED ? *s_open : 0;
-      constexpr int EACH = cfg::SPLIT ? 2 : 1;                 // a warp's tiles: every one, or every other one
-      uint32_t it = cfg::SPLIT ? ew >> 3 : 0;
+      constexpr int EACH = SPLIT ? 2 : 1;                 // a warp's tiles: every one, or every other one
+      uint32_t it = SPLIT ? ew >> 3 : 0;
       for (long long w = blockIdx.x + (long long)it * gridDim.x; w < n_work; w += (long long)EACH * gridDim.x, it += EACH) {
         const long long tile = (MODE == 0) ? w * a.stride : w;
         const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
@@ -553,23 +553,39 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap map_corpus, const __grid_cons
   }
 }
 
-template <int MODE, bool I8, int NQ, bool BIAS>
+template <int MODE, bool I8, int NQ, bool BIAS, bool SPLIT>
 phx_status launch_scan_tc(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, int grid, int* err_flag,
                           cudaStream_t stream, std::string& err) {
   const int kblk = a.row_bytes / 128;
   const size_t smem = (size_t)kblk * NQ * 128 + (size_t)scan_stages(BIAS, kblk) * kblk * TC_ROWS * 128 + scan_bias_bytes(BIAS, NQ) + 2 * 256 * 4 + 64 + 128 * 16 + TC_CWARPS * (QCAP * 16 + 128) + 256 + 1024;
   static SmemLimit limit;
-  PHX_CUDA_TRY(limit.raise(scan_tc_kernel<MODE, I8, NQ, BIAS>, 226 * 1024), err);
-  PHX_CUDA_TRY(launch_programmatic(scan_tc_kernel<MODE, I8, NQ, BIAS>, grid, scan_threads(BIAS), smem, stream, map_corpus, map_users, a, err_flag), err);
+  PHX_CUDA_TRY(limit.raise(scan_tc_kernel<MODE, I8, NQ, BIAS, SPLIT>, 226 * 1024), err);
+  PHX_CUDA_TRY(launch_programmatic(scan_tc_kernel<MODE, I8, NQ, BIAS, SPLIT>, grid, scan_threads(BIAS), smem, stream, map_corpus, map_users, a, err_flag), err);
   return PHX_OK;
 }
+// Collect passes of up to 64 queries: int8 rows while no more than a dozen of a tile are expected to pass for some query - the tests of more hold
+// the eight warps up - and any rows for up to 16 queries, whose tests half of the warps would be without otherwise.  Whole calls, us, every warp on
+// every tile / split: int8 rows, 64 queries, k = 1000: 12.5 M rows 389 / 339, 4 M 161 / 149 (six of a tile), 2 M 113 / 117 (twelve), 1 M 90 / 101, 500 k 78 / 90; 33
+// queries: 12.5 M 357 / 315, 2 M 107 / 99, 1 M 84 / 83 (twelve), 150 k 58 / 62; 16 queries: 500 k 66 / 56, 150 k 54 / 48.  bf16 rows, whose copies
+// take longer than the tests where few pass: 64 queries, k = 1000: 12.5 M 479 / 480, 1 M 91 / 103, 150 k 71 / 81; 16 queries: 500 k 63 / 56, 150 k 53 / 47.
+bool split_tiles(const TcScanArgs& a, double expected) {
+  return a.B <= 16 || (a.row_scale != nullptr && expected * a.B * TC_ROWS <= 12.0 * (double)a.rows);
+}
 template <int MODE, bool I8, bool BIAS>
-phx_status launch_scan_nq(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, int grid, int* err_flag,
+phx_status launch_scan_nq(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, double expected, int grid, int* err_flag,
                           cudaStream_t stream, std::string& err) {
   // query columns: the multiple of 64 that holds the batch (the tensor core and the consumers work on all NQ of them)
-  if (a.B <= 64) return launch_scan_tc<MODE, I8, 64, BIAS>(map_corpus, map_users, a, grid, err_flag, stream, err);
-  if (a.B <= 128) return launch_scan_tc<MODE, I8, 128, BIAS>(map_corpus, map_users, a, grid, err_flag, stream, err);
-  return launch_scan_tc<MODE, I8, 256, BIAS>(map_corpus, map_users, a, grid, err_flag, stream, err);
+  if (a.B <= 64) {
+    if constexpr (MODE == 1) {
+      if (split_tiles(a, expected)) {
+        dispatch_note(DK_FORM_SCAN_SPLIT);
+        return launch_scan_tc<MODE, I8, 64, BIAS, true>(map_corpus, map_users, a, grid, err_flag, stream, err);
+      }
+    }
+    return launch_scan_tc<MODE, I8, 64, BIAS, false>(map_corpus, map_users, a, grid, err_flag, stream, err);
+  }
+  if (a.B <= 128) return launch_scan_tc<MODE, I8, 128, BIAS, false>(map_corpus, map_users, a, grid, err_flag, stream, err);
+  return launch_scan_tc<MODE, I8, 256, BIAS, false>(map_corpus, map_users, a, grid, err_flag, stream, err);
 }
 
 }  // namespace
@@ -585,20 +601,20 @@ phx_status tc_scan_make_maps(CUtensorMap* map_corpus, CUtensorMap* map_users, co
 }
 
 phx_status tc_scan_launch(const CUtensorMap& map_corpus, const CUtensorMap& map_users, const TcScanArgs& a, int mode,
-                          int num_sms, int* err_flag, cudaStream_t stream, std::string& err) {
+                          double expected, int num_sms, int* err_flag, cudaStream_t stream, std::string& err) {
   const long long n_tiles = (a.rows + TC_ROWS - 1) / TC_ROWS;
   const long long n_work = (mode == 0) ? (n_tiles + a.stride - 1) / a.stride : n_tiles;
   const int grid = (int)(n_work < num_sms ? n_work : num_sms);
   if (grid <= 0) return PHX_OK;
   const bool i8 = a.row_scale != nullptr;
   if (mode == 0)
-    return i8 ? launch_scan_nq<0, true, false>(map_corpus, map_users, a, grid, err_flag, stream, err)
-              : launch_scan_nq<0, false, false>(map_corpus, map_users, a, grid, err_flag, stream, err);
-  if (!i8) return launch_scan_nq<1, false, false>(map_corpus, map_users, a, grid, err_flag, stream, err);
+    return i8 ? launch_scan_nq<0, true, false>(map_corpus, map_users, a, expected, grid, err_flag, stream, err)
+              : launch_scan_nq<0, false, false>(map_corpus, map_users, a, expected, grid, err_flag, stream, err);
+  if (!i8) return launch_scan_nq<1, false, false>(map_corpus, map_users, a, expected, grid, err_flag, stream, err);
   // Scales below zero turn the order of the sums round, and the sign of a sum says nothing in a corpus that has one: every group is
   // open, or the bias is left out (one such row, 12.5 M rows, device us open / without: 256 queries 1545 / 1103, 100 847 / 690, one 539 / 589)
-  return a.scales_negative && a.B > 64 ? launch_scan_nq<1, true, false>(map_corpus, map_users, a, grid, err_flag, stream, err)
-                           : launch_scan_nq<1, true, true>(map_corpus, map_users, a, grid, err_flag, stream, err);
+  return a.scales_negative && a.B > 64 ? launch_scan_nq<1, true, false>(map_corpus, map_users, a, expected, grid, err_flag, stream, err)
+                           : launch_scan_nq<1, true, true>(map_corpus, map_users, a, expected, grid, err_flag, stream, err);
 }
 
 }  // namespace phx
