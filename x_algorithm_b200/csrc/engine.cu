@@ -246,7 +246,6 @@ phx_status dev_alloc(phx_engine* e, Tp** p, size_t count) {
   return PHX_OK;
 }
 
-// Results of `rows` candidates as one block: f64 scores, log-probabilities, continuous values, each on a 256-byte boundary
 // Up to this size a host-buffer call has the device write its results straight to pinned memory.  A copy costs its bytes and, behind
 // or in front of a kernel, 5 to 10 us of hand-over between the engines; larger results are worth copying in chunks, so that the
 // host can take one while the next is on the bus.  Inputs are read from pinned memory at every size.  Whole calls, us, copies both ways /
@@ -254,6 +253,7 @@ phx_status dev_alloc(phx_engine* e, Tp** p, size_t count) {
 // 1.1 MB 302 / 282 / 268; 606 KB, 2.3 MB 503 / 523 / - (inputs alone 485); inputs alone, 1.4 MB 1054 -> 1018, 2.9 MB 1986 -> 1924.
 // Packed results are laid out request by request: from half a megabyte on that is worth overlapping (1.1 MB: 500 direct, 491 copied).
 constexpr size_t DIRECT_OUT_BYTES = 1280u << 10, DIRECT_OUT_PACKED_BYTES = 512u << 10;
+// Results of `rows` candidates as one block: f64 scores, log-probabilities, continuous values, each on a 256-byte boundary
 struct OutLayout {
   size_t lp_off, cont_off, bytes;
   OutLayout(size_t rows, int V, int NC) {

@@ -564,11 +564,11 @@ phx_status launch_t(const GemmPlan& p, const GemmRope& rope, const GemmNorm& nor
       e = cudaOccupancyMaxActiveClusters(&n, kern, &lc);
       lc.numAttrs = all_attrs;
       max_pairs = n < num_sms / 2 ? n : num_sms / 2;
-      if (d < LAUNCH_MAX_DEVICES) pairs_of[d].store(max_pairs, std::memory_order_relaxed);
+      if (d >= 0 && d < LAUNCH_MAX_DEVICES) pairs_of[d].store(max_pairs, std::memory_order_relaxed);
     }
     return e;
   }), err);
-  if (PAIR && max_pairs == 0 && dev < LAUNCH_MAX_DEVICES) max_pairs = pairs_of[dev].load(std::memory_order_relaxed);
+  if (PAIR && max_pairs == 0 && dev >= 0 && dev < LAUNCH_MAX_DEVICES) max_pairs = pairs_of[dev].load(std::memory_order_relaxed);
   if (PAIR && max_pairs <= 0) { err = "gemm: the device cannot hold a CTA pair of this kernel"; return PHX_E_CUDA; }
   constexpr int TILE_M = PAIR ? 2 * BM : BM;
   const int n_tiles = (p.N + BN - 1) / BN;
@@ -604,12 +604,12 @@ phx_status launch_e(const GemmPlan& p, int epilogue, const GemmRope& rp, const G
   return PHX_E_ARG;
 }
 
-// ---- small problems: one 128 x BN tile per CTA -----------------------------------------------------------------------
+// ---- small problems: one TM x BN tile per CTA ------------------------------------------------------------------------
 // For calls whose 128 x BN tiles (BN = 64 or 128) do not outnumber the SMs: one request, or a few.  Such a GEMM is a chain of
 // latencies - launch, first operand bytes, k-steps, epilogue, last store - and the pair kernel above pays most of them on
-// a dozen CTA pairs.  Here every tile has a CTA of its own, no cluster hand-shake, at most two CTAs fit an SM, so the next
-// kernel's CTAs set up (and, for weights that nothing rewrites, fetch the W half of their ring) under the tail of this
-// one; each epilogue thread owns half a row's slab, has its residual / statistics loads in flight under the main loop and
+// a dozen CTA pairs.  Here every tile (128 rows, or 64: low_tiles) has a CTA of its own and there is no cluster hand-shake.  Two CTAs with
+// shallow rings fit an SM, so that the next kernel's set up (and, for weights that nothing rewrites, fetch the W half of their ring) under the
+// tail of this one; a CTA with a deep ring has an SM to itself (deep_ring).  Each epilogue thread owns half a row's slab, has its residual / statistics loads in flight under the main loop and
 // stores its 64 bytes straight to global memory.
 //   warp 0 TMA producer, warp 1 MMA issuer, then BN / 32 epilogue groups of four warps: group g takes the half g & 1 of
 //   64-column slab g >> 1 (RoPE: the column pairs of pass g & 1)
@@ -634,7 +634,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   constexpr bool RES = (EPI == EPI_RESIDUAL);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t ss_base = smem_base + cfg::STAGES * cfg::STAGE_BYTES;     // [slab][128] first halves of the row sums
+  const uint32_t ss_base = smem_base + cfg::STAGES * cfg::STAGE_BYTES;     // [slab][TM] first halves of the row sums
   const uint32_t bars = ss_base + (BN / 64) * TM * 4;
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (cfg::STAGES + s); };
@@ -854,8 +854,8 @@ phx_status launch_small_d(const GemmPlan& p, const CUtensorMap& map_b64, bf16* C
 // A deep ring has its SM for itself; a shallow one leaves room for a CTA of the kernel behind.  Deep from K = 1024 on, and from 512 where the
 // kernel behind finds SMs free anyway or has few CTAs.  Forwards of 1 to 16 requests on the device, us, shallow / deep from K = 1024 / from 512 /
 // as here: eight layers of D = 512 and 106 rows a request, one 248 / 222 / 216 / 216, three 242 / 219 / 213 / 213, 118 rows, 16 requests 383 / 336 /
-// 324 / 324; 640 rows, one request 276 / 251 / 254 / 250; D = 1024, two layers of 275 rows, six requests 210 / 168.
-// (Each kernel ends without a look at the error flag in all but the first figure of each.)
+// 324 / 324; 640 rows, one request 276 / 251 / 254 / 250; D = 1024, two layers of 275 rows, six requests 210 / 168.  (The shallow figures are of
+// kernels that still read the error flag as their last act, 0.5 us each - see gave_up.)
 bool deep_ring(int K, int epilogue, long long tiles, int num_sms) {
   return K >= 1024 || (K >= 512 && (epilogue == EPI_RESIDUAL || 3 * tiles <= 2 * num_sms));
 }

@@ -349,17 +349,20 @@ phx_status launch_heads_mma(const HeadsArgs& a, long long rows, cudaStream_t str
   const long long strips = (rows + 15) / 16;
   const size_t params = (size_t)NT * 8 * (a.D + HM_WPAD) * sizeof(bf16) + (size_t)a.D * sizeof(float);
   const size_t strip_smem = params + (size_t)16 * NT * 8 * (sizeof(float) + sizeof(double)) + 64 + (size_t)16 * (a.D + HM_WPAD) * sizeof(bf16);
-  // Three CTAs of a strip each fit an SM's registers (one or two its shared memory from D = 768 on); about two rounds of them and a warp a strip
-  // are level.  Kernel at 20 outputs, us, eight warps a strip up to 296 strips and then one / this: D = 512: 32 strips 14.7 / 10.7, 288: 18.7 / 14.7;
-  // beyond the line 768: 22.9 / 22.8, 2048: 27.0 / 45.4, 8192: 92 / 164; D = 1024: 32 strips 20.7 / 14.7, 300: 31.1 / 24.9; D = 128: 8 strips
-  // 10.6 / 10.5, beyond 3750: 29.0 / 39.3.
+  // Three CTAs of a strip each fit an SM's registers, of wide rows two or one its shared memory, so that the line below is one to three rounds of
+  // them: each round takes less than a warp a strip, or four, take with all strips at once.  Kernel, us, sixteen warps / four / one, at 148, 296 and
+  // 444 strips: D = 512, 20 outputs 12.6 / 18.9 / 20.9, 12.7 / 22.9 / 22.9, 14.8 / 23.0 / 22.9; D = 1024, 30 outputs 16.9 / 39.3 / 39.4, 18.9 / 39.4 / 39.4, 29.2 / 63.9 /
+  // 39.4; D = 1280, 20 outputs 18.9 / 39.4 / 37.3, 20.9 / 39.4 / 39.3, 33.2 / 66.0 / 41.4; D = 1280, 30 outputs (one CTA an SM from here on) 20.9 / 45.5 /
+  // 45.5, 29.1 / 47.6 / 45.5, 39.4 / 78.2 / 49.6; D = 1536 18.9 / 45.5 / 41.4, 29.1 / 47.6 / 41.4, 39.4 / 80.3 / 45.5; D = 2048 23.0 / 49.6 / 49.6, 37.3 / 90.4 /
+  // 55.7, 51.7 / 131.6 / 57.8.  Beyond the line one warp a strip: D = 512, 20 outputs, sixteen / one: 768 strips 22.8 / 22.9, 2048 45.4 / 27.0, 8192 164 / 92.
   static SmemLimit limit16, limit4, limit1;
-  if (strips <= 3 * 148 && strip_smem <= HEADS_SMEM_MAX)
+  const int sms = device_sms();
+  if (strips <= 3LL * sms && strip_smem <= HEADS_SMEM_MAX)
     return launch_heads(heads_strip_kernel<NT>, limit16, a, strips, HS_WARPS * 32, strip_smem, stream, err);
-  if (strips <= 2 * 148)
+  if (strips <= 2LL * sms)
     return launch_heads(heads_mma_kernel<NT, 4>, limit4, a, strips, 4 * 32, params + (size_t)16 * NT * 8 * (4 * sizeof(float) + sizeof(double)), stream, err);
   const long long blocks = (strips + HM_WARPS - 1) / HM_WARPS;
-  return launch_heads(heads_mma_kernel<NT, 1>, limit1, a, blocks < 148 * 3 ? blocks : 148 * 3, HM_WARPS * 32,
+  return launch_heads(heads_mma_kernel<NT, 1>, limit1, a, blocks < 3LL * sms ? blocks : 3LL * sms, HM_WARPS * 32,
                       params + (size_t)16 * NT * 8 * HM_WARPS * (sizeof(float) + sizeof(double)), stream, err);
 }
 
