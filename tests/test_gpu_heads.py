@@ -12,10 +12,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("opts,B,C", [(dict(), 240, 31), (dict(num_actions=7), 160, 47), (dict(num_actions=14, num_continuous=2), 500, 17),
                                       (dict(num_actions=30, num_continuous=2), 240, 32),
                                       (dict(emb_size=2432, num_q_heads=2, num_kv_heads=2, key_size=32), 150, 33)])
-def test_heads_same_bits_for_any_number_of_rows(monkeypatch, opts, B, C):
+def test_heads_same_bits_for_any_number_of_rows(opts, B, C):
     """More strips than the small calls' kernel takes, against the same requests a few at a time."""
-    if "emb_size" in opts:
-        monkeypatch.setenv("PHX_NORM", "separate")     # row statistics of such widths follow the token kernel's share of a warp
     assert B * C > 3 * 148 * 16 or "emb_size" in opts
     ocfg, w, rows_fn, eng = make_pair(max_batch=B, num_layers=1, history_len=9, num_candidates=C, **opts)
     b = po.make_batch(ocfg, B, seed=6, ragged=True)

@@ -5,7 +5,7 @@ against the oracle, and both heads kernels against each other."""
 import numpy as np
 import pytest
 
-from helpers import make_pair, rel_l2, to_inputs
+from helpers import assert_heads_close, make_pair, rel_l2, to_inputs
 from oracle import phoenix_oracle as po
 
 pytestmark = pytest.mark.gpu
@@ -30,6 +30,28 @@ def test_tokens_a_warp(monkeypatch, B, S, C, D, H, pack):
     eng.close()
     np.testing.assert_array_equal(got.log_probs, want.log_probs)
     np.testing.assert_array_equal(got.continuous, want.continuous)
+
+
+@pytest.mark.parametrize("D", [2048, 2112, 2432])
+@pytest.mark.parametrize("build", ["plain", "general", "project"])
+def test_rows_with_more_than_32_statistics(monkeypatch, D, build):
+    """A row's sum of squares goes to slot 0 of D / 64 and the others to zero, all of them: what the forward before left in a slot (the sums of its
+    last layer) is no part of the next one's first norm."""
+    if build == "general":
+        monkeypatch.setenv("PHX_DEBUG_TAPS", "1")
+    kw = dict(token_combine="project") if build == "project" else {}
+    ocfg, w, rows_fn, eng = make_pair(max_batch=6, emb_size=D, num_layers=1, num_q_heads=2, num_kv_heads=2, key_size=32, history_len=9,
+                                      num_candidates=20, **kw)
+    a, b = (po.make_batch(ocfg, n, seed=n, ragged=True) for n in (4, 6))
+    first = eng.rank(to_inputs(a))
+    eng.rank(to_inputs(b))
+    again = eng.rank(to_inputs(a))
+    np.testing.assert_array_equal(again.log_probs, first.log_probs)
+    np.testing.assert_array_equal(again.continuous, first.continuous)
+    lp, cont, logits = po.rank_forward(ocfg, w, rows_fn, a)
+    valid = a.cand_post_ids != 0
+    assert_heads_close(again.log_probs[valid], again.continuous[valid], logits[valid], cont[valid], tol=TOL)
+    eng.close()
 
 
 @pytest.mark.parametrize("S,D,B", [(140, 256, 3), (144, 256, 3), (33, 128, 5), (200, 256, 2)])   # 72 KB of rows and statistics: 142 x 256

@@ -86,6 +86,11 @@ __device__ __forceinline__ void cont_add(const TokenBuildArgs& a, const float (*
   }
 }
 
+// A row's statistics for the first fused RMSNorm: its sum of squares in slot 0, zero in the others (D / 64 slots, more than 32 of them from D = 2112 on)
+__device__ __forceinline__ void store_row_ss(float* slots, int n, int lane, float ss) {
+  for (int i = lane; i < n; i += 32) slots[i] = i == 0 ? ss : 0.f;
+}
+
 __global__ void __launch_bounds__(256, 3) build_tokens_kernel(TokenBuildArgs a) {
   // (no early launch signal here: the GEMM behind this kernel would park its CTAs - registers and all - on the SMs
   // while this bandwidth-bound kernel still needs every warp slot it can get)
@@ -218,7 +223,7 @@ __global__ void __launch_bounds__(256, 3) build_tokens_kernel(TokenBuildArgs a) 
   if (a.row_ss) {   // statistics of the bf16 row for the first fused RMSNorm
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) row_ss += __shfl_xor_sync(0xffffffffu, row_ss, o);
-    if (lane < a.ss_slots) a.row_ss[orow * a.ss_slots + lane] = (lane == 0) ? row_ss : 0.f;
+    store_row_ss(a.row_ss + orow * a.ss_slots, a.ss_slots, lane, row_ss);
   }
 }
 
@@ -315,7 +320,7 @@ __global__ void __launch_bounds__(256, SL == 8 ? 2 : 3) build_tokens_bulk_kernel
       float ss = row_ss;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      if (lane < a.ss_slots) a.row_ss[(long long)p.row * a.ss_slots + lane] = (lane == 0) ? ss : 0.f;
+      store_row_ss(a.row_ss + (long long)p.row * a.ss_slots, a.ss_slots, lane, ss);
     }
   };
   const int span = (a.D + 255) & ~255;    // columns of a token's walk
@@ -393,7 +398,7 @@ __global__ void __launch_bounds__(256) finish_tokens_kernel(const bf16* __restri
   if (a.row_ss) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) row_ss += __shfl_xor_sync(0xffffffffu, row_ss, o);
-    if (lane < a.ss_slots) a.row_ss[orow * a.ss_slots + lane] = (lane == 0) ? row_ss : 0.f;
+    store_row_ss(a.row_ss + orow * a.ss_slots, a.ss_slots, lane, row_ss);
   }
 }
 
