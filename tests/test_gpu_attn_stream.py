@@ -7,14 +7,14 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def reference(q, k, v, seg, S, scale):
+def reference(q, k, v, seg, S, scale, cap=lambda x: x):
     import torch
     q, k, v = q.float(), k.float(), v.float()
     g = q.shape[2] // k.shape[2]
     k, v = k.repeat_interleave(g, 2), v.repeat_interleave(g, 2)
-    s = torch.einsum("bqhd,bkhd->bhqk", q, k[:, :S]) * scale
+    s = cap(torch.einsum("bqhd,bkhd->bhqk", q, k[:, :S]) * scale)
     s = s.masked_fill((seg[:, None, None, :S] != 1), -math.inf)
-    own = ((q * k).sum(-1) * scale).permute(0, 2, 1)[..., None].masked_fill((seg != -1)[:, None, :, None], -math.inf)
+    own = cap((q * k).sum(-1) * scale).permute(0, 2, 1)[..., None].masked_fill((seg != -1)[:, None, :, None], -math.inf)
     p = torch.nan_to_num(torch.softmax(torch.cat((s, own), -1), -1))
     o = torch.einsum("bhqk,bkhd->bqhd", p[..., :S], v[:, :S]) + p[..., S:].permute(0, 2, 1, 3) * v
     return o * (seg != 0)[:, :, None, None]
@@ -99,4 +99,27 @@ def test_rows_of_a_tile_follow_the_rounds(monkeypatch, dh, H, Hk, B, S, C, low):
     want = reference(q, k, v, seg, S, 1.0 / math.sqrt(dh))
     assert bool((got[seg == 0] == 0).all())
     assert (got.float() - want).abs().max() <= 2.0 ** -7 * v.float().abs().max()          # as above
+    assert torch.linalg.norm(got.float() - want) <= 2.0 ** -8 * torch.linalg.norm(want)
+
+
+@pytest.mark.parametrize("method", [1, 2])
+@pytest.mark.parametrize("dh,H,Hk", [(128, 4, 2), (64, 4, 4)])
+@pytest.mark.parametrize("S,C", [(0, 70), (63, 64), (129, 63), (192, 200), (330, 5)])
+def test_streaming_with_capped_logits(monkeypatch, S, C, dh, H, Hk, method):
+    """Soft sign and tanh at a cap that the larger logits feel, whole and half blocks of keys."""
+    import torch
+    from x_algorithm_b200.engine import dispatch_counts, ranker_attention
+    monkeypatch.setenv("PHX_ATTN", "tcgen05")
+    B, T, cap = 2, S + C, 2.0
+    g = torch.Generator(device="cuda").manual_seed(S * 131 + C)
+    q, k, v = (torch.randn(B, T, h, dh, device="cuda", generator=g).to(torch.bfloat16) for h in (H, Hk, Hk))
+    seg = torch.ones((B, T), dtype=torch.int32, device="cuda")
+    seg[:, S:] = -1
+    seg[1, S // 2: S // 2 + 9] = 0
+    before = dispatch_counts()["attn.tcgen05"]
+    got, _ = ranker_attention(q, k, v, seg, S, 1.0 / math.sqrt(dh), cap, method)
+    assert dispatch_counts()["attn.tcgen05"] == before + 1
+    capped = (lambda x: x / (1 + x.abs() / cap)) if method == 1 else (lambda x: cap * torch.tanh(x / cap))
+    want = reference(q, k, v, seg, S, 1.0 / math.sqrt(dh), capped)
+    assert (got.float() - want).abs().max() <= 2.0 ** -7 * v.float().abs().max()          # as without a cap: the logits stay fp32
     assert torch.linalg.norm(got.float() - want) <= 2.0 ** -8 * torch.linalg.norm(want)
