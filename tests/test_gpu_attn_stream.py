@@ -123,3 +123,29 @@ def test_streaming_with_capped_logits(monkeypatch, S, C, dh, H, Hk, method):
     want = reference(q, k, v, seg, S, 1.0 / math.sqrt(dh), capped)
     assert (got.float() - want).abs().max() <= 2.0 ** -7 * v.float().abs().max()          # as without a cap: the logits stay fp32
     assert torch.linalg.norm(got.float() - want) <= 2.0 ** -8 * torch.linalg.norm(want)
+
+
+@pytest.mark.parametrize("impl,dh,H,Hk,B,S,C", [
+    ("mma", 32, 4, 2, 3, 105, 20), ("mma", 64, 8, 8, 1, 223, 349), ("mma", 128, 4, 1, 2, 300, 40), ("mma", 64, 8, 8, 40, 200, 300), ("mma", 64, 2, 2, 2, 90, 0),
+    ("strip", 64, 8, 2, 8, 17, 173), ("strip", 64, 4, 4, 40, 120, 15), ("strip", 64, 4, 1, 25, 128, 428), ("pingpong", 64, 8, 8, 26, 96, 374),
+    ("pingpong", 64, 8, 8, 20, 128, 130), ("pingpong", 64, 8, 2, 20, 40, 0), ("resident", 64, 4, 4, 3, 100, 200), ("tcgen05", 64, 8, 8, 2, 200, 60),
+    ("tcgen05", 128, 8, 2, 2, 70, 60)])
+def test_history_rows_marked_as_candidates_attend_to_themselves(monkeypatch, impl, dh, H, Hk, B, S, C):
+    """allowed(q, k) = history key, or the row itself (ranker_attention_utils.py:16-56): also for rows in front of the candidates, whatever tile or
+    strip they share, in every kernel."""
+    import torch
+    from x_algorithm_b200.engine import ranker_attention
+    monkeypatch.setenv("PHX_ATTN", impl)
+    g = torch.Generator(device="cuda").manual_seed(S * 131 + C)
+    T = S + C
+    q, k, v = (torch.randn(B, T, h, dh, device="cuda", generator=g).to(torch.bfloat16) for h in (H, Hk, Hk))
+    seg = torch.ones((B, T), dtype=torch.int32, device="cuda")
+    seg[:, S:] = -1
+    r = torch.rand((B, T), device="cuda", generator=g)
+    seg[r < 0.3] = 0
+    seg[r > 0.9] = -1
+    got, _ = ranker_attention(q, k, v, seg, S, 1.0 / math.sqrt(dh))
+    want = reference(q, k, v, seg, S, 1.0 / math.sqrt(dh))
+    assert bool((got[seg == 0] == 0).all())
+    assert (got.float() - want).abs().max() <= 2.0 ** -7 * v.float().abs().max()          # as above
+    assert torch.linalg.norm(got.float() - want) <= 2.0 ** -8 * torch.linalg.norm(want)

@@ -139,16 +139,19 @@ __global__ void __launch_bounds__(32 * WARPS) ranker_attention_kernel(AttnArgs a
 #pragma unroll
   for (int i = 0; i < 2; ++i) segq[i] = (rq[i] < T) ? a.seg[trow(rq[i])] : 0;
   const int seg_key = load_key(0, 2);
-  for (int c = threadIdx.x; c < ROWS * CH; c += THREADS) {
-    const int r = c / CH, dc = (c % CH) * 8;
-    const bool ok = (q0 + r) < T;
-    const long long tok = trow(ok ? q0 + r : 0);
-    cp16((uint32_t)__cvta_generic_to_shared(sq + r * LD + dc), a.q + tok * a.q_tok_stride + a.q_col(h) + dc, ok);
-    if (has_cand) {
-      cp16((uint32_t)__cvta_generic_to_shared(sks + r * LD + dc), kbase + tok * a.k_tok_stride + dc, ok);
-      cp16((uint32_t)__cvta_generic_to_shared(svs + r * LD + dc), vbase + tok * a.v_tok_stride + dc, ok);
+  auto copy_rows = [&](bool q, bool own) {     // the tile's Q rows, its own K and V rows
+    for (int c = threadIdx.x; c < ROWS * CH; c += THREADS) {
+      const int r = c / CH, dc = (c % CH) * 8;
+      const bool ok = (q0 + r) < T;
+      const long long tok = trow(ok ? q0 + r : 0);
+      if (q) cp16((uint32_t)__cvta_generic_to_shared(sq + r * LD + dc), a.q + tok * a.q_tok_stride + a.q_col(h) + dc, ok);
+      if (own) {
+        cp16((uint32_t)__cvta_generic_to_shared(sks + r * LD + dc), kbase + tok * a.k_tok_stride + dc, ok);
+        cp16((uint32_t)__cvta_generic_to_shared(svs + r * LD + dc), vbase + tok * a.v_tok_stride + dc, ok);
+      }
     }
-  }
+  };
+  copy_rows(true, has_cand);
   if (n_blocks > 0) load_block(0, 0);
   cp_commit();
   if (n_blocks > 1) load_block(1, 1);
@@ -274,7 +277,18 @@ __global__ void __launch_bounds__(32 * WARPS) ranker_attention_kernel(AttnArgs a
   }
 
   // ---- self key of candidate rows: one more online-softmax step with a per-row dot product ------------
-  if (has_cand) {
+  // (a row in front of the candidates that is marked as one attends to itself all the same; its tile did not expect it)
+  bool self = has_cand;
+  if (!has_cand) {
+    self = __syncthreads_or(segq[0] == -1 || segq[1] == -1);
+    if (self) {
+      copy_rows(false, true);
+      cp_commit();
+      cp_wait<0>();
+      __syncthreads();
+    }
+  }
+  if (self) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const bool is_cand = segq[i] == -1;
@@ -603,7 +617,15 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) ranker_attention_strip_kernel(
     // diagonal P block against the strip's own V rows.
     cp_wait<1>();      // the strip's own K/V rows (requested one tile ago) have landed; the next Q may still be in flight
     __syncwarp();
-    if (has_cand) {
+    bool self = has_cand;
+    if (!has_cand && __any_sync(0xffffffffu, segq[0] == -1 || segq[1] == -1)) {   // rows in front of the candidates that are marked as such
+      load_own_kv(tile);
+      cp_commit();
+      cp_wait<0>();
+      __syncwarp();
+      self = true;
+    }
+    if (self) {
       float sd[2][4];
 #pragma unroll
       for (int j = 0; j < 2; ++j) { sd[j][0] = sd[j][1] = sd[j][2] = sd[j][3] = 0.f; }

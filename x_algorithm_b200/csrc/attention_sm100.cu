@@ -757,7 +757,9 @@ struct PingArgs {
 // the eight tensor maps of a launch: Q / K / V / out over the history block and over the candidate block
 struct PingMaps { CUtensorMap qh, qc, kh, vh, kc, vc, oh, oc; };
 
-template <bool CAP>
+// OWN: history rows may be marked as candidates (AttnArgs::marked_history); 256 x 8 x (125 of 128 + 510 of 512) rows 141.8 -> 143.5 us with it, level where
+// every history row is a key
+template <bool CAP, bool OWN>
 __global__ void __launch_bounds__(PP_THREADS, 1)
 ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs a) {
   constexpr int DH = 64;
@@ -965,6 +967,12 @@ ranker_attention_pingpong_kernel(const __grid_constant__ PingMaps maps, PingArgs
         all_ok = (kmask[0] & kmask[1] & kmask[2] & kmask[3]) == 0xffffffffu;
         mask_li = cur.li;
       }
+      if (OWN && !all_ok) {
+        // a history row marked as a candidate attends to itself: key r of the one history tile, which is no key to the others
+        const uint32_t own = cur.seg == -1 && !cur.cand ? 1u << lane : 0u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) kmask[i] = mask_words[w * 4 + i] | (i == quad ? own : 0u);
+      }
 
       mbar_wait(s_full(w), ph, verr);
       tc_fence_after();
@@ -1132,11 +1140,11 @@ phx_status cached_map3d(CUtensorMap* out, const bf16* ptr, long long cols, long 
   return PHX_OK;
 }
 
-template <bool CAP>
+template <bool CAP, bool OWN>
 phx_status launch_pingpong(const AttnArgs& a, int* err_flag, int num_sms, cudaStream_t stream, std::string& err) {
   const size_t smem = (size_t)(4 + 3 * PP_NQ) * SLAB + 64 + 192 + 1024;
   static SmemLimit limit;
-  PHX_CUDA_TRY(limit.raise(ranker_attention_pingpong_kernel<CAP>, (int)smem), err);
+  PHX_CUDA_TRY(limit.raise(ranker_attention_pingpong_kernel<CAP, OWN>, (int)smem), err);
   const int n_hist = a.hist_len < a.T ? a.hist_len : a.T;
   const int n_cand = a.T - n_hist;
   PingArgs p;
@@ -1194,7 +1202,7 @@ phx_status launch_pingpong(const AttnArgs& a, int* err_flag, int num_sms, cudaSt
   }
   const long long tiles = (long long)p.n_items * ((p.skip_hist ? 0 : (n_hist + QT - 1) / QT) + (n_cand + QT - 1) / QT);
   const int grid = (int)(tiles < num_sms ? tiles : num_sms);
-  ranker_attention_pingpong_kernel<CAP><<<grid, PP_THREADS, smem, stream>>>(pm, p);
+  ranker_attention_pingpong_kernel<CAP, OWN><<<grid, PP_THREADS, smem, stream>>>(pm, p);
   PHX_CUDA_TRY(cudaGetLastError(), err);
   return PHX_OK;
 }
@@ -1282,7 +1290,8 @@ phx_status ranker_attention_pingpong_launch(const AttnArgs& a, int* err_flag, cu
   const int num_sms = device_sms();
   dispatch_note(DK_ATTN_PINGPONG);
   const bool cap = a.cap_method != 0 && a.cap > 0.f;
-  return cap ? launch_pingpong<true>(a, err_flag, num_sms, stream, err) : launch_pingpong<false>(a, err_flag, num_sms, stream, err);
+  if (a.marked_history) return cap ? launch_pingpong<true, true>(a, err_flag, num_sms, stream, err) : launch_pingpong<false, true>(a, err_flag, num_sms, stream, err);
+  return cap ? launch_pingpong<true, false>(a, err_flag, num_sms, stream, err) : launch_pingpong<false, false>(a, err_flag, num_sms, stream, err);
 }
 
 // the streaming kernel: head dim 64 or 128, any grouping of the q heads, plain or split rows (not packed ones)

@@ -321,6 +321,7 @@ struct AttnArgs {
   int B, T, Hq, Hkv, dh, hist_len;
   float sm_scale, cap;
   int cap_method;
+  int marked_history = 1;   // rows in front of the candidates may be marked as such (seg -1); 0: the caller knows that none is
   int* err_flag;         // int in device or pinned memory, raised by a bounded wait that ran out (tcgen05 path); null = mma.sync path only
   // Split token layout (token_row): q / k / v / out / seg rows are the B * hist_len history rows followed by the
   // candidate rows.  q_start > 0: query rows below it are not computed (candidate-only layers).

@@ -490,7 +490,7 @@ phx_status layer_attention(phx_engine* e, int B, int Tt, int hist_len, bool spli
   aa.cap = c.attn_logit_cap;
   aa.cap_method = (c.attn_logit_cap > 0.f) ? c.cap_method : 0;
   aa.err_flag = e->err_flag;
-  aa.split = split ? 1 : 0; aa.q_start = q_start;
+  aa.split = split ? 1 : 0; aa.q_start = q_start; aa.marked_history = 0;
   aa.pack = pack_map(pk);
   e->last_launches++;
   ProfScope ps(e, KC_ATTN);
